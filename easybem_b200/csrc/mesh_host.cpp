@@ -123,49 +123,77 @@ void host_topology(HostMesh* m)
   }
 
   // Near pairs per test triangle (sorted by trial index), DL slots per row.
+  // Marks replace set operations: seen[j] = i once triangle j is a candidate of
+  // row i, and slot[v] (with owner[v] = i) is vertex v's place in row i's
+  // column list, so only the ~13 candidates and ~12 columns are sorted.
+  const size_t guess = 14 * (size_t)ne;
   m->sl_rowptr.assign(ne + 1, 0);
   m->sl_col.clear();
+  m->sl_col.reserve(guess);
   m->pair_i.clear();
+  m->pair_i.reserve(guess);
   m->pair_kind.clear();
+  m->pair_kind.reserve(guess);
   m->dl_rowptr.assign(ne + 1, 0);
   m->dl_col.clear();
-  std::vector<int> cand;
-  std::vector<std::pair<int, int>> dl_entries;  // (column, entry id)
+  m->dl_col.reserve(guess);
+  std::vector<int> seen(ne, -1), owner(nv, -1), slot(nv), cand, cols, first, entry_col;
   long long near_incl_repeat = 0;
   std::vector<int> contrib_ptr(1, 0), contrib;
+  contrib_ptr.reserve(guess);
+  contrib.reserve(3 * guess);
   for (int i = 0; i < ne; i++) {
     cand.clear();
     for (int k = 0; k < 3; k++) {
       const int v = m->elems[3 * i + k];
-      for (int p = vptr[v]; p < vptr[v + 1]; p++) cand.push_back(vtri[p]);
+      for (int p = vptr[v]; p < vptr[v + 1]; p++)
+        if (seen[vtri[p]] != i) {
+          seen[vtri[p]] = i;
+          cand.push_back(vtri[p]);
+        }
     }
     std::sort(cand.begin(), cand.end());
-    cand.erase(std::unique(cand.begin(), cand.end()), cand.end());
     near_incl_repeat += (long long)cand.size();
-    dl_entries.clear();
+    cols.clear();
+    entry_col.clear();
+    const int p0 = (int)m->sl_col.size();
     for (int j : cand) {
       const PairGeom g = classify_pair(&m->elems[3 * i], &m->elems[3 * j], i == j);
       if (g.kind == kPairRepeat) continue;  // a repeated triangle contributes nothing
-      const int p = (int)m->sl_col.size();
       m->sl_col.push_back(j);
       m->pair_i.push_back(i);
       m->pair_kind.push_back((int8_t)g.kind);
       if (g.kind == kPairVertex || g.kind == kPairEdge) {
         int slots[3];
         dl_trial_slots(g, slots);
-        for (int k = 0; k < 3; k++) dl_entries.push_back({m->elems[3 * j + slots[k]], 3 * p + k});
+        for (int k = 0; k < 3; k++) {
+          const int v = m->elems[3 * j + slots[k]];
+          entry_col.push_back(v);
+          if (owner[v] != i) {
+            owner[v] = i;
+            cols.push_back(v);
+          }
+        }
+      } else {
+        entry_col.insert(entry_col.end(), 3, -1);
       }
     }
     m->sl_rowptr[i + 1] = (int)m->sl_col.size();
-    std::sort(dl_entries.begin(), dl_entries.end());
-    for (size_t e = 0; e < dl_entries.size(); e++) {
-      if (e == 0 || dl_entries[e].first != dl_entries[e - 1].first) {
-        if (e > 0) contrib_ptr.push_back((int)contrib.size());
-        m->dl_col.push_back(dl_entries[e].first);
-      }
-      contrib.push_back(dl_entries[e].second);
+    // entries 3 pair + k by column, ascending within each column
+    std::sort(cols.begin(), cols.end());
+    first.assign(cols.size() + 1, 0);
+    for (size_t c = 0; c < cols.size(); c++) slot[cols[c]] = (int)c;
+    for (int v : entry_col)
+      if (v >= 0) first[slot[v] + 1]++;
+    for (size_t c = 0; c < cols.size(); c++) {
+      first[c + 1] += first[c];
+      m->dl_col.push_back(cols[c]);
+      contrib_ptr.push_back((int)contrib.size() + first[c + 1]);
     }
-    if (!dl_entries.empty()) contrib_ptr.push_back((int)contrib.size());
+    const size_t base = contrib.size();
+    contrib.resize(base + first[cols.size()]);
+    for (size_t e = 0; e < entry_col.size(); e++)
+      if (entry_col[e] >= 0) contrib[base + first[slot[entry_col[e]]]++] = 3 * p0 + (int)e;
     m->dl_rowptr[i + 1] = (int)m->dl_col.size();
   }
   m->dl_contrib_ptr.swap(contrib_ptr);
