@@ -321,13 +321,9 @@ static int build_static(Mesh* m)
     const int v = h.elems[3 * h.perm[s] + k];
     return mk3(h.nodes[3 * v], h.nodes[3 * v + 1], h.nodes[3 * v + 2]);
   };
-  // cell bounding spheres (centre = mean centroid, radius over all vertices)
   for (int c = 0; c < h.ncells; c++) {
-    const d3 cc = mk3(h.cell_center[3 * c], h.cell_center[3 * c + 1], h.cell_center[3 * c + 2]);
-    double r2 = 0.0;
-    for (int s = c * kCell; s < std::min(ne, (c + 1) * kCell); s++)
-      for (int k = 0; k < 3; k++) r2 = std::max(r2, dot3(vertex(s, k) - cc, vertex(s, k) - cc));
-    ccent[c] = dq{cc.x, cc.y, cc.z, std::sqrt(r2) * (1.0 + 1e-12)};
+    const double* b = &h.cell_ball[4 * (size_t)c];
+    ccent[c] = dq{b[0], b[1], b[2], b[3]};
   }
   for (int s = 0; s < ne; s++) {
     d3 P[3];
@@ -381,16 +377,10 @@ static int build_static(Mesh* m)
   auto item_spheres = [&](int n, std::vector<dq>& out) {
     for (size_t t = 0; t < out.size(); t++) {
       const int i0 = (int)t * n, i1 = std::min(h.nitems, i0 + n);
-      d3 c = mk3(0, 0, 0);
-      for (int it = i0; it < i1; it++) c = c + mk3(tcent[it].x, tcent[it].y, tcent[it].z);
-      c = (1.0 / (i1 - i0)) * c;
-      double r2 = 0.0;
-      for (int it = i0; it < i1; it++)
-        for (int k = 0; k < 3; k++) {
-          const d3 v = vertex(it / h.nchunk, k);
-          r2 = std::max(r2, dot3(v - c, v - c));
-        }
-      out[t] = dq{c.x, c.y, c.z, std::sqrt(r2) * (1.0 + 1e-12)};
+      double b[4];
+      if (h.nchunk == 1 && n == kCell) std::copy_n(&h.cell_ball[4 * t], 4, b);  // a cell's own triangles
+      else vertex_ball(h, i0 / h.nchunk, (i1 - 1) / h.nchunk + 1, b);
+      out[t] = dq{b[0], b[1], b[2], b[3]};
     }
   };
   item_spheres(kTT, ttile);

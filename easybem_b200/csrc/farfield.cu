@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kTT, far_min_blocks<T, NSL, ND, P1T>())
     const int ti = w.tgt0 + threadIdx.x;
     const bool active = ti < md.nitems;
     const int tsel = active ? ti : w.tgt0;
-    // separation test per warp (the warp's items are consecutive in Morton order)
+    // separation test per warp (the warp's items are consecutive in sorted order)
     const dq tile = md.twarp[tsel / kWarpItems];
 
     // target points relative to the triangle centroid are re-read per cell
@@ -292,7 +292,7 @@ __device__ __forceinline__ void prep_point(const ApplyArgs& A, long long idx)
   }
 }
 
-// Output rows in sorted (Morton) order, kFinalizeLanes threads per row: the
+// Output rows in sorted order, kFinalizeLanes threads per row: the
 // lanes take every kFinalizeLanes-th partial slot and CSR entry, then add
 // their sums in a fixed shuffle tree (deterministic). Sorted order makes the
 // partial-sum reads of neighbouring rows contiguous; the row's original index

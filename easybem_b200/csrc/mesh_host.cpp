@@ -19,15 +19,77 @@ void target_split(int Q, int* K, int* nchunk)
   *nchunk = (Q + 7) / 8;
 }
 
-static uint64_t spread21(uint64_t x)
+int split_cells(int ncells)
 {
-  x &= 0x1fffff;
-  x = (x | x << 32) & 0x1f00000000ffffULL;
-  x = (x | x << 16) & 0x1f0000ff0000ffULL;
-  x = (x | x << 8) & 0x100f00f00f00f00fULL;
-  x = (x | x << 4) & 0x10c30c30c30c30c3ULL;
-  x = (x | x << 2) & 0x1249249249249249ULL;
-  return x;
+  // larger ranges split at whole 128-triangle target tiles (4 cells); small
+  // ones in the middle, so that no part is a sliver
+  const int half = (ncells + 1) / 2;
+  return ncells > 32 ? (half + 3) / 4 * 4 : half;
+}
+
+struct Centroid {
+  double c[3];
+  int i;
+};
+
+// Recursive bisection: t[0, n) is halved at a whole number of cells across
+// the longest side of its box until one cell is left.
+static void bisect(Centroid* t, int n)
+{
+  const int ncells = (n + kCell - 1) / kCell;
+  if (ncells <= 1) return;
+  double lo[3] = {t[0].c[0], t[0].c[1], t[0].c[2]}, hi[3] = {lo[0], lo[1], lo[2]};
+  for (int k = 1; k < n; k++)
+    for (int d = 0; d < 3; d++) {
+      lo[d] = std::min(lo[d], t[k].c[d]);
+      hi[d] = std::max(hi[d], t[k].c[d]);
+    }
+  int ax = 0;
+  for (int d = 1; d < 3; d++)
+    if (hi[d] - lo[d] > hi[ax] - lo[ax]) ax = d;
+  const int m = split_cells(ncells) * kCell;  // < n: the right part holds at least one cell
+  std::nth_element(t, t + m, t + n, [ax](const Centroid& a, const Centroid& b) {
+    return a.c[ax] < b.c[ax] || (a.c[ax] == b.c[ax] && a.i < b.i);
+  });
+  bisect(t, m);
+  bisect(t + m, n - m);
+}
+
+void vertex_ball(const HostMesh& m, int s0, int s1, double* ball)
+{
+  thread_local std::vector<d3> p;
+  p.clear();
+  for (int s = s0; s < s1; s++)
+    for (int k = 0; k < 3; k++) {
+      const double* v = &m.nodes[3 * (size_t)m.elems[3 * (size_t)m.perm[s] + k]];
+      p.push_back(mk3(v[0], v[1], v[2]));
+    }
+  d3 lo = p[0], hi = p[0];
+  for (const d3& v : p) {
+    lo = mk3(std::min(lo.x, v.x), std::min(lo.y, v.y), std::min(lo.z, v.z));
+    hi = mk3(std::max(hi.x, v.x), std::max(hi.y, v.y), std::max(hi.z, v.z));
+  }
+  d3 c = 0.5 * (lo + hi);
+  double best = -1.0;
+  for (int it = 0; it <= 4; it++) {
+    double r2 = -1.0;
+    d3 far = c;
+    for (const d3& v : p) {
+      const double e2 = dot3(v - c, v - c);
+      if (e2 > r2) {
+        r2 = e2;
+        far = v;
+      }
+    }
+    if (best < 0.0 || r2 < best) {
+      best = r2;
+      ball[0] = c.x;
+      ball[1] = c.y;
+      ball[2] = c.z;
+    }
+    c = c + (1.0 / (it + 4.0)) * (far - c);
+  }
+  ball[3] = std::sqrt(best) * (1.0 + 1e-12);
 }
 
 int prepare_host_mesh(int nv, const double* nodes, int ne, const int* elems1, int order, HostMesh* m,
@@ -64,45 +126,24 @@ int prepare_host_mesh(int nv, const double* nodes, int ne, const int* elems1, in
       return set_error(EB_ERR_MESH, "triangle " + std::to_string(i) + " is degenerate (zero area)");
   }
 
-  // Morton order of centroids.
-  std::vector<double> cent(3 * (size_t)ne);
-  double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-  for (int i = 0; i < ne; i++)
-    for (int d = 0; d < 3; d++) {
-      const int* f = &m->elems[3 * i];
-      const double c = (nodes[3 * f[0] + d] + nodes[3 * f[1] + d] + nodes[3 * f[2] + d]) / 3.0;
-      cent[3 * i + d] = c;
-      lo[d] = std::min(lo[d], c);
-      hi[d] = std::max(hi[d], c);
-    }
-  double ext = std::max({hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2], 1e-300});
-  std::vector<std::pair<uint64_t, int>> keys(ne);
+  // order by recursive bisection of the centroids
+  std::vector<Centroid> cent(ne);
   for (int i = 0; i < ne; i++) {
-    uint64_t k = 0;
-    for (int d = 0; d < 3; d++) {
-      double s = (cent[3 * i + d] - lo[d]) / ext;
-      uint64_t q = (uint64_t)std::min(2097151.0, std::max(0.0, s * 2097151.0));
-      k |= spread21(q) << d;
-    }
-    keys[i] = {k, i};
+    const int* f = &m->elems[3 * i];
+    for (int d = 0; d < 3; d++) cent[i].c[d] = (nodes[3 * f[0] + d] + nodes[3 * f[1] + d] + nodes[3 * f[2] + d]) / 3.0;
+    cent[i].i = i;
   }
-  std::sort(keys.begin(), keys.end());
+  bisect(cent.data(), ne);
   m->perm.resize(ne);
   m->iperm.resize(ne);
   for (int s = 0; s < ne; s++) {
-    m->perm[s] = keys[s].second;
-    m->iperm[keys[s].second] = s;
+    m->perm[s] = cent[s].i;
+    m->iperm[cent[s].i] = s;
   }
   m->ncells = (ne + kCell - 1) / kCell;
-  m->cell_center.assign(3 * (size_t)m->ncells, 0.0);
-  for (int c = 0; c < m->ncells; c++) {
-    const int s0 = c * kCell, s1 = std::min(ne, s0 + kCell);
-    for (int d = 0; d < 3; d++) {
-      double acc = 0.0;
-      for (int s = s0; s < s1; s++) acc += cent[3 * m->perm[s] + d];
-      m->cell_center[3 * c + d] = acc / (s1 - s0);
-    }
-  }
+  m->cell_ball.resize(4 * (size_t)m->ncells);
+  for (int c = 0; c < m->ncells; c++)
+    vertex_ball(*m, c * kCell, std::min(ne, (c + 1) * kCell), &m->cell_ball[4 * (size_t)c]);
   target_split(m->Q, &m->K, &m->nchunk);
   m->nitems = ne * m->nchunk;
   if (topology) host_topology(m);

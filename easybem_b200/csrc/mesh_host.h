@@ -3,7 +3,7 @@
 // Replaces the reference's host topology (src/meshTopology.cpp:22-261, an
 // O(ne * nedges) edge search) and its per-matvec host pair enumeration
 // (src/BEM3dLaplaceGPU.cu:1224-1260) with one O(ne log ne) pass at mesh
-// creation: triangles are reordered along a Morton curve of their centroids,
+// creation: triangles are reordered by recursive bisection of their centroids,
 // grouped in cells of kCell consecutive triangles (the far-field source
 // granularity), and the near pairs (triangles sharing at least one vertex)
 // are listed once in CSR form for the Sauter-Schwab correction.
@@ -24,10 +24,15 @@ struct HostMesh {
   std::vector<double> nodes;  // [nv][3]
   std::vector<int> elems;     // [ne][3], 0-based
 
-  // Morton order: perm[s] = original index of sorted triangle s; iperm inverse.
+  // Sorted order: perm[s] = original index of sorted triangle s; iperm inverse.
+  // Recursive bisection across the longest side of the centroids' box, at
+  // multiples of kCell (split_cells), so cells and the ranges of the bisection
+  // are compact patches. Cells of a Morton curve jump across its faces: on
+  // the perturbed icosphere L5 47 cells lay within twice the sum of the radii
+  // of a cell, against 16 here.
   std::vector<int> perm, iperm;
   int ncells = 0;
-  std::vector<double> cell_center;  // [ncells][3]
+  std::vector<double> cell_ball;  // [ncells][4]: centre and radius of a ball around the cell's vertices
 
   // Target items: a triangle's Q points split into chunks of at most K points.
   int K = 0;        // target points per item (compile-time kernel width)
@@ -51,7 +56,13 @@ struct HostMesh {
   long long far_cell_tri_pairs = 0, near_cell_tri_pairs = 0;
 };
 
-// Validates and prepares (Morton order, cells, target items and, when
+// Cells of the first half of a range of ncells cells in the bisection.
+int split_cells(int ncells);
+// Centre and radius of a small ball around the vertices of sorted triangles
+// [s0, s1): the box centre, moved towards the farthest vertex four times.
+void vertex_ball(const HostMesh& m, int s0, int s1, double* ball);
+
+// Validates and prepares (sorted order, cells, target items and, when
 // topology is set, the near-pair CSR through host_topology); returns EB_OK or
 // an error status with a message.
 int prepare_host_mesh(int nv, const double* nodes, int ne, const int* elems1, int order, HostMesh* m,
