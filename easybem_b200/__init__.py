@@ -27,7 +27,7 @@ __all__ = ["Mesh", "Batch", "Solver", "Server", "solve", "EasyBemError", "init_g
 
 
 # far-field engines of the fused mixed SL+DL apply (EB_FAR_* in easybem_gpu.h)
-FAR_ENGINES = {"cuda": 0, "tensor": 1, "sym": 2, "sym_all": 3}
+FAR_ENGINES = {"cuda": 0, "tensor": 1, "sym": 2, "sym_all": 3, "tree": 4}
 
 
 def precision_code(precision) -> int:

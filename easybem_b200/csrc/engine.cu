@@ -3,6 +3,7 @@
 #include "engine.h"
 #include "farfield_sym.h"
 #include "farfield_tc.h"
+#include "farfield_tree.h"
 
 #include <algorithm>
 #include <chrono>
@@ -325,6 +326,7 @@ static int build_static(Mesh* m)
     const double* b = &h.cell_ball[4 * (size_t)c];
     ccent[c] = dq{b[0], b[1], b[2], b[3]};
   }
+  h.cell_rho.assign(h.ncells, 0.0);
   for (int s = 0; s < ne; s++) {
     d3 P[3];
     for (int k = 0; k < 3; k++) P[k] = vertex(s, k);
@@ -346,6 +348,7 @@ static int build_static(Mesh* m)
       wjtab[(size_t)s * Q + b] = h.quad.tw[b] * J;
       const d3 yr = y - cc;
       pos64[(size_t)s * Q + b] = dq{-2.0 * yr.x, -2.0 * yr.y, -2.0 * yr.z, dot3(yr, yr)};
+      h.cell_rho[cell] = std::max(h.cell_rho[cell], dot3(yr, yr));
       const float fx = (float)yr.x, fy = (float)yr.y, fz = (float)yr.z;
       const double y2 = (double)fx * fx + (double)fy * fy + (double)fz * fz;
       pos32[(size_t)s * Q + b] = make_float4(-2.0f * fx, -2.0f * fy, -2.0f * fz, (float)y2);
@@ -371,6 +374,7 @@ static int build_static(Mesh* m)
       }
     }
   }
+  for (double& r : h.cell_rho) r = std::sqrt(r) * (1.0 + 1e-12);
   // bounding spheres over the triangles of n consecutive target items: per
   // tile of kTT (the tensor-core kernel's test) and per warp of kWarpItems
   // (the CUDA-core kernel's: a tighter sphere leaves fewer cells "near")
@@ -539,6 +543,7 @@ int mesh_set_plan(Mesh* m, int items_per_sm, int tile)
   m->tc_var.grid = 0;
   m->sym_var.desc.release();
   m->sym_var.grid = 0;
+  if (m->tree) m->tree->scratch.clear();  // descriptors hold the record pointer
   m->rec.release();
   m->partial.release();
   return build_items(m);
@@ -663,13 +668,14 @@ bool sym_eligible(const Mesh* m, bool fp32, int nsl, int nd, bool fp64_internal)
   // the partial slots take (nsl + nd) ne^2 / 128 * 8 bytes: meshes whose slots
   // would pass kSymMaxSlotBytes keep the ordered-pair kernels (whose slots
   // grow with the work split, not with ne^2)
-  const bool engine = (m->plan.engine == 2 && (fp32 || fp64_internal)) || m->plan.engine == 3;
+  const bool engine = ((m->plan.engine == 2 || m->plan.engine == 4) && (fp32 || fp64_internal)) || m->plan.engine == 3;
   return engine && far_sym_variant(fp32, nsl, nd) && m->h.Q == kSymRule && m->h.K == kSymRule &&
          m->h.nchunk == 1 && sym_slot_bytes(m->h, nsl + nd) <= kSymMaxSlotBytes;
 }
 
 long long mesh_far_slots(const Mesh* m, bool fp32, int nsl, int nd)
 {
+  if (m->tree && m->tree->usable && m->plan.engine == 4 && tree_eligible(const_cast<Mesh*>(m), fp32, nsl, nd)) return tree_far_slots(m);
   if (sym_eligible(m, fp32, nsl, nd)) {
     const int r = far_sym_cells_per_item(kSymCellsPerItem);
     long long n = 0;
@@ -816,7 +822,8 @@ int mesh_apply(Mesh* m, int precision, int nsl, int nd, const double* d_t, const
     var.smem = smem;
     var.src_tile = desc.src_tile;
   }
-  const bool sym = sym_eligible(m, fp32, nsl, nd);
+  const bool tree = tree_eligible(m, fp32, nsl, nd);
+  const bool sym = !tree && sym_eligible(m, fp32, nsl, nd);
   ApplyArgs A = mesh_apply_args(m, fp32, m->rec.p, m->partial.as<double>(), d_t, h.ne, d_u, d_v, h.ne, d_q);
   EB_CUDA(prep_launch(fp32, nsl, nd, A, st));
   if (m->profile && !m->ev0) {
@@ -824,7 +831,10 @@ int mesh_apply(Mesh* m, int precision, int nsl, int nd, const double* d_t, const
     EB_CUDA(cudaEventCreate(&m->ev1));
     EB_CUDA(cudaEventCreate(&m->ev2));
   }
-  if (sym) {
+  if (tree) {
+    m->sym_used = m->tc_used = false;
+    EB_CHECK(tree_far_apply(m, fp32, nsl, nd, &A, st));
+  } else if (sym) {
     EB_CHECK(sym_far_apply(m, fp32, nsl, nd, st));
     A.partial = m->sym_partial.as<double>();
     A.nsplit = m->sym_nsplit;
@@ -1124,9 +1134,9 @@ int eb_mesh_set_far_engine(eb_mesh mesh, int engine)
 {
   if (!mesh) return set_error(EB_ERR_INVALID, "null mesh");
   if (engine != EB_FAR_CUDA_CORES && engine != EB_FAR_TENSOR_CORES && engine != EB_FAR_SYMMETRIC &&
-      engine != EB_FAR_SYMMETRIC_ALL)
-    return set_error(EB_ERR_INVALID, "engine must be EB_FAR_CUDA_CORES, EB_FAR_TENSOR_CORES, EB_FAR_SYMMETRIC or "
-                                     "EB_FAR_SYMMETRIC_ALL");
+      engine != EB_FAR_SYMMETRIC_ALL && engine != EB_FAR_TREE)
+    return set_error(EB_ERR_INVALID, "engine must be EB_FAR_CUDA_CORES, EB_FAR_TENSOR_CORES, EB_FAR_SYMMETRIC, "
+                                     "EB_FAR_SYMMETRIC_ALL or EB_FAR_TREE");
   mesh->m->plan.engine = engine;
   return EB_OK;
 }
@@ -1135,7 +1145,8 @@ int eb_mesh_get_far_engine(eb_mesh mesh, int precision, int* engine)
 {
   if (!mesh || !engine) return set_error(EB_ERR_INVALID, "null argument");
   const bool fp32 = precision == EB_PREC_MIXED;
-  *engine = eb::tc_eligible(mesh->m, fp32, 1, 1)    ? EB_FAR_TENSOR_CORES
+  *engine = eb::tree_eligible(mesh->m, fp32, 1, 1)  ? EB_FAR_TREE
+            : eb::tc_eligible(mesh->m, fp32, 1, 1)  ? EB_FAR_TENSOR_CORES
             : eb::sym_eligible(mesh->m, fp32, 1, 1) ? EB_FAR_SYMMETRIC
                                                     : EB_FAR_CUDA_CORES;
   return EB_OK;

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <vector>
 
 #include "farfield.cuh"
@@ -88,7 +89,8 @@ struct DevBuf {
 
 // Launch plan of the far field for one mesh (tile shape and work split).
 struct FarPlan {
-  int engine = 2;         // 0: CUDA-core far kernel; 1: tensor-core kernel, 2: symmetric kernel, where the variant has one
+  int engine = 4;         // 0: CUDA-core far kernel; 1: tensor-core kernel, 2: symmetric kernel, 3: that for FP64 too, where
+                          // the variant has one; 4: the tree where it pays, else as 2
   int items_per_sm = 32;  // work items per SM the source ranges are cut into (load balance)
   int tile = 0;           // source triangles per shared-memory tile (0: the variant's default)
   int src_tile = kTS;     // tile of the last launch
@@ -96,6 +98,8 @@ struct FarPlan {
   int grid = 0;           // persistent CTAs of the last launch
   size_t smem = 0;
 };
+
+struct TreeMesh;  // farfield_tree.h
 
 struct Mesh {
   HostMesh h;
@@ -145,6 +149,8 @@ struct Mesh {
   int sym_nitems = 0, sym_nsplit = 0;
   Variant sym_var;
   bool sym_used = false;  // the last apply ran the symmetric kernel
+  // tree far field (engine 4), made on the first apply that takes it
+  std::shared_ptr<TreeMesh> tree;
   // host seconds of mesh creation: topology and pairs, static tables, near
   // field, and within the tables their device allocation and copy
   double setup_s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};

@@ -316,6 +316,7 @@ __device__ __forceinline__ double lanes_sum(double v)
 
 __device__ __forceinline__ size_t partial_offset(const ApplyArgs& A, int k)
 {
+  if (A.slot_off) return (size_t)k * kCell;
   if (A.nchunk == 1) return (size_t)k * A.nitems;
   const int sp = k / A.nchunk;
   return (size_t)sp * A.nitems + (k - sp * A.nchunk);
@@ -364,9 +365,15 @@ __device__ __forceinline__ void finalize_row(const ApplyArgs& A, int row_block)
     i = A.perm[s];
     scale = A.trin[s].w * (0.25 / M_PI);
     // far partial sums of row s: slot k of output c at c*stride + offset(k) + s*nchunk
-    const size_t stride = (size_t)A.nsplit * A.nitems;
+    size_t stride = (size_t)A.nsplit * A.nitems;
     const double* base = A.partial + (size_t)s * A.nchunk;
-    const int nparts = A.sym_cells > 0 ? sym_row_slots(s, A.ne, A.sym_cells) : A.nsplit * A.nchunk;
+    int nparts = A.sym_cells > 0 ? sym_row_slots(s, A.ne, A.sym_cells) : A.nsplit * A.nchunk;
+    if (A.slot_off) {
+      const int c = s / kCell, k0 = A.slot_off[c];
+      nparts = A.slot_off[c + 1] - k0;
+      stride = (size_t)A.slot_off[(A.ne + kCell - 1) / kCell] * kCell;
+      base = A.partial + (size_t)k0 * kCell + (s - c * kCell);
+    }
     int k = lane;
     for (; k + (kFinPipe - 1) * kFinalizeLanes < nparts; k += kFinPipe * kFinalizeLanes) {
       double x[kFinPipe][NO];

@@ -148,6 +148,9 @@ struct ApplyArgs {
   // nsplit slots); row s of tile T = s / kTT then has T + 1 + (its tile's upper
   // items) slots, and the rest are never written nor read
   int sym_cells = 0;
+  // tree far field: slots of cell c's rows are slot_off[c] .. slot_off[c + 1]),
+  // each kCell rows long (null: the layouts above)
+  const int* slot_off = nullptr;
 };
 
 // Partial slots a row of the symmetric plan holds (sorted row s, ne rows,

@@ -1,0 +1,1203 @@
+// Tree far field: the sum over all pairs of quadrature points in time
+// proportional to their number (7-point rule).
+//
+// Clusters of triangles (the nodes of the bisection that orders the mesh) are
+// paired as in tree_plan.h. Between separated clusters the kernel 1/|x - y| is
+// expanded in solid harmonics; close cells are summed point by point with the
+// inner loops of the symmetric far field. Harmonics are normalised so that
+// rotations act unitarily (C = sqrt(4 pi / (2n + 1)) Y):
+//
+//   R_n^m(x) = |x|^n C_n^m,   S_n^m(x) = |x|^-(n+1) C_n^m,
+//   1/|x - y| = sum_nm conj(R_n^m(y)) S_n^m(x),  |y| < |x|,
+//
+// a cluster's multipole is A_n^m = sum q R_n^m(y - c) / rho^n (rho its radius;
+// every stored coefficient is of the size of the charges whatever the mesh's
+// units), a double-layer source of strength s and normal n enters as
+// s (n.grad) R_n^m, and a local expansion gives phi = Re sum L_n^m conj(R_n^m).
+// Only m >= 0 is kept (the sums are real).
+//
+//   points -> multipoles   tree_p2m_kernel   one CTA per cell
+//   multipoles upward      tree_move_kernel<kUp>, three levels per launch
+//   multipoles -> locals   tree_move_kernel<kAcross>
+//   locals downward        tree_move_kernel<kDown>, all ancestors at once
+//   locals -> points       tree_l2p_kernel, into the last partial slot
+//   close cells            tree_near_kernel, one warp per task
+//
+// Moving an expansion along a vector d costs 2 p^3 multiply-adds instead of
+// p^4: it is rotated so that d becomes the z axis, moved along z (which
+// couples only equal m) and rotated back. The rotation about y splits into
+// rotations about z (a phase per m) and the constant rotation about y by 90
+// degrees: Ry(90) Rz(theta) Ry(-90) Rz(90 - phi) takes d to z. The matrix of
+// Ry(90) couples only half of the orders of a degree, real and imaginary
+// parts apart, and that of Ry(-90) differs by a sign per degree.
+//
+// Every sum runs in a fixed order on fixed lanes and every slot has one
+// writer, so results are bitwise reproducible.
+#include "farfield_tree.h"
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <mutex>
+
+#include "farfield_sym_eval.cuh"
+
+namespace eb {
+
+namespace {
+
+enum Move { kUp, kAcross, kDown };
+
+constexpr int kMoveWarps = 4;
+
+// Constant tables of one order (device pointers).
+//
+// Order of an expansion's (p + 1)^2 real coefficients in shared memory
+// ("grouped"): degree by degree, real parts of even m, real parts of odd m,
+// imaginary parts of even m, of odd m; so each output of Ry(90) reads one
+// contiguous group. Along z ("m-major"): for each m the real parts of degrees
+// m..p, then the imaginary ones. The matrices are padded per round of 32
+// outputs: entry [offset of the round + k * 32 + lane].
+struct TreeTables {
+  const double *bmat, *tmat[3];
+  const int2 *bround, *tround;  // (offset, length)
+  const int* bout;  // grouped output: first input | m-major position << 11 | sign of Ry(-90) << 22
+  const int* tout;  // m-major output: first input | grouped position << 11 | (n - m) << 22
+  const int* pair;  // (n, m): grouped position of re | of im << 10 | m << 20 | n << 25
+  const double2* rec;  // (n, m): R_n^m = rec.x z R_{n-1}^m - rec.y r^2 R_{n-2}^m (n > m)
+};
+
+template <int P>
+struct TreeShape {
+  static constexpr int kCoef = (P + 1) * (P + 1);
+  static constexpr int kRounds = (kCoef + 31) / 32;
+  static constexpr int kPairs = tree_pairs(P);
+  static constexpr int kPairRounds = (kPairs + 31) / 32;
+  static constexpr int kBuf = kCoef + P + 2;  // zero padding behind the last group
+};
+
+template <int NC>
+struct alignas(8 * NC) Vec {
+  double v[NC];
+};
+
+__device__ __forceinline__ int tree_pair(int n, int m) { return n * (n + 1) / 2 + m; }
+
+// Block b's entry among the meshes and its index there.
+__device__ __forceinline__ int tree_entry(const int* __restrict__ off, int n, int& b)
+{
+  if (n == 1) return 0;
+  int lo = 0, hi = n;  // off[lo] <= b < off[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (off[mid] <= b) lo = mid;
+    else hi = mid;
+  }
+  b -= off[lo];
+  return lo;
+}
+
+// ---------------------------------------------------------------------------
+// Moves.
+
+// dst = Ry(+-90) src; TO_M writes m-major positions.
+template <int P, int NC, bool BACK, bool TO_M>
+__device__ __forceinline__ void turn(const TreeTables& tab, const Vec<NC>* src, Vec<NC>* dst, int lane)
+{
+  using Sh = TreeShape<P>;
+#pragma unroll 1
+  for (int r = 0; r < Sh::kRounds; ++r) {
+    const int2 rd = tab.bround[r];
+    const int o = r * 32 + lane;
+    const int info = o < Sh::kCoef ? tab.bout[o] : 0;
+    const Vec<NC>* s = src + (info & 2047);
+    const double* mat = tab.bmat + rd.x + lane;
+    Vec<NC> acc;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc.v[c] = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < rd.y; ++k) {
+      const double b = mat[k * 32];
+      const Vec<NC> x = s[k];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc.v[c] += b * x.v[c];
+    }
+    if (o < Sh::kCoef) {
+      if (BACK && (info >> 22 & 1)) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) acc.v[c] = -acc.v[c];
+      }
+      dst[TO_M ? info >> 11 & 2047 : o] = acc;
+    }
+  }
+  __syncwarp();
+}
+
+// dst (grouped) = the move along z applied to src (m-major); pw: powers of
+// the step over the radius (not kAcross).
+template <int P, int NC, int MODE>
+__device__ __forceinline__ void along_z(const TreeTables& tab, const double* pw, const Vec<NC>* src, Vec<NC>* dst,
+                                        int lane)
+{
+  using Sh = TreeShape<P>;
+#pragma unroll 1
+  for (int r = 0; r < Sh::kRounds; ++r) {
+    const int2 rd = tab.tround[r];
+    const int o = r * 32 + lane;
+    const int info = o < Sh::kCoef ? tab.tout[o] : 0;
+    const int j = info >> 22;
+    const Vec<NC>* s = src + (info & 2047);
+    const double* mat = tab.tmat[MODE] + rd.x + lane;
+    Vec<NC> acc;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc.v[c] = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < rd.y; ++k) {
+      double b = mat[k * 32];
+      if (MODE != kAcross) b *= pw[abs(j - k)];
+      const Vec<NC> x = s[k];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc.v[c] += b * x.v[c];
+    }
+    if (o < Sh::kCoef) dst[info >> 11 & 2047] = acc;
+  }
+  __syncwarp();
+}
+
+// Rotation about z in place: (n, m) times e^{i m alpha} (SIGN +1) or its conjugate.
+template <int P, int NC, int SIGN>
+__device__ __forceinline__ void phase(const TreeTables& tab, const double2* e, Vec<NC>* buf, int lane)
+{
+  using Sh = TreeShape<P>;
+#pragma unroll 1
+  for (int i = lane; i < Sh::kPairs; i += 32) {
+    const int info = tab.pair[i];
+    const int m = info >> 20 & 31;
+    if (m == 0) continue;
+    const double2 f = e[m];
+    const double fi = SIGN * f.y;
+    Vec<NC>& re = buf[info & 1023];
+    Vec<NC>& im = buf[info >> 10 & 1023];
+    const Vec<NC> a = re, b = im;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      re.v[c] = a.v[c] * f.x - b.v[c] * fi;
+      im.v[c] = a.v[c] * fi + b.v[c] * f.x;
+    }
+  }
+  __syncwarp();
+}
+
+// b^k by squaring, k < 32
+__device__ __forceinline__ double power(double b, int k)
+{
+  double r = 1.0;
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    if (k >> i & 1) r *= b;
+    b *= b;
+  }
+  return r;
+}
+
+__device__ __forceinline__ double2 power(double2 b, int k)
+{
+  double2 r = make_double2(1.0, 0.0);
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    if (k >> i & 1) r = make_double2(r.x * b.x - r.y * b.y, r.x * b.y + r.y * b.x);
+    b = make_double2(b.x * b.x - b.y * b.y, 2.0 * b.x * b.y);
+  }
+  return r;
+}
+
+template <int P, int NC>
+constexpr size_t move_smem()
+{
+  return kMoveWarps * (2 * TreeShape<P>::kBuf * sizeof(Vec<NC>) + (P + 2) * 2 * (sizeof(double2) + sizeof(double)));
+}
+
+// One CTA per target node: its four warps take every fourth source, each a
+// whole move; the warps' sums are added in warp order.
+template <int P, int NC, int MODE>
+__global__ void __launch_bounds__(32 * kMoveWarps)
+    tree_move_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh, int pass, TreeTables tab)
+{
+  using Sh = TreeShape<P>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  int k = blockIdx.x;
+  const TreeDesc& d = descs[tree_entry(off, nmesh, k)];
+  if (d.far.active && *d.far.active == 0) return;
+  const TreeMovesDev mv = MODE == kUp ? d.up[pass] : MODE == kAcross ? d.m2l : d.down;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  Vec<NC>* bufs = reinterpret_cast<Vec<NC>*>(smem_raw);
+  Vec<NC>* b0 = bufs + warp * 2 * Sh::kBuf;
+  Vec<NC>* b1 = b0 + Sh::kBuf;
+  double2* ephi = reinterpret_cast<double2*>(bufs + kMoveWarps * 2 * Sh::kBuf) + warp * 2 * (P + 2);
+  double2* eth = ephi + P + 2;
+  double* pin = reinterpret_cast<double*>(reinterpret_cast<double2*>(bufs + kMoveWarps * 2 * Sh::kBuf) +
+                                          kMoveWarps * 2 * (P + 2)) + warp * 2 * (P + 2);
+  double* pout = pin + P + 2;
+  for (int i = lane; i < Sh::kBuf - Sh::kCoef; i += 32)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) b0[Sh::kCoef + i].v[c] = b1[Sh::kCoef + i].v[c] = 0.0;
+
+  const int tgt = mv.tgt[k];
+  const dq bt = d.ball[tgt];
+  const size_t cstride = (size_t)d.nnodes * Sh::kPairs;
+  const size_t col0 = (size_t)blockIdx.y * NC * cstride;
+  const double2* from = (MODE == kDown ? d.local : d.multipole) + col0;
+  double2* to = (MODE == kUp ? d.multipole : d.local) + col0;
+  Vec<NC> sre[Sh::kPairRounds], sim[Sh::kPairRounds];
+#pragma unroll
+  for (int r = 0; r < Sh::kPairRounds; ++r)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) sre[r].v[c] = sim[r].v[c] = 0.0;
+
+#pragma unroll 1
+  for (int s = mv.ptr[k] + warp; s < mv.ptr[k + 1]; s += kMoveWarps) {
+    const int src = mv.src[s];
+    const dq bs = d.ball[src];
+    // the vector that becomes the z axis: from the source's centre to the
+    // target's, reversed for a multipole (its points move the other way)
+    const double sg = MODE == kUp ? -1.0 : 1.0;
+    const double dx = sg * (bt.x - bs.x), dy = sg * (bt.y - bs.y), dz = sg * (bt.z - bs.z);
+    const double h2 = dx * dx + dy * dy, h = sqrt(h2), dist = sqrt(h2 + dz * dz);
+    const double cphi = h > 0.0 ? dx / h : 1.0, sphi = h > 0.0 ? dy / h : 0.0;
+    const double cth = dist > 0.0 ? dz / dist : 1.0, sth = dist > 0.0 ? h / dist : 0.0;
+    // kAcross: rho_s / d in, rho_t / d out; kUp: rho_s / rho_t in, d / rho_t
+    // between; kDown: d / rho_s between, rho_t / rho_s out
+    const double in = MODE == kAcross ? bs.w / dist : MODE == kUp ? bs.w / bt.w : dist / bs.w;
+    const double out = MODE == kAcross ? bt.w / dist : MODE == kUp ? dist / bt.w : bt.w / bs.w;
+    if (lane <= P) {
+      ephi[lane] = power(make_double2(sphi, cphi), lane);  // e^{i (90 - phi)}
+      eth[lane] = power(make_double2(cth, sth), lane);
+      pin[lane] = power(in, lane);
+      pout[lane] = power(out, lane);
+    }
+    __syncwarp();
+    const double2* a = from + (size_t)src * Sh::kPairs;
+#pragma unroll 1
+    for (int i = lane; i < Sh::kPairs; i += 32) {
+      const int info = tab.pair[i];
+      const int m = info >> 20 & 31;
+      const double2 f = ephi[m];
+      const double w = MODE == kDown ? 1.0 : pin[info >> 25];
+      const double fr = w * f.x, fi = w * f.y;
+      Vec<NC> re, im;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const double2 x = a[c * cstride + i];
+        re.v[c] = x.x * fr - x.y * fi;
+        im.v[c] = x.x * fi + x.y * fr;
+      }
+      b0[info & 1023] = re;
+      if (m > 0) b0[info >> 10 & 1023] = im;
+    }
+    __syncwarp();
+    turn<P, NC, true, false>(tab, b0, b1, lane);
+    phase<P, NC, 1>(tab, eth, b1, lane);
+    turn<P, NC, false, true>(tab, b1, b0, lane);
+    along_z<P, NC, MODE>(tab, MODE == kUp ? pout : pin, b0, b1, lane);
+    turn<P, NC, true, false>(tab, b1, b0, lane);
+    phase<P, NC, -1>(tab, eth, b0, lane);
+    turn<P, NC, false, false>(tab, b0, b1, lane);
+    const double unit = MODE == kAcross ? 1.0 / dist : 1.0;
+#pragma unroll
+    for (int r = 0; r < Sh::kPairRounds; ++r) {
+      const int i = r * 32 + lane;
+      if (i < Sh::kPairs) {
+        const int info = tab.pair[i];
+        const double2 f = ephi[info >> 20 & 31];
+        const double w = MODE == kUp ? 1.0 : unit * pout[info >> 25];
+        const Vec<NC> re = b1[info & 1023], im = b1[info >> 10 & 1023];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          sre[r].v[c] += w * (re.v[c] * f.x + im.v[c] * f.y);
+          sim[r].v[c] += w * (im.v[c] * f.x - re.v[c] * f.y);
+        }
+      }
+    }
+    __syncwarp();
+  }
+  // add the warps' sums in warp order
+  double2* mine = reinterpret_cast<double2*>(b0);  // kPairs * NC double2 fit the two buffers
+#pragma unroll
+  for (int r = 0; r < Sh::kPairRounds; ++r) {
+    const int i = r * 32 + lane;
+    if (i < Sh::kPairs)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) mine[c * Sh::kPairs + i] = make_double2(sre[r].v[c], sim[r].v[c]);
+  }
+  __syncthreads();
+  const bool add = MODE == kDown && d.has_local[tgt];
+  for (int i = threadIdx.x; i < Sh::kPairs * NC; i += 32 * kMoveWarps) {
+    const int c = i / Sh::kPairs, q = i - c * Sh::kPairs;
+    double2* t = to + c * cstride + (size_t)tgt * Sh::kPairs + q;
+    double2 v = add ? *t : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int w = 0; w < kMoveWarps; ++w) {
+      const double2 x = reinterpret_cast<const double2*>(bufs + w * 2 * Sh::kBuf)[i];
+      v.x += x.x;
+      v.y += x.y;
+    }
+    *t = v;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Points and expansions. Four warps per cell, one lane per triangle with its
+// seven points in registers; warp w runs the orders m = w, w + 4, ... of the
+// recurrences in n. Both directions use w_a-weighted sums over a triangle's
+// points: sources need sum_b q_b R(y_b), targets sum_a w_a phi(x_a).
+
+constexpr int kCellWarps = 4;
+constexpr int kSumRows = 8, kSumStride = 36;  // conflict-free rows of the lane sums
+
+struct CellPoints {
+  double x[kQ], y[kQ], z[kQ], r2[kQ];
+};
+
+__device__ __forceinline__ void load_points(const TreeDesc& d, int tri, double inv_rho, CellPoints& p)
+{
+#pragma unroll
+  for (int a = 0; a < kQ; ++a) {
+    const dq q = d.pos[(size_t)tri * kQ + a];
+    p.x[a] = -0.5 * q.x * inv_rho;
+    p.y[a] = -0.5 * q.y * inv_rho;
+    p.z[a] = -0.5 * q.z * inv_rho;
+    p.r2[a] = p.x[a] * p.x[a] + p.y[a] * p.y[a] + p.z[a] * p.z[a];
+  }
+}
+
+// Runs fn(n, m, re, im) over degrees n = m .. P of this warp's orders m, with
+// the harmonics of the kQ points in re, im.
+template <int P, typename F>
+__device__ __forceinline__ void each_harmonic(const TreeTables& tab, const CellPoints& p, int warp, F&& fn)
+{
+  double dr[kQ], di[kQ];  // R_m^m
+#pragma unroll
+  for (int a = 0; a < kQ; ++a) {
+    dr[a] = 1.0;
+    di[a] = 0.0;
+  }
+#pragma unroll 1
+  for (int m = 0; m <= P; ++m) {
+    if (m > 0) {
+      const double f = -sqrt((2.0 * m - 1.0) / (2.0 * m));
+#pragma unroll
+      for (int a = 0; a < kQ; ++a) {
+        const double t = f * (p.x[a] * dr[a] - p.y[a] * di[a]);
+        di[a] = f * (p.x[a] * di[a] + p.y[a] * dr[a]);
+        dr[a] = t;
+      }
+    }
+    if ((m & (kCellWarps - 1)) != warp) continue;
+    double r1[kQ], i1[kQ], r0[kQ], i0[kQ];
+#pragma unroll
+    for (int a = 0; a < kQ; ++a) {
+      r1[a] = dr[a];
+      i1[a] = di[a];
+      r0[a] = i0[a] = 0.0;
+    }
+    fn(m, m, r1, i1);
+#pragma unroll 1
+    for (int n = m + 1; n <= P; ++n) {
+      const double2 c = tab.rec[tree_pair(n, m)];
+#pragma unroll
+      for (int a = 0; a < kQ; ++a) {
+        const double az = c.x * p.z[a], br = c.y * p.r2[a];
+        const double tr = az * r1[a] - br * r0[a], ti = az * i1[a] - br * i0[a];
+        r0[a] = r1[a];
+        i0[a] = i1[a];
+        r1[a] = tr;
+        i1[a] = ti;
+      }
+      fn(n, m, r1, i1);
+    }
+  }
+}
+
+// Multipoles of one cell: NSL single-layer columns (they share sum_b w_b J
+// R(y_b)), and for ND = 1 the double-layer column blockIdx.y.
+template <int P, int NSL, int ND>
+__global__ void __launch_bounds__(32 * kCellWarps)
+    tree_p2m_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh, ApplyArgs one,
+                    const ApplyArgs* __restrict__ many, TreeTables tab)
+{
+  constexpr int kPairs = tree_pairs(P);
+  constexpr int kRows = 2 * NSL + 6 * ND;
+  static_assert(kRows <= kSumRows, "one row of lane sums per value");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* s_red = reinterpret_cast<double*>(smem_raw) + (threadIdx.x >> 5) * kSumRows * kSumStride;
+  double* s_sum = reinterpret_cast<double*>(smem_raw) + kCellWarps * kSumRows * kSumStride;  // [kRows][kPairs]
+  int cell = blockIdx.x;
+  const int e = tree_entry(off, nmesh, cell);
+  const TreeDesc& d = descs[e];
+  if (d.far.active && *d.far.active == 0) return;
+  const ApplyArgs& A = many ? many[e] : one;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double rho = d.ball[cell].w;
+  const int tri = cell * kCell + lane;
+  const bool on = tri < A.ne;
+  const int sel = on ? tri : cell * kCell;
+  CellPoints p;
+  load_points(d, sel, 1.0 / rho, p);
+  double wj[kQ], s[kQ], t[NSL > 0 ? NSL : 1], nrm[3] = {0.0, 0.0, 0.0};
+  const int orig = A.perm[sel];
+#pragma unroll
+  for (int a = 0; a < kQ; ++a) wj[a] = on ? A.wj[(size_t)sel * kQ + a] : 0.0;
+#pragma unroll
+  for (int c = 0; c < NSL; ++c) t[c] = A.t[(size_t)c * A.tstride + orig];
+  if constexpr (ND > 0) {
+    const int4 v = A.svid[sel];
+    const double* u = A.u + (size_t)blockIdx.y * A.ustride;
+    const double u0 = u[v.x], u1 = u[v.y], u2 = u[v.z];
+#pragma unroll
+    for (int a = 0; a < kQ; ++a) {
+      const double e1 = A.bary[2 * a], e2 = A.bary[2 * a + 1];
+      s[a] = wj[a] * ((1.0 - e1 - e2) * u0 + e1 * u1 + e2 * u2);
+    }
+    const dq n = A.trin[sel];
+    nrm[0] = n.x; nrm[1] = n.y; nrm[2] = n.z;
+  }
+  each_harmonic<P>(tab, p, warp, [&](int n, int m, const double (&re)[kQ], const double (&im)[kQ]) {
+    int row = 0;
+    if constexpr (NSL > 0) {
+      double hr = 0.0, hi = 0.0;
+#pragma unroll
+      for (int a = 0; a < kQ; ++a) {
+        hr += wj[a] * re[a];
+        hi += wj[a] * im[a];
+      }
+#pragma unroll
+      for (int c = 0; c < NSL; ++c) {
+        s_red[row++ * kSumStride + lane] = hr * t[c];
+        s_red[row++ * kSumStride + lane] = hi * t[c];
+      }
+    }
+    if constexpr (ND > 0) {
+      double gr = 0.0, gi = 0.0;
+#pragma unroll
+      for (int a = 0; a < kQ; ++a) {
+        gr += s[a] * re[a];
+        gi += s[a] * im[a];
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        s_red[row++ * kSumStride + lane] = gr * nrm[k];
+        s_red[row++ * kSumStride + lane] = gi * nrm[k];
+      }
+    }
+    __syncwarp();
+    // four lanes add a row of 32
+    const int r = lane >> 2, part = lane & 3;
+    double v = 0.0;
+    if (r < kRows)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v += s_red[r * kSumStride + part + 4 * k];
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    if (part == 0 && r < kRows) s_sum[r * kPairs + tree_pair(n, m)] = v;
+    __syncwarp();
+  });
+  __syncthreads();
+  const size_t cstride = (size_t)d.nnodes * kPairs;
+  double2* out = d.multipole + (size_t)cell * kPairs;
+  for (int i = threadIdx.x; i < kPairs; i += 32 * kCellWarps) {
+#pragma unroll
+    for (int c = 0; c < NSL; ++c)
+      out[c * cstride + i] = make_double2(s_sum[2 * c * kPairs + i], s_sum[(2 * c + 1) * kPairs + i]);
+    if constexpr (ND > 0) {
+      // (n.grad) R_n^m from the moments G^k = sum s n_k R of degree n - 1
+      const double* g = s_sum + 2 * NSL * kPairs;
+      const int info = tab.pair[i];
+      const int m = info >> 20 & 31, n = info >> 25;
+      double ar = 0.0, ai = 0.0;
+      if (n > 0) {
+        if (m < n) {
+          const int j = tree_pair(n - 1, m);
+          const double f = sqrt((double)((n - m) * (n + m)));
+          ar += f * g[4 * kPairs + j];
+          ai += f * g[5 * kPairs + j];
+        }
+        {  // -1/2 (G^x + i G^y)_{n-1}^{m-1}
+          const double f = -0.5 * sqrt((double)((n + m) * (n + m - 1)));
+          double xr = 0.0, xi = 0.0, yr = 0.0, yi = 0.0;
+          if (m > 0) {
+            const int j = tree_pair(n - 1, m - 1);
+            xr = g[j]; xi = g[kPairs + j]; yr = g[2 * kPairs + j]; yi = g[3 * kPairs + j];
+          } else if (n > 1) {  // order -1: minus the conjugate of order 1
+            const int j = tree_pair(n - 1, 1);
+            xr = -g[j]; xi = g[kPairs + j]; yr = -g[2 * kPairs + j]; yi = g[3 * kPairs + j];
+          }
+          ar += f * (xr - yi);
+          ai += f * (xi + yr);
+        }
+        if (m + 1 < n) {  // +1/2 (G^x - i G^y)_{n-1}^{m+1}
+          const double f = 0.5 * sqrt((double)((n - m) * (n - m - 1)));
+          const int j = tree_pair(n - 1, m + 1);
+          ar += f * (g[j] + g[3 * kPairs + j]);
+          ai += f * (g[kPairs + j] - g[2 * kPairs + j]);
+        }
+        ar /= rho;
+        ai /= rho;
+      }
+      out[((size_t)NSL + blockIdx.y) * cstride + i] = make_double2(ar, ai);
+    }
+  }
+}
+
+template <int P, int NSL, int ND>
+constexpr size_t p2m_smem()
+{
+  return sizeof(double) * (kCellWarps * kSumRows * kSumStride + (2 * NSL + 6 * ND) * tree_pairs(P));
+}
+
+// Far sums of one cell's rows: sum_a w_a phi_c(x_a) for every column c.
+template <int P, int NC>
+__global__ void __launch_bounds__(32 * kCellWarps)
+    tree_l2p_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh, TreeTables tab)
+{
+  constexpr int kPairs = tree_pairs(P);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* s_loc = reinterpret_cast<double2*>(smem_raw);  // [NC][kPairs]
+  __shared__ double s_part[kCellWarps][NC][kCell];
+  int cell = blockIdx.x;
+  const TreeDesc& d = descs[tree_entry(off, nmesh, cell)];
+  if (d.far.active && *d.far.active == 0) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < kPairs * NC; i += 32 * kCellWarps) {
+    const int c = i / kPairs, q = i - c * kPairs;
+    double2 v = d.local[((size_t)c * d.nnodes + cell) * kPairs + q];
+    if (tab.pair[q] >> 20 & 31) {  // orders m and -m
+      v.x *= 2.0;
+      v.y *= 2.0;
+    }
+    s_loc[i] = v;
+  }
+  const int tri = cell * kCell + lane;
+  const bool on = tri < d.far.ne;
+  const int sel = on ? tri : cell * kCell;
+  CellPoints p;
+  load_points(d, sel, 1.0 / d.ball[cell].w, p);
+  double w[kQ], phi[NC];
+#pragma unroll
+  for (int a = 0; a < kQ; ++a) w[a] = d.far.tgt64[(size_t)sel * kQ + a].w;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) phi[c] = 0.0;
+  __syncthreads();
+  each_harmonic<P>(tab, p, warp, [&](int n, int m, const double (&re)[kQ], const double (&im)[kQ]) {
+    double hr = 0.0, hi = 0.0;
+#pragma unroll
+    for (int a = 0; a < kQ; ++a) {
+      hr += w[a] * re[a];
+      hi += w[a] * im[a];
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const double2 l = s_loc[c * kPairs + tree_pair(n, m)];
+      phi[c] += l.x * hr + l.y * hi;
+    }
+  });
+#pragma unroll
+  for (int c = 0; c < NC; ++c) s_part[warp][c][lane] = phi[c];
+  __syncthreads();
+  if (warp == 0) {
+    const size_t stride = (size_t)d.slot_off[d.ncells] * kCell;
+    double* out = d.partial + (size_t)(d.slot_off[cell + 1] - 1) * kCell + lane;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      double v = 0.0;
+#pragma unroll
+      for (int k = 0; k < kCellWarps; ++k) v += s_part[k][c][lane];
+      out[c * stride] = v;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Close cells: one warp per task, a lane per target triangle, the source cell
+// staged in shared memory; every unordered pair of cells once, both orders
+// (the transposed sums of a source cell go to its slot), a cell with itself
+// in forward order.
+
+template <typename T, int NSL, int ND>
+constexpr int near_sources() { return sizeof(T) == 4 ? kCell : kCell / 2; }  // sources per reduction
+
+template <typename T, int NSL, int ND>
+constexpr size_t near_red_row()  // bytes of a lane's transposed sums, padded
+{
+  return sizeof(T) == 4 ? (ND > 0 ? 16 * (kCell / 2 + 1) : 8 * (kCell / 2 * NSL + 1))
+                        : (ND > 0 ? 16 * (kCell / 2 + 1) : 8 * (kCell / 2 * NSL + 1));
+}
+
+template <typename T, int NSL, int ND>
+constexpr size_t near_smem()
+{
+  return (size_t)kCell * kQ * kNrec * 4 * sizeof(T) + kCell * near_red_row<T, NSL, ND>();
+}
+
+template <typename T, int NSL, int ND>
+__global__ void __launch_bounds__(32, 8)
+    tree_near_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh)
+{
+  using S = typename Slot<T>::type;
+  constexpr bool F32 = sizeof(T) == 4;
+  constexpr int NO = NSL + ND;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int4 s_vid[kCell];
+  __shared__ dq s_nrm[ND ? kCell : 1];
+  __shared__ S s_plane[ND ? kCell : 1];
+  S* s_rec = reinterpret_cast<S*>(smem_raw);
+  unsigned char* s_red = smem_raw + (size_t)kCell * kQ * kNrec * 4 * sizeof(T);
+  const int lane = threadIdx.x;
+  unsigned char* my_red = s_red + lane * near_red_row<T, NSL, ND>();
+  int k = blockIdx.x;
+  const TreeDesc& d = descs[tree_entry(off, nmesh, k)];
+  const FarMeshDesc& md = d.far;
+  if (md.active && *md.active == 0) return;
+  const int4 task = d.tasks[k];
+  const int ti = task.x * kCell + lane;
+  const bool active = ti < md.ne;
+  const int tsel = active ? ti : task.x * kCell;
+  const dq ball = md.twarp[task.x];
+  double cen[3], nrm[3] = {0.0, 0.0, 0.0}, pin = 0.0;
+  {
+    const dq c = md.tcent[tsel];
+    cen[0] = c.x; cen[1] = c.y; cen[2] = c.z;
+    if constexpr (ND > 0) {
+      const dq n = md.snrm[tsel];
+      nrm[0] = n.x; nrm[1] = n.y; nrm[2] = n.z;
+      pin = n.w;
+    }
+  }
+  const int4 tv = active ? md.tvid[tsel] : make_int4(-1, -1, -1, 0);
+  const S* grec = reinterpret_cast<const S*>(md.rec);
+  const size_t stride = (size_t)d.slot_off[d.ncells] * kCell;
+  T hi[NO], lo[NO];
+#pragma unroll
+  for (int c = 0; c < NO; ++c) hi[c] = lo[c] = 0;
+
+#pragma unroll 1
+  for (int e = task.y; e < task.z; ++e) {
+    const int2 en = d.entries[e];
+    const int cell = en.x, t0 = cell * kCell;
+    const int ns = min(kCell, md.ne - t0);
+    {
+      const S* g = grec + (size_t)t0 * kQ * kNrec;
+      if constexpr (F32) {  // source-pair layout, as the symmetric kernel stages it
+        constexpr int per = kQ * kNrec;
+        const int nstage = ((ns + 1) >> 1) * per;
+        for (int i = lane; i < nstage; i += 32) {
+          const int p = i / per, rem = i - p * per;
+          const float4 a = g[(size_t)(2 * p) * per + rem];
+          float4 c;
+          if (2 * p + 1 < ns) c = g[(size_t)(2 * p + 1) * per + rem];
+          else c = rem % kNrec == 0 ? make_float4(0.f, 0.f, 0.f, 1.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+          s_rec[2 * i] = make_float4(a.x, c.x, a.y, c.y);
+          s_rec[2 * i + 1] = make_float4(a.z, c.z, a.w, c.w);
+        }
+        if ((ns & 1) && lane == 0) {
+          s_vid[ns] = make_int4(-1, -1, -1, 0);
+          if constexpr (ND > 0) {
+            s_nrm[ns] = dq{0.0, 0.0, 0.0, 0.0};
+            s_plane[ns] = make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+        }
+      } else {
+        for (int i = lane; i < ns * kQ * kNrec; i += 32) s_rec[i] = g[i];
+      }
+      if (lane < ns) {
+        s_vid[lane] = md.svid[t0 + lane];
+        if constexpr (ND > 0) {
+          s_nrm[lane] = md.snrm[t0 + lane];
+          if constexpr (F32) s_plane[lane] = md.splane32[t0 + lane];
+          else s_plane[lane] = md.splane64[t0 + lane];
+        }
+      }
+    }
+    __syncwarp();
+    const dq cc = md.ccent[cell];
+    const double ddx = cc.x - ball.x, ddy = cc.y - ball.y, ddz = cc.z - ball.z;
+    const double rr = kFarRatio * (cc.w + ball.w);
+    const bool far = ddx * ddx + ddy * ddy + ddz * ddz > rr * rr;
+    const T o[3] = {(T)(cc.x - cen[0]), (T)(cc.y - cen[1]), (T)(cc.z - cen[2])};
+    T xs[kQ], ys[kQ], zs[kQ], q2[kQ], wq[kQ], part[NO];
+#pragma unroll
+    for (int a = 0; a < kQ; ++a) {
+      S p;
+      if constexpr (F32) p = md.tgt32[(size_t)tsel * kQ + a];
+      else p = md.tgt64[(size_t)tsel * kQ + a];
+      xs[a] = p.x - o[0]; ys[a] = p.y - o[1]; zs[a] = p.z - o[2];
+      q2[a] = xs[a] * xs[a] + ys[a] * ys[a] + zs[a] * zs[a];
+      wq[a] = p.w;
+    }
+    const double c3[3] = {cc.x, cc.y, cc.z};
+#pragma unroll
+    for (int c = 0; c < NO; ++c) part[c] = 0;
+    if (cell == task.x) {
+      T sl[NSL][kQ], dl[1][kQ];
+#pragma unroll
+      for (int a = 0; a < kQ; ++a) {
+        dl[0][a] = 0;
+#pragma unroll
+        for (int c = 0; c < NSL; ++c) sl[c][a] = 0;
+      }
+      if (active) {
+        if constexpr (F32)
+          eval_cell_sp<kQ, kQ, NSL, ND, false>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm,
+                                               sl, dl);
+        else
+          eval_cell<T, kQ, kQ, NSL, ND, false>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm,
+                                               sl, dl);
+      }
+#pragma unroll
+      for (int a = 0; a < kQ; ++a) {
+#pragma unroll
+        for (int c = 0; c < NSL; ++c) part[c] += wq[a] * sl[c][a];
+        if constexpr (ND > 0) part[NSL] += wq[a] * dl[0][a];
+      }
+    } else {
+      constexpr int kSrc = near_sources<T, NSL, ND>();
+#pragma unroll 1
+      for (int h = 0; h < ns; h += kSrc) {
+        const int h1 = min(ns, h + kSrc);
+        if (active) {
+          // the target's strengths (SL + DL: s_a, c_a) and charges
+          if constexpr (ND > 0) {
+            T ca[kQ], cd[kQ], dl[kQ], slw = 0;
+#pragma unroll
+            for (int a = 0; a < kQ; ++a) {
+              const S st = grec[((size_t)tsel * kQ + a) * kNrec + 1];
+              cd[a] = st.x;
+              ca[a] = st.y;
+              dl[a] = 0;
+            }
+            if constexpr (F32) {
+              float4* red = reinterpret_cast<float4*>(my_red);
+              if (far) eval_cell_sym<true>(s_rec, s_vid, s_nrm, s_plane, h, h1, tv, xs, ys, zs, q2, ca, cd, wq, o, cen,
+                                           nrm, c3, pin, slw, dl, red);
+              else eval_cell_sym<false>(s_rec, s_vid, s_nrm, s_plane, h, h1, tv, xs, ys, zs, q2, ca, cd, wq, o, cen,
+                                        nrm, c3, pin, slw, dl, red);
+            } else {
+              double2* red = reinterpret_cast<double2*>(my_red);
+              if (far) eval_cell_sym64<true>(s_rec, s_vid, s_nrm, s_plane, h, h1, tv, xs, ys, zs, q2, ca, cd, wq, o,
+                                             cen, nrm, c3, pin, slw, dl, red);
+              else eval_cell_sym64<false>(s_rec, s_vid, s_nrm, s_plane, h, h1, tv, xs, ys, zs, q2, ca, cd, wq, o, cen,
+                                          nrm, c3, pin, slw, dl, red);
+            }
+            part[0] += slw;
+#pragma unroll
+            for (int a = 0; a < kQ; ++a) part[NSL] += wq[a] * dl[a];
+          } else {
+            T cw[NSL][kQ], om[kQ], slw[NSL];
+#pragma unroll
+            for (int a = 0; a < kQ; ++a) {
+              om[a] = wq[a] / wq[0];
+              const S st = grec[((size_t)tsel * kQ + a) * kNrec + 1];
+#pragma unroll
+              for (int c = 0; c < NSL; ++c) cw[c][a] = wq[0] * comp(st, c);
+            }
+#pragma unroll
+            for (int c = 0; c < NSL; ++c) slw[c] = 0;
+            if constexpr (F32) {
+              float2* red = reinterpret_cast<float2*>(my_red);
+              if (far) eval_cell_sym_sl<NSL, true>(s_rec, s_vid, h, h1, tv, xs, ys, zs, q2, cw, om, wq, slw, red);
+              else eval_cell_sym_sl<NSL, false>(s_rec, s_vid, h, h1, tv, xs, ys, zs, q2, cw, om, wq, slw, red);
+            } else {
+              double* red = reinterpret_cast<double*>(my_red);
+              if (far) eval_cell_sym64_sl<NSL, true>(s_rec, s_vid, h, h1, tv, xs, ys, zs, q2, cw, om, wq, slw, red);
+              else eval_cell_sym64_sl<NSL, false>(s_rec, s_vid, h, h1, tv, xs, ys, zs, q2, cw, om, wq, slw, red);
+            }
+#pragma unroll
+            for (int c = 0; c < NSL; ++c) part[c] += slw[c];
+          }
+        } else {
+          for (size_t i = 0; i < near_red_row<T, NSL, ND>() / 8; ++i) reinterpret_cast<double*>(my_red)[i] = 0.0;
+        }
+        __syncwarp();
+        // lane l adds source triangle h + l over the 32 target lanes in order
+        constexpr size_t row = near_red_row<T, NSL, ND>() / sizeof(T);
+        const T* rf = reinterpret_cast<const T*>(s_red);
+        if (h + lane < h1) {
+#pragma unroll
+          for (int c = 0; c < NO; ++c) {
+            // FP32 sums of a triangle pair are interleaved
+            int at;
+            if constexpr (F32) at = ND > 0 ? (lane >> 1) * 4 + 2 * c + (lane & 1) : ((lane >> 1) * NSL + c) * 2 + (lane & 1);
+            else at = lane * NO + c;
+            T v0 = 0, v1 = 0, v2 = 0, v3 = 0;
+#pragma unroll 4
+            for (int t = 0; t < 32; t += 4) {
+              v0 += rf[(t + 0) * row + at];
+              v1 += rf[(t + 1) * row + at];
+              v2 += rf[(t + 2) * row + at];
+              v3 += rf[(t + 3) * row + at];
+            }
+            d.partial[c * stride + (size_t)en.y * kCell + h + lane] = (double)((v0 + v1) + (v2 + v3));
+          }
+        }
+        __syncwarp();
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < NO; ++c) {
+      if constexpr (F32) two_sum_add(hi[c], lo[c], part[c]);
+      else hi[c] += part[c];
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int c = 0; c < NO; ++c)
+    d.partial[c * stride + (size_t)task.w * kCell + lane] = active ? (double)hi[c] + (double)lo[c] : 0.0;
+}
+
+// ---------------------------------------------------------------------------
+// Tables (host, extended precision).
+
+using ld = long double;
+
+std::vector<std::vector<ld>> half_turns(int P)
+{
+  // d^n_{m'm}(90 degrees), [n][(m' + n) (2n + 1) + m + n], by the three-term
+  // recurrence in n (stable upward) from n = max(|m|, |m'|)
+  std::vector<std::vector<ld>> d(P + 1);
+  for (int n = 0; n <= P; n++) d[n].assign((size_t)(2 * n + 1) * (2 * n + 1), 0.0L);
+  auto binom = [](int n, int k) {
+    ld v = 1.0L;
+    for (int i = 1; i <= k; i++) v = v * (n - k + i) / i;
+    return v;
+  };
+  for (int a = -P; a <= P; a++)
+    for (int b = -P; b <= P; b++) {
+      const int l0 = std::max(std::abs(a), std::abs(b));
+      const ld half = std::pow(0.5L, l0);
+      ld cur;
+      if (a == l0) cur = std::sqrt(binom(2 * l0, l0 + b)) * half * ((l0 - b) & 1 ? -1 : 1);
+      else if (a == -l0) cur = std::sqrt(binom(2 * l0, l0 + b)) * half;
+      else if (b == l0) cur = std::sqrt(binom(2 * l0, l0 + a)) * half;
+      else cur = std::sqrt(binom(2 * l0, l0 + a)) * half * ((l0 + a) & 1 ? -1 : 1);
+      ld prev = 0.0L;
+      for (int n = l0; n <= P; n++) {
+        d[n][(size_t)(a + n) * (2 * n + 1) + b + n] = cur;
+        ld next = 0.0L;
+        if (n > 0)
+          next = ((2 * n + 1) * (ld)(-a * b) * cur -
+                  (n + 1) * std::sqrt((ld)(n * n - a * a) * (n * n - b * b)) * prev) /
+                 (n * std::sqrt((ld)((n + 1) * (n + 1) - a * a) * ((n + 1) * (n + 1) - b * b)));
+        prev = cur;
+        cur = next;
+      }
+    }
+  return d;
+}
+
+struct HostTables {
+  std::vector<double> bmat, tmat[3];
+  std::vector<int2> bround, tround;
+  std::vector<int> bout, tout, pair;
+  std::vector<double2> rec;
+};
+
+HostTables make_tables(int P)
+{
+  HostTables h;
+  const int ncoef = (P + 1) * (P + 1), rounds = (ncoef + 31) / 32;
+  auto even = [](int n) { return n / 2 + 1; };
+  auto pos = [&](int n, int m, int im) {
+    const int base = n * n + (im ? n + 1 : 0), e = even(n) - im;
+    return base + (m & 1 ? e + (m - 1) / 2 : m / 2 - im);
+  };
+  std::vector<int> mbase(2 * (P + 1));
+  for (int m = 0, at = 0; m <= P; m++)
+    for (int im = 0; im < (m ? 2 : 1); im++) {
+      mbase[2 * m + im] = at;
+      at += P + 1 - m;
+    }
+  struct Out {
+    int n, m, im;
+  };
+  std::vector<Out> grouped(ncoef), major(ncoef);
+  for (int n = 0; n <= P; n++)
+    for (int m = 0; m <= n; m++)
+      for (int im = 0; im < (m ? 2 : 1); im++) {
+        grouped[pos(n, m, im)] = Out{n, m, im};
+        major[mbase[2 * m + im] + n - m] = Out{n, m, im};
+      }
+  // Ry(90)
+  const auto d = half_turns(P);
+  std::vector<std::vector<double>> rows(ncoef);
+  h.bout.resize(ncoef);
+  for (int o = 0; o < ncoef; o++) {
+    const Out q = grouped[o];
+    const int par = (q.n + q.m + q.im) & 1;
+    int first = -1;
+    for (int m = par; m <= q.n; m += 2) {
+      if (q.im && m == 0) continue;
+      if (first < 0) first = pos(q.n, m, q.im);
+      const ld* row = &d[q.n][(size_t)(q.m + q.n) * (2 * q.n + 1)];
+      const ld minus = (m & 1 ? -1 : 1) * row[q.n - m];
+      rows[o].push_back((double)(m == 0 ? row[q.n] : q.im ? row[q.n + m] - minus : row[q.n + m] + minus));
+    }
+    const int sign = (q.n + q.im) & 1;
+    h.bout[o] = std::max(first, 0) | (mbase[2 * q.m + q.im] + q.n - q.m) << 11 | sign << 22;
+  }
+  auto pad = [&](const std::vector<std::vector<double>>& r, std::vector<double>& mat, std::vector<int2>* rounds_out) {
+    for (int k = 0; k < rounds; k++) {
+      size_t len = 0;
+      for (int o = 32 * k; o < std::min(ncoef, 32 * k + 32); o++) len = std::max(len, r[o].size());
+      if (rounds_out) rounds_out->push_back(make_int2((int)mat.size(), (int)len));
+      for (size_t j = 0; j < len; j++)
+        for (int o = 32 * k; o < 32 * k + 32; o++)
+          mat.push_back(o < ncoef && j < r[o].size() ? r[o][j] : 0.0);
+    }
+  };
+  pad(rows, h.bmat, &h.bround);
+  // along z
+  std::vector<ld> fact(2 * P + 2, 1.0L);
+  for (int k = 1; k < 2 * P + 2; k++) fact[k] = fact[k - 1] * k;
+  auto norm = [&](int n, int m) { return std::sqrt(fact[n - m] * fact[n + m]); };
+  h.tout.resize(ncoef);
+  for (int mode = 0; mode < 3; mode++) {
+    for (auto& r : rows) r.clear();
+    for (int o = 0; o < ncoef; o++) {
+      const Out q = major[o];
+      h.tout[o] = mbase[2 * q.m + q.im] | pos(q.n, q.m, q.im) << 11 | (q.n - q.m) << 22;
+      for (int k = q.m; k <= P; k++) {
+        ld v = 0.0L;
+        if (mode == kAcross) v = ((q.n + q.m) & 1 ? -1 : 1) * fact[q.n + k] / (norm(q.n, q.m) * norm(k, q.m));
+        else if (mode == kUp && k <= q.n) v = norm(q.n, q.m) / (norm(k, q.m) * fact[q.n - k]);
+        else if (mode == kDown && k >= q.n) v = norm(k, q.m) / (norm(q.n, q.m) * fact[k - q.n]);
+        rows[o].push_back((double)v);
+      }
+    }
+    pad(rows, h.tmat[mode], mode == 0 ? &h.tround : nullptr);
+  }
+  h.rec.assign(tree_pairs(P), make_double2(0.0, 0.0));
+  for (int n = 0; n <= P; n++)
+    for (int m = 0; m <= n; m++) {
+      h.pair.push_back(pos(n, m, 0) | (m ? pos(n, m, 1) : ncoef) << 10 | m << 20 | n << 25);
+      if (n > m) {
+        const double q = (double)(n * n - m * m);
+        h.rec[n * (n + 1) / 2 + m] =
+            make_double2((2 * n - 1) / std::sqrt(q), std::sqrt(((n - 1.0) * (n - 1.0) - m * m) / q));
+      }
+    }
+  return h;
+}
+
+// One set per device and order, made on first use and kept for the process
+// (0.4 MB for both orders).
+int tables_for(int device, int P, TreeTables* out)
+{
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, TreeTables> known;
+  std::lock_guard<std::mutex> g(mu);
+  const auto it = known.find({device, P});
+  if (it != known.end()) {
+    *out = it->second;
+    return EB_OK;
+  }
+  const HostTables h = make_tables(P);
+  std::vector<unsigned char> host;
+  auto add = [&](const auto& v) {
+    const size_t at = (host.size() + 15) & ~(size_t)15;
+    host.resize(at + v.size() * sizeof(v[0]));
+    std::memcpy(host.data() + at, v.data(), v.size() * sizeof(v[0]));
+    return at;
+  };
+  const size_t at[] = {add(h.bmat), add(h.tmat[0]), add(h.tmat[1]), add(h.tmat[2]), add(h.bround),
+                       add(h.tround), add(h.bout),  add(h.tout),    add(h.pair),    add(h.rec)};
+  auto buf = std::make_unique<DevBuf>();
+  EB_CHECK(buf->alloc(host.size()));
+  EB_CHECK(copy_h2d(buf->p, host.data(), host.size()));
+  const unsigned char* p = static_cast<const unsigned char*>(buf.release()->p);  // kept
+  TreeTables t;
+  t.bmat = reinterpret_cast<const double*>(p + at[0]);
+  for (int k = 0; k < 3; k++) t.tmat[k] = reinterpret_cast<const double*>(p + at[1 + k]);
+  t.bround = reinterpret_cast<const int2*>(p + at[4]);
+  t.tround = reinterpret_cast<const int2*>(p + at[5]);
+  t.bout = reinterpret_cast<const int*>(p + at[6]);
+  t.tout = reinterpret_cast<const int*>(p + at[7]);
+  t.pair = reinterpret_cast<const int*>(p + at[8]);
+  t.rec = reinterpret_cast<const double2*>(p + at[9]);
+  known[{device, P}] = t;
+  *out = t;
+  return EB_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Launches.
+
+template <typename... Args>
+cudaError_t start(void (*fn)(Args...), dim3 grid, int block, size_t smem, cudaStream_t st, Args... args)
+{
+  if (grid.x == 0) return cudaSuccess;
+  if (smem > 32 * 1024) {  // per device: set on every launch (a host-side call)
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  fn<<<grid, block, smem, st>>>(args...);
+  return cudaGetLastError();
+}
+
+// Block counts of each kernel over the meshes of a launch and, for more than
+// one mesh, the first block of each (device).
+struct TreeGrid {
+  int nmesh = 1;
+  const int *cells = nullptr, *m2l = nullptr, *tasks = nullptr, *up[kTreePasses] = {};
+  int ncells = 0, nm2l = 0, ntasks = 0, nup[kTreePasses] = {};
+};
+
+template <int P, typename T, int NSL, int ND>
+int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const ApplyArgs* many, const TreeTables& tab,
+               cudaStream_t st)
+{
+  constexpr int NC = NSL + ND;
+  // columns moved together: two share the matrices' loads while the buffers
+  // of a CTA stay small (order 14: 34 KB)
+  constexpr int MC = P <= 16 && NC % 2 == 0 ? 2 : 1;
+  const dim3 b(32 * kMoveWarps);
+  EB_CUDA(start(tree_p2m_kernel<P, NSL, ND>, dim3(g.ncells), 32 * kCellWarps, p2m_smem<P, NSL, ND>(), st, d, g.cells,
+                g.nmesh, one, many, tab));
+  for (int s = 0; s < kTreePasses; s++)
+    EB_CUDA(start(tree_move_kernel<P, MC, kUp>, dim3(g.nup[s], NC / MC), b.x, move_smem<P, MC>(), st, d, g.up[s],
+                  g.nmesh, s, tab));
+  EB_CUDA(start(tree_move_kernel<P, MC, kAcross>, dim3(g.nm2l, NC / MC), b.x, move_smem<P, MC>(), st, d, g.m2l, g.nmesh,
+                0, tab));
+  EB_CUDA(start(tree_move_kernel<P, MC, kDown>, dim3(g.ncells, NC / MC), b.x, move_smem<P, MC>(), st, d, g.cells,
+                g.nmesh, 0, tab));
+  EB_CUDA(start(tree_l2p_kernel<P, NC>, dim3(g.ncells), 32 * kCellWarps, sizeof(double2) * NC * tree_pairs(P), st, d,
+                g.cells, g.nmesh, tab));
+  EB_CUDA(start(tree_near_kernel<T, NSL, ND>, dim3(g.ntasks), 32, near_smem<T, NSL, ND>(), st, d, g.tasks, g.nmesh));
+  return EB_OK;
+}
+
+bool tree_variant(int nsl, int nd) { return (nsl == 1 && nd == 1) || (nd == 0 && (nsl == 1 || nsl == 3 || nsl == 4)); }
+
+int launch_variant(bool fp32, int nsl, int nd, const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one,
+                   const ApplyArgs* many, int device, cudaStream_t st)
+{
+  TreeTables tab;
+  EB_CHECK(tables_for(device, fp32 ? kTreeOrder32 : kTreeOrder64, &tab));
+#define EB_TREE(NSL, ND)                                                                        \
+  if (nsl == NSL && nd == ND)                                                                   \
+    return fp32 ? launch_all<kTreeOrder32, float, NSL, ND>(d, g, one, many, tab, st)            \
+                : launch_all<kTreeOrder64, double, NSL, ND>(d, g, one, many, tab, st);
+  EB_TREE(1, 1)
+  EB_TREE(1, 0)
+  EB_TREE(3, 0)
+  EB_TREE(4, 0)
+#undef EB_TREE
+  return set_error(EB_ERR_INVALID, "no tree far field for this operator combination");
+}
+
+}  // namespace
+
+// Smallest mesh (cells) that takes the tree.
+#ifndef EB_TREE_MIN32
+#define EB_TREE_MIN32 256
+#endif
+#ifndef EB_TREE_MIN64
+#define EB_TREE_MIN64 320
+#endif
+
+bool tree_eligible(Mesh* m, bool fp32, int nsl, int nd)
+{
+  const HostMesh& h = m->h;
+  if (m->plan.engine != 4 || !tree_variant(nsl, nd) || h.Q != kSymRule || h.K != kSymRule || h.nchunk != 1 ||
+      h.ncells < (fp32 ? EB_TREE_MIN32 : EB_TREE_MIN64))
+    return false;
+  if (!m->tree) {
+    auto t = std::make_shared<TreeMesh>();
+    t->usable = make_tree_plan(h, &t->plan);
+    m->tree = t;
+  }
+  return m->tree->usable;
+}
+
+static int upload_lists(TreeMesh* t)
+{
+  if (t->lists.p) return EB_OK;
+  const TreePlan& p = t->plan;
+  std::vector<unsigned char> host;
+  auto add = [&](const auto& v) {
+    const size_t at = (host.size() + 15) & ~(size_t)15;
+    host.resize(at + std::max<size_t>(1, v.size()) * sizeof(v[0]));
+    if (!v.empty()) std::memcpy(host.data() + at, v.data(), v.size() * sizeof(v[0]));
+    return at;
+  };
+  const size_t ball = add(p.ball), has = add(p.has_local), tasks = add(p.tasks), entries = add(p.entries),
+               slots = add(p.slot_off);
+  struct At {
+    size_t tgt, ptr, src;
+  };
+  auto moves = [&](const TreeMoves& m) { return At{add(m.tgt), add(m.ptr), add(m.src)}; };
+  At up[kTreePasses];
+  for (int s = 0; s < kTreePasses; s++) up[s] = moves(p.up[s]);
+  const At m2l = moves(p.m2l), down = moves(p.down);
+  EB_CHECK(t->lists.alloc(host.size()));
+  EB_CHECK(copy_h2d(t->lists.p, host.data(), host.size()));
+  const unsigned char* q = static_cast<const unsigned char*>(t->lists.p);
+  auto dev = [&](const At& a) {
+    return TreeMovesDev{reinterpret_cast<const int*>(q + a.tgt), reinterpret_cast<const int*>(q + a.ptr),
+                        reinterpret_cast<const int*>(q + a.src)};
+  };
+  TreeDesc& d = t->base;
+  d.ball = reinterpret_cast<const dq*>(q + ball);
+  d.has_local = reinterpret_cast<const char*>(q + has);
+  d.tasks = reinterpret_cast<const int4*>(q + tasks);
+  d.entries = reinterpret_cast<const int2*>(q + entries);
+  d.slot_off = reinterpret_cast<const int*>(q + slots);
+  for (int s = 0; s < kTreePasses; s++) {
+    d.up[s] = dev(up[s]);
+    d.nup[s] = (int)p.up[s].tgt.size();
+  }
+  d.m2l = dev(m2l);
+  d.down = dev(down);
+  d.nnodes = p.nnodes;
+  d.ncells = p.ncells;
+  d.ntasks = (int)p.tasks.size();
+  d.nm2l = (int)p.m2l.tgt.size();
+  return EB_OK;
+}
+
+long long tree_far_slots(const Mesh* m) { return (long long)m->tree->plan.slot_off.back() * kCell; }
+
+int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream_t st)
+{
+  TreeMesh* t = m->tree.get();
+  EB_CHECK(upload_lists(t));
+  std::unique_ptr<TreeScratch>& sc = t->scratch[(fp32 ? 64 : 0) + nsl * 5 + nd];
+  if (!sc) {
+    auto s = std::make_unique<TreeScratch>();
+    const int cols = nsl + nd;
+    const size_t bytes = sizeof(double2) * (size_t)cols * t->plan.nnodes * tree_pairs(fp32 ? kTreeOrder32 : kTreeOrder64);
+    EB_CHECK(s->multipole.alloc(bytes));
+    EB_CHECK(s->local.alloc(bytes));
+    EB_CHECK(s->partial.alloc(sizeof(double) * (size_t)cols * tree_far_slots(m)));
+    TreeDesc d = t->base;
+    d.far = mesh_far_desc(m, fp32, nsl, nd, m->rec.p, s->partial.as<double>());
+    d.pos = m->pos64.as<dq>();
+    d.multipole = s->multipole.as<double2>();
+    d.local = s->local.as<double2>();
+    d.partial = s->partial.as<double>();
+    EB_CHECK(s->desc.alloc(sizeof d));
+    EB_CHECK(copy_h2d(s->desc.p, &d, sizeof d));
+    s->host = d;
+    sc = std::move(s);
+  }
+  const TreeDesc& d = sc->host;
+  A->partial = d.partial;
+  A->slot_off = d.slot_off;
+  TreeGrid g;
+  g.ncells = d.ncells;
+  g.nm2l = d.nm2l;
+  g.ntasks = d.ntasks;
+  std::copy_n(d.nup, kTreePasses, g.nup);
+  if (m->profile) EB_CUDA(cudaEventRecord(m->ev0, st));
+  return launch_variant(fp32, nsl, nd, sc->desc.as<TreeDesc>(), g, *A, nullptr, m->device, st);
+}
+
+}  // namespace eb

@@ -33,6 +33,7 @@ struct HostMesh {
   std::vector<int> perm, iperm;
   int ncells = 0;
   std::vector<double> cell_ball;  // [ncells][4]: centre and radius of a ball around the cell's vertices
+  std::vector<double> cell_rho;   // [ncells]: the ball's radius over the quadrature points only (with the static tables)
 
   // Target items: a triangle's Q points split into chunks of at most K points.
   int K = 0;        // target points per item (compile-time kernel width)

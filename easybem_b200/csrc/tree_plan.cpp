@@ -1,0 +1,205 @@
+#include "tree_plan.h"
+
+#include <algorithm>
+#include <cmath>
+#include <functional>
+#include <utility>
+
+namespace eb {
+
+namespace {
+
+struct Node {
+  int lo, hi;      // cells
+  int left, right; // children (-1: a cell)
+  int parent;
+  int height;      // 0 for a cell
+};
+
+// A small ball around the balls of cells [lo, hi): the centre of their box,
+// moved towards the farthest ball.
+dq ball_of(const std::vector<dq>& cell, int lo, int hi)
+{
+  d3 a = mk3(1e300, 1e300, 1e300), b = mk3(-1e300, -1e300, -1e300);
+  for (int c = lo; c < hi; c++) {
+    const dq& q = cell[c];
+    a = mk3(std::min(a.x, q.x - q.w), std::min(a.y, q.y - q.w), std::min(a.z, q.z - q.w));
+    b = mk3(std::max(b.x, q.x + q.w), std::max(b.y, q.y + q.w), std::max(b.z, q.z + q.w));
+  }
+  d3 m = 0.5 * (a + b);
+  dq best{0.0, 0.0, 0.0, -1.0};
+  for (int it = 0; it <= 6; it++) {
+    double r = -1.0;
+    d3 far = m;
+    for (int c = lo; c < hi; c++) {
+      const d3 v = mk3(cell[c].x, cell[c].y, cell[c].z) - m;
+      const double d = std::sqrt(dot3(v, v)) + cell[c].w;
+      if (d > r) {
+        r = d;
+        far = mk3(cell[c].x, cell[c].y, cell[c].z);
+      }
+    }
+    if (best.w < 0.0 || r < best.w) best = dq{m.x, m.y, m.z, r};
+    m = m + (1.0 / (it + 4.0)) * (far - m);
+  }
+  best.w *= 1.0 + 1e-12;
+  return best;
+}
+
+}  // namespace
+
+bool make_tree_plan(const HostMesh& h, TreePlan* plan)
+{
+  TreePlan& p = *plan;
+  const int nc = h.ncells;
+  p.ncells = nc;
+  std::vector<Node> nodes(nc);
+  for (int c = 0; c < nc; c++) nodes[c] = Node{c, c + 1, -1, -1, -1, 0};
+  std::function<int(int, int)> build = [&](int lo, int hi) {
+    if (hi - lo == 1) return lo;
+    const int mid = lo + split_cells(hi - lo);
+    const int l = build(lo, mid), r = build(mid, hi);
+    const int k = (int)nodes.size();
+    nodes.push_back(Node{lo, hi, l, r, -1, 1 + std::max(nodes[l].height, nodes[r].height)});
+    nodes[l].parent = nodes[r].parent = k;
+    return k;
+  };
+  const int root = build(0, nc);
+  if (nodes[root].height > kTreePasses * kTreeLevelsPerPass) return false;
+  const int nn = p.nnodes = (int)nodes.size();
+  p.ball.resize(nn);
+  for (int c = 0; c < nc; c++) {
+    const double* b = &h.cell_ball[4 * (size_t)c];
+    p.ball[c] = dq{b[0], b[1], b[2], std::max(h.cell_rho[c], 1e-3 * b[3])};
+  }
+  for (int k = nc; k < nn; k++) p.ball[k] = ball_of(p.ball, nodes[k].lo, nodes[k].hi);
+
+  // the tree against itself
+  std::vector<std::pair<int, int>> far;
+  std::vector<std::vector<int>> near(nc);  // later cells close to each cell
+  const long long limit = std::max<long long>(4 * nc, (long long)nc * nc / 16);
+  long long nnear = 0;
+  std::vector<std::pair<int, int>> stack(1, {root, root});
+  while (!stack.empty()) {
+    const auto [a, b] = stack.back();
+    stack.pop_back();
+    const Node &A = nodes[a], &B = nodes[b];
+    if (a == b) {
+      if (A.left < 0) continue;
+      stack.push_back({A.left, A.right});
+      stack.push_back({A.left, A.left});
+      stack.push_back({A.right, A.right});
+      continue;
+    }
+    const dq &x = p.ball[a], &y = p.ball[b];
+    const d3 d = mk3(x.x - y.x, x.y - y.y, x.z - y.z);
+    const double s = (x.w + y.w) / kTreeTheta;
+    if (dot3(d, d) > s * s) {
+      far.push_back({a, b});
+    } else if (A.left < 0 && B.left < 0) {
+      near[std::min(a, b)].push_back(std::max(a, b));
+      if (++nnear > limit) return false;
+    } else if (B.left < 0 || (A.left >= 0 && x.w >= y.w)) {
+      stack.push_back({A.left, b});
+      stack.push_back({A.right, b});
+    } else {
+      stack.push_back({a, B.left});
+      stack.push_back({a, B.right});
+    }
+  }
+
+  // separated pairs in both directions, by target
+  std::vector<int> count(nn + 1, 0);
+  for (const auto& f : far) {
+    count[f.first + 1]++;
+    count[f.second + 1]++;
+  }
+  for (int k = 0; k < nn; k++) count[k + 1] += count[k];
+  std::vector<int> fill(count.begin(), count.end() - 1), src(2 * far.size());
+  std::vector<char> used(nn, 0);  // its multipole is read
+  for (const auto& f : far) {
+    src[fill[f.first]++] = f.second;
+    src[fill[f.second]++] = f.first;
+    used[f.first] = used[f.second] = 1;
+  }
+  p.has_local.assign(nn, 0);
+  // targets with the longest lists first (the last wave then holds short ones)
+  std::vector<int> order;
+  for (int k = 0; k < nn; k++)
+    if (count[k + 1] > count[k]) {
+      order.push_back(k);
+      p.has_local[k] = 1;
+    }
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int a, int b) { return count[a + 1] - count[a] > count[b + 1] - count[b]; });
+  for (int k : order) {
+    p.m2l.tgt.push_back(k);
+    std::sort(src.begin() + count[k], src.begin() + count[k + 1]);
+    p.m2l.src.insert(p.m2l.src.end(), src.begin() + count[k], src.begin() + count[k + 1]);
+    p.m2l.ptr.push_back((int)p.m2l.src.size());
+  }
+
+  // upward: pass s forms the nodes of heights (s L, (s + 1) L] from their
+  // descendants of height at most s L (the topmost on each path)
+  std::vector<int> byheight;
+  for (int k = nc; k < nn; k++) byheight.push_back(k);
+  std::stable_sort(byheight.begin(), byheight.end(), [&](int a, int b) { return nodes[a].height > nodes[b].height; });
+  std::vector<std::vector<int>> sources(nn);
+  for (int k : byheight) {  // from the top: a used node makes its sources used
+    if (!used[k]) continue;
+    const int base = (nodes[k].height - 1) / kTreeLevelsPerPass * kTreeLevelsPerPass;
+    std::function<void(int)> gather = [&](int j) {
+      if (nodes[j].height <= base) {
+        sources[k].push_back(j);
+        used[j] = 1;
+        return;
+      }
+      gather(nodes[j].left);
+      gather(nodes[j].right);
+    };
+    gather(k);
+  }
+  for (int k = nc; k < nn; k++) {
+    if (!used[k]) continue;
+    TreeMoves& u = p.up[(nodes[k].height - 1) / kTreeLevelsPerPass];
+    u.tgt.push_back(k);
+    u.src.insert(u.src.end(), sources[k].begin(), sources[k].end());
+    u.ptr.push_back((int)u.src.size());
+  }
+
+  // downward: every cell from all its ancestors with a local expansion
+  for (int c = 0; c < nc; c++) {
+    p.down.tgt.push_back(c);
+    for (int k = nodes[c].parent; k >= 0; k = nodes[k].parent)
+      if (p.has_local[k]) p.down.src.push_back(k);
+    p.down.ptr.push_back((int)p.down.src.size());
+  }
+
+  // close pairs: transposed slots first, then one forward slot per task, then
+  // the far slot
+  std::vector<int> trans(nc, 0), chunks(nc);
+  for (int c = 0; c < nc; c++) {
+    std::sort(near[c].begin(), near[c].end());
+    for (int j : near[c]) trans[j]++;
+    chunks[c] = ((int)near[c].size() + 1 + kTreeNearChunk - 1) / kTreeNearChunk;
+  }
+  p.slot_off.assign(nc + 1, 0);
+  for (int c = 0; c < nc; c++) p.slot_off[c + 1] = p.slot_off[c] + trans[c] + chunks[c] + 1;
+  std::vector<int> next(p.slot_off.begin(), p.slot_off.end() - 1);
+  for (int c = 0; c < nc; c++) {
+    const int e0 = (int)p.entries.size();
+    p.entries.push_back(make_int2(c, -1));
+    for (int j : near[c]) p.entries.push_back(make_int2(j, next[j]++));
+    const int e1 = (int)p.entries.size();
+    int slot = p.slot_off[c] + trans[c];
+    for (int e = e0; e < e1; e += kTreeNearChunk)
+      p.tasks.push_back(make_int4(c, e, std::min(e1, e + kTreeNearChunk), slot++));
+  }
+  // the larger tasks first; those that start with the diagonal are the first
+  // chunks of their cells
+  std::stable_sort(p.tasks.begin(), p.tasks.end(),
+                   [](const int4& a, const int4& b) { return a.z - a.y > b.z - b.y; });
+  return true;
+}
+
+}  // namespace eb

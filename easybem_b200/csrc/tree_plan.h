@@ -1,0 +1,56 @@
+// Cluster tree of a mesh's far field (host side): the cells of the sorted
+// order are the leaves, the ranges of the bisection the inner nodes.
+//
+// A pair of nodes is separated when the sum of its radii is below kTreeTheta
+// times the distance of its centres. The traversal of the tree against itself
+// splits all cell pairs exactly once into separated node pairs (evaluated
+// through multipole and local expansions) and close cell pairs (evaluated
+// point by point).
+#pragma once
+
+#include <vector>
+
+#include "farfield.cuh"
+#include "mesh_host.h"
+
+namespace eb {
+
+// Separation: measured on the perturbed icosphere L5 and a torus, random
+// densities, far sum against the whole sum. At 0.5, order 14: 1.9e-10 (SL) and
+// 6.8e-9 (DL); order 24: 3.4e-15 and 3.5e-14. A wider ratio trades close cell
+// pairs (16 a cell at 0.5, 11 at 0.6) for higher orders (18 at 0.6 for the
+// accuracy of 14 at 0.5).
+constexpr double kTreeTheta = 0.5;
+// Translations into one node run on four warps; the upward pass covers three
+// levels of the tree per launch (eight descendants a node, two per warp).
+constexpr int kTreeLevelsPerPass = 3;
+constexpr int kTreePasses = 6;  // enough for 2^18 cells
+// Close cell pairs per near task (one warp's work; the diagonal counts).
+constexpr int kTreeNearChunk = 4;
+
+// Expansions moved into node tgt[k] from nodes src[ptr[k] .. ptr[k + 1]).
+struct TreeMoves {
+  std::vector<int> tgt, ptr = {0}, src;
+};
+
+struct TreePlan {
+  int ncells = 0, nnodes = 0;  // nodes 0 .. ncells - 1 are the cells
+  std::vector<dq> ball;        // centre; radius over the quadrature points
+  TreeMoves up[kTreePasses];   // multipoles of descendants into inner nodes
+  TreeMoves m2l;               // multipoles of separated nodes into locals
+  TreeMoves down;              // locals of the ancestors into every cell
+  std::vector<char> has_local; // per node: it is a target of m2l
+  // close pairs: every unordered pair of cells once (sym), with the slot that
+  // takes the transposed sums; a task is (cell, first entry, last entry, slot
+  // of its forward sums); slots of cell c are slot_off[c] .. slot_off[c + 1]),
+  // the last one for the far sum
+  std::vector<int4> tasks;
+  std::vector<int2> entries;
+  std::vector<int> slot_off;
+};
+
+// False when more than an eighth of all cell pairs are close (the tree would
+// not pay): the plan is then incomplete.
+bool make_tree_plan(const HostMesh& h, TreePlan* plan);
+
+}  // namespace eb

@@ -366,6 +366,13 @@ int eb_mesh_get_plan(eb_mesh mesh, int* items_per_sm, int* src_tile, int* nsplit
  * residuals take the symmetric kernel on the default engine); get reports
  * EB_FAR_SYMMETRIC for an FP64 apply on this engine. */
 #define EB_FAR_SYMMETRIC_ALL 3
+/* The default of a new mesh: separated clusters of triangles through multipole
+ * and local expansions, close cells of 32 triangles point by point with the
+ * EB_FAR_SYMMETRIC inner loops, so an apply costs O(nelems). Taken by meshes
+ * large enough to gain (7-point rule; SL+DL and the SL with 1, 3 or 4 columns),
+ * EB_FAR_SYMMETRIC's rules otherwise. The expansion orders keep the truncation
+ * below the rounding of the point sums in either precision. */
+#define EB_FAR_TREE 4
 int eb_mesh_set_far_engine(eb_mesh mesh, int engine);
 int eb_mesh_get_far_engine(eb_mesh mesh, int precision, int* engine);
 /* Pipe work per well-separated quadrature pair of the fused mixed SL+DL far

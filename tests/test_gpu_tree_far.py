@@ -1,0 +1,118 @@
+"""The tree far field (EB_FAR_TREE, the default engine of larger meshes).
+
+Against the CPU oracle on sampled rows and against the symmetric kernels on
+every row. FP64 is held to 1e-12 (the bar of the FP64 engines), mixed to 1e-6.
+The sizes put the last cell at 1 and 31 triangles, split the bisection
+unevenly and lie just above the smallest size that takes the tree; the shapes
+are closed, open, in two distant parts, thin, graded, and in units far from
+one (every expansion coefficient is scaled by its cluster's radius).
+"""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+from easybem_b200 import meshes
+
+pytestmark = pytest.mark.gpu
+
+FP64_TOL, MIXED_TOL = 1e-12, 1e-6
+
+
+def _cut(v, f, ne):
+    """The first ne triangles (an open surface)."""
+    return v, f[:ne]
+
+
+def _two(n_u):
+    v, f = meshes.torus(n_u, 0.3)
+    return np.vstack([v, 0.4 * v + np.array([7.0, -3.0, 1.0])]), np.vstack([f, f + len(v)])
+
+
+def _graded(level):
+    v, f = meshes.icosphere(level)
+    return v * np.array([3.0, 0.6, 0.15]) * (0.05 + np.exp(-2.0 * (1 + v[:, :1]))), f
+
+
+MESHES = {
+    "torus206": lambda: meshes.torus(206, 0.25),            # 21,012 triangles: last cell of 20
+    "cut12801": lambda: _cut(*meshes.torus(206, 0.25), 12801),  # last cell of 1
+    "cut12831": lambda: _cut(*meshes.torus(206, 0.25), 12831),  # last cell of 31
+    "cut16416": lambda: _cut(*meshes.perturbed_icosphere(5, seed=3), 16416),
+    "two": lambda: _two(165),
+    "graded": lambda: _graded(5),
+}
+
+
+def _vectors(nodes, elems, seed):
+    rng = np.random.default_rng(seed)
+    return rng.normal(size=len(elems)), rng.normal(size=len(nodes))
+
+
+@pytest.mark.parametrize("name", list(MESHES))
+def test_tree_matches_oracle_and_symmetric_kernels(gpu_lib, oracle, name):
+    oracle.set_order(4)
+    nodes, elems = MESHES[name]()
+    t, u = _vectors(nodes, elems, len(name))
+    rows = np.sort(np.random.default_rng(1).choice(len(elems), 48, replace=False)).astype(np.int32)
+    vo, qo = oracle.apply_rows(nodes, elems, t, u, rows)
+    with gpu_lib.Mesh(nodes, elems) as m:
+        assert m.far_engine("mixed") == "tree" and m.far_engine("fp64") == "tree"
+        for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL)):
+            m.set_far_engine("tree")
+            v, q = m.apply_sl_dl(t, u, precision=prec)
+            assert rel_l2(v[rows], vo) < tol and rel_l2(q[rows], qo) < tol
+            v2, q2 = m.apply_sl_dl(t, u, precision=prec)
+            assert np.array_equal(v, v2) and np.array_equal(q, q2)
+            vs = m.apply_sl(t, precision=prec)
+            assert rel_l2(vs[rows], vo) < tol
+            d = m.apply_hypersingular(u, precision=prec)
+            m.set_far_engine("sym_all")
+            vd, qd = m.apply_sl_dl(t, u, precision=prec)
+            assert rel_l2(v, vd) < tol and rel_l2(q, qd) < tol
+            assert rel_l2(d, m.apply_hypersingular(u, precision=prec)) < 10 * tol  # differences of V's columns
+
+
+@pytest.mark.parametrize("unit", [1e-9, 1e6])
+def test_tree_in_other_units(gpu_lib, unit):
+    nodes, elems = meshes.torus(180, 0.3)
+    t, u = _vectors(nodes, elems, 5)
+    with gpu_lib.Mesh(nodes, elems) as a, gpu_lib.Mesh(nodes * unit, elems) as b:
+        assert b.far_engine("fp64") == "tree"
+        # the FP32 point sums have an absolute floor of 1e-12 in distance: at
+        # 1e-9 they are no reference
+        for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL))[:1 if unit < 1e-6 else 2]:
+            v, q = a.apply_sl_dl(t, u, precision=prec)
+            w, r = b.apply_sl_dl(t, u, precision=prec)
+            assert rel_l2(w / unit ** 3, v) < tol and rel_l2(r / unit ** 2, q) < tol
+
+
+def test_meshes_without_separated_clusters_keep_the_direct_sum(gpu_lib):
+    """A tube of long strips: every cell spans it, nearly all cells are close."""
+    n = 8200
+    a = 2 * np.pi * np.arange(n) / n
+    ring = np.stack([np.cos(a), np.sin(a), np.zeros(n)], 1)
+    nodes = np.vstack([ring - [0, 0, 20.0], ring + [0, 0, 20.0]])
+    i, j = np.arange(n), (np.arange(n) + 1) % n
+    elems = (np.vstack([np.stack([i, j, n + j], 1), np.stack([i, n + j, n + i], 1)]) + 1).astype(np.int32)
+    t, u = _vectors(nodes, elems, 9)
+    with gpu_lib.Mesh(nodes, elems) as m:
+        for prec, engine in (("mixed", "sym"), ("fp64", "cuda")):
+            m.set_far_engine("tree")
+            assert m.far_engine(prec) == engine
+            v, q = m.apply_sl_dl(t, u, precision=prec)
+            m.set_far_engine(engine)
+            w, r = m.apply_sl_dl(t, u, precision=prec)
+            assert np.array_equal(v, w) and np.array_equal(q, r)
+
+
+def test_tree_follows_plan_changes_and_small_meshes_stay_direct(gpu_lib):
+    nodes, elems = meshes.torus(170, 0.3)
+    t, u = _vectors(nodes, elems, 6)
+    with gpu_lib.Mesh(nodes, elems) as m:
+        v, q = m.apply_sl_dl(t, u)
+        m.set_plan(64)  # releases the records that the tree's descriptors point to
+        w, r = m.apply_sl_dl(t, u)
+        assert np.array_equal(v, w) and np.array_equal(q, r)
+    nodes, elems = meshes.icosphere(3)
+    with gpu_lib.Mesh(nodes, elems) as m:
+        assert m.far_engine("mixed") == "sym" and m.far_engine("fp64") == "cuda"
