@@ -48,37 +48,15 @@ namespace {
 
 enum Move { kUp, kAcross, kDown };
 
-constexpr int kMoveWarps = 4;
-
-// Constant tables of one order (device pointers).
-//
-// Order of an expansion's (p + 1)^2 real coefficients in shared memory
-// ("grouped"): degree by degree, real parts of even m, real parts of odd m,
-// imaginary parts of even m, of odd m; so each output of Ry(90) reads one
-// contiguous group. Along z ("m-major"): for each m the real parts of degrees
-// m..p, then the imaginary ones. The matrices are padded per round of 32
-// outputs: entry [offset of the round + k * 32 + lane].
+// Constant tables of one order (device pointers). The matrices are stored as
+// mma operand fragments: lane l holds output slot 8 t + (l / 8) + 4 (l / 4 % 2)
+// and input slot 4 k + l % 4 of tile t and step k (zeros outside):
+//   Ry(90), per degree: [part][output parity][t][k], slots as in the kernel;
+//   along z, per order m: [t][k], slot = n - m.
 struct TreeTables {
   const double *bmat, *tmat[3];
-  const int2 *bround, *tround;  // (offset, length)
-  const int* bout;  // grouped output: first input | m-major position << 11 | sign of Ry(-90) << 22
-  const int* tout;  // m-major output: first input | grouped position << 11 | (n - m) << 22
-  const int* pair;  // (n, m): grouped position of re | of im << 10 | m << 20 | n << 25
+  const int* pair;     // (n, m): m | n << 8
   const double2* rec;  // (n, m): R_n^m = rec.x z R_{n-1}^m - rec.y r^2 R_{n-2}^m (n > m)
-};
-
-template <int P>
-struct TreeShape {
-  static constexpr int kCoef = (P + 1) * (P + 1);
-  static constexpr int kRounds = (kCoef + 31) / 32;
-  static constexpr int kPairs = tree_pairs(P);
-  static constexpr int kPairRounds = (kPairs + 31) / 32;
-  static constexpr int kBuf = kCoef + P + 2;  // zero padding behind the last group
-};
-
-template <int NC>
-struct alignas(8 * NC) Vec {
-  double v[NC];
 };
 
 __device__ __forceinline__ int tree_pair(int n, int m) { return n * (n + 1) / 2 + m; }
@@ -98,95 +76,60 @@ __device__ __forceinline__ int tree_entry(const int* __restrict__ off, int n, in
 }
 
 // ---------------------------------------------------------------------------
-// Moves.
+// Moves. A CTA owns one target node and takes its sources eight at a time; an
+// mma m8n8k4 multiplies the eight sources' coefficients (rows) with eight
+// outputs of a constant matrix, for every column. A warp owns whole degrees
+// for the rotations and whole orders for the move along z:
+//
+//   per degree  load, phase, Ry(-90), phase, Ry(90)     -> shared memory
+//   per order   along z, in place
+//   per degree  Ry(-90), phase, Ry(90), phase           -> running sums
+//
+// A pair whose radii are small against its distance needs fewer degrees: those
+// beyond its order (TreeMoves::src) are left out of all stages.
+//
+// The result fragment of an mma (a lane has source lane / 4, outputs 2j and
+// 2j + 1, j = lane % 4) is the operand fragment of the next one when the
+// output columns stand for slots j and j + 4, so the chain of a degree stays
+// in registers. Coefficient slots of one parity of m: m = 2 slot + parity,
+// slot = 4 el + j; real and imaginary parts sit in the same slots (the
+// imaginary part of m = 0 is a zero row and column).
+//
+// Measured on the SL+DL apply at 81,920 triangles (105,000 moves, two columns;
+// mixed / FP64): one warp per source with scalar multiply-adds 3.5 / 39 ms
+// (order 30); batched vectors, a lane per output 3.0 / 12.3 (the shared-memory
+// pipe 95 % busy: two wavefronts per 32 products); mma with all stages through
+// shared memory 3.4 / 13.0 (latency of the matrix loads); chains in registers
+// 2.55 / 12.1; degrees by separation 2.50 / 10.8; degrees specialised by parity
+// and size, so that slots are not selected at run time, 2.17 / 8.8. The mma
+// pipe itself sustains 64 multiply-adds per clock and SM, as DFMA does.
 
-// dst = Ry(+-90) src; TO_M writes m-major positions.
-template <int P, int NC, bool BACK, bool TO_M>
-__device__ __forceinline__ void turn(const TreeTables& tab, const Vec<NC>* src, Vec<NC>* dst, int lane)
+constexpr int kBatch = 8;  // sources of a batch
+
+template <int P, int NC>
+struct MoveShape {
+  // Larger orders: two columns share the matrix loads of one CTA of eight
+  // warps (113 KB); a single column runs two CTAs of four. Measured, 81,920
+  // triangles, SL+DL FP64: 8.78 ms against 8.96 with a column per CTA.
+  static constexpr int kWarps = P > 16 && NC == 2 ? 8 : 4;
+  static constexpr int kCtas = P <= 16 ? 3 : NC == 2 ? 1 : 2;
+  static constexpr int kThreads = 32 * kWarps;
+  static constexpr int kEls = 2 * ((P / 2 + 8) / 8);  // slot groups of four per parity, even
+  static constexpr int kRows = 2 * tree_pairs(P);     // real rows m-major, then imaginary rows
+  static constexpr size_t smem() { return sizeof(double) * (kBatch + 1) * kRows * NC; }
+};
+
+__device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b)
 {
-  using Sh = TreeShape<P>;
-#pragma unroll 1
-  for (int r = 0; r < Sh::kRounds; ++r) {
-    const int2 rd = tab.bround[r];
-    const int o = r * 32 + lane;
-    const int info = o < Sh::kCoef ? tab.bout[o] : 0;
-    const Vec<NC>* s = src + (info & 2047);
-    const double* mat = tab.bmat + rd.x + lane;
-    Vec<NC> acc;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) acc.v[c] = 0.0;
-#pragma unroll 4
-    for (int k = 0; k < rd.y; ++k) {
-      const double b = mat[k * 32];
-      const Vec<NC> x = s[k];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) acc.v[c] += b * x.v[c];
-    }
-    if (o < Sh::kCoef) {
-      if (BACK && (info >> 22 & 1)) {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) acc.v[c] = -acc.v[c];
-      }
-      dst[TO_M ? info >> 11 & 2047 : o] = acc;
-    }
-  }
-  __syncwarp();
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c0), "+d"(c1)
+      : "d"(a), "d"(b));
 }
 
-// dst (grouped) = the move along z applied to src (m-major); pw: powers of
-// the step over the radius (not kAcross).
-template <int P, int NC, int MODE>
-__device__ __forceinline__ void along_z(const TreeTables& tab, const double* pw, const Vec<NC>* src, Vec<NC>* dst,
-                                        int lane)
-{
-  using Sh = TreeShape<P>;
-#pragma unroll 1
-  for (int r = 0; r < Sh::kRounds; ++r) {
-    const int2 rd = tab.tround[r];
-    const int o = r * 32 + lane;
-    const int info = o < Sh::kCoef ? tab.tout[o] : 0;
-    const int j = info >> 22;
-    const Vec<NC>* s = src + (info & 2047);
-    const double* mat = tab.tmat[MODE] + rd.x + lane;
-    Vec<NC> acc;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) acc.v[c] = 0.0;
-#pragma unroll 4
-    for (int k = 0; k < rd.y; ++k) {
-      double b = mat[k * 32];
-      if (MODE != kAcross) b *= pw[abs(j - k)];
-      const Vec<NC> x = s[k];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) acc.v[c] += b * x.v[c];
-    }
-    if (o < Sh::kCoef) dst[info >> 11 & 2047] = acc;
-  }
-  __syncwarp();
-}
+__host__ __device__ constexpr int order_row(int P, int m) { return m * (P + 1) - m * (m - 1) / 2; }  // of (m, m)
 
-// Rotation about z in place: (n, m) times e^{i m alpha} (SIGN +1) or its conjugate.
-template <int P, int NC, int SIGN>
-__device__ __forceinline__ void phase(const TreeTables& tab, const double2* e, Vec<NC>* buf, int lane)
-{
-  using Sh = TreeShape<P>;
-#pragma unroll 1
-  for (int i = lane; i < Sh::kPairs; i += 32) {
-    const int info = tab.pair[i];
-    const int m = info >> 20 & 31;
-    if (m == 0) continue;
-    const double2 f = e[m];
-    const double fi = SIGN * f.y;
-    Vec<NC>& re = buf[info & 1023];
-    Vec<NC>& im = buf[info >> 10 & 1023];
-    const Vec<NC> a = re, b = im;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      re.v[c] = a.v[c] * f.x - b.v[c] * fi;
-      im.v[c] = a.v[c] * fi + b.v[c] * f.x;
-    }
-  }
-  __syncwarp();
-}
+// Slots of a parity in degree n.
+__device__ __forceinline__ int slots_of(int n, int par) { return par ? (n + 1) >> 1 : (n >> 1) + 1; }
 
 // b^k by squaring, k < 32
 __device__ __forceinline__ double power(double b, int k)
@@ -200,148 +143,330 @@ __device__ __forceinline__ double power(double b, int k)
   return r;
 }
 
+__device__ __forceinline__ double2 cmul(double2 a, double2 b)
+{
+  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+
 __device__ __forceinline__ double2 power(double2 b, int k)
 {
   double2 r = make_double2(1.0, 0.0);
 #pragma unroll
   for (int i = 0; i < 5; ++i) {
-    if (k >> i & 1) r = make_double2(r.x * b.x - r.y * b.y, r.x * b.y + r.y * b.x);
-    b = make_double2(b.x * b.x - b.y * b.y, 2.0 * b.x * b.y);
+    if (k >> i & 1) r = cmul(r, b);
+    b = cmul(b, b);
   }
   return r;
 }
 
-template <int P, int NC>
-constexpr size_t move_smem()
+// e[par][el] = base^m of this lane's slots.
+template <int E>
+__device__ __forceinline__ void lane_phases(double2 base, int j, double2 (&e)[2][E])
 {
-  return kMoveWarps * (2 * TreeShape<P>::kBuf * sizeof(Vec<NC>) + (P + 2) * 2 * (sizeof(double2) + sizeof(double)));
+  const double2 b2 = cmul(base, base), b4 = cmul(b2, b2), b8 = cmul(b4, b4);
+  e[0][0] = power(b2, j);
+#pragma unroll
+  for (int el = 0; el < E; ++el) {
+    if (el > 0) e[0][el] = cmul(e[0][el - 1], b8);
+    e[1][el] = cmul(e[0][el], base);
+  }
 }
 
-// One CTA per target node: its four warps take every fourth source, each a
-// whole move; the warps' sums are added in warp order.
+// One degree's coefficients of NC columns: real and imaginary parts, parity, slot group.
+template <int NC, int E>
+struct Degree {
+  double x[NC][2][2][E];
+};
+
+// x = Ry(90) x for a degree n of parity ODD with at most 4 EN slots per parity
+// (frag: its matrix, stored for E slot groups).
+template <int NC, int E, int EN, int ODD>
+__device__ __forceinline__ void turn(const double* __restrict__ frag, int n, Degree<NC, EN>& d)
+{
+  Degree<NC, EN> y;
+#pragma unroll
+  for (int part = 0; part < 2; ++part)
+#pragma unroll
+    for (int par = 0; par < 2; ++par) {
+      constexpr int kTiles = (EN + 1) / 2;
+      const int from = (ODD + par + part) & 1;
+      const bool last = slots_of(n, from) > 4 * (EN - 1);  // the last step has inputs
+#pragma unroll
+      for (int t = 0; t < kTiles; ++t) {
+        double c0[NC], c1[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) c0[c] = c1[c] = 0.0;
+        const double* f = frag + (((part * 2 + par) * (E / 2) + t) * E) * 32;
+#pragma unroll
+        for (int k = 0; k < EN; ++k)
+          if (k < EN - 1 || EN == 1 || last) {
+            const double b = __ldg(f + 32 * k);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) mma_f64(c0[c], c1[c], d.x[c][part][from][k], b);
+          }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          y.x[c][part][par][2 * t] = c0[c];
+          if (2 * t + 1 < EN) y.x[c][part][par][2 * t + 1] = c1[c];
+        }
+      }
+    }
+  d = y;
+}
+
+// x = scale x e^{+-i m alpha}; MIRROR: of (re, -im) (Ry(-90) is Ry(90) times
+// (-1)^n for real and -(-1)^n for imaginary parts)
+template <int NC, int E, int EN, int SIGN, bool MIRROR>
+__device__ __forceinline__ void phase(const double2 (&e)[2][E], double scale, Degree<NC, EN>& d)
+{
+#pragma unroll
+  for (int par = 0; par < 2; ++par)
+#pragma unroll
+    for (int el = 0; el < EN; ++el) {
+      const double fr = MIRROR ? e[par][el].x : scale * e[par][el].x, fi = MIRROR ? e[par][el].y : scale * e[par][el].y;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const double re = d.x[c][0][par][el], im = d.x[c][1][par][el];
+        const double si = (MIRROR ? -1.0 : 1.0) * SIGN, sc = MIRROR ? -1.0 : 1.0, ss = SIGN;
+        d.x[c][0][par][el] = re * fr - si * (im * fi);
+        d.x[c][1][par][el] = ss * (re * fi) + sc * (im * fr);
+      }
+    }
+}
+
+// Stage of a degree before the move along z: coefficients a (pair (n, 0) of
+// column 0) into the rows of zb.
+template <int P, int NC, int EN, int ODD>
+__device__ __forceinline__ void before_z(const TreeTables& tab, int n, bool on, const double2* __restrict__ a,
+                                         size_t cstride, const double2 (&ephi)[2][MoveShape<P, NC>::kEls],
+                                         const double2 (&eth)[2][MoveShape<P, NC>::kEls], double scale, int vec, int j,
+                                         int lane, double* zb)
+{
+  using Mv = MoveShape<P, NC>;
+  constexpr int E = Mv::kEls, kPairs = tree_pairs(P);
+  Degree<NC, EN> x;
+#pragma unroll
+  for (int par = 0; par < 2; ++par)
+#pragma unroll
+    for (int el = 0; el < EN; ++el) {
+      const int m = 2 * (4 * el + j) + par;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const double2 v = on && m <= n ? a[c * cstride + m] : make_double2(0.0, 0.0);
+        x.x[c][0][par][el] = v.x;
+        x.x[c][1][par][el] = v.y;
+      }
+    }
+  const double* frag = tab.bmat + (size_t)n * (2 * E * E) * 32 + lane;
+  phase<NC, E, EN, 1, false>(ephi, ODD ? -scale : scale, x);
+  turn<NC, E, EN, ODD>(frag, n, x);
+  phase<NC, E, EN, 1, true>(eth, 1.0, x);
+  turn<NC, E, EN, ODD>(frag, n, x);
+#pragma unroll
+  for (int par = 0; par < 2; ++par)
+#pragma unroll
+    for (int el = 0; el < EN; ++el) {
+      const int m = 2 * (4 * el + j) + par;
+      if (m <= n) {
+        double* r = zb + (order_row(P, m) + n - m) * kBatch + vec;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          r[c * Mv::kRows * kBatch] = x.x[c][0][par][el];
+          r[(c * Mv::kRows + kPairs) * kBatch] = x.x[c][1][par][el];
+        }
+      }
+    }
+}
+
+// Stage of a degree after the move along z: rows of zb turned back, added over
+// the eight sources and onto acc ([column][part][pair]).
+template <int P, int NC, int EN, int ODD>
+__device__ __forceinline__ void after_z(const TreeTables& tab, int n, const double2 (&ephi)[2][MoveShape<P, NC>::kEls],
+                                        const double2 (&eth)[2][MoveShape<P, NC>::kEls], double scale, int vec, int j,
+                                        int lane, const double* zb, double* acc)
+{
+  using Mv = MoveShape<P, NC>;
+  constexpr int E = Mv::kEls, kPairs = tree_pairs(P);
+  Degree<NC, EN> x;
+#pragma unroll
+  for (int par = 0; par < 2; ++par)
+#pragma unroll
+    for (int el = 0; el < EN; ++el) {
+      const int m = 2 * (4 * el + j) + par;
+      const double* r = zb + (order_row(P, m) + n - m) * kBatch + vec;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        x.x[c][0][par][el] = m <= n ? r[c * Mv::kRows * kBatch] : 0.0;
+        x.x[c][1][par][el] = m <= n ? r[(c * Mv::kRows + kPairs) * kBatch] : 0.0;
+      }
+    }
+  const double* frag = tab.bmat + (size_t)n * (2 * E * E) * 32 + lane;
+  turn<NC, E, EN, ODD>(frag, n, x);
+  phase<NC, E, EN, -1, true>(eth, 1.0, x);
+  turn<NC, E, EN, ODD>(frag, n, x);
+  phase<NC, E, EN, -1, false>(ephi, ODD ? -scale : scale, x);
+  // halving the values per lane at each step: lane bit 4 keeps the part, bit 3
+  // the parity, bit 2 the slot group's low bit
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    double u[2][EN], w[EN];
+#pragma unroll
+    for (int par = 0; par < 2; ++par)
+#pragma unroll
+      for (int el = 0; el < EN; ++el) {
+        const double keep = b4 ? x.x[c][1][par][el] : x.x[c][0][par][el];
+        const double give = b4 ? x.x[c][0][par][el] : x.x[c][1][par][el];
+        u[par][el] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+      }
+#pragma unroll
+    for (int el = 0; el < EN; ++el) {
+      const double keep = b3 ? u[1][el] : u[0][el], give = b3 ? u[0][el] : u[1][el];
+      w[el] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+    }
+    double* to = acc + (2 * c + (lane >> 4)) * kPairs + tree_pair(n, 0);
+    if constexpr (EN == 1) {
+      const double v = w[0] + __shfl_xor_sync(0xffffffffu, w[0], 4);
+      const int m = 2 * j + (lane >> 3 & 1);
+      if (!b2 && m <= n) to[m] += v;
+    } else {
+#pragma unroll
+      for (int i = 0; i < EN / 2; ++i) {
+        const double keep = b2 ? w[2 * i + 1] : w[2 * i], give = b2 ? w[2 * i] : w[2 * i + 1];
+        const double v = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+        const int m = 2 * (4 * (2 * i + (lane >> 2 & 1)) + j) + (lane >> 3 & 1);
+        if (m <= n) to[m] += v;
+      }
+    }
+  }
+}
+
 template <int P, int NC, int MODE>
-__global__ void __launch_bounds__(32 * kMoveWarps)
+__global__ void __launch_bounds__(MoveShape<P, NC>::kThreads, MoveShape<P, NC>::kCtas)
     tree_move_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh, int pass, TreeTables tab)
 {
-  using Sh = TreeShape<P>;
+  using Mv = MoveShape<P, NC>;
+  constexpr int kPairs = tree_pairs(P), W = Mv::kWarps, E = Mv::kEls, KT = (P + 4) / 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  int k = blockIdx.x;
-  const TreeDesc& d = descs[tree_entry(off, nmesh, k)];
+  double* zb = reinterpret_cast<double*>(smem_raw);     // [column][row][source]
+  double* acc = zb + (size_t)kBatch * Mv::kRows * NC;   // [column][part][pair]
+  int node = blockIdx.x;
+  const TreeDesc& d = descs[tree_entry(off, nmesh, node)];
   if (d.far.active && *d.far.active == 0) return;
   const TreeMovesDev mv = MODE == kUp ? d.up[pass] : MODE == kAcross ? d.m2l : d.down;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  Vec<NC>* bufs = reinterpret_cast<Vec<NC>*>(smem_raw);
-  Vec<NC>* b0 = bufs + warp * 2 * Sh::kBuf;
-  Vec<NC>* b1 = b0 + Sh::kBuf;
-  double2* ephi = reinterpret_cast<double2*>(bufs + kMoveWarps * 2 * Sh::kBuf) + warp * 2 * (P + 2);
-  double2* eth = ephi + P + 2;
-  double* pin = reinterpret_cast<double*>(reinterpret_cast<double2*>(bufs + kMoveWarps * 2 * Sh::kBuf) +
-                                          kMoveWarps * 2 * (P + 2)) + warp * 2 * (P + 2);
-  double* pout = pin + P + 2;
-  for (int i = lane; i < Sh::kBuf - Sh::kCoef; i += 32)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) b0[Sh::kCoef + i].v[c] = b1[Sh::kCoef + i].v[c] = 0.0;
-
-  const int tgt = mv.tgt[k];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, vec = lane >> 2, j = lane & 3;
+  for (int i = threadIdx.x; i < 2 * NC * kPairs; i += Mv::kThreads) acc[i] = 0.0;
+  const int tgt = mv.tgt[node];
   const dq bt = d.ball[tgt];
-  const size_t cstride = (size_t)d.nnodes * Sh::kPairs;
-  const size_t col0 = (size_t)blockIdx.y * NC * cstride;
+  const size_t cstride = (size_t)d.nnodes * kPairs, col0 = blockIdx.y * NC * cstride;
   const double2* from = (MODE == kDown ? d.local : d.multipole) + col0;
-  double2* to = (MODE == kUp ? d.multipole : d.local) + col0;
-  Vec<NC> sre[Sh::kPairRounds], sim[Sh::kPairRounds];
-#pragma unroll
-  for (int r = 0; r < Sh::kPairRounds; ++r)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) sre[r].v[c] = sim[r].v[c] = 0.0;
+  const int n0 = (P - warp) % W;  // this warp's degrees: n0, n0 + W, ...
+  __syncthreads();
 
+  const int end = mv.ptr[node + 1];
 #pragma unroll 1
-  for (int s = mv.ptr[k] + warp; s < mv.ptr[k + 1]; s += kMoveWarps) {
-    const int src = mv.src[s];
+  for (int first = mv.ptr[node]; first < end; first += kBatch) {
+    const bool on = first + vec < end;
+    // the list is sorted by the order its pairs need: the first one decides
+    const int order = ((P + 1) * (int)((unsigned)mv.src[first] >> 24) + 254) / 255 - 1;
+    const int src = mv.src[on ? first + vec : first] & 0xffffff;
     const dq bs = d.ball[src];
+    const double2* a = from + (size_t)src * kPairs;
     // the vector that becomes the z axis: from the source's centre to the
     // target's, reversed for a multipole (its points move the other way)
     const double sg = MODE == kUp ? -1.0 : 1.0;
     const double dx = sg * (bt.x - bs.x), dy = sg * (bt.y - bs.y), dz = sg * (bt.z - bs.z);
     const double h2 = dx * dx + dy * dy, h = sqrt(h2), dist = sqrt(h2 + dz * dz);
-    const double cphi = h > 0.0 ? dx / h : 1.0, sphi = h > 0.0 ? dy / h : 0.0;
-    const double cth = dist > 0.0 ? dz / dist : 1.0, sth = dist > 0.0 ? h / dist : 0.0;
-    // kAcross: rho_s / d in, rho_t / d out; kUp: rho_s / rho_t in, d / rho_t
-    // between; kDown: d / rho_s between, rho_t / rho_s out
-    const double in = MODE == kAcross ? bs.w / dist : MODE == kUp ? bs.w / bt.w : dist / bs.w;
-    const double out = MODE == kAcross ? bt.w / dist : MODE == kUp ? dist / bt.w : bt.w / bs.w;
-    if (lane <= P) {
-      ephi[lane] = power(make_double2(sphi, cphi), lane);  // e^{i (90 - phi)}
-      eth[lane] = power(make_double2(cth, sth), lane);
-      pin[lane] = power(in, lane);
-      pout[lane] = power(out, lane);
-    }
-    __syncwarp();
-    const double2* a = from + (size_t)src * Sh::kPairs;
+    const double rd = 1.0 / dist, rh = h > 0.0 ? 1.0 / h : 0.0;
+    double2 ephi[2][E], eth[2][E];
+    lane_phases(h > 0.0 ? make_double2(dy * rh, dx * rh) : make_double2(0.0, 1.0), j, ephi);  // e^{i (90 - phi)}
+    lane_phases(make_double2(dz * rd, h * rd), j, eth);
+    // degrees scale with the radii their coefficients are stored for and with
+    // the step: to the power -n on the side of irregular or moved multipoles,
+    // n on the other
+    const double in = MODE == kDown ? dist / bs.w : bs.w * rd;
+    const double out = MODE == kUp ? dist / bt.w : bt.w * rd;
+    double scale = power(in, n0), step = power(in, W);
 #pragma unroll 1
-    for (int i = lane; i < Sh::kPairs; i += 32) {
-      const int info = tab.pair[i];
-      const int m = info >> 20 & 31;
-      const double2 f = ephi[m];
-      const double w = MODE == kDown ? 1.0 : pin[info >> 25];
-      const double fr = w * f.x, fi = w * f.y;
-      Vec<NC> re, im;
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const double2 x = a[c * cstride + i];
-        re.v[c] = x.x * fr - x.y * fi;
-        im.v[c] = x.x * fi + x.y * fr;
+    for (int n = n0; n <= order; n += W, scale *= step) {
+      const double2* an = a + tree_pair(n, 0);
+      if (n < 4 * E) {  // half of the slot groups
+        if (n & 1) before_z<P, NC, E / 2, 1>(tab, n, on, an, cstride, ephi, eth, scale, vec, j, lane, zb);
+        else before_z<P, NC, E / 2, 0>(tab, n, on, an, cstride, ephi, eth, scale, vec, j, lane, zb);
+      } else {
+        if (n & 1) before_z<P, NC, E, 1>(tab, n, on, an, cstride, ephi, eth, scale, vec, j, lane, zb);
+        else before_z<P, NC, E, 0>(tab, n, on, an, cstride, ephi, eth, scale, vec, j, lane, zb);
       }
-      b0[info & 1023] = re;
-      if (m > 0) b0[info >> 10 & 1023] = im;
     }
-    __syncwarp();
-    turn<P, NC, true, false>(tab, b0, b1, lane);
-    phase<P, NC, 1>(tab, eth, b1, lane);
-    turn<P, NC, false, true>(tab, b1, b0, lane);
-    along_z<P, NC, MODE>(tab, MODE == kUp ? pout : pin, b0, b1, lane);
-    turn<P, NC, true, false>(tab, b1, b0, lane);
-    phase<P, NC, -1>(tab, eth, b0, lane);
-    turn<P, NC, false, false>(tab, b0, b1, lane);
-    const double unit = MODE == kAcross ? 1.0 / dist : 1.0;
+    __syncthreads();
+
+#pragma unroll 1
+    for (int q = 0; q * W <= order; ++q) {
+      const int m = q & 1 ? (q + 1) * W - 1 - warp : q * W + warp;
+      if (m > order) continue;
+      const int len = order + 1 - m, steps = (len + 3) >> 2, tiles = (len + 7) >> 3;
+      const double* frag = tab.tmat[MODE] + (size_t)m * (KT * ((KT + 1) / 2)) * 32 + lane;
+      double* r = zb + (order_row(P, m) + j) * kBatch + vec;
+      double a2[NC][2][KT];
 #pragma unroll
-    for (int r = 0; r < Sh::kPairRounds; ++r) {
-      const int i = r * 32 + lane;
-      if (i < Sh::kPairs) {
-        const int info = tab.pair[i];
-        const double2 f = ephi[info >> 20 & 31];
-        const double w = MODE == kUp ? 1.0 : unit * pout[info >> 25];
-        const Vec<NC> re = b1[info & 1023], im = b1[info >> 10 & 1023];
+      for (int k = 0; k < KT; ++k)
+        if (k < steps) {
+          const bool in_range = 4 * k + j < len;
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          sre[r].v[c] += w * (re.v[c] * f.x + im.v[c] * f.y);
-          sim[r].v[c] += w * (im.v[c] * f.x - re.v[c] * f.y);
+          for (int c = 0; c < NC; ++c)
+#pragma unroll
+            for (int part = 0; part < 2; ++part)
+              a2[c][part][k] = in_range ? r[(c * Mv::kRows + part * kPairs + 4 * k) * kBatch] : 0.0;
         }
+#pragma unroll
+      for (int t = 0; t < (KT + 1) / 2; ++t)
+        if (t < tiles) {
+          double y[NC][2][2];
+#pragma unroll
+          for (int c = 0; c < NC; ++c) y[c][0][0] = y[c][0][1] = y[c][1][0] = y[c][1][1] = 0.0;
+#pragma unroll
+          for (int k = 0; k < KT; ++k)
+            if (k < steps) {
+              const double b = __ldg(frag + (t * KT + k) * 32);
+#pragma unroll
+              for (int c = 0; c < NC; ++c) {
+                mma_f64(y[c][0][0], y[c][0][1], a2[c][0][k], b);
+                mma_f64(y[c][1][0], y[c][1][1], a2[c][1][k], b);
+              }
+            }
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            if (8 * t + 4 * h + j < len)
+#pragma unroll
+              for (int c = 0; c < NC; ++c) {
+                r[(c * Mv::kRows + 8 * t + 4 * h) * kBatch] = y[c][0][h];
+                r[(c * Mv::kRows + kPairs + 8 * t + 4 * h) * kBatch] = y[c][1][h];
+              }
+        }
+    }
+    __syncthreads();
+
+    scale = on ? (MODE == kAcross ? rd : 1.0) * power(out, n0) : 0.0;
+    step = power(out, W);
+#pragma unroll 1
+    for (int n = n0; n <= order; n += W, scale *= step) {
+      if (n < 4 * E) {
+        if (n & 1) after_z<P, NC, E / 2, 1>(tab, n, ephi, eth, scale, vec, j, lane, zb, acc);
+        else after_z<P, NC, E / 2, 0>(tab, n, ephi, eth, scale, vec, j, lane, zb, acc);
+      } else {
+        if (n & 1) after_z<P, NC, E, 1>(tab, n, ephi, eth, scale, vec, j, lane, zb, acc);
+        else after_z<P, NC, E, 0>(tab, n, ephi, eth, scale, vec, j, lane, zb, acc);
       }
     }
-    __syncwarp();
+    __syncthreads();
   }
-  // add the warps' sums in warp order
-  double2* mine = reinterpret_cast<double2*>(b0);  // kPairs * NC double2 fit the two buffers
-#pragma unroll
-  for (int r = 0; r < Sh::kPairRounds; ++r) {
-    const int i = r * 32 + lane;
-    if (i < Sh::kPairs)
-#pragma unroll
-      for (int c = 0; c < NC; ++c) mine[c * Sh::kPairs + i] = make_double2(sre[r].v[c], sim[r].v[c]);
-  }
-  __syncthreads();
   const bool add = MODE == kDown && d.has_local[tgt];
-  for (int i = threadIdx.x; i < Sh::kPairs * NC; i += 32 * kMoveWarps) {
-    const int c = i / Sh::kPairs, q = i - c * Sh::kPairs;
-    double2* t = to + c * cstride + (size_t)tgt * Sh::kPairs + q;
-    double2 v = add ? *t : make_double2(0.0, 0.0);
-#pragma unroll
-    for (int w = 0; w < kMoveWarps; ++w) {
-      const double2 x = reinterpret_cast<const double2*>(bufs + w * 2 * Sh::kBuf)[i];
-      v.x += x.x;
-      v.y += x.y;
-    }
-    *t = v;
+  double2* to = (MODE == kUp ? d.multipole : d.local) + col0 + (size_t)tgt * kPairs;
+  for (int it = threadIdx.x; it < NC * kPairs; it += Mv::kThreads) {
+    const int c = it / kPairs, i = it - c * kPairs;
+    double2* t = to + c * cstride + i;
+    const double2 old = add ? *t : make_double2(0.0, 0.0);
+    *t = make_double2(old.x + acc[2 * c * kPairs + i], old.y + acc[(2 * c + 1) * kPairs + i]);
   }
 }
 
@@ -512,7 +637,7 @@ __global__ void __launch_bounds__(32 * kCellWarps)
       // (n.grad) R_n^m from the moments G^k = sum s n_k R of degree n - 1
       const double* g = s_sum + 2 * NSL * kPairs;
       const int info = tab.pair[i];
-      const int m = info >> 20 & 31, n = info >> 25;
+      const int m = info & 255, n = info >> 8;
       double ar = 0.0, ai = 0.0;
       if (n > 0) {
         if (m < n) {
@@ -570,7 +695,7 @@ __global__ void __launch_bounds__(32 * kCellWarps)
   for (int i = threadIdx.x; i < kPairs * NC; i += 32 * kCellWarps) {
     const int c = i / kPairs, q = i - c * kPairs;
     double2 v = d.local[((size_t)c * d.nnodes + cell) * kPairs + q];
-    if (tab.pair[q] >> 20 & 31) {  // orders m and -m
+    if (tab.pair[q] & 255) {  // orders m and -m
       v.x *= 2.0;
       v.y *= 2.0;
     }
@@ -895,89 +1020,56 @@ std::vector<std::vector<ld>> half_turns(int P)
 
 struct HostTables {
   std::vector<double> bmat, tmat[3];
-  std::vector<int2> bround, tround;
-  std::vector<int> bout, tout, pair;
+  std::vector<int> pair;
   std::vector<double2> rec;
 };
+
+// Appends the fragment of tile t and step k of a block's matrix.
+template <typename F>
+void add_fragment(std::vector<double>& mat, int t, int k, F&& entry)
+{
+  for (int lane = 0; lane < 32; lane++)
+    mat.push_back((double)entry(8 * t + (lane >> 3) + 4 * (lane >> 2 & 1), 4 * k + (lane & 3)));
+}
 
 HostTables make_tables(int P)
 {
   HostTables h;
-  const int ncoef = (P + 1) * (P + 1), rounds = (ncoef + 31) / 32;
-  auto even = [](int n) { return n / 2 + 1; };
-  auto pos = [&](int n, int m, int im) {
-    const int base = n * n + (im ? n + 1 : 0), e = even(n) - im;
-    return base + (m & 1 ? e + (m - 1) / 2 : m / 2 - im);
-  };
-  std::vector<int> mbase(2 * (P + 1));
-  for (int m = 0, at = 0; m <= P; m++)
-    for (int im = 0; im < (m ? 2 : 1); im++) {
-      mbase[2 * m + im] = at;
-      at += P + 1 - m;
-    }
-  struct Out {
-    int n, m, im;
-  };
-  std::vector<Out> grouped(ncoef), major(ncoef);
-  for (int n = 0; n <= P; n++)
-    for (int m = 0; m <= n; m++)
-      for (int im = 0; im < (m ? 2 : 1); im++) {
-        grouped[pos(n, m, im)] = Out{n, m, im};
-        major[mbase[2 * m + im] + n - m] = Out{n, m, im};
-      }
-  // Ry(90)
+  const int els = 2 * ((P / 2 + 8) / 8), kt = (P + 4) / 4;
   const auto d = half_turns(P);
-  std::vector<std::vector<double>> rows(ncoef);
-  h.bout.resize(ncoef);
-  for (int o = 0; o < ncoef; o++) {
-    const Out q = grouped[o];
-    const int par = (q.n + q.m + q.im) & 1;
-    int first = -1;
-    for (int m = par; m <= q.n; m += 2) {
-      if (q.im && m == 0) continue;
-      if (first < 0) first = pos(q.n, m, q.im);
-      const ld* row = &d[q.n][(size_t)(q.m + q.n) * (2 * q.n + 1)];
-      const ld minus = (m & 1 ? -1 : 1) * row[q.n - m];
-      rows[o].push_back((double)(m == 0 ? row[q.n] : q.im ? row[q.n + m] - minus : row[q.n + m] + minus));
-    }
-    const int sign = (q.n + q.im) & 1;
-    h.bout[o] = std::max(first, 0) | (mbase[2 * q.m + q.im] + q.n - q.m) << 11 | sign << 22;
-  }
-  auto pad = [&](const std::vector<std::vector<double>>& r, std::vector<double>& mat, std::vector<int2>* rounds_out) {
-    for (int k = 0; k < rounds; k++) {
-      size_t len = 0;
-      for (int o = 32 * k; o < std::min(ncoef, 32 * k + 32); o++) len = std::max(len, r[o].size());
-      if (rounds_out) rounds_out->push_back(make_int2((int)mat.size(), (int)len));
-      for (size_t j = 0; j < len; j++)
-        for (int o = 32 * k; o < 32 * k + 32; o++)
-          mat.push_back(o < ncoef && j < r[o].size() ? r[o][j] : 0.0);
-    }
-  };
-  pad(rows, h.bmat, &h.bround);
-  // along z
+  for (int n = 0; n <= P; n++)
+    for (int part = 0; part < 2; part++)
+      for (int par = 0; par < 2; par++)
+        for (int t = 0; t < els / 2; t++)
+          for (int k = 0; k < els; k++)
+            add_fragment(h.bmat, t, k, [&](int row, int col) -> ld {
+              const int a = 2 * row + par, m = 2 * col + ((n + par + part) & 1);
+              if (a > n || m > n || (part && (a == 0 || m == 0))) return 0.0L;
+              const ld* r = &d[n][(size_t)(a + n) * (2 * n + 1)];
+              if (m == 0) return r[n];
+              const ld minus = (m & 1 ? -1 : 1) * r[n - m];
+              return part ? r[n + m] - minus : r[n + m] + minus;
+            });
+  // along z; the powers of the step over the radii are applied to the
+  // coefficients before and after
   std::vector<ld> fact(2 * P + 2, 1.0L);
   for (int k = 1; k < 2 * P + 2; k++) fact[k] = fact[k - 1] * k;
   auto norm = [&](int n, int m) { return std::sqrt(fact[n - m] * fact[n + m]); };
-  h.tout.resize(ncoef);
-  for (int mode = 0; mode < 3; mode++) {
-    for (auto& r : rows) r.clear();
-    for (int o = 0; o < ncoef; o++) {
-      const Out q = major[o];
-      h.tout[o] = mbase[2 * q.m + q.im] | pos(q.n, q.m, q.im) << 11 | (q.n - q.m) << 22;
-      for (int k = q.m; k <= P; k++) {
-        ld v = 0.0L;
-        if (mode == kAcross) v = ((q.n + q.m) & 1 ? -1 : 1) * fact[q.n + k] / (norm(q.n, q.m) * norm(k, q.m));
-        else if (mode == kUp && k <= q.n) v = norm(q.n, q.m) / (norm(k, q.m) * fact[q.n - k]);
-        else if (mode == kDown && k >= q.n) v = norm(k, q.m) / (norm(q.n, q.m) * fact[k - q.n]);
-        rows[o].push_back((double)v);
-      }
-    }
-    pad(rows, h.tmat[mode], mode == 0 ? &h.tround : nullptr);
-  }
+  for (int mode = 0; mode < 3; mode++)
+    for (int m = 0; m <= P; m++)
+      for (int t = 0; t < (kt + 1) / 2; t++)
+        for (int s = 0; s < kt; s++)
+          add_fragment(h.tmat[mode], t, s, [&](int row, int col) -> ld {
+            const int n = m + row, k = m + col;
+            if (n > P || k > P) return 0.0L;
+            if (mode == kAcross) return ((n + m) & 1 ? -1 : 1) * fact[n + k] / (norm(n, m) * norm(k, m));
+            if (mode == kUp) return k <= n ? norm(n, m) / (norm(k, m) * fact[n - k]) : 0.0L;
+            return k >= n ? norm(k, m) / (norm(n, m) * fact[k - n]) : 0.0L;
+          });
   h.rec.assign(tree_pairs(P), make_double2(0.0, 0.0));
   for (int n = 0; n <= P; n++)
     for (int m = 0; m <= n; m++) {
-      h.pair.push_back(pos(n, m, 0) | (m ? pos(n, m, 1) : ncoef) << 10 | m << 20 | n << 25);
+      h.pair.push_back(m | n << 8);
       if (n > m) {
         const double q = (double)(n * n - m * m);
         h.rec[n * (n + 1) / 2 + m] =
@@ -1007,8 +1099,7 @@ int tables_for(int device, int P, TreeTables* out)
     std::memcpy(host.data() + at, v.data(), v.size() * sizeof(v[0]));
     return at;
   };
-  const size_t at[] = {add(h.bmat), add(h.tmat[0]), add(h.tmat[1]), add(h.tmat[2]), add(h.bround),
-                       add(h.tround), add(h.bout),  add(h.tout),    add(h.pair),    add(h.rec)};
+  const size_t at[] = {add(h.bmat), add(h.tmat[0]), add(h.tmat[1]), add(h.tmat[2]), add(h.pair), add(h.rec)};
   auto buf = std::make_unique<DevBuf>();
   EB_CHECK(buf->alloc(host.size()));
   EB_CHECK(copy_h2d(buf->p, host.data(), host.size()));
@@ -1016,12 +1107,8 @@ int tables_for(int device, int P, TreeTables* out)
   TreeTables t;
   t.bmat = reinterpret_cast<const double*>(p + at[0]);
   for (int k = 0; k < 3; k++) t.tmat[k] = reinterpret_cast<const double*>(p + at[1 + k]);
-  t.bround = reinterpret_cast<const int2*>(p + at[4]);
-  t.tround = reinterpret_cast<const int2*>(p + at[5]);
-  t.bout = reinterpret_cast<const int*>(p + at[6]);
-  t.tout = reinterpret_cast<const int*>(p + at[7]);
-  t.pair = reinterpret_cast<const int*>(p + at[8]);
-  t.rec = reinterpret_cast<const double2*>(p + at[9]);
+  t.pair = reinterpret_cast<const int*>(p + at[4]);
+  t.rec = reinterpret_cast<const double2*>(p + at[5]);
   known[{device, P}] = t;
   *out = t;
   return EB_OK;
@@ -1055,18 +1142,17 @@ int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const
                cudaStream_t st)
 {
   constexpr int NC = NSL + ND;
-  // columns moved together: two share the matrices' loads while the buffers
-  // of a CTA stay small (order 14: 34 KB)
-  constexpr int MC = P <= 16 && NC % 2 == 0 ? 2 : 1;
-  const dim3 b(32 * kMoveWarps);
+  constexpr int MC = NC % 2 == 0 ? 2 : 1;  // columns of a CTA
+  using Mv = MoveShape<P, MC>;
+  const dim3 b(Mv::kThreads);
   EB_CUDA(start(tree_p2m_kernel<P, NSL, ND>, dim3(g.ncells), 32 * kCellWarps, p2m_smem<P, NSL, ND>(), st, d, g.cells,
                 g.nmesh, one, many, tab));
   for (int s = 0; s < kTreePasses; s++)
-    EB_CUDA(start(tree_move_kernel<P, MC, kUp>, dim3(g.nup[s], NC / MC), b.x, move_smem<P, MC>(), st, d, g.up[s],
+    EB_CUDA(start(tree_move_kernel<P, MC, kUp>, dim3(g.nup[s], NC / MC), b.x, Mv::smem(), st, d, g.up[s],
                   g.nmesh, s, tab));
-  EB_CUDA(start(tree_move_kernel<P, MC, kAcross>, dim3(g.nm2l, NC / MC), b.x, move_smem<P, MC>(), st, d, g.m2l, g.nmesh,
+  EB_CUDA(start(tree_move_kernel<P, MC, kAcross>, dim3(g.nm2l, NC / MC), b.x, Mv::smem(), st, d, g.m2l, g.nmesh,
                 0, tab));
-  EB_CUDA(start(tree_move_kernel<P, MC, kDown>, dim3(g.ncells, NC / MC), b.x, move_smem<P, MC>(), st, d, g.cells,
+  EB_CUDA(start(tree_move_kernel<P, MC, kDown>, dim3(g.ncells, NC / MC), b.x, Mv::smem(), st, d, g.cells,
                 g.nmesh, 0, tab));
   EB_CUDA(start(tree_l2p_kernel<P, NC>, dim3(g.ncells), 32 * kCellWarps, sizeof(double2) * NC * tree_pairs(P), st, d,
                 g.cells, g.nmesh, tab));

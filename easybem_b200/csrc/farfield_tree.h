@@ -18,7 +18,7 @@ namespace eb {
 #define EB_TREE_ORDER32 14
 #endif
 #ifndef EB_TREE_ORDER64
-#define EB_TREE_ORDER64 30
+#define EB_TREE_ORDER64 28
 #endif
 constexpr int kTreeOrder32 = EB_TREE_ORDER32;  // mixed applies
 constexpr int kTreeOrder64 = EB_TREE_ORDER64;  // FP64 applies

@@ -65,14 +65,31 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
     return k;
   };
   const int root = build(0, nc);
-  if (nodes[root].height > kTreePasses * kTreeLevelsPerPass) return false;
+  if (nodes[root].height > kTreePasses * kTreeLevelsPerPass || (int)nodes.size() >= kTreeMaxNodes) return false;
   const int nn = p.nnodes = (int)nodes.size();
   p.ball.resize(nn);
   for (int c = 0; c < nc; c++) {
     const double* b = &h.cell_ball[4 * (size_t)c];
     p.ball[c] = dq{b[0], b[1], b[2], std::max(h.cell_rho[c], 1e-3 * b[3])};
   }
-  for (int k = nc; k < nn; k++) p.ball[k] = ball_of(p.ball, nodes[k].lo, nodes[k].hi);
+  // a move scales with the inverse distance of the two centres, so an inner
+  // node's centre keeps away from those of its descendants (symmetric meshes
+  // put them at the same point)
+  std::function<bool(int, int)> clear = [&](int k, int j) {
+    const dq &x = p.ball[k], &y = p.ball[j];
+    const d3 v = mk3(x.x - y.x, x.y - y.y, x.z - y.z);
+    const double s = kTreeMinStep * x.w;
+    if (dot3(v, v) < s * s) return false;
+    return nodes[j].left < 0 || (clear(k, nodes[j].left) && clear(k, nodes[j].right));
+  };
+  for (int k = nc; k < nn; k++) {
+    const dq b = ball_of(p.ball, nodes[k].lo, nodes[k].hi);
+    p.ball[k] = b;
+    for (int t = 1; t < 64 && !(clear(k, nodes[k].left) && clear(k, nodes[k].right)); t++) {
+      const double a = 2.4 * t, z = std::cos(1.7 * t), r = std::sqrt(1.0 - z * z), s = 0.004 * t * b.w;
+      p.ball[k] = dq{b.x + s * r * std::cos(a), b.y + s * r * std::sin(a), b.z + s * z, b.w + s};
+    }
+  }
 
   // the tree against itself
   std::vector<std::pair<int, int>> far;
@@ -134,8 +151,15 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
                    [&](int a, int b) { return count[a + 1] - count[a] > count[b + 1] - count[b]; });
   for (int k : order) {
     p.m2l.tgt.push_back(k);
-    std::sort(src.begin() + count[k], src.begin() + count[k + 1]);
-    p.m2l.src.insert(p.m2l.src.end(), src.begin() + count[k], src.begin() + count[k + 1]);
+    for (int q = count[k]; q < count[k + 1]; q++) {
+      const dq &x = p.ball[k], &y = p.ball[src[q]];
+      const d3 v = mk3(x.x - y.x, x.y - y.y, x.z - y.z);
+      const double share = std::log(kTreeTheta) / std::log((x.w + y.w) / std::sqrt(dot3(v, v)));
+      const int f = std::min(255, std::max(1, (int)std::ceil(255.0 * share)));
+      p.m2l.src.push_back((int)((unsigned)f << 24 | (unsigned)src[q]));
+    }
+    std::sort(p.m2l.src.end() - (count[k + 1] - count[k]), p.m2l.src.end(),
+              [](int a, int b) { return (unsigned)a >> 24 != (unsigned)b >> 24 ? (unsigned)a >> 24 > (unsigned)b >> 24 : a < b; });
     p.m2l.ptr.push_back((int)p.m2l.src.size());
   }
 
@@ -163,7 +187,7 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
     if (!used[k]) continue;
     TreeMoves& u = p.up[(nodes[k].height - 1) / kTreeLevelsPerPass];
     u.tgt.push_back(k);
-    u.src.insert(u.src.end(), sources[k].begin(), sources[k].end());
+    for (int j : sources[k]) u.src.push_back((int)(255u << 24 | (unsigned)j));
     u.ptr.push_back((int)u.src.size());
   }
 
@@ -171,7 +195,7 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
   for (int c = 0; c < nc; c++) {
     p.down.tgt.push_back(c);
     for (int k = nodes[c].parent; k >= 0; k = nodes[k].parent)
-      if (p.has_local[k]) p.down.src.push_back(k);
+      if (p.has_local[k]) p.down.src.push_back((int)(255u << 24 | (unsigned)k));
     p.down.ptr.push_back((int)p.down.src.size());
   }
 

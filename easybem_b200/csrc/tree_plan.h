@@ -21,14 +21,22 @@ namespace eb {
 // pairs (16 a cell at 0.5, 11 at 0.6) for higher orders (18 at 0.6 for the
 // accuracy of 14 at 0.5).
 constexpr double kTreeTheta = 0.5;
-// Translations into one node run on four warps; the upward pass covers three
-// levels of the tree per launch (eight descendants a node, two per warp).
+// Least distance of a node's centre from its descendants' centres, over its radius.
+constexpr double kTreeMinStep = 1e-3;
+// The upward pass covers three levels of the tree per launch (up to eight
+// descendants a node).
 constexpr int kTreeLevelsPerPass = 3;
 constexpr int kTreePasses = 6;  // enough for 2^18 cells
+constexpr int kTreeMaxNodes = 1 << 24;
 // Close cell pairs per near task (one warp's work; the diagonal counts).
 constexpr int kTreeNearChunk = 4;
 
-// Expansions moved into node tgt[k] from nodes src[ptr[k] .. ptr[k + 1]).
+// Expansions moved into node tgt[k] from nodes src[ptr[k] .. ptr[k + 1]). The
+// upper 8 bits of a source are the share f / 255 of the degrees that its pair
+// needs: an expansion of order p is used up to (p + 1) f / 255 - 1 (rounded
+// up). With radii r and distance d the truncation falls as (r / d)^(order + 1),
+// so f = ln(kTreeTheta) / ln(r / d) gives every pair the bound of the closest
+// ones (0.8 on average: half of the work). Sorted by f, largest first.
 struct TreeMoves {
   std::vector<int> tgt, ptr = {0}, src;
 };
