@@ -675,7 +675,8 @@ bool sym_eligible(const Mesh* m, bool fp32, int nsl, int nd, bool fp64_internal)
 
 long long mesh_far_slots(const Mesh* m, bool fp32, int nsl, int nd)
 {
-  if (m->tree && m->tree->usable && m->plan.engine == 4 && tree_eligible(const_cast<Mesh*>(m), fp32, nsl, nd)) return tree_far_slots(m);
+  if (m->tree && m->tree->usable && m->plan.engine == 4 && tree_eligible(const_cast<Mesh*>(m), fp32, nsl, nd))
+    return tree_far_slots(m, nd);
   if (sym_eligible(m, fp32, nsl, nd)) {
     const int r = far_sym_cells_per_item(kSymCellsPerItem);
     long long n = 0;

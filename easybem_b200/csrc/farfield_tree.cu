@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(32 * kCellWarps)
   __syncthreads();
   if (warp == 0) {
     const size_t stride = (size_t)d.slot_off[d.ncells] * kCell;
-    double* out = d.partial + (size_t)(d.slot_off[cell + 1] - 1) * kCell + lane;
+    double* out = d.partial + d.first_col * stride + (size_t)(d.slot_off[cell + 1] - 1) * kCell + lane;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       double v = 0.0;
@@ -978,6 +978,113 @@ __global__ void __launch_bounds__(32, 8)
     d.partial[c * stride + (size_t)task.w * kCell + lane] = active ? (double)hi[c] + (double)lo[c] : 0.0;
 }
 
+// The same in forward order only, for ND double-layer columns: every cell
+// against all its close cells (the full lists). With four columns a pair costs
+// 15 operations in either order; two symmetric passes of two columns, the most
+// whose sums fit the registers, cost the same.
+template <typename T, int ND>
+__global__ void __launch_bounds__(32, 8)
+    tree_near_dl_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh)
+{
+  using S = typename Slot<T>::type;
+  constexpr bool F32 = sizeof(T) == 4;
+  constexpr int NREC = rec_slots(0, ND);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int4 s_vid[kCell];
+  __shared__ dq s_nrm[kCell];
+  __shared__ S s_plane[kCell];
+  S* s_rec = reinterpret_cast<S*>(smem_raw);
+  const int lane = threadIdx.x;
+  int k = blockIdx.x;
+  const TreeDesc& d = descs[tree_entry(off, nmesh, k)];
+  const FarMeshDesc& md = d.far;
+  if (md.active && *md.active == 0) return;
+  const int4 task = d.tasks[k];
+  const int ti = task.x * kCell + lane;
+  const bool active = ti < md.ne;
+  const int tsel = active ? ti : task.x * kCell;
+  const dq ball = md.twarp[task.x], cd = md.tcent[tsel], nd = md.tnrm[tsel];
+  const double cen[3] = {cd.x, cd.y, cd.z}, nrm[3] = {nd.x, nd.y, nd.z};
+  const int4 tv = active ? md.tvid[tsel] : make_int4(-1, -1, -1, 0);
+  const S* grec = reinterpret_cast<const S*>(md.rec);
+  T hi[ND], lo[ND];
+#pragma unroll
+  for (int c = 0; c < ND; ++c) hi[c] = lo[c] = 0;
+#pragma unroll 1
+  for (int e = task.y; e < task.z; ++e) {
+    const int cell = d.entries[e].x, t0 = cell * kCell;
+    const int ns = min(kCell, md.ne - t0);
+    const S* g = grec + (size_t)t0 * kQ * NREC;
+    if constexpr (F32) {  // source-pair layout
+      constexpr int per = kQ * NREC;
+      const int nstage = ((ns + 1) >> 1) * per;
+      for (int i = lane; i < nstage; i += 32) {
+        const int p = i / per, rem = i - p * per;
+        const float4 a = g[(size_t)(2 * p) * per + rem];
+        float4 c;
+        if (2 * p + 1 < ns) c = g[(size_t)(2 * p + 1) * per + rem];
+        else c = rem % NREC == 0 ? make_float4(0.f, 0.f, 0.f, 1.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+        s_rec[2 * i] = make_float4(a.x, c.x, a.y, c.y);
+        s_rec[2 * i + 1] = make_float4(a.z, c.z, a.w, c.w);
+      }
+      if ((ns & 1) && lane == 0) {
+        s_vid[ns] = make_int4(-1, -1, -1, 0);
+        s_nrm[ns] = dq{0.0, 0.0, 0.0, 0.0};
+        s_plane[ns] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    } else {
+      for (int i = lane; i < ns * kQ * NREC; i += 32) s_rec[i] = g[i];
+    }
+    if (lane < ns) {
+      s_vid[lane] = md.svid[t0 + lane];
+      s_nrm[lane] = md.snrm[t0 + lane];
+      if constexpr (F32) s_plane[lane] = md.splane32[t0 + lane];
+      else s_plane[lane] = md.splane64[t0 + lane];
+    }
+    __syncwarp();
+    if (active) {
+      const dq cc = md.ccent[cell];
+      const double ddx = cc.x - ball.x, ddy = cc.y - ball.y, ddz = cc.z - ball.z;
+      const double rr = kFarRatio * (cc.w + ball.w);
+      const bool far = ddx * ddx + ddy * ddy + ddz * ddz > rr * rr;
+      const T o[3] = {(T)(cc.x - cen[0]), (T)(cc.y - cen[1]), (T)(cc.z - cen[2])};
+      T xs[kQ], ys[kQ], zs[kQ], q2[kQ], wq[kQ], sl[1][kQ], dl[ND][kQ];
+#pragma unroll
+      for (int a = 0; a < kQ; ++a) {
+        S p;
+        if constexpr (F32) p = md.tgt32[(size_t)tsel * kQ + a];
+        else p = md.tgt64[(size_t)tsel * kQ + a];
+        xs[a] = p.x - o[0]; ys[a] = p.y - o[1]; zs[a] = p.z - o[2];
+        q2[a] = xs[a] * xs[a] + ys[a] * ys[a] + zs[a] * zs[a];
+        wq[a] = p.w;
+        sl[0][a] = 0;
+#pragma unroll
+        for (int c = 0; c < ND; ++c) dl[c][a] = 0;
+      }
+      if constexpr (F32) {
+        if (far) eval_cell_sp<kQ, kQ, 0, ND, true>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+        else eval_cell_sp<kQ, kQ, 0, ND, false>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+      } else {
+        if (far) eval_cell<T, kQ, kQ, 0, ND, true>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+        else eval_cell<T, kQ, kQ, 0, ND, false>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+      }
+#pragma unroll
+      for (int c = 0; c < ND; ++c) {
+        T part = 0;
+#pragma unroll
+        for (int a = 0; a < kQ; ++a) part += wq[a] * dl[c][a];
+        if constexpr (F32) two_sum_add(hi[c], lo[c], part);
+        else hi[c] += part;
+      }
+    }
+    __syncwarp();
+  }
+  const size_t stride = (size_t)d.slot_off[d.ncells] * kCell;
+#pragma unroll
+  for (int c = 0; c < ND; ++c)
+    d.partial[c * stride + (size_t)task.w * kCell + lane] = active ? (double)hi[c] + (double)lo[c] : 0.0;
+}
+
 // ---------------------------------------------------------------------------
 // Tables (host, extended precision).
 
@@ -1139,14 +1246,26 @@ struct TreeGrid {
 
 template <int P, typename T, int NSL, int ND>
 int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const ApplyArgs* many, const TreeTables& tab,
-               cudaStream_t st)
+               const TreeSide& side, cudaStream_t st)
 {
   constexpr int NC = NSL + ND;
   constexpr int MC = NC % 2 == 0 ? 2 : 1;  // columns of a CTA
+  constexpr int PD = ND > 0 ? 1 : 0;       // double-layer columns of a multipole CTA
   using Mv = MoveShape<P, MC>;
   const dim3 b(Mv::kThreads);
-  EB_CUDA(start(tree_p2m_kernel<P, NSL, ND>, dim3(g.ncells), 32 * kCellWarps, p2m_smem<P, NSL, ND>(), st, d, g.cells,
-                g.nmesh, one, many, tab));
+  EB_CUDA(cudaEventRecord(side.fork, st));
+  EB_CUDA(cudaStreamWaitEvent(side.st, side.fork, 0));
+  // a single double layer runs the SL+DL sums with zero charges (their records
+  // hold zeros there; 1 of 9 or 14 operations), several the forward form
+  if constexpr (ND > 1)
+    EB_CUDA(start(tree_near_dl_kernel<T, ND>, dim3(g.ntasks), 32, (size_t)kCell * kQ * rec_slots(0, ND) * 4 * sizeof(T),
+                  side.st, d, g.tasks, g.nmesh));
+  else
+    EB_CUDA(start(tree_near_kernel<T, ND ? 1 : NSL, ND>, dim3(g.ntasks), 32, near_smem<T, ND ? 1 : NSL, ND>(), side.st, d,
+                  g.tasks, g.nmesh));
+  EB_CUDA(cudaEventRecord(side.join, side.st));
+  EB_CUDA(start(tree_p2m_kernel<P, NSL, PD>, dim3(g.ncells, ND > 1 ? ND : 1), 32 * kCellWarps, p2m_smem<P, NSL, PD>(), st,
+                d, g.cells, g.nmesh, one, many, tab));
   for (int s = 0; s < kTreePasses; s++)
     EB_CUDA(start(tree_move_kernel<P, MC, kUp>, dim3(g.nup[s], NC / MC), b.x, Mv::smem(), st, d, g.up[s],
                   g.nmesh, s, tab));
@@ -1156,25 +1275,30 @@ int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const
                 g.nmesh, 0, tab));
   EB_CUDA(start(tree_l2p_kernel<P, NC>, dim3(g.ncells), 32 * kCellWarps, sizeof(double2) * NC * tree_pairs(P), st, d,
                 g.cells, g.nmesh, tab));
-  EB_CUDA(start(tree_near_kernel<T, NSL, ND>, dim3(g.ntasks), 32, near_smem<T, NSL, ND>(), st, d, g.tasks, g.nmesh));
+  EB_CUDA(cudaStreamWaitEvent(st, side.join, 0));
   return EB_OK;
 }
 
-bool tree_variant(int nsl, int nd) { return (nsl == 1 && nd == 1) || (nd == 0 && (nsl == 1 || nsl == 3 || nsl == 4)); }
+bool tree_variant(int nsl, int nd)
+{
+  return nd == 0 ? nsl == 1 || nsl == 3 || nsl == 4 : nsl == 0 ? nd == 1 || nd == 4 : nsl == 1 && nd == 1;
+}
 
 int launch_variant(bool fp32, int nsl, int nd, const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one,
-                   const ApplyArgs* many, int device, cudaStream_t st)
+                   const ApplyArgs* many, int device, const TreeSide& side, cudaStream_t st)
 {
   TreeTables tab;
   EB_CHECK(tables_for(device, fp32 ? kTreeOrder32 : kTreeOrder64, &tab));
 #define EB_TREE(NSL, ND)                                                                        \
   if (nsl == NSL && nd == ND)                                                                   \
-    return fp32 ? launch_all<kTreeOrder32, float, NSL, ND>(d, g, one, many, tab, st)            \
-                : launch_all<kTreeOrder64, double, NSL, ND>(d, g, one, many, tab, st);
+    return fp32 ? launch_all<kTreeOrder32, float, NSL, ND>(d, g, one, many, tab, side, st)            \
+                : launch_all<kTreeOrder64, double, NSL, ND>(d, g, one, many, tab, side, st);
   EB_TREE(1, 1)
   EB_TREE(1, 0)
   EB_TREE(3, 0)
   EB_TREE(4, 0)
+  EB_TREE(0, 1)
+  EB_TREE(0, 4)
 #undef EB_TREE
   return set_error(EB_ERR_INVALID, "no tree far field for this operator combination");
 }
@@ -1214,8 +1338,9 @@ static int upload_lists(TreeMesh* t)
     if (!v.empty()) std::memcpy(host.data() + at, v.data(), v.size() * sizeof(v[0]));
     return at;
   };
-  const size_t ball = add(p.ball), has = add(p.has_local), tasks = add(p.tasks), entries = add(p.entries),
-               slots = add(p.slot_off);
+  const size_t ball = add(p.ball), has = add(p.has_local), tasks = add(p.sym.tasks), entries = add(p.sym.entries),
+               slots = add(p.sym.slot_off), ftasks = add(p.fwd.tasks), fentries = add(p.fwd.entries),
+               fslots = add(p.fwd.slot_off);
   struct At {
     size_t tgt, ptr, src;
   };
@@ -1236,6 +1361,9 @@ static int upload_lists(TreeMesh* t)
   d.tasks = reinterpret_cast<const int4*>(q + tasks);
   d.entries = reinterpret_cast<const int2*>(q + entries);
   d.slot_off = reinterpret_cast<const int*>(q + slots);
+  t->fwd_tasks = reinterpret_cast<const int4*>(q + ftasks);
+  t->fwd_entries = reinterpret_cast<const int2*>(q + fentries);
+  t->fwd_slot_off = reinterpret_cast<const int*>(q + fslots);
   for (int s = 0; s < kTreePasses; s++) {
     d.up[s] = dev(up[s]);
     d.nup[s] = (int)p.up[s].tgt.size();
@@ -1244,26 +1372,59 @@ static int upload_lists(TreeMesh* t)
   d.down = dev(down);
   d.nnodes = p.nnodes;
   d.ncells = p.ncells;
-  d.ntasks = (int)p.tasks.size();
+  d.ntasks = (int)p.sym.tasks.size();
   d.nm2l = (int)p.m2l.tgt.size();
   return EB_OK;
 }
 
-long long tree_far_slots(const Mesh* m) { return (long long)m->tree->plan.slot_off.back() * kCell; }
+int TreeSide::create()
+{
+  if (st) return EB_OK;
+  int least = 0, greatest = 0;
+  EB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  EB_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+  EB_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+  EB_CUDA(cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, least));
+  return EB_OK;
+}
+
+TreeSide::~TreeSide()
+{
+  if (st) cudaStreamDestroy(st);
+  if (fork) cudaEventDestroy(fork);
+  if (join) cudaEventDestroy(join);
+}
+
+// Close pairs of a variant in both orders at once, or forward only.
+static bool tree_forward(int nd) { return nd > 1; }
+
+long long tree_far_slots(const Mesh* m, int nd)
+{
+  const TreePlan& p = m->tree->plan;
+  return (long long)(tree_forward(nd) ? p.fwd : p.sym).slot_off.back() * kCell;
+}
 
 int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream_t st)
 {
   TreeMesh* t = m->tree.get();
   EB_CHECK(upload_lists(t));
+  EB_CHECK(t->side.create());
   std::unique_ptr<TreeScratch>& sc = t->scratch[(fp32 ? 64 : 0) + nsl * 5 + nd];
   if (!sc) {
     auto s = std::make_unique<TreeScratch>();
-    const int cols = nsl + nd;
+    const int cols = nsl + nd, slot_cols = nd == 1 ? 2 : cols;  // a DL alone leaves the SL column unused
     const size_t bytes = sizeof(double2) * (size_t)cols * t->plan.nnodes * tree_pairs(fp32 ? kTreeOrder32 : kTreeOrder64);
     EB_CHECK(s->multipole.alloc(bytes));
     EB_CHECK(s->local.alloc(bytes));
-    EB_CHECK(s->partial.alloc(sizeof(double) * (size_t)cols * tree_far_slots(m)));
+    EB_CHECK(s->partial.alloc(sizeof(double) * (size_t)slot_cols * tree_far_slots(m, nd)));
     TreeDesc d = t->base;
+    if (tree_forward(nd)) {
+      d.tasks = t->fwd_tasks;
+      d.entries = t->fwd_entries;
+      d.slot_off = t->fwd_slot_off;
+      d.ntasks = (int)t->plan.fwd.tasks.size();
+    }
+    d.first_col = slot_cols - cols;
     d.far = mesh_far_desc(m, fp32, nsl, nd, m->rec.p, s->partial.as<double>());
     d.pos = m->pos64.as<dq>();
     d.multipole = s->multipole.as<double2>();
@@ -1275,7 +1436,7 @@ int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream
     sc = std::move(s);
   }
   const TreeDesc& d = sc->host;
-  A->partial = d.partial;
+  A->partial = d.partial + (size_t)d.first_col * tree_far_slots(m, nd);
   A->slot_off = d.slot_off;
   TreeGrid g;
   g.ncells = d.ncells;
@@ -1283,7 +1444,7 @@ int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream
   g.ntasks = d.ntasks;
   std::copy_n(d.nup, kTreePasses, g.nup);
   if (m->profile) EB_CUDA(cudaEventRecord(m->ev0, st));
-  return launch_variant(fp32, nsl, nd, sc->desc.as<TreeDesc>(), g, *A, nullptr, m->device, st);
+  return launch_variant(fp32, nsl, nd, sc->desc.as<TreeDesc>(), g, *A, nullptr, m->device, t->side, st);
 }
 
 }  // namespace eb

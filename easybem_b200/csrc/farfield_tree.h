@@ -47,6 +47,7 @@ struct TreeDesc {
   double* partial;           // [columns][slots][kCell]
   int nnodes, ncells;
   int ntasks, nm2l, nup[kTreePasses];
+  int first_col;             // of partial: 1 for a double layer alone (column 0: its zero single layer)
 };
 
 // Scratch and descriptor of one variant, made on its first apply and kept.
@@ -55,12 +56,30 @@ struct TreeScratch {
   TreeDesc host;
 };
 
+// The close pairs' stream: they run beside the expansions (the FP32 pipe and
+// MUFU beside FP64 mma in a mixed apply), forked from and joined to the
+// apply's stream, at the least priority so that the shorter kernels of the
+// expansions take freed SMs first.
+struct TreeSide {
+  cudaStream_t st = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  TreeSide() = default;
+  TreeSide(const TreeSide&) = delete;
+  TreeSide& operator=(const TreeSide&) = delete;
+  ~TreeSide();
+  int create();  // no-op when made
+};
+
 // A mesh's tree, made on the first apply that takes it.
 struct TreeMesh {
   bool usable = false;
   TreePlan plan;
   DevBuf lists;  // one allocation
   TreeDesc base; // static pointers
+  const int4* fwd_tasks;      // TreePlan::fwd
+  const int2* fwd_entries;
+  const int* fwd_slot_off;
+  TreeSide side;
   std::map<int, std::unique_ptr<TreeScratch>> scratch;
 };
 
@@ -71,6 +90,6 @@ bool tree_eligible(Mesh* m, bool fp32, int nsl, int nd);
 // (A.partial and A.slot_off are set for the finalize).
 int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream_t st);
 // Partial slots (summed over the rows, per output).
-long long tree_far_slots(const Mesh* m);
+long long tree_far_slots(const Mesh* m, int nd);
 
 }  // namespace eb

@@ -200,29 +200,39 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
   }
 
   // close pairs: transposed slots first, then one forward slot per task, then
-  // the far slot
-  std::vector<int> trans(nc, 0), chunks(nc);
+  // the far slot; the larger tasks first
+  std::vector<std::vector<int>> all(nc);
   for (int c = 0; c < nc; c++) {
     std::sort(near[c].begin(), near[c].end());
-    for (int j : near[c]) trans[j]++;
-    chunks[c] = ((int)near[c].size() + 1 + kTreeNearChunk - 1) / kTreeNearChunk;
+    for (int j : near[c]) {
+      all[c].push_back(j);
+      all[j].push_back(c);
+    }
   }
-  p.slot_off.assign(nc + 1, 0);
-  for (int c = 0; c < nc; c++) p.slot_off[c + 1] = p.slot_off[c] + trans[c] + chunks[c] + 1;
-  std::vector<int> next(p.slot_off.begin(), p.slot_off.end() - 1);
-  for (int c = 0; c < nc; c++) {
-    const int e0 = (int)p.entries.size();
-    p.entries.push_back(make_int2(c, -1));
-    for (int j : near[c]) p.entries.push_back(make_int2(j, next[j]++));
-    const int e1 = (int)p.entries.size();
-    int slot = p.slot_off[c] + trans[c];
-    for (int e = e0; e < e1; e += kTreeNearChunk)
-      p.tasks.push_back(make_int4(c, e, std::min(e1, e + kTreeNearChunk), slot++));
-  }
-  // the larger tasks first; those that start with the diagonal are the first
-  // chunks of their cells
-  std::stable_sort(p.tasks.begin(), p.tasks.end(),
-                   [](const int4& a, const int4& b) { return a.z - a.y > b.z - b.y; });
+  auto lists = [&](const std::vector<std::vector<int>>& close, bool both, TreeNear& out) {
+    std::vector<int> trans(nc, 0);
+    if (both)
+      for (int c = 0; c < nc; c++)
+        for (int j : close[c]) trans[j]++;
+    out.slot_off.assign(nc + 1, 0);
+    for (int c = 0; c < nc; c++)
+      out.slot_off[c + 1] =
+          out.slot_off[c] + trans[c] + ((int)close[c].size() + kTreeNearChunk) / kTreeNearChunk + 1;
+    std::vector<int> next(out.slot_off.begin(), out.slot_off.end() - 1);
+    for (int c = 0; c < nc; c++) {
+      const int e0 = (int)out.entries.size();
+      out.entries.push_back(make_int2(c, -1));
+      for (int j : close[c]) out.entries.push_back(make_int2(j, both ? next[j]++ : -1));
+      const int e1 = (int)out.entries.size();
+      int slot = out.slot_off[c] + trans[c];
+      for (int e = e0; e < e1; e += kTreeNearChunk)
+        out.tasks.push_back(make_int4(c, e, std::min(e1, e + kTreeNearChunk), slot++));
+    }
+    std::stable_sort(out.tasks.begin(), out.tasks.end(),
+                     [](const int4& a, const int4& b) { return a.z - a.y > b.z - b.y; });
+  };
+  lists(near, true, p.sym);
+  lists(all, false, p.fwd);
   return true;
 }
 

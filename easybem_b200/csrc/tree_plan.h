@@ -41,6 +41,16 @@ struct TreeMoves {
   std::vector<int> tgt, ptr = {0}, src;
 };
 
+// Close cell pairs. A task is (cell, first entry, last entry, slot of its
+// forward sums), an entry (other cell, slot of the transposed sums or -1); the
+// slots of cell c are slot_off[c] .. slot_off[c + 1]), the last one for the
+// far sum.
+struct TreeNear {
+  std::vector<int4> tasks;
+  std::vector<int2> entries;
+  std::vector<int> slot_off;
+};
+
 struct TreePlan {
   int ncells = 0, nnodes = 0;  // nodes 0 .. ncells - 1 are the cells
   std::vector<dq> ball;        // centre; radius over the quadrature points
@@ -48,13 +58,8 @@ struct TreePlan {
   TreeMoves m2l;               // multipoles of separated nodes into locals
   TreeMoves down;              // locals of the ancestors into every cell
   std::vector<char> has_local; // per node: it is a target of m2l
-  // close pairs: every unordered pair of cells once (sym), with the slot that
-  // takes the transposed sums; a task is (cell, first entry, last entry, slot
-  // of its forward sums); slots of cell c are slot_off[c] .. slot_off[c + 1]),
-  // the last one for the far sum
-  std::vector<int4> tasks;
-  std::vector<int2> entries;
-  std::vector<int> slot_off;
+  TreeNear sym;  // every unordered pair of cells once
+  TreeNear fwd;  // every ordered pair
 };
 
 // False when more than an eighth of all cell pairs are close (the tree would

@@ -66,10 +66,28 @@ def test_tree_matches_oracle_and_symmetric_kernels(gpu_lib, oracle, name):
             vs = m.apply_sl(t, precision=prec)
             assert rel_l2(vs[rows], vo) < tol
             d = m.apply_hypersingular(u, precision=prec)
+            qs = m.apply_dl(u, precision=prec)
+            assert rel_l2(qs[rows], qo) < tol
             m.set_far_engine("sym_all")
             vd, qd = m.apply_sl_dl(t, u, precision=prec)
             assert rel_l2(v, vd) < tol and rel_l2(q, qd) < tol
             assert rel_l2(d, m.apply_hypersingular(u, precision=prec)) < 10 * tol  # differences of V's columns
+
+
+@pytest.mark.parametrize("name", ["cut12801", "two"])
+@pytest.mark.parametrize("nrhs", [1, 3, 5])
+def test_tree_right_hand_sides(gpu_lib, name, nrhs):
+    """b = 1/2 M g + K g: one column, a padded group of four, four and one."""
+    nodes, elems = MESHES[name]()
+    g = np.random.default_rng(nrhs).normal(size=(nrhs, len(nodes)))
+    with gpu_lib.Mesh(nodes, elems) as m:
+        for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL)):
+            m.set_far_engine("tree")
+            b = m.dirichlet_rhs(g, prec)
+            m.set_far_engine("cuda")
+            c = m.dirichlet_rhs(g, prec)
+            for k in range(nrhs):
+                assert rel_l2(b[k], c[k]) < tol
 
 
 @pytest.mark.parametrize("unit", [1e-9, 1e6])
