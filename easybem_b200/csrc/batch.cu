@@ -54,10 +54,17 @@ int Batch::build(const std::vector<BatchEntry*>& entries, bool fp32, int nsl, in
   Q_ = entries[0]->mesh->h.Q;
   K_ = entries[0]->mesh->h.K;
   const int n = (int)entries.size();
-  tc_ = fp32 && nsl_ == 1 && nd_ == 1;
-  for (BatchEntry* be : entries) tc_ = tc_ && tc_eligible(be->mesh, fp32, 1, 1);
-  sym_ = !tc_;
-  for (BatchEntry* be : entries) sym_ = sym_ && sym_eligible(be->mesh, fp32, nsl_, nd_, sym_fp64);
+  std::vector<char> tree(n);
+  for (int e = 0; e < n; e++) tree[e] = tree_eligible(entries[e]->mesh, fp32, nsl_, nd_);
+  ntree_ = (int)std::count(tree.begin(), tree.end(), 1);
+  tc_ = fp32 && nsl_ == 1 && nd_ == 1 && ntree_ < n;
+  for (int e = 0; e < n; e++)
+    if (!tree[e]) tc_ = tc_ && tc_eligible(entries[e]->mesh, fp32, 1, 1);
+  sym_ = !tc_ && ntree_ < n;
+  for (int e = 0; e < n; e++)
+    if (!tree[e]) sym_ = sym_ && sym_eligible(entries[e]->mesh, fp32, nsl_, nd_, sym_fp64);
+  std::vector<TreeDesc> tdesc;
+  std::vector<ApplyArgs> tree_args;
   std::vector<TcPrepArgs> targs;
   std::vector<int> toff(1, 0);
   std::vector<FarMeshDesc> desc(n);
@@ -76,7 +83,7 @@ int Batch::build(const std::vector<BatchEntry*>& entries, bool fp32, int nsl, in
     if (nd_ && !be->uin.p) return set_error(EB_ERR_INVALID, "batch entry without DL columns");
     desc[e] = mesh_far_desc(m, fp32, nsl_, nd_, be->rec.p, be->partial.as<double>());
     desc[e].active = d_flags ? d_flags + e : nullptr;
-    if (tc_) {
+    if (tc_ && !tree[e]) {
       EB_CHECK(ensure_tc_static(m));
       EB_CHECK(be->tc_be.alloc(far_tc_operand_bytes(h.ncells)));
       EB_CHECK(be->tc_charge.alloc(far_tc_charge_bytes(h.ncells)));
@@ -89,7 +96,7 @@ int Batch::build(const std::vector<BatchEntry*>& entries, bool fp32, int nsl, in
     }
     std::vector<WorkItem> sym_items;
     int sym_nsplit = 0;
-    if (sym_) {  // the mesh's symmetric work list and its own zeroed partial slots
+    if (sym_ && !tree[e]) {  // the mesh's symmetric work list and its own zeroed partial slots
       sym_nsplit = far_sym_items(h.nitems, h.ncells, kSymBatchCellsPerItem, sym_items);
       const size_t bytes = sizeof(double) * (size_t)(nsl_ + nd_) * (size_t)sym_nsplit * h.nitems;
       if (be->sym_partial.bytes < bytes) {  // no zeroing: the finalize reads only written slots
@@ -100,12 +107,31 @@ int Batch::build(const std::vector<BatchEntry*>& entries, bool fp32, int nsl, in
       desc[e].nsplit = sym_nsplit;
       desc[e].src_tile = kTS;
     }
-    src_tile = std::min(src_tile, desc[e].src_tile);
+    if (tree[e]) {
+      // both precisions of a solver share the entry's buffers: size them for the larger order
+      const size_t bytes = tree_expansion_bytes(m, std::max(kTreeOrder32, kTreeOrder64), nsl_ + nd_);
+      if (bytes) {
+        EB_CHECK(be->tree_multipole.alloc(bytes));
+        EB_CHECK(be->tree_local.alloc(bytes));
+      }
+      EB_CHECK(be->tree_partial.alloc(tree_partial_bytes(m, nsl_, nd_)));
+      TreeDesc d;
+      EB_CHECK(tree_desc(m, fp32, nsl_, nd_, be->rec.p, be->tree_multipole.p, be->tree_local.p,
+                         be->tree_partial.as<double>(), &d));
+      d.far.active = desc[e].active;
+      tdesc.push_back(d);
+    } else {
+      src_tile = std::min(src_tile, desc[e].src_tile);
+    }
     args[e] = mesh_apply_args(m, fp32, be->rec.p, be->partial.as<double>(), nsl_ ? be->tin.as<double>() : nullptr,
                               h.ne, nd_ ? be->uin.as<double>() : nullptr, nsl_ ? be->vout.as<double>() : nullptr,
                               h.ne, nd_ ? be->qout.as<double>() : nullptr);
     args[e].active = d_flags ? d_flags + e : nullptr;
-    if (sym_) {
+    if (tree[e]) {
+      args[e].partial = tdesc.back().partial;
+      args[e].slot_off = tdesc.back().slot_off;
+      tree_args.push_back(args[e]);
+    } else if (sym_) {
       args[e].partial = be->sym_partial.as<double>();
       args[e].nsplit = sym_nsplit;
       args[e].sym_cells = far_sym_cells_per_item(kSymBatchCellsPerItem);
@@ -113,6 +139,7 @@ int Batch::build(const std::vector<BatchEntry*>& entries, bool fp32, int nsl, in
     poff[e + 1] = poff[e] + (int)(((long long)h.ne * h.Q + kPrepBlock - 1) / kPrepBlock);
     foff[e + 1] = foff[e] + (h.ne + kFinalizeRows - 1) / kFinalizeRows;
     quad_pairs_ += h.far_quad_pairs;
+    if (tree[e]) continue;
     for (WorkItem w : sym_ ? sym_items : m->items_host) {
       w.mesh = e;
       const long long tg = std::min(kTT, h.nitems - w.tgt0);
@@ -129,6 +156,8 @@ int Batch::build(const std::vector<BatchEntry*>& entries, bool fp32, int nsl, in
   std::vector<WorkItem> flat(items.size());
   for (size_t k = 0; k < items.size(); k++) flat[k] = items[k].second;
   nitems_ = (int)flat.size();
+  cudaGetDevice(&device_);
+  if (ntree_ > 0) EB_CHECK(build_tree(tdesc, tree_args));
   prep_blocks_ = poff[n];
   fin_blocks_ = foff[n];
 
@@ -173,6 +202,44 @@ int Batch::build(const std::vector<BatchEntry*>& entries, bool fp32, int nsl, in
   return EB_OK;
 }
 
+int Batch::build_tree(const std::vector<TreeDesc>& desc, const std::vector<ApplyArgs>& args)
+{
+  const int n = (int)desc.size();
+  std::vector<int> off;
+  // first blocks of one kernel's entries; returns its block count
+  auto blocks = [&](auto&& count) {
+    int at = 0;
+    for (int k = 0; k < n; k++) {
+      off.push_back(at);
+      at += count(desc[k]);
+    }
+    off.push_back(at);
+    return at;
+  };
+  TreeGrid g;
+  g.nmesh = n;
+  g.ntasks = blocks([](const TreeDesc& d) { return d.ntasks; });
+  g.ncells = blocks([](const TreeDesc& d) { return d.multipole ? d.ncells : 0; });
+  g.nm2l = blocks([](const TreeDesc& d) { return d.multipole ? d.nm2l : 0; });
+  for (int s = 0; s < kTreePasses; s++) g.nup[s] = blocks([s](const TreeDesc& d) { return d.multipole ? d.nup[s] : 0; });
+  g.expansions = g.ncells > 0;
+  EB_CHECK(tree_off_.alloc(sizeof(int) * off.size()));
+  EB_CHECK(copy_h2d(tree_off_.p, off.data(), sizeof(int) * off.size()));
+  const int* o = tree_off_.as<int>();
+  g.tasks = o;
+  g.cells = o + (n + 1);
+  g.m2l = o + 2 * (n + 1);
+  for (int s = 0; s < kTreePasses; s++) g.up[s] = o + (3 + s) * (n + 1);
+  EB_CHECK(tree_desc_.alloc(sizeof(TreeDesc) * n));
+  EB_CHECK(copy_h2d(tree_desc_.p, desc.data(), sizeof(TreeDesc) * n));
+  EB_CHECK(tree_args_.alloc(sizeof(ApplyArgs) * n));
+  EB_CHECK(copy_h2d(tree_args_.p, args.data(), sizeof(ApplyArgs) * n));
+  if (g.expansions) EB_CHECK(tree_tables(fp32_, device_));
+  EB_CHECK(tree_side_.create());
+  tree_grid_ = g;
+  return EB_OK;
+}
+
 int Batch::check_error()
 {
   if (!tc_ || !tc_err_.p) return EB_OK;
@@ -191,8 +258,13 @@ int Batch::run(cudaStream_t st, int reserve_sms)
   const int grid = reserve_sms > 0 ? std::min(grid_, free_sms * occ_) : grid_;
   EB_CUDA(prep_launch_batch(fp32_, nsl_, nd_, args_.as<ApplyArgs>(), prep_off_.as<int>(), n, prep_blocks_, st));
   if (tc_) EB_CUDA(far_tc_prep_dl_batch(tc_args_.as<TcPrepArgs>(), tc_off_.as<int>(), n, tc_blocks_, st));
-  EB_CUDA(cudaMemsetAsync(counter_.p, 0, sizeof(int), st));
-  if (tc_)
+  if (ntree_ > 0)
+    EB_CHECK(tree_launch(fp32_, nsl_, nd_, tree_desc_.as<TreeDesc>(), tree_grid_, ApplyArgs{}, tree_args_.as<ApplyArgs>(),
+                         device_, tree_side_, st));
+  if (nitems_ > 0) EB_CUDA(cudaMemsetAsync(counter_.p, 0, sizeof(int), st));
+  if (nitems_ == 0) {
+    // every entry is on the tree
+  } else if (tc_)
     EB_CUDA(far_tc_launch(desc_.as<FarMeshDesc>(), items_.as<WorkItem>(), nitems_, counter_.as<int>(),
                           tc_err_.as<int>(), grid, st));
   else if (sym_)

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "farfield_tree.h"
 
 namespace eb {
 
@@ -29,6 +30,7 @@ struct BatchEntry {
   DevBuf uin, qout;     // DL density [nnodes] and DL output [nelems] (batches with a DL column)
   DevBuf tc_be, tc_charge;  // tensor-core DL operand and charges (tensor-core SL+DL batches)
   DevBuf sym_partial;       // symmetric batches: partial slots (one per tile, row and output)
+  DevBuf tree_multipole, tree_local, tree_partial;  // entries on the tree
   int index = -1;       // position in the current batch
 };
 
@@ -63,6 +65,7 @@ class Batch {
   long long quad_pairs() const { return quad_pairs_; }
 
  private:
+  int build_tree(const std::vector<TreeDesc>& desc, const std::vector<ApplyArgs>& args);
   std::vector<BatchEntry*> entries_;
   bool fp32_ = true;
   int nsl_ = kBatchCols;
@@ -72,6 +75,14 @@ class Batch {
   DevBuf tc_args_, tc_off_, tc_err_;
   bool sym_ = false;  // symmetric far field (fused FP32 SL+DL, 7-point rule, engine 2 on every mesh)
   int tc_blocks_ = 0;
+  // entries whose mesh takes the tree, whatever the others take (an entry's
+  // result does not depend on its neighbours): their kernels run beside the
+  // merged far-field launch of the rest
+  int ntree_ = 0;
+  DevBuf tree_desc_, tree_args_, tree_off_;
+  TreeGrid tree_grid_;
+  TreeSide tree_side_;
+  int device_ = 0;
   int nitems_ = 0, grid_ = 0, occ_ = 1, nsm_ = 148, prep_blocks_ = 0, fin_blocks_ = 0, K_ = 0, Q_ = 0;
   size_t smem_ = 0;
   long long quad_pairs_ = 0;

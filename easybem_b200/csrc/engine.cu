@@ -485,6 +485,7 @@ static int build_near(Mesh* m)
       e1 = cudaGetLastError();
     }
   }  // temporaries released on st
+  tree_prepare(m);  // host work beside the kernels
   e2 = cudaStreamSynchronize(st);
   cudaStreamDestroy(st);
   EB_CHECK(rc);
@@ -675,8 +676,7 @@ bool sym_eligible(const Mesh* m, bool fp32, int nsl, int nd, bool fp64_internal)
 
 long long mesh_far_slots(const Mesh* m, bool fp32, int nsl, int nd)
 {
-  if (m->tree && m->tree->usable && m->plan.engine == 4 && tree_eligible(const_cast<Mesh*>(m), fp32, nsl, nd))
-    return tree_far_slots(m, nd);
+  if (tree_eligible(m, fp32, nsl, nd) && (nd <= 1 || !m->tree->fwd.slot_off.empty())) return tree_far_slots(m, nd);
   if (sym_eligible(m, fp32, nsl, nd)) {
     const int r = far_sym_cells_per_item(kSymCellsPerItem);
     long long n = 0;
@@ -1146,7 +1146,7 @@ int eb_mesh_get_far_engine(eb_mesh mesh, int precision, int* engine)
 {
   if (!mesh || !engine) return set_error(EB_ERR_INVALID, "null argument");
   const bool fp32 = precision == EB_PREC_MIXED;
-  *engine = eb::tree_eligible(mesh->m, fp32, 1, 1)  ? EB_FAR_TREE
+  *engine = eb::tree_eligible(mesh->m, fp32, 1, 1)        ? (mesh->m->tree->plan.all_close ? EB_FAR_SYMMETRIC : EB_FAR_TREE)
             : eb::tc_eligible(mesh->m, fp32, 1, 1)  ? EB_FAR_TENSOR_CORES
             : eb::sym_eligible(mesh->m, fp32, 1, 1) ? EB_FAR_SYMMETRIC
                                                     : EB_FAR_CUDA_CORES;

@@ -149,7 +149,7 @@ struct Mesh {
   int sym_nitems = 0, sym_nsplit = 0;
   Variant sym_var;
   bool sym_used = false;  // the last apply ran the symmetric kernel
-  // tree far field (engine 4), made on the first apply that takes it
+  // tree far field (engine 4)
   std::shared_ptr<TreeMesh> tree;
   // host seconds of mesh creation: topology and pairs, static tables, near
   // field, and within the tables their device allocation and copy

@@ -1236,14 +1236,6 @@ cudaError_t start(void (*fn)(Args...), dim3 grid, int block, size_t smem, cudaSt
   return cudaGetLastError();
 }
 
-// Block counts of each kernel over the meshes of a launch and, for more than
-// one mesh, the first block of each (device).
-struct TreeGrid {
-  int nmesh = 1;
-  const int *cells = nullptr, *m2l = nullptr, *tasks = nullptr, *up[kTreePasses] = {};
-  int ncells = 0, nm2l = 0, ntasks = 0, nup[kTreePasses] = {};
-};
-
 template <int P, typename T, int NSL, int ND>
 int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const ApplyArgs* many, const TreeTables& tab,
                const TreeSide& side, cudaStream_t st)
@@ -1253,16 +1245,21 @@ int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const
   constexpr int PD = ND > 0 ? 1 : 0;       // double-layer columns of a multipole CTA
   using Mv = MoveShape<P, MC>;
   const dim3 b(Mv::kThreads);
-  EB_CUDA(cudaEventRecord(side.fork, st));
-  EB_CUDA(cudaStreamWaitEvent(side.st, side.fork, 0));
+  // close pairs beside the expansions; with nothing to run beside, on st itself
+  cudaStream_t near = g.expansions ? side.st : st;
+  if (g.expansions) {
+    EB_CUDA(cudaEventRecord(side.fork, st));
+    EB_CUDA(cudaStreamWaitEvent(side.st, side.fork, 0));
+  }
   // a single double layer runs the SL+DL sums with zero charges (their records
   // hold zeros there; 1 of 9 or 14 operations), several the forward form
   if constexpr (ND > 1)
     EB_CUDA(start(tree_near_dl_kernel<T, ND>, dim3(g.ntasks), 32, (size_t)kCell * kQ * rec_slots(0, ND) * 4 * sizeof(T),
-                  side.st, d, g.tasks, g.nmesh));
+                  near, d, g.tasks, g.nmesh));
   else
-    EB_CUDA(start(tree_near_kernel<T, ND ? 1 : NSL, ND>, dim3(g.ntasks), 32, near_smem<T, ND ? 1 : NSL, ND>(), side.st, d,
+    EB_CUDA(start(tree_near_kernel<T, ND ? 1 : NSL, ND>, dim3(g.ntasks), 32, near_smem<T, ND ? 1 : NSL, ND>(), near, d,
                   g.tasks, g.nmesh));
+  if (!g.expansions) return EB_OK;
   EB_CUDA(cudaEventRecord(side.join, side.st));
   EB_CUDA(start(tree_p2m_kernel<P, NSL, PD>, dim3(g.ncells, ND > 1 ? ND : 1), 32 * kCellWarps, p2m_smem<P, NSL, PD>(), st,
                 d, g.cells, g.nmesh, one, many, tab));
@@ -1284,11 +1281,13 @@ bool tree_variant(int nsl, int nd)
   return nd == 0 ? nsl == 1 || nsl == 3 || nsl == 4 : nsl == 0 ? nd == 1 || nd == 4 : nsl == 1 && nd == 1;
 }
 
-int launch_variant(bool fp32, int nsl, int nd, const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one,
-                   const ApplyArgs* many, int device, const TreeSide& side, cudaStream_t st)
+}  // namespace
+
+int tree_launch(bool fp32, int nsl, int nd, const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one,
+                const ApplyArgs* many, int device, const TreeSide& side, cudaStream_t st)
 {
-  TreeTables tab;
-  EB_CHECK(tables_for(device, fp32 ? kTreeOrder32 : kTreeOrder64, &tab));
+  TreeTables tab = {};
+  if (g.expansions) EB_CHECK(tables_for(device, fp32 ? kTreeOrder32 : kTreeOrder64, &tab));
 #define EB_TREE(NSL, ND)                                                                        \
   if (nsl == NSL && nd == ND)                                                                   \
     return fp32 ? launch_all<kTreeOrder32, float, NSL, ND>(d, g, one, many, tab, side, st)            \
@@ -1303,28 +1302,18 @@ int launch_variant(bool fp32, int nsl, int nd, const TreeDesc* d, const TreeGrid
   return set_error(EB_ERR_INVALID, "no tree far field for this operator combination");
 }
 
-}  // namespace
-
-// Smallest mesh (cells) that takes the tree.
-#ifndef EB_TREE_MIN32
-#define EB_TREE_MIN32 256
-#endif
-#ifndef EB_TREE_MIN64
-#define EB_TREE_MIN64 320
-#endif
-
-bool tree_eligible(Mesh* m, bool fp32, int nsl, int nd)
+void tree_prepare(Mesh* m)
 {
   const HostMesh& h = m->h;
-  if (m->plan.engine != 4 || !tree_variant(nsl, nd) || h.Q != kSymRule || h.K != kSymRule || h.nchunk != 1 ||
-      h.ncells < (fp32 ? EB_TREE_MIN32 : EB_TREE_MIN64))
-    return false;
-  if (!m->tree) {
-    auto t = std::make_shared<TreeMesh>();
-    t->usable = make_tree_plan(h, &t->plan);
-    m->tree = t;
-  }
-  return m->tree->usable;
+  if (h.Q != kSymRule || h.K != kSymRule || h.nchunk != 1) return;
+  m->tree = std::make_shared<TreeMesh>();
+  m->tree->usable = make_tree_plan(h, &m->tree->plan);
+}
+
+bool tree_eligible(const Mesh* m, bool fp32, int nsl, int nd)
+{
+  return m->plan.engine == 4 && m->tree && m->tree->usable && tree_variant(nsl, nd) &&
+         (fp32 || m->h.ncells >= kTreeMinCells64);
 }
 
 static int upload_lists(TreeMesh* t)
@@ -1339,8 +1328,7 @@ static int upload_lists(TreeMesh* t)
     return at;
   };
   const size_t ball = add(p.ball), has = add(p.has_local), tasks = add(p.sym.tasks), entries = add(p.sym.entries),
-               slots = add(p.sym.slot_off), ftasks = add(p.fwd.tasks), fentries = add(p.fwd.entries),
-               fslots = add(p.fwd.slot_off);
+               slots = add(p.sym.slot_off);
   struct At {
     size_t tgt, ptr, src;
   };
@@ -1361,9 +1349,6 @@ static int upload_lists(TreeMesh* t)
   d.tasks = reinterpret_cast<const int4*>(q + tasks);
   d.entries = reinterpret_cast<const int2*>(q + entries);
   d.slot_off = reinterpret_cast<const int*>(q + slots);
-  t->fwd_tasks = reinterpret_cast<const int4*>(q + ftasks);
-  t->fwd_entries = reinterpret_cast<const int2*>(q + fentries);
-  t->fwd_slot_off = reinterpret_cast<const int*>(q + fslots);
   for (int s = 0; s < kTreePasses; s++) {
     d.up[s] = dev(up[s]);
     d.nup[s] = (int)p.up[s].tgt.size();
@@ -1400,39 +1385,97 @@ static bool tree_forward(int nd) { return nd > 1; }
 
 long long tree_far_slots(const Mesh* m, int nd)
 {
-  const TreePlan& p = m->tree->plan;
-  return (long long)(tree_forward(nd) ? p.fwd : p.sym).slot_off.back() * kCell;
+  const TreeMesh& t = *m->tree;
+  return (long long)(tree_forward(nd) ? t.fwd : t.plan.sym).slot_off.back() * kCell;
+}
+
+static int upload_forward(TreeMesh* t)
+{
+  if (t->fwd_lists.p) return EB_OK;
+  TreeNear& f = t->fwd;
+  make_near_lists(t->plan, false, &f);
+  const size_t a = f.tasks.size() * sizeof(int4), b = f.entries.size() * sizeof(int2), c = f.slot_off.size() * sizeof(int);
+  std::vector<unsigned char> host(a + b + c);
+  std::memcpy(host.data(), f.tasks.data(), a);
+  std::memcpy(host.data() + a, f.entries.data(), b);
+  std::memcpy(host.data() + a + b, f.slot_off.data(), c);
+  EB_CHECK(t->fwd_lists.alloc(host.size()));
+  return copy_h2d(t->fwd_lists.p, host.data(), host.size());
+}
+
+int tree_tables(bool fp32, int device)
+{
+  TreeTables tab;
+  return tables_for(device, fp32 ? kTreeOrder32 : kTreeOrder64, &tab);
+}
+
+size_t tree_expansion_bytes(const Mesh* m, int order, int cols)
+{
+  return m->tree->plan.all_close ? 0 : sizeof(double2) * (size_t)cols * m->tree->plan.nnodes * tree_pairs(order);
+}
+
+// A double layer alone leaves the single layer's column unused.
+static int slot_columns(int nsl, int nd) { return nd == 1 ? 2 : nsl + nd; }
+
+size_t tree_partial_bytes(const Mesh* m, int nsl, int nd)
+{
+  return sizeof(double) * (size_t)slot_columns(nsl, nd) * tree_far_slots(m, nd);
+}
+
+int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, void* local, double* partial,
+              TreeDesc* out)
+{
+  TreeMesh* t = m->tree.get();
+  EB_CHECK(upload_lists(t));
+  TreeDesc d = t->base;
+  if (tree_forward(nd)) {
+    EB_CHECK(upload_forward(t));
+    d.tasks = t->fwd_lists.as<int4>();
+    d.entries = reinterpret_cast<const int2*>(d.tasks + t->fwd.tasks.size());
+    d.slot_off = reinterpret_cast<const int*>(d.entries + t->fwd.entries.size());
+    d.ntasks = (int)t->fwd.tasks.size();
+  }
+  d.far = mesh_far_desc(m, fp32, nsl, nd, rec, partial);
+  d.pos = m->pos64.as<dq>();
+  d.multipole = static_cast<double2*>(multipole);
+  d.local = static_cast<double2*>(local);
+  d.partial = partial;
+  d.first_col = slot_columns(nsl, nd) - nsl - nd;
+  *out = d;
+  return EB_OK;
+}
+
+size_t tree_bytes(const Mesh* m)
+{
+  if (!m->tree) return 0;
+  size_t b = m->tree->lists.bytes + m->tree->fwd_lists.bytes;
+  for (const auto& s : m->tree->scratch)
+    b += s.second->multipole.bytes + s.second->local.bytes + s.second->partial.bytes + s.second->desc.bytes;
+  return b;
+}
+
+void tree_release_scratch(Mesh* m)
+{
+  if (m->tree) m->tree->scratch.clear();
 }
 
 int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream_t st)
 {
   TreeMesh* t = m->tree.get();
-  EB_CHECK(upload_lists(t));
-  EB_CHECK(t->side.create());
+  if (!t->plan.all_close) EB_CHECK(t->side.create());
   std::unique_ptr<TreeScratch>& sc = t->scratch[(fp32 ? 64 : 0) + nsl * 5 + nd];
   if (!sc) {
     auto s = std::make_unique<TreeScratch>();
-    const int cols = nsl + nd, slot_cols = nd == 1 ? 2 : cols;  // a DL alone leaves the SL column unused
-    const size_t bytes = sizeof(double2) * (size_t)cols * t->plan.nnodes * tree_pairs(fp32 ? kTreeOrder32 : kTreeOrder64);
-    EB_CHECK(s->multipole.alloc(bytes));
-    EB_CHECK(s->local.alloc(bytes));
-    EB_CHECK(s->partial.alloc(sizeof(double) * (size_t)slot_cols * tree_far_slots(m, nd)));
-    TreeDesc d = t->base;
-    if (tree_forward(nd)) {
-      d.tasks = t->fwd_tasks;
-      d.entries = t->fwd_entries;
-      d.slot_off = t->fwd_slot_off;
-      d.ntasks = (int)t->plan.fwd.tasks.size();
+    if (tree_forward(nd)) EB_CHECK(upload_forward(t));  // its slots are counted below
+    const size_t bytes = tree_expansion_bytes(m, fp32 ? kTreeOrder32 : kTreeOrder64, nsl + nd);
+    if (bytes) {
+      EB_CHECK(s->multipole.alloc(bytes));
+      EB_CHECK(s->local.alloc(bytes));
     }
-    d.first_col = slot_cols - cols;
-    d.far = mesh_far_desc(m, fp32, nsl, nd, m->rec.p, s->partial.as<double>());
-    d.pos = m->pos64.as<dq>();
-    d.multipole = s->multipole.as<double2>();
-    d.local = s->local.as<double2>();
-    d.partial = s->partial.as<double>();
-    EB_CHECK(s->desc.alloc(sizeof d));
-    EB_CHECK(copy_h2d(s->desc.p, &d, sizeof d));
-    s->host = d;
+    EB_CHECK(s->partial.alloc(tree_partial_bytes(m, nsl, nd)));
+    EB_CHECK(tree_desc(m, fp32, nsl, nd, m->rec.p, s->multipole.p, s->local.p, s->partial.as<double>(), &s->host));
+    EB_CHECK(s->desc.alloc(sizeof(TreeDesc)));
+    EB_CHECK(copy_h2d(s->desc.p, &s->host, sizeof(TreeDesc)));
     sc = std::move(s);
   }
   const TreeDesc& d = sc->host;
@@ -1442,9 +1485,10 @@ int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream
   g.ncells = d.ncells;
   g.nm2l = d.nm2l;
   g.ntasks = d.ntasks;
+  g.expansions = !t->plan.all_close;
   std::copy_n(d.nup, kTreePasses, g.nup);
   if (m->profile) EB_CUDA(cudaEventRecord(m->ev0, st));
-  return launch_variant(fp32, nsl, nd, sc->desc.as<TreeDesc>(), g, *A, nullptr, m->device, t->side, st);
+  return tree_launch(fp32, nsl, nd, sc->desc.as<TreeDesc>(), g, *A, nullptr, m->device, t->side, st);
 }
 
 }  // namespace eb

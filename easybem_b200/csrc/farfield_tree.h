@@ -70,26 +70,54 @@ struct TreeSide {
   int create();  // no-op when made
 };
 
-// A mesh's tree, made on the first apply that takes it.
+// Block counts of each kernel over the meshes of a launch and, for more than
+// one mesh, the first block of each (device).
+struct TreeGrid {
+  int nmesh = 1;
+  const int *cells = nullptr, *m2l = nullptr, *tasks = nullptr, *up[kTreePasses] = {};
+  int ncells = 0, nm2l = 0, ntasks = 0, nup[kTreePasses] = {};
+  bool expansions = true;
+};
+
+// A mesh's tree: the plan of a new mesh, the rest with the first apply.
 struct TreeMesh {
   bool usable = false;
   TreePlan plan;
   DevBuf lists;  // one allocation
   TreeDesc base; // static pointers
-  const int4* fwd_tasks;      // TreePlan::fwd
-  const int2* fwd_entries;
-  const int* fwd_slot_off;
+  // close pairs in forward order, made with the first variant that needs them
+  TreeNear fwd;
+  DevBuf fwd_lists;
   TreeSide side;
   std::map<int, std::unique_ptr<TreeScratch>> scratch;
 };
 
-// True when mesh m applies this far-field variant through the tree; makes the
-// tree (host work and one upload) the first time the rules allow it.
-bool tree_eligible(Mesh* m, bool fp32, int nsl, int nd);
+// The tree of mesh m when its size allows one (host work, done while the GPU
+// computes the near field of a new mesh).
+void tree_prepare(Mesh* m);
+// True when mesh m applies this far-field variant through the tree.
+bool tree_eligible(const Mesh* m, bool fp32, int nsl, int nd);
 // The far field of mesh m: expansions and close pairs into the partial slots
 // (A.partial and A.slot_off are set for the finalize).
 int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream_t st);
 // Partial slots (summed over the rows, per output).
 long long tree_far_slots(const Mesh* m, int nd);
+// Descriptor of mesh m for one variant over the given scratch (tree_scratch_bytes);
+// uploads the mesh's lists the first time.
+int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, void* local, double* partial,
+              TreeDesc* out);
+// Bytes of one of the two expansion buffers, and of the partial slots.
+size_t tree_expansion_bytes(const Mesh* m, int order, int cols);
+size_t tree_partial_bytes(const Mesh* m, int nsl, int nd);
+// The kernels of the meshes of g: descriptors d, arguments one (a single mesh)
+// or many (device).
+int tree_launch(bool fp32, int nsl, int nd, const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one,
+                const ApplyArgs* many, int device, const TreeSide& side, cudaStream_t st);
+// Makes the constant tables that a launch needs (before a stream capture).
+int tree_tables(bool fp32, int device);
+// Device bytes of the mesh's tree and its single-mesh scratch; gives the
+// scratch back (no work on the mesh in flight).
+size_t tree_bytes(const Mesh* m);
+void tree_release_scratch(Mesh* m);
 
 }  // namespace eb

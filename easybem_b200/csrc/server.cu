@@ -32,6 +32,8 @@
 #include <vector>
 
 #include "solver.h"
+#include "farfield_sym.h"
+#include "farfield_tree.h"
 
 eb::Mesh* eb_mesh_internal(eb_mesh handle);
 
@@ -52,7 +54,16 @@ static size_t mesh_resident_bytes(const Mesh* m)
                           &m->dl_col, &m->dl_val, &m->rec, &m->partial, &m->counter, &m->items, &m->io_t,
                           &m->io_u, &m->io_v, &m->io_q, &m->pc_val};
   for (const DevBuf* d : bufs) b += d->bytes;
-  return b;
+  return b + tree_bytes(m);
+}
+
+// Device bytes of the solver entries' far-field scratch for nrhs right-hand sides.
+static size_t batch_far_bytes(const Mesh* m, int nrhs)
+{
+  const size_t entries = ((size_t)nrhs + kBatchCols - 1) / kBatchCols;
+  if (tree_eligible(m, true, kBatchCols, 0))
+    return entries * (2 * tree_expansion_bytes(m, kTreeOrder64, kBatchCols) + tree_partial_bytes(m, kBatchCols, 0));
+  return sym_eligible(m, true, kBatchCols, 0) ? entries * sym_slot_bytes(m->h, kBatchCols) : 0;
 }
 
 // Estimate before the mesh exists: ~13 near pairs per triangle (SL + DL CSR
@@ -66,7 +77,12 @@ static size_t estimate_bytes(int nv, int ne, int order, int nrhs, int restart)
   const size_t solver = (size_t)nrhs * ne * 8 * (restart + 4) + ((size_t)nrhs + 3) / 4 * ne * (Q * 64 + 160);
   // the symmetric far field's partial slots: kBatchCols outputs per 128-triangle tile and row
   const size_t slots = (size_t)kBatchCols * (((size_t)ne + kTT - 1) / kTT + 1) * ne * 8;
-  return mesh + solver + slots;
+  // the tree's expansions (two buffers of two nodes per cell) and close-pair
+  // slots (~30 per cell), per group of kBatchCols right-hand sides
+  const size_t cells = ((size_t)ne + kCell - 1) / kCell;
+  const size_t tree = ((size_t)nrhs + 3) / 4 * kBatchCols * cells *
+                      (2 * 2 * tree_pairs(kTreeOrder64) * sizeof(double2) + 30 * kCell * sizeof(double));
+  return mesh + solver + std::max(slots, Q == kSymRule ? tree : 0);
 }
 
 struct Request {
@@ -329,6 +345,7 @@ class Server {
         b.resize((size_t)r->nrhs * r->ne);
         rc = eb_dirichlet_rhs_prec(m, opt_.rhs_precision, r->nrhs, r->g.data(), b.data());
       }
+      if (m) tree_release_scratch(eb_mesh_internal(m));  // the solver's entries have their own
       const double t2 = now_ms();
       if (rc == EB_OK && opt_.precond) rc = ensure_near_precond(eb_mesh_internal(m));
       const double t3 = now_ms();
@@ -353,9 +370,7 @@ class Server {
       // replace the estimate by the measured footprint
       const size_t actual = mesh_resident_bytes(eb_mesh_internal(m)) +
                             (size_t)r->nrhs * pool_.device_bytes_per_system(eb_mesh_internal(m)) +
-                            (sym_eligible(eb_mesh_internal(m), true, kBatchCols, 0)
-                                 ? sym_slot_bytes(eb_mesh_internal(m)->h, kBatchCols)
-                                 : 0);
+                            batch_far_bytes(eb_mesh_internal(m), r->nrhs);
       used_ = used_ - r->bytes + actual;
       r->bytes = actual;
       r->mesh = m;

@@ -46,13 +46,85 @@ dq ball_of(const std::vector<dq>& cell, int lo, int hi)
   return best;
 }
 
+// True when the centre of node k keeps kTreeMinStep of its radius from those of
+// node j and its descendants.
+bool clear_of(const std::vector<Node>& nodes, const std::vector<dq>& ball, int k, int j)
+{
+  const dq &x = ball[k], &y = ball[j];
+  const d3 v = mk3(x.x - y.x, x.y - y.y, x.z - y.z);
+  const double s = kTreeMinStep * x.w;
+  if (dot3(v, v) < s * s) return false;
+  return nodes[j].left < 0 || (clear_of(nodes, ball, k, nodes[j].left) && clear_of(nodes, ball, k, nodes[j].right));
+}
+
+// Pairs (c, j) as rows c of ascending j.
+struct Rows {
+  std::vector<int> ptr, col;
+  Rows(int n, const std::vector<std::pair<int, int>>& pairs, bool both) : ptr(n + 1, 0)
+  {
+    for (const auto& q : pairs) {
+      ptr[q.first + 1]++;
+      if (both) ptr[q.second + 1]++;
+    }
+    for (int k = 0; k < n; k++) ptr[k + 1] += ptr[k];
+    std::vector<int> fill(ptr.begin(), ptr.end() - 1);
+    col.resize(ptr[n]);
+    for (const auto& q : pairs) {
+      col[fill[q.first]++] = q.second;
+      if (both) col[fill[q.second]++] = q.first;
+    }
+    for (int k = 0; k < n; k++) std::sort(col.begin() + ptr[k], col.begin() + ptr[k + 1]);
+  }
+};
+
 }  // namespace
+
+void make_near_lists(const TreePlan& plan, bool both, TreeNear* out)
+{
+  // transposed slots first, then one forward slot per task, then the far slot
+  const int nc = plan.ncells;
+  const Rows close(nc, plan.near, !both);
+  const int pairs = nc + (int)close.col.size();
+  const int chunk = std::min(kTreeNearChunk, std::max(1, pairs / kTreeNearTasks));
+  const int far_slots = plan.all_close ? 0 : 1;
+  std::vector<int> trans(nc, 0);
+  if (both)
+    for (int j : close.col) trans[j]++;
+  out->slot_off.assign(nc + 1, 0);
+  for (int c = 0; c < nc; c++)
+    out->slot_off[c + 1] =
+        out->slot_off[c] + trans[c] + (close.ptr[c + 1] - close.ptr[c] + chunk) / chunk + far_slots;
+  std::vector<int> next(out->slot_off.begin(), out->slot_off.end() - 1);
+  out->entries.reserve(close.col.size() + nc);
+  for (int c = 0; c < nc; c++) {
+    const int e0 = (int)out->entries.size();
+    out->entries.push_back(make_int2(c, -1));
+    for (int q = close.ptr[c]; q < close.ptr[c + 1]; q++)
+      out->entries.push_back(make_int2(close.col[q], both ? next[close.col[q]]++ : -1));
+    const int e1 = (int)out->entries.size();
+    int slot = out->slot_off[c] + trans[c];
+    for (int e = e0; e < e1; e += chunk)
+      out->tasks.push_back(make_int4(c, e, std::min(e1, e + chunk), slot++));
+  }
+  // the larger tasks first
+  std::stable_sort(out->tasks.begin(), out->tasks.end(),
+                   [](const int4& a, const int4& b) { return a.z - a.y > b.z - b.y; });
+}
 
 bool make_tree_plan(const HostMesh& h, TreePlan* plan)
 {
   TreePlan& p = *plan;
   const int nc = h.ncells;
   p.ncells = nc;
+  auto all_close = [&] {
+    p.all_close = true;
+    p.near.clear();
+    for (int c = 0; c < nc; c++)
+      for (int j = c + 1; j < nc; j++) p.near.push_back({c, j});
+    make_near_lists(p, true, &p.sym);
+    return true;
+  };
+  if (nc < kTreeMinCells) return all_close();
   std::vector<Node> nodes(nc);
   for (int c = 0; c < nc; c++) nodes[c] = Node{c, c + 1, -1, -1, -1, 0};
   std::function<int(int, int)> build = [&](int lo, int hi) {
@@ -75,27 +147,25 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
   // a move scales with the inverse distance of the two centres, so an inner
   // node's centre keeps away from those of its descendants (symmetric meshes
   // put them at the same point)
-  std::function<bool(int, int)> clear = [&](int k, int j) {
-    const dq &x = p.ball[k], &y = p.ball[j];
-    const d3 v = mk3(x.x - y.x, x.y - y.y, x.z - y.z);
-    const double s = kTreeMinStep * x.w;
-    if (dot3(v, v) < s * s) return false;
-    return nodes[j].left < 0 || (clear(k, nodes[j].left) && clear(k, nodes[j].right));
-  };
   for (int k = nc; k < nn; k++) {
     const dq b = ball_of(p.ball, nodes[k].lo, nodes[k].hi);
     p.ball[k] = b;
-    for (int t = 1; t < 64 && !(clear(k, nodes[k].left) && clear(k, nodes[k].right)); t++) {
+    for (int t = 1; t < 64 && !(clear_of(nodes, p.ball, k, nodes[k].left) && clear_of(nodes, p.ball, k, nodes[k].right)); t++) {
       const double a = 2.4 * t, z = std::cos(1.7 * t), r = std::sqrt(1.0 - z * z), s = 0.004 * t * b.w;
       p.ball[k] = dq{b.x + s * r * std::cos(a), b.y + s * r * std::sin(a), b.z + s * z, b.w + s};
     }
   }
 
   // the tree against itself
-  std::vector<std::pair<int, int>> far;
-  std::vector<std::vector<int>> near(nc);  // later cells close to each cell
-  const long long limit = std::max<long long>(4 * nc, (long long)nc * nc / 16);
-  long long nnear = 0;
+  struct Far {
+    int a, b;
+    unsigned key;  // 255 - f: sorts the pairs that need most degrees first
+  };
+  std::vector<Far> far;
+  far.reserve(32 * (size_t)nc);
+  std::vector<std::pair<int, int>> near;  // close cells, the earlier one first
+  near.reserve(20 * (size_t)nc);
+  const long long limit = (long long)nc * nc / 6;
   std::vector<std::pair<int, int>> stack(1, {root, root});
   while (!stack.empty()) {
     const auto [a, b] = stack.back();
@@ -110,12 +180,13 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
     }
     const dq &x = p.ball[a], &y = p.ball[b];
     const d3 d = mk3(x.x - y.x, x.y - y.y, x.z - y.z);
-    const double s = (x.w + y.w) / kTreeTheta;
-    if (dot3(d, d) > s * s) {
-      far.push_back({a, b});
+    const double r = x.w + y.w, d2 = dot3(d, d);
+    if (d2 * (kTreeTheta * kTreeTheta) > r * r) {
+      const double share = 2.0 * std::log(kTreeTheta) / std::log(r * r / d2);
+      far.push_back({a, b, 255u - (unsigned)std::min(255.0, std::max(1.0, std::ceil(255.0 * share)))});
     } else if (A.left < 0 && B.left < 0) {
-      near[std::min(a, b)].push_back(std::max(a, b));
-      if (++nnear > limit) return false;
+      near.push_back({std::min(a, b), std::max(a, b)});
+      if ((long long)near.size() > limit) return nc <= kTreeAllCloseCells && all_close();
     } else if (B.left < 0 || (A.left >= 0 && x.w >= y.w)) {
       stack.push_back({A.left, b});
       stack.push_back({A.right, b});
@@ -125,19 +196,21 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
     }
   }
 
-  // separated pairs in both directions, by target
+  // separated pairs in both directions, by target, each list sorted by
+  // (255 - f, source)
   std::vector<int> count(nn + 1, 0);
-  for (const auto& f : far) {
-    count[f.first + 1]++;
-    count[f.second + 1]++;
+  for (const Far& f : far) {
+    count[f.a + 1]++;
+    count[f.b + 1]++;
   }
   for (int k = 0; k < nn; k++) count[k + 1] += count[k];
-  std::vector<int> fill(count.begin(), count.end() - 1), src(2 * far.size());
+  std::vector<int> fill(count.begin(), count.end() - 1);
+  std::vector<unsigned> src(2 * far.size());
   std::vector<char> used(nn, 0);  // its multipole is read
-  for (const auto& f : far) {
-    src[fill[f.first]++] = f.second;
-    src[fill[f.second]++] = f.first;
-    used[f.first] = used[f.second] = 1;
+  for (const Far& f : far) {
+    src[fill[f.a]++] = f.key << 24 | (unsigned)f.b;
+    src[fill[f.b]++] = f.key << 24 | (unsigned)f.a;
+    used[f.a] = used[f.b] = 1;
   }
   p.has_local.assign(nn, 0);
   // targets with the longest lists first (the last wave then holds short ones)
@@ -149,17 +222,11 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
     }
   std::stable_sort(order.begin(), order.end(),
                    [&](int a, int b) { return count[a + 1] - count[a] > count[b + 1] - count[b]; });
+  p.m2l.src.reserve(src.size());
   for (int k : order) {
+    std::sort(src.begin() + count[k], src.begin() + count[k + 1]);
     p.m2l.tgt.push_back(k);
-    for (int q = count[k]; q < count[k + 1]; q++) {
-      const dq &x = p.ball[k], &y = p.ball[src[q]];
-      const d3 v = mk3(x.x - y.x, x.y - y.y, x.z - y.z);
-      const double share = std::log(kTreeTheta) / std::log((x.w + y.w) / std::sqrt(dot3(v, v)));
-      const int f = std::min(255, std::max(1, (int)std::ceil(255.0 * share)));
-      p.m2l.src.push_back((int)((unsigned)f << 24 | (unsigned)src[q]));
-    }
-    std::sort(p.m2l.src.end() - (count[k + 1] - count[k]), p.m2l.src.end(),
-              [](int a, int b) { return (unsigned)a >> 24 != (unsigned)b >> 24 ? (unsigned)a >> 24 > (unsigned)b >> 24 : a < b; });
+    for (int q = count[k]; q < count[k + 1]; q++) p.m2l.src.push_back((int)((255u - (src[q] >> 24)) << 24 | (src[q] & 0xffffffu)));
     p.m2l.ptr.push_back((int)p.m2l.src.size());
   }
 
@@ -199,40 +266,8 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
     p.down.ptr.push_back((int)p.down.src.size());
   }
 
-  // close pairs: transposed slots first, then one forward slot per task, then
-  // the far slot; the larger tasks first
-  std::vector<std::vector<int>> all(nc);
-  for (int c = 0; c < nc; c++) {
-    std::sort(near[c].begin(), near[c].end());
-    for (int j : near[c]) {
-      all[c].push_back(j);
-      all[j].push_back(c);
-    }
-  }
-  auto lists = [&](const std::vector<std::vector<int>>& close, bool both, TreeNear& out) {
-    std::vector<int> trans(nc, 0);
-    if (both)
-      for (int c = 0; c < nc; c++)
-        for (int j : close[c]) trans[j]++;
-    out.slot_off.assign(nc + 1, 0);
-    for (int c = 0; c < nc; c++)
-      out.slot_off[c + 1] =
-          out.slot_off[c] + trans[c] + ((int)close[c].size() + kTreeNearChunk) / kTreeNearChunk + 1;
-    std::vector<int> next(out.slot_off.begin(), out.slot_off.end() - 1);
-    for (int c = 0; c < nc; c++) {
-      const int e0 = (int)out.entries.size();
-      out.entries.push_back(make_int2(c, -1));
-      for (int j : close[c]) out.entries.push_back(make_int2(j, both ? next[j]++ : -1));
-      const int e1 = (int)out.entries.size();
-      int slot = out.slot_off[c] + trans[c];
-      for (int e = e0; e < e1; e += kTreeNearChunk)
-        out.tasks.push_back(make_int4(c, e, std::min(e1, e + kTreeNearChunk), slot++));
-    }
-    std::stable_sort(out.tasks.begin(), out.tasks.end(),
-                     [](const int4& a, const int4& b) { return a.z - a.y > b.z - b.y; });
-  };
-  lists(near, true, p.sym);
-  lists(all, false, p.fwd);
+  p.near.swap(near);
+  make_near_lists(p, true, &p.sym);
   return true;
 }
 

@@ -8,6 +8,7 @@
 // point by point).
 #pragma once
 
+#include <utility>
 #include <vector>
 
 #include "farfield.cuh"
@@ -28,8 +29,21 @@ constexpr double kTreeMinStep = 1e-3;
 constexpr int kTreeLevelsPerPass = 3;
 constexpr int kTreePasses = 6;  // enough for 2^18 cells
 constexpr int kTreeMaxNodes = 1 << 24;
-// Close cell pairs per near task (one warp's work; the diagonal counts).
+// Close cell pairs per near task (one warp's work; the diagonal counts): at
+// most kTreeNearChunk, fewer while that leaves less than kTreeNearTasks tasks
+// (four warps on each of the 592 SM quarters).
 constexpr int kTreeNearChunk = 4;
+constexpr int kTreeNearTasks = 4 * 592;
+// Smaller meshes (cells) have no separated clusters worth an expansion: all
+// their cell pairs are close. Up to here the near tasks alone also beat the
+// symmetric kernel, whose items (a 128-triangle tile against 8 cells) leave
+// SMs idle.
+constexpr int kTreeMinCells = 100;
+constexpr int kTreeAllCloseCells = 140;
+// Least cells of an FP64 apply on the tree: below, a pair of cells (22 us on an
+// SM quarter) is too coarse a task, and the ordered-pair kernel's finer items
+// finish first (512 triangles, SL+DL: 69 us against 96; 1,200: 134 against 121).
+constexpr int kTreeMinCells64 = 28;
 
 // Expansions moved into node tgt[k] from nodes src[ptr[k] .. ptr[k + 1]). The
 // upper 8 bits of a source are the share f / 255 of the degrees that its pair
@@ -44,7 +58,7 @@ struct TreeMoves {
 // Close cell pairs. A task is (cell, first entry, last entry, slot of its
 // forward sums), an entry (other cell, slot of the transposed sums or -1); the
 // slots of cell c are slot_off[c] .. slot_off[c + 1]), the last one for the
-// far sum.
+// far sum (if there is one).
 struct TreeNear {
   std::vector<int4> tasks;
   std::vector<int2> entries;
@@ -53,17 +67,21 @@ struct TreeNear {
 
 struct TreePlan {
   int ncells = 0, nnodes = 0;  // nodes 0 .. ncells - 1 are the cells
+  bool all_close = false;      // no expansions: every cell pair in near
   std::vector<dq> ball;        // centre; radius over the quadrature points
   TreeMoves up[kTreePasses];   // multipoles of descendants into inner nodes
   TreeMoves m2l;               // multipoles of separated nodes into locals
   TreeMoves down;              // locals of the ancestors into every cell
   std::vector<char> has_local; // per node: it is a target of m2l
+  std::vector<std::pair<int, int>> near;  // close cells, the earlier one first
   TreeNear sym;  // every unordered pair of cells once
-  TreeNear fwd;  // every ordered pair
 };
 
-// False when more than an eighth of all cell pairs are close (the tree would
-// not pay): the plan is then incomplete.
+// False when more than a third of all cell pairs are close in a mesh of more
+// than kTreeAllCloseCells (the tree would not pay): the plan is then incomplete.
 bool make_tree_plan(const HostMesh& h, TreePlan* plan);
+// Tasks and slots of a plan's close pairs: every unordered pair once (both),
+// or every ordered pair.
+void make_near_lists(const TreePlan& plan, bool both, TreeNear* out);
 
 }  // namespace eb

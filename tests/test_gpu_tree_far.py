@@ -123,7 +123,7 @@ def test_meshes_without_separated_clusters_keep_the_direct_sum(gpu_lib):
             assert np.array_equal(v, w) and np.array_equal(q, r)
 
 
-def test_tree_follows_plan_changes_and_small_meshes_stay_direct(gpu_lib):
+def test_tree_follows_plan_changes(gpu_lib):
     nodes, elems = meshes.torus(170, 0.3)
     t, u = _vectors(nodes, elems, 6)
     with gpu_lib.Mesh(nodes, elems) as m:
@@ -131,6 +131,33 @@ def test_tree_follows_plan_changes_and_small_meshes_stay_direct(gpu_lib):
         m.set_plan(64)  # releases the records that the tree's descriptors point to
         w, r = m.apply_sl_dl(t, u)
         assert np.array_equal(v, w) and np.array_equal(q, r)
-    nodes, elems = meshes.icosphere(3)
+
+
+@pytest.mark.parametrize("ne", [1, 31, 32, 33, 127, 864, 865, 1280, 3199, 3201, 4000])
+def test_small_meshes_sum_all_cell_pairs(gpu_lib, oracle, ne):
+    """Cells that all lie close: one cell, whole and ragged last cells, both
+    sides of the smallest tree."""
+    oracle.set_order(4)
+    nodes, elems = meshes.torus(100, 0.3)
+    nodes, elems = _cut(nodes, elems, ne)
+    t, u = _vectors(nodes, elems, ne)
+    rows = np.sort(np.random.default_rng(1).choice(ne, min(ne, 64), replace=False)).astype(np.int32)
+    vo, qo = oracle.apply_rows(nodes, elems, t, u, rows)
+    g = np.stack([u, u[::-1], 2 * u])
     with gpu_lib.Mesh(nodes, elems) as m:
-        assert m.far_engine("mixed") == "sym" and m.far_engine("fp64") == "cuda"
+        if ne < 3200:
+            assert m.far_engine("mixed") == "sym" and m.far_engine("fp64") == ("sym" if ne > 27 * 32 else "cuda")
+        for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL)):
+            m.set_far_engine("tree")
+            v, q = m.apply_sl_dl(t, u, precision=prec)
+            vs, qs, b, d = m.apply_sl(t, prec), m.apply_dl(u, prec), m.dirichlet_rhs(g, prec), m.apply_hypersingular(u, prec)
+            assert rel_l2(v[rows], vo) < tol and rel_l2(vs[rows], vo) < tol
+            m.set_far_engine("cuda")
+            w, r = m.apply_sl_dl(t, u, precision=prec)
+            c, e = m.dirichlet_rhs(g, prec), m.apply_hypersingular(u, prec)
+            if ne == 1:  # no pair but the triangle with itself: K u = 0
+                assert not q.any() and not qs.any() and not r.any()
+            else:
+                assert rel_l2(q[rows], qo) < tol and rel_l2(qs[rows], qo) < tol
+                assert rel_l2(d, e) < 10 * tol
+            assert rel_l2(b, c) < tol
