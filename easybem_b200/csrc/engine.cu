@@ -792,6 +792,18 @@ int mesh_check_far_error(Mesh* m)
   return set_error(EB_ERR_TIMEOUT, "tensor-core far field: a bounded wait for the tensor cores ran out");
 }
 
+// Scratch sized once for the largest variant, so device pointers captured in
+// descriptors (and in CUDA graphs) stay valid.
+int ensure_apply_scratch(Mesh* m)
+{
+  const HostMesh& h = m->h;
+  if (!m->rec.p) {
+    EB_CHECK(m->rec.alloc((size_t)h.ne * h.Q * kMaxRecSlots * sizeof(dq)));
+    EB_CHECK(m->partial.alloc(sizeof(double) * (size_t)kMaxOutputs * m->plan.nsplit * h.nitems));
+  }
+  return EB_OK;
+}
+
 int mesh_apply(Mesh* m, int precision, int nsl, int nd, const double* d_t, const double* d_u, double* d_v,
                double* d_q, cudaStream_t st)
 {
@@ -803,12 +815,7 @@ int mesh_apply(Mesh* m, int precision, int nsl, int nd, const double* d_t, const
   if (!far_variant_supported(nsl, nd)) return set_error(EB_ERR_INVALID, "unsupported operator combination");
   if ((nsl > 0 && (!d_t || !d_v)) || (dl && (!d_u || !d_q))) return set_error(EB_ERR_INVALID, "null vector");
   const int nrec = rec_slots(nsl, nd);
-  // Scratch sized once for the largest variant, so device pointers captured
-  // in descriptors (and in CUDA graphs) stay valid.
-  if (!m->rec.p) {
-    EB_CHECK(m->rec.alloc((size_t)h.ne * h.Q * kMaxRecSlots * sizeof(dq)));
-    EB_CHECK(m->partial.alloc(sizeof(double) * (size_t)kMaxOutputs * m->plan.nsplit * h.nitems));
-  }
+  EB_CHECK(ensure_apply_scratch(m));
   Mesh::Variant& var = m->variants[(fp32 ? 64 : 0) + nsl * 5 + nd];
   if (!var.desc.p) {
     const FarMeshDesc desc = mesh_far_desc(m, fp32, nsl, nd, m->rec.p, m->partial.as<double>());
@@ -1124,8 +1131,13 @@ int eb_evaluate_potential(eb_mesh mesh, int precision, int npts, const double* p
   EB_CUDA(cudaMemcpyAsync(m->io_t.p, t, sizeof(double) * ne, cudaMemcpyHostToDevice, st));
   EB_CUDA(cudaMemcpyAsync(m->io_u.p, u, sizeof(double) * nv, cudaMemcpyHostToDevice, st));
   EB_CUDA(cudaMemcpyAsync(m->io_pts.p, pts, sizeof(double) * 3 * (size_t)npts, cudaMemcpyHostToDevice, st));
-  EB_CHECK(eb::mesh_evaluate_potential(m, precision, npts, m->io_pts.as<double>(), m->io_t.as<double>(),
-                                       m->io_u.as<double>(), m->io_pot.as<double>(), st));
+  if ((precision == EB_PREC_MIXED || precision == EB_PREC_FP64) &&
+      eb::tree_points_eligible(m, precision == EB_PREC_MIXED, npts))
+    EB_CHECK(eb::tree_evaluate(m, precision == EB_PREC_MIXED, npts, pts, m->io_pts.as<double>(), m->io_t.as<double>(),
+                               m->io_u.as<double>(), m->io_pot.as<double>(), st));
+  else
+    EB_CHECK(eb::mesh_evaluate_potential(m, precision, npts, m->io_pts.as<double>(), m->io_t.as<double>(),
+                                         m->io_u.as<double>(), m->io_pot.as<double>(), st));
   EB_CUDA(cudaMemcpyAsync(out, m->io_pot.p, sizeof(double) * (size_t)npts, cudaMemcpyDeviceToHost, st));
   EB_CUDA(cudaStreamSynchronize(st));
   return EB_OK;

@@ -189,6 +189,10 @@ int ensure_tc_static(Mesh* m);
 // EB_ERR_TIMEOUT (and the flag cleared) if the last tensor-core launch on m
 // gave up a bounded wait; EB_OK otherwise. The stream must be synchronised.
 int mesh_check_far_error(Mesh* m);
+// The record and partial-sum scratch of single-mesh calls.
+int ensure_apply_scratch(Mesh* m);
+// The mixed potential evaluation sums cells within this many radii of a point in FP64.
+constexpr double kPotNear = 2.5;
 // Device-pointer apply: t has nsl columns (stride ne), v likewise; u has nd
 // DL columns (stride nnodes), q likewise (stride ne).
 int mesh_apply(Mesh* m, int precision, int nsl, int nd, const double* d_t, const double* d_u, double* d_v,

@@ -39,6 +39,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "farfield_sym_eval.cuh"
 
@@ -367,9 +368,10 @@ __global__ void __launch_bounds__(MoveShape<P, NC>::kThreads, MoveShape<P, NC>::
 #pragma unroll 1
   for (int first = mv.ptr[node]; first < end; first += kBatch) {
     const bool on = first + vec < end;
-    // the list is sorted by the order its pairs need: the first one decides
-    const int order = ((P + 1) * (int)((unsigned)mv.src[first] >> 24) + 254) / 255 - 1;
-    const int src = mv.src[on ? first + vec : first] & 0xffffff;
+    const int entry = mv.src[on ? first + vec : first];
+    // the batch runs to the highest order that one of its pairs needs
+    const int order = ((P + 1) * (int)__reduce_max_sync(0xffffffffu, (unsigned)entry >> 24) + 254) / 255 - 1;
+    const int src = entry & 0xffffff;
     const dq bs = d.ball[src];
     const double2* a = from + (size_t)src * kPairs;
     // the vector that becomes the z axis: from the source's centre to the
@@ -544,8 +546,9 @@ __device__ __forceinline__ void each_harmonic(const TreeTables& tab, const CellP
 }
 
 // Multipoles of one cell: NSL single-layer columns (they share sum_b w_b J
-// R(y_b)), and for ND = 1 the double-layer column blockIdx.y.
-template <int P, int NSL, int ND>
+// R(y_b)), and for ND = 1 the double-layer column blockIdx.y. DIFF: one
+// column, single minus double layer (the representation formula).
+template <int P, int NSL, int ND, bool DIFF = false>
 __global__ void __launch_bounds__(32 * kCellWarps)
     tree_p2m_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh, ApplyArgs one,
                     const ApplyArgs* __restrict__ many, TreeTables tab)
@@ -630,9 +633,10 @@ __global__ void __launch_bounds__(32 * kCellWarps)
   const size_t cstride = (size_t)d.nnodes * kPairs;
   double2* out = d.multipole + (size_t)cell * kPairs;
   for (int i = threadIdx.x; i < kPairs; i += 32 * kCellWarps) {
+    if constexpr (!DIFF)
 #pragma unroll
-    for (int c = 0; c < NSL; ++c)
-      out[c * cstride + i] = make_double2(s_sum[2 * c * kPairs + i], s_sum[(2 * c + 1) * kPairs + i]);
+      for (int c = 0; c < NSL; ++c)
+        out[c * cstride + i] = make_double2(s_sum[2 * c * kPairs + i], s_sum[(2 * c + 1) * kPairs + i]);
     if constexpr (ND > 0) {
       // (n.grad) R_n^m from the moments G^k = sum s n_k R of degree n - 1
       const double* g = s_sum + 2 * NSL * kPairs;
@@ -668,7 +672,8 @@ __global__ void __launch_bounds__(32 * kCellWarps)
         ar /= rho;
         ai /= rho;
       }
-      out[((size_t)NSL + blockIdx.y) * cstride + i] = make_double2(ar, ai);
+      if constexpr (DIFF) out[i] = make_double2(s_sum[i] - ar, s_sum[kPairs + i] - ai);
+      else out[((size_t)NSL + blockIdx.y) * cstride + i] = make_double2(ar, ai);
     }
   }
 }
@@ -1281,6 +1286,502 @@ bool tree_variant(int nsl, int nd)
   return nd == 0 ? nsl == 1 || nsl == 3 || nsl == 4 : nsl == 0 ? nd == 1 || nd == 4 : nsl == 1 && nd == 1;
 }
 
+// ---------------------------------------------------------------------------
+// Potentials at points off the surface: groups of at most 32 points, each from
+// one cube of an octree along a Hilbert curve, take the separated nodes through
+// local expansions of their own (the combination V t - W u as one column) and
+// the close cells point by point: in FP64, in a mixed evaluation in FP32 unless
+// the point lies within kPotNear radii of the cell (the rule of the direct
+// evaluation).
+
+constexpr int kGroup = 32;
+constexpr int kCurveBits = 7;  // per dimension: two 11-bit passes of the host's radix sort
+
+// Position of every point on the Hilbert curve through 2^kCurveBits cells per
+// side (J. Skilling, "Programming the Hilbert curve", AIP Conf. Proc. 707
+// (2004) 381); points outside or not finite go to the nearest side or 0.
+__global__ void curve_kernel(int n, const double* __restrict__ pts, double ox, double oy, double oz, double inv,
+                             unsigned* __restrict__ code)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double top = (1 << kCurveBits) - 1;
+  const double o[3] = {ox, oy, oz};
+  unsigned x[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double v = (pts[3 * (size_t)i + d] - o[d]) * inv;
+    x[d] = v > 0.0 ? (unsigned)fmin(v, top) : 0u;
+  }
+#pragma unroll
+  for (unsigned q = 1u << (kCurveBits - 1); q > 1; q >>= 1) {
+    const unsigned p = q - 1;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      if (x[d] & q) {
+        x[0] ^= p;
+      } else {
+        const unsigned t = (x[0] ^ x[d]) & p;
+        x[0] ^= t;
+        x[d] ^= t;
+      }
+    }
+  }
+  x[1] ^= x[0];
+  x[2] ^= x[1];
+  unsigned t = 0;
+#pragma unroll
+  for (unsigned q = 1u << (kCurveBits - 1); q > 1; q >>= 1)
+    if (x[2] & q) t ^= q - 1;
+  unsigned c = 0;
+#pragma unroll
+  for (int b = kCurveBits - 1; b >= 0; --b)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) c = c << 1 | ((x[d] ^ t) >> b & 1);
+  code[i] = c;
+}
+
+// Ball of every group (one warp each): box centre, largest distance, at least
+// min_radius (points that coincide).
+__global__ void group_ball_kernel(int ngroups, const int* __restrict__ gptr, const double* __restrict__ pts,
+                                  const int* __restrict__ perm, double min_radius, dq* __restrict__ ball)
+{
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (g >= ngroups) return;
+  const int i = perm[min(gptr[g] + lane, gptr[g + 1] - 1)];
+  const double p[3] = {pts[3 * (size_t)i], pts[3 * (size_t)i + 1], pts[3 * (size_t)i + 2]};
+  double c[3], r2 = 0.0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    double lo = p[d], hi = p[d];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    c[d] = 0.5 * (lo + hi);
+    r2 += (p[d] - c[d]) * (p[d] - c[d]);
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(0xffffffffu, r2, o));
+  if (lane == 0) ball[g] = dq{c[0], c[1], c[2], fmax(sqrt(r2) * (1.0 + 1e-12), min_radius)};
+}
+
+constexpr int kPointCells = 4;  // close cells of a task
+constexpr int kListWarps = 4;
+constexpr int kListStack = 1024;  // 32 nodes leave and at most 64 children enter: at most 32 (height + 1)
+static_assert(32 * (kTreePasses * kTreeLevelsPerPass + 2) <= kListStack, "stack of the deepest tree");
+
+// The tree against every group, a warp per group testing 32 nodes at a time:
+// separated nodes that have a multipole and close cells, counted (FILL false)
+// or written at the scanned offsets.
+template <bool FILL>
+__global__ void __launch_bounds__(32 * kListWarps)
+    group_lists_kernel(int ngroups, int root, int ncells, double theta, const dq* __restrict__ nodes,
+                       const char* __restrict__ formed, const int2* __restrict__ child, const dq* __restrict__ ball,
+                       int* __restrict__ far_ptr, int* __restrict__ near_ptr, int* __restrict__ task_ptr,
+                       int* __restrict__ far, int* __restrict__ near)
+{
+  __shared__ int s_stack[kListWarps][kListStack];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = blockIdx.x * kListWarps + warp;
+  if (g >= ngroups) return;
+  int* stack = s_stack[warp];
+  const unsigned below = (1u << lane) - 1;
+  const dq b = ball[g];
+  int nf = FILL ? far_ptr[g] : 0, nn = FILL ? near_ptr[g] : 0, top = 1;
+  if (lane == 0) stack[0] = root;
+  __syncwarp();
+  while (top > 0) {
+    const int take = min(32, top);
+    const int k = lane < take ? stack[top - 1 - lane] : -1;
+    top -= take;
+    __syncwarp();
+    bool is_far = false, is_near = false;
+    double d2 = 0.0, r = 0.0;
+    if (k >= 0) {
+      const dq x = nodes[k];
+      const double dx = x.x - b.x, dy = x.y - b.y, dz = x.z - b.z;
+      d2 = dx * dx + dy * dy + dz * dz;
+      r = x.w + b.w;
+      is_far = formed[k] && d2 * (theta * theta) > r * r;
+      is_near = !is_far && k < ncells;
+    }
+    const bool split = k >= 0 && !is_far && !is_near;
+    const unsigned mf = __ballot_sync(0xffffffffu, is_far), mn = __ballot_sync(0xffffffffu, is_near);
+    const unsigned ms = __ballot_sync(0xffffffffu, split);
+    if (FILL && is_far) {
+      const double share = 2.0 * log(theta) / log(r * r / d2);
+      far[nf + __popc(mf & below)] = (int)((unsigned)fmin(255.0, fmax(1.0, ceil(255.0 * share))) << 24 | (unsigned)k);
+    }
+    if (FILL && is_near) near[nn + __popc(mn & below)] = k;
+    if (split) {
+      const int2 c = child[k - ncells];
+      const int at = top + 2 * __popc(ms & below);
+      stack[at] = c.x;
+      stack[at + 1] = c.y;
+    }
+    nf += __popc(mf);
+    nn += __popc(mn);
+    top += 2 * __popc(ms);
+    __syncwarp();
+  }
+  if (!FILL && lane == 0) {
+    far_ptr[g] = nf;
+    near_ptr[g] = nn;
+    task_ptr[g] = (nn + kPointCells - 1) / kPointCells;
+  }
+}
+
+// Exclusive sums of a[0, n), b[0, n) and c[0, n) in place, totals at [n] (one block).
+__global__ void __launch_bounds__(1024) scan_lists_kernel(int n, int* __restrict__ a, int* __restrict__ b,
+                                                          int* __restrict__ c)
+{
+  __shared__ int warps[3][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int* v[3] = {a, b, c};
+  int base[3] = {0, 0, 0};
+  for (int i0 = 0; i0 < n; i0 += 1024) {
+    const int i = i0 + threadIdx.x;
+    int x[3], s[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      s[k] = x[k] = i < n ? v[k][i] : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, s[k], o);
+        if (lane >= o) s[k] += y;
+      }
+      if (lane == 31) warps[k][w] = s[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      int before = base[k];
+      for (int j = 0; j < 32; ++j) {
+        if (j < w) before += warps[k][j];
+        base[k] += warps[k][j];
+      }
+      if (i < n) v[k][i] = before + s[k] - x[k];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x < 3) v[threadIdx.x][n] = base[threadIdx.x];
+}
+
+__global__ void iota_kernel(int n, int first, int* __restrict__ v)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) v[i] = first + i;
+}
+
+constexpr int kPointWarps = 4;
+
+// One close cell's sum at a point in FP64, (xs, ys, zs) relative to its centre.
+__device__ __forceinline__ double point_cell64(double xs, double ys, double zs, const dq* __restrict__ rec,
+                                               const dq* __restrict__ plane, int ns)
+{
+  double part = 0.0;
+#pragma unroll 1
+  for (int s = 0; s < ns; ++s) {
+    const dq pn = plane[s];
+    const double d = xs * pn.x + (ys * pn.y + (zs * pn.z - pn.w));
+    double sl = 0.0, acc = 0.0;
+    const dq* r = rec + (size_t)s * kQ * kNrec;
+#pragma unroll
+    for (int k = 0; k < kQ; ++k) {
+      const dq p0 = r[2 * k], p1 = r[2 * k + 1];
+      const double ex = xs + 0.5 * p0.x, ey = ys + 0.5 * p0.y, ez = zs + 0.5 * p0.z;
+      const double inv = rsq_f64(ex * ex + ey * ey + ez * ez);
+      sl += p1.y * inv;
+      acc += (inv * inv) * (p1.x * inv);
+    }
+    part += sl - d * acc;
+  }
+  return part;
+}
+
+// Close cells of the groups: a warp per task (kPointCells cells of one group),
+// a lane per point, the cells staged one at a time (F32: FP32 records; the
+// lanes close to the cell read the FP64 ones from global memory instead).
+// part[task][lane] is the task's sum.
+template <bool F32>
+__global__ void __launch_bounds__(32 * kPointWarps)
+    points_near_kernel(int ngroups, int ntasks, const int* __restrict__ gptr, const double* __restrict__ pts,
+                       const int* __restrict__ perm, const int* __restrict__ task_ptr, const int* __restrict__ near_ptr,
+                       const int* __restrict__ near, int ne, const float4* __restrict__ rec32,
+                       const float4* __restrict__ plane32, const dq* __restrict__ rec64, const dq* __restrict__ plane64,
+                       const dq* __restrict__ ccent, double* __restrict__ part_out)
+{
+  using S = typename std::conditional<F32, float4, dq>::type;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ S s_plane[kPointWarps][kCell];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int task = blockIdx.x * kPointWarps + warp;
+  if (task >= ntasks) return;  // warps are independent
+  S* s_rec = reinterpret_cast<S*>(smem_raw) + (size_t)warp * kCell * kQ * kNrec;
+  int g = 0;
+  for (int hi = ngroups; hi - g > 1;) {  // task_ptr[g] <= task < task_ptr[hi]
+    const int mid = (g + hi) >> 1;
+    if (task_ptr[mid] <= task) g = mid;
+    else hi = mid;
+  }
+  const int p = perm[min(gptr[g] + lane, gptr[g + 1] - 1)];
+  const double px = pts[3 * (size_t)p], py = pts[3 * (size_t)p + 1], pz = pts[3 * (size_t)p + 2];
+  const int e0 = near_ptr[g] + (task - task_ptr[g]) * kPointCells, e1 = min(near_ptr[g + 1], e0 + kPointCells);
+  double sum = 0.0;
+  float hi = 0.f, lo = 0.f;
+#pragma unroll 1
+  for (int e = e0; e < e1; ++e) {
+    const int cell = near[e], t0 = cell * kCell, ns = min(kCell, ne - t0);
+    const dq cc = ccent[cell];
+    const double xs = px - cc.x, ys = py - cc.y, zs = pz - cc.z;
+    const dq* r64 = rec64 + (size_t)t0 * kQ * kNrec;
+    if constexpr (F32) {
+      for (int i = lane; i < ns * kQ * kNrec; i += 32) s_rec[i] = rec32[(size_t)t0 * kQ * kNrec + i];
+      if (lane < ns) s_plane[warp][lane] = plane32[t0 + lane];
+      __syncwarp();
+      if (xs * xs + ys * ys + zs * zs < kPotNear * kPotNear * cc.w * cc.w) {
+        sum += point_cell64(xs, ys, zs, r64, plane64 + t0, ns);
+      } else {
+        const float X = (float)xs, Y = (float)ys, Z = (float)zs;
+        float part = 0.f;
+#pragma unroll 1
+        for (int s = 0; s < ns; ++s) {
+          const float4 pn = s_plane[warp][s];
+          const float d = X * pn.x + (Y * pn.y + (Z * pn.z - pn.w));
+          float sl = 0.f, acc = 0.f;
+          const float4* r = s_rec + (size_t)s * kQ * kNrec;
+#pragma unroll
+          for (int k = 0; k < kQ; ++k) {
+            const float4 p0 = r[2 * k], p1 = r[2 * k + 1];
+            const float ex = X + 0.5f * p0.x, ey = Y + 0.5f * p0.y, ez = Z + 0.5f * p0.z;
+            const float inv = rsq(ex * ex + ey * ey + ez * ez);
+            sl += p1.y * inv;
+            acc += (inv * inv) * (p1.x * inv);
+          }
+          part += sl - d * acc;
+        }
+        two_sum_add(hi, lo, part);
+      }
+    } else {
+      for (int i = lane; i < ns * kQ * kNrec; i += 32) s_rec[i] = r64[i];
+      if (lane < ns) s_plane[warp][lane] = plane64[t0 + lane];
+      __syncwarp();
+      sum += point_cell64(xs, ys, zs, s_rec, s_plane[warp], ns);
+    }
+    __syncwarp();
+  }
+  part_out[(size_t)task * 32 + lane] = sum + ((double)hi + (double)lo);
+}
+
+// Potentials of one group per warp, a lane per point: the local expansion and
+// the sums of the group's tasks in order.
+template <int P>
+__global__ void __launch_bounds__(32 * kPointWarps)
+    tree_points_kernel(int ngroups, const int* __restrict__ gptr, const double* __restrict__ pts,
+                       const int* __restrict__ perm, const dq* __restrict__ ball, const double2* __restrict__ local,
+                       const int* __restrict__ task_ptr, const double* __restrict__ part_in, TreeTables tab,
+                       double* __restrict__ out)
+{
+  constexpr int kPairs = tree_pairs(P);
+  __shared__ double2 s_all[kPointWarps][kPairs];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = blockIdx.x * kPointWarps + warp;
+  if (g >= ngroups) return;  // warps are independent
+  double2* s_loc = s_all[warp];
+  for (int i = lane; i < kPairs; i += 32) s_loc[i] = local[(size_t)g * kPairs + i];
+  const bool on = gptr[g] + lane < gptr[g + 1];
+  const int p = perm[min(gptr[g] + lane, gptr[g + 1] - 1)];
+  const dq b = ball[g];
+  const double x = (pts[3 * (size_t)p] - b.x) / b.w, y = (pts[3 * (size_t)p + 1] - b.y) / b.w;
+  const double z = (pts[3 * (size_t)p + 2] - b.z) / b.w, r2 = x * x + y * y + z * z;
+  __syncwarp();
+  double sum = 0.0;
+  double dr = 1.0, di = 0.0;
+#pragma unroll 1
+  for (int m = 0; m <= P; ++m) {
+    if (m > 0) {
+      const double f = -sqrt((2.0 * m - 1.0) / (2.0 * m));
+      const double t = f * (x * dr - y * di);
+      di = f * (x * di + y * dr);
+      dr = t;
+    }
+    double r1 = dr, i1 = di, r0 = 0.0, i0 = 0.0, part = 0.0;
+#pragma unroll 4
+    for (int d = m; d <= P; ++d) {
+      const int q = tree_pair(d, m);
+      if (d > m) {
+        const double2 c = tab.rec[q];
+        const double az = c.x * z, br = c.y * r2;
+        const double tr = az * r1 - br * r0, ti = az * i1 - br * i0;
+        r0 = r1;
+        i0 = i1;
+        r1 = tr;
+        i1 = ti;
+      }
+      const double2 l = s_loc[q];
+      part += l.x * r1 + l.y * i1;
+    }
+    sum += m > 0 ? 2.0 * part : part;
+  }
+  const int end = task_ptr[g + 1];
+  for (int k = task_ptr[g]; k < end; ++k) sum += part_in[(size_t)k * 32 + lane];
+  if (on) out[p] = sum * (0.25 / M_PI);
+}
+
+// Sorted order of the points by code (stable two-pass radix sort).
+void order_points(const std::vector<unsigned>& code, std::vector<int>* perm)
+{
+  const size_t n = code.size();
+  constexpr int kBits = 11, kBins = 1 << kBits;
+  static_assert(3 * kCurveBits <= 2 * kBits, "two passes cover the code");
+  std::vector<int> a(n), cnt(kBins + 1);
+  perm->resize(n);
+  for (int pass = 0; pass < 2; pass++) {
+    std::fill(cnt.begin(), cnt.end(), 0);
+    for (size_t i = 0; i < n; i++) cnt[(code[i] >> (pass * kBits) & (kBins - 1)) + 1]++;
+    for (int k = 0; k < kBins; k++) cnt[k + 1] += cnt[k];
+    for (size_t i = 0; i < n; i++) {
+      const int p = pass ? a[i] : (int)i;
+      (pass ? *perm : a)[cnt[code[p] >> (pass * kBits) & (kBins - 1)]++] = p;
+    }
+  }
+}
+
+// First points of the groups in sorted order: the octree's cubes are split
+// while they hold more than kGroup points; small neighbours of one parent join.
+void split_groups(const std::vector<unsigned>& code, const std::vector<int>& perm, int lo, int hi, int level,
+                  std::vector<int>* gptr)
+{
+  if (hi - lo <= kGroup || level == kCurveBits) {
+    for (int i = lo; i < hi; i += kGroup) gptr->push_back(i);
+    return;
+  }
+  const int shift = 3 * (kCurveBits - 1 - level);
+  auto digit = [&](int i) { return code[perm[i]] >> shift & 7; };
+  int start = lo;  // of the open group
+  for (int i = lo; i < hi;) {
+    const unsigned c = digit(i);
+    const int end = (int)(std::partition_point(perm.begin() + i, perm.begin() + hi,
+                                               [&](int p) { return (code[p] >> shift & 7) == c; }) - perm.begin());
+    if (end - i > kGroup) {
+      if (i > start) gptr->push_back(start);
+      split_groups(code, perm, i, end, level + 1, gptr);
+      start = end;
+    } else if (end - start > kGroup) {
+      gptr->push_back(start);
+      start = i;
+    }
+    i = end;
+  }
+  if (hi > start) gptr->push_back(start);
+}
+
+template <int P>
+int evaluate_order(Mesh* m, int n, const double* pts, const double* d_pts, const ApplyArgs& A, const float4* rec32,
+                   const dq* rec64, double* d_out, cudaStream_t st)
+{
+  TreeMesh* t = m->tree.get();
+  TreePoints& w = t->points;
+  const TreePlan& plan = t->plan;
+  constexpr int kPairs = tree_pairs(P);
+  TreeTables tab;
+  EB_CHECK(tables_for(m->device, P, &tab));
+  // positions on the curve first: the host sorts them while the GPU forms the multipoles
+  double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+  for (int i = 0; i < n; i++)
+    for (int d = 0; d < 3; d++) {
+      const double v = pts[3 * (size_t)i + d];
+      if (!std::isfinite(v)) continue;
+      lo[d] = std::min(lo[d], v);
+      hi[d] = std::max(hi[d], v);
+    }
+  const double ext = std::max({hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2], 1e-300});
+  EB_CHECK(w.code.alloc(sizeof(unsigned) * (size_t)n));
+  EB_CHECK(w.perm.alloc(sizeof(int) * (size_t)n));
+  EB_CHECK(w.multipole.alloc(sizeof(double2) * (size_t)plan.nnodes * kPairs));
+  EB_CHECK(w.desc.alloc(2 * sizeof(TreeDesc)));
+  curve_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, d_pts, lo[0], lo[1], lo[2], ((1 << kCurveBits) - 1e-6) / ext,
+                                                w.code.as<unsigned>());
+  EB_CUDA(cudaGetLastError());
+  std::vector<unsigned> code(n);
+  EB_CUDA(cudaMemcpyAsync(code.data(), w.code.p, sizeof(unsigned) * (size_t)n, cudaMemcpyDeviceToHost, st));
+  EB_CUDA(cudaStreamSynchronize(st));  // the codes are here
+  TreeDesc d[2];
+  EB_CHECK(tree_desc(m, false, 1, 1, m->rec.p, w.multipole.p, nullptr, nullptr, &d[0]));
+  TreeDesc* dd = w.desc.as<TreeDesc>();
+  EB_CUDA(cudaMemcpyAsync(dd, &d[0], sizeof(TreeDesc), cudaMemcpyHostToDevice, st));
+  using Mv = MoveShape<P, 1>;
+  EB_CUDA(start(tree_p2m_kernel<P, 1, 1, true>, dim3(plan.ncells), 32 * kCellWarps, p2m_smem<P, 1, 1>(), st,
+                (const TreeDesc*)dd, (const int*)nullptr, 1, A, (const ApplyArgs*)nullptr, tab));
+  for (int s = 0; s < kTreePasses; s++)
+    EB_CUDA(start(tree_move_kernel<P, 1, kUp>, dim3(d[0].nup[s]), Mv::kThreads, Mv::smem(), st, (const TreeDesc*)dd,
+                  (const int*)nullptr, 1, s, tab));
+  std::vector<int> perm;
+  order_points(code, &perm);
+  std::vector<int> gptr;
+  split_groups(code, perm, 0, n, 0, &gptr);
+  const int ngroups = (int)gptr.size();
+  gptr.push_back(n);
+  perm.insert(perm.end(), gptr.begin(), gptr.end());  // one copy
+  EB_CHECK(w.perm.alloc(sizeof(int) * perm.size()));
+  EB_CHECK(w.ptr.alloc(sizeof(int) * 4 * ((size_t)ngroups + 1)));
+  EB_CHECK(w.ball.alloc(sizeof(dq) * ((size_t)plan.nnodes + ngroups)));
+  EB_CHECK(w.local.alloc(sizeof(double2) * ((size_t)plan.nnodes + ngroups) * kPairs));
+  EB_CUDA(cudaMemcpyAsync(w.perm.p, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice, st));
+  const int* d_perm = w.perm.as<int>();
+  const int* d_gptr = d_perm + n;
+  int* far_ptr = w.ptr.as<int>();
+  int* near_ptr = far_ptr + ngroups + 1;
+  int* task_ptr = near_ptr + ngroups + 1;
+  int* ids = task_ptr + ngroups + 1;
+  // the groups as targets: nodes nnodes, nnodes + 1, ...
+  dq* gball = w.ball.as<dq>() + plan.nnodes;
+  d[1] = d[0];
+  d[1].ball = w.ball.as<dq>();
+  d[1].local = w.local.as<double2>();
+  d[1].m2l.tgt = ids;
+  d[1].m2l.ptr = far_ptr;
+  EB_CUDA(cudaMemcpyAsync(w.ball.p, d[0].ball, sizeof(dq) * plan.nnodes, cudaMemcpyDeviceToDevice, st));
+  const double root = plan.ball[plan.nnodes - 1].w, theta = P <= kTreeOrder32 ? kTreePointTheta32 : kTreePointTheta64;
+  group_ball_kernel<<<(ngroups + 3) / 4, 128, 0, st>>>(ngroups, d_gptr, d_pts, d_perm, 1e-4 * root, gball);
+  const int gb = (ngroups + kListWarps - 1) / kListWarps;
+  group_lists_kernel<false><<<gb, 32 * kListWarps, 0, st>>>(ngroups, plan.nnodes - 1, plan.ncells, theta, d[0].ball,
+                                                            t->formed, t->children, gball, far_ptr, near_ptr, task_ptr,
+                                                            nullptr, nullptr);
+  scan_lists_kernel<<<1, 1024, 0, st>>>(ngroups, far_ptr, near_ptr, task_ptr);
+  iota_kernel<<<(ngroups + 255) / 256, 256, 0, st>>>(ngroups, plan.nnodes, ids);
+  EB_CUDA(cudaGetLastError());
+  int total[3];
+  EB_CUDA(cudaMemcpyAsync(&total[0], far_ptr + ngroups, sizeof(int), cudaMemcpyDeviceToHost, st));
+  EB_CUDA(cudaMemcpyAsync(&total[1], near_ptr + ngroups, sizeof(int), cudaMemcpyDeviceToHost, st));
+  EB_CUDA(cudaMemcpyAsync(&total[2], task_ptr + ngroups, sizeof(int), cudaMemcpyDeviceToHost, st));
+  EB_CUDA(cudaStreamSynchronize(st));
+  EB_CHECK(w.part.alloc(sizeof(double) * 32 * (size_t)std::max(1, total[2])));
+  EB_CHECK(w.far.alloc(sizeof(int) * std::max(1, total[0])));
+  EB_CHECK(w.near.alloc(sizeof(int) * std::max(1, total[1])));
+  d[1].m2l.src = w.far.as<int>();
+  EB_CUDA(cudaMemcpyAsync(dd + 1, &d[1], sizeof(TreeDesc), cudaMemcpyHostToDevice, st));
+  group_lists_kernel<true><<<gb, 32 * kListWarps, 0, st>>>(ngroups, plan.nnodes - 1, plan.ncells, theta, d[0].ball,
+                                                           t->formed, t->children, gball, far_ptr, near_ptr,
+                                                           task_ptr, w.far.as<int>(), w.near.as<int>());
+  EB_CUDA(cudaGetLastError());
+  EB_CUDA(start(tree_move_kernel<P, 1, kAcross>, dim3(ngroups), Mv::kThreads, Mv::smem(), st, (const TreeDesc*)(dd + 1),
+                (const int*)nullptr, 1, 0, tab));
+  constexpr bool F32 = P <= kTreeOrder32;
+  EB_CUDA(start(points_near_kernel<F32>, dim3((total[2] + kPointWarps - 1) / kPointWarps), 32 * kPointWarps,
+                (size_t)kPointWarps * kCell * kQ * kNrec * (F32 ? sizeof(float4) : sizeof(dq)), st, ngroups, total[2],
+                d_gptr, d_pts, d_perm, (const int*)task_ptr, (const int*)near_ptr, (const int*)w.near.as<int>(), m->h.ne,
+                rec32, (const float4*)m->splane32.as<float4>(), rec64, (const dq*)m->splane64.as<dq>(),
+                (const dq*)m->ccent.as<dq>(), w.part.as<double>()));
+  EB_CUDA(start(tree_points_kernel<P>, dim3((ngroups + kPointWarps - 1) / kPointWarps), 32 * kPointWarps, 0, st, ngroups,
+                d_gptr, d_pts, d_perm, (const dq*)gball,
+                (const double2*)(w.local.as<double2>() + (size_t)plan.nnodes * kPairs), (const int*)task_ptr,
+                (const double*)w.part.as<double>(), tab, d_out));
+  EB_CUDA(cudaStreamSynchronize(st));  // perm and d are read by the copies
+  return EB_OK;
+}
+
 }  // namespace
 
 int tree_launch(bool fp32, int nsl, int nd, const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one,
@@ -1327,7 +1828,7 @@ static int upload_lists(TreeMesh* t)
     if (!v.empty()) std::memcpy(host.data() + at, v.data(), v.size() * sizeof(v[0]));
     return at;
   };
-  const size_t ball = add(p.ball), has = add(p.has_local), tasks = add(p.sym.tasks), entries = add(p.sym.entries),
+  const size_t child = add(p.child), formed = add(p.formed), ball = add(p.ball), has = add(p.has_local), tasks = add(p.sym.tasks), entries = add(p.sym.entries),
                slots = add(p.sym.slot_off);
   struct At {
     size_t tgt, ptr, src;
@@ -1344,6 +1845,8 @@ static int upload_lists(TreeMesh* t)
                         reinterpret_cast<const int*>(q + a.src)};
   };
   TreeDesc& d = t->base;
+  t->children = reinterpret_cast<const int2*>(q + child);
+  t->formed = reinterpret_cast<const char*>(q + formed);
   d.ball = reinterpret_cast<const dq*>(q + ball);
   d.has_local = reinterpret_cast<const char*>(q + has);
   d.tasks = reinterpret_cast<const int4*>(q + tasks);
@@ -1443,6 +1946,28 @@ int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, v
   d.first_col = slot_columns(nsl, nd) - nsl - nd;
   *out = d;
   return EB_OK;
+}
+
+bool tree_points_eligible(const Mesh* m, bool fp32, int npts)
+{
+  const double pairs = (double)npts * m->h.ne;
+  return m->plan.engine == 4 && m->tree && m->tree->usable && !m->tree->plan.all_close &&
+         (fp32 ? pairs >= kTreePointPairs32 : pairs >= kTreePointPairs64 && m->h.ne >= kTreePointTriangles64);
+}
+
+int tree_evaluate(Mesh* m, bool fp32, int npts, const double* pts, const double* d_pts, const double* d_t,
+                  const double* d_u, double* d_out, cudaStream_t st)
+{
+  // FP64 records in either precision (the cells closest to a point), FP32 ones beside them
+  DevBuf& rec = m->pot_rec64;
+  EB_CHECK(rec.alloc((size_t)m->h.ne * m->h.Q * rec_slots(1, 1) * sizeof(dq)));
+  const ApplyArgs A = mesh_apply_args(m, false, rec.p, nullptr, d_t, m->h.ne, d_u, nullptr, m->h.ne, nullptr);
+  EB_CUDA(prep_launch(false, 1, 1, A, st));
+  if (!fp32) return evaluate_order<kTreeOrder64>(m, npts, pts, d_pts, A, nullptr, rec.as<dq>(), d_out, st);
+  EB_CHECK(ensure_apply_scratch(m));
+  const ApplyArgs A32 = mesh_apply_args(m, true, m->rec.p, nullptr, d_t, m->h.ne, d_u, nullptr, m->h.ne, nullptr);
+  EB_CUDA(prep_launch(true, 1, 1, A32, st));
+  return evaluate_order<kTreeOrder32>(m, npts, pts, d_pts, A, m->rec.as<float4>(), rec.as<dq>(), d_out, st);
 }
 
 size_t tree_bytes(const Mesh* m)

@@ -70,6 +70,11 @@ struct TreeSide {
   int create();  // no-op when made
 };
 
+// Scratch of the potential evaluation.
+struct TreePoints {
+  DevBuf code, perm, multipole, local, ball, ptr, far, near, part, desc;
+};
+
 // Block counts of each kernel over the meshes of a launch and, for more than
 // one mesh, the first block of each (device).
 struct TreeGrid {
@@ -88,6 +93,9 @@ struct TreeMesh {
   // close pairs in forward order, made with the first variant that needs them
   TreeNear fwd;
   DevBuf fwd_lists;
+  const int2* children = nullptr;  // of the inner nodes (device)
+  const char* formed = nullptr;    // TreePlan::formed (device)
+  TreePoints points;
   TreeSide side;
   std::map<int, std::unique_ptr<TreeScratch>> scratch;
 };
@@ -113,6 +121,11 @@ size_t tree_partial_bytes(const Mesh* m, int nsl, int nd);
 // or many (device).
 int tree_launch(bool fp32, int nsl, int nd, const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one,
                 const ApplyArgs* many, int device, const TreeSide& side, cudaStream_t st);
+// Potentials V t - W u at npts points (pts host, d_pts the same on the device)
+// through the tree. Waits for the stream.
+bool tree_points_eligible(const Mesh* m, bool fp32, int npts);
+int tree_evaluate(Mesh* m, bool fp32, int npts, const double* pts, const double* d_pts, const double* d_t,
+                  const double* d_u, double* d_out, cudaStream_t st);
 // Makes the constant tables that a launch needs (before a stream capture).
 int tree_tables(bool fp32, int device);
 // Device bytes of the mesh's tree and its single-mesh scratch; gives the

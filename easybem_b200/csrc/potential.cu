@@ -29,7 +29,6 @@
 namespace eb {
 
 constexpr int kPotThreads = 128;
-constexpr double kPotNear = 2.5;  // cells within this many radii of a point are summed in FP64
 
 // One cell's contribution to u(x) in FP64 from FP64 records ([ne*Q][2] dq)
 // and planes, (xs, ys, zs) = x relative to the cell centre.
@@ -235,10 +234,7 @@ int mesh_evaluate_potential(Mesh* m, int precision, int npts, const double* d_pt
     return set_error(EB_ERR_INVALID, "precision must be EB_PREC_FP64 or EB_PREC_MIXED");
   if (npts < 1) return EB_OK;
   // source records of the fused SL+DL variant (slot1 = (s, c))
-  if (!m->rec.p) {
-    EB_CHECK(m->rec.alloc((size_t)h.ne * h.Q * kMaxRecSlots * sizeof(dq)));
-    EB_CHECK(m->partial.alloc(sizeof(double) * (size_t)kMaxOutputs * m->plan.nsplit * h.nitems));
-  }
+  EB_CHECK(ensure_apply_scratch(m));
   const ApplyArgs A = mesh_apply_args(m, fp32, m->rec.p, nullptr, d_t, h.ne, d_u, nullptr, h.ne, nullptr);
   EB_CUDA(prep_launch(fp32, 1, true, A, st));
   if (fp32) {  // FP64 records for the cells close to a point

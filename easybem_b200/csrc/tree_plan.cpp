@@ -139,6 +139,7 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
   const int root = build(0, nc);
   if (nodes[root].height > kTreePasses * kTreeLevelsPerPass || (int)nodes.size() >= kTreeMaxNodes) return false;
   const int nn = p.nnodes = (int)nodes.size();
+  for (int k = nc; k < nn; k++) p.child.push_back(make_int2(nodes[k].left, nodes[k].right));
   p.ball.resize(nn);
   for (int c = 0; c < nc; c++) {
     const double* b = &h.cell_ball[4 * (size_t)c];
@@ -257,6 +258,9 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
     for (int j : sources[k]) u.src.push_back((int)(255u << 24 | (unsigned)j));
     u.ptr.push_back((int)u.src.size());
   }
+
+  p.formed.swap(used);
+  std::fill(p.formed.begin(), p.formed.begin() + nc, 1);
 
   // downward: every cell from all its ancestors with a local expansion
   for (int c = 0; c < nc; c++) {

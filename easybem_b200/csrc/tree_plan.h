@@ -29,6 +29,22 @@ constexpr double kTreeMinStep = 1e-3;
 constexpr int kTreeLevelsPerPass = 3;
 constexpr int kTreePasses = 6;  // enough for 2^18 cells
 constexpr int kTreeMaxNodes = 1 << 24;
+// Points x triangles from which the potential evaluation takes the tree, and
+// least triangles in FP64 (whose point sums are only 1.5 to 3 times dearer
+// than in the mixed evaluation, while the moves cost eight times the work).
+// Measured, direct -> tree (ms): mixed 5,940 triangles 2,000 points 0.41 -> 0.45,
+// 4,000 0.76 -> 0.47; FP64 17,860 x 4,000 1.09 -> 1.11, 8,000 1.97 -> 1.47;
+// 3,280 x 100,000 4.34 -> 4.53.
+constexpr double kTreePointPairs32 = 2e7, kTreePointPairs64 = 1e8;
+constexpr int kTreePointTriangles64 = 5000;
+// Separation of a group of points from a node. Potentials in the volume are
+// small against the contributions that cancel in them (rough double-layer
+// densities above all), so the same orders need smaller ratios than the
+// applies. Error against 64-bit sums, 50,000 points inside an icosphere L5
+// (the direct sums: 8.3e-8 mixed, 7.1e-16 FP64): at 0.5 1.8e-7 and 1.5e-12, at
+// 0.45 2.8e-8 and 5.2e-14, at 0.4 1.5e-15, at 0.35 5.1e-16 in FP64.
+constexpr double kTreePointTheta32 = 0.45;
+constexpr double kTreePointTheta64 = 0.35;
 // Close cell pairs per near task (one warp's work; the diagonal counts): at
 // most kTreeNearChunk, fewer while that leaves less than kTreeNearTasks tasks
 // (four warps on each of the 592 SM quarters).
@@ -69,10 +85,12 @@ struct TreePlan {
   int ncells = 0, nnodes = 0;  // nodes 0 .. ncells - 1 are the cells
   bool all_close = false;      // no expansions: every cell pair in near
   std::vector<dq> ball;        // centre; radius over the quadrature points
+  std::vector<int2> child;     // of node ncells + k
   TreeMoves up[kTreePasses];   // multipoles of descendants into inner nodes
   TreeMoves m2l;               // multipoles of separated nodes into locals
   TreeMoves down;              // locals of the ancestors into every cell
   std::vector<char> has_local; // per node: it is a target of m2l
+  std::vector<char> formed;    // per node: the upward passes form its multipole
   std::vector<std::pair<int, int>> near;  // close cells, the earlier one first
   TreeNear sym;  // every unordered pair of cells once
 };

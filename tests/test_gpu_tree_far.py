@@ -161,3 +161,39 @@ def test_small_meshes_sum_all_cell_pairs(gpu_lib, oracle, ne):
                 assert rel_l2(q[rows], qo) < tol and rel_l2(qs[rows], qo) < tol
                 assert rel_l2(d, e) < 10 * tol
             assert rel_l2(b, c) < tol
+
+
+@pytest.mark.parametrize("npts", [2000, 5000, 5017, 20000])
+@pytest.mark.parametrize("name", ["torus206", "graded", "two"])
+def test_tree_potentials(gpu_lib, oracle, name, npts):
+    """Points far away, in the volume and close to the surface, several of them
+    the same; ragged last groups. One point that is not finite leaves the
+    others alone."""
+    oracle.set_order(4)
+    nodes, elems = MESHES[name]()
+    t, u = _vectors(nodes, elems, npts)
+    rng = np.random.default_rng(npts)
+    c = nodes.mean(axis=0)
+    size = np.linalg.norm(nodes - c, axis=1).max()
+    pts = c + size * rng.uniform(-1.5, 1.5, size=(npts, 3))
+    k = rng.integers(0, len(elems), size=npts // 4)
+    tri = nodes[elems[k] - 1]
+    nrm = np.cross(tri[:, 1] - tri[:, 0], tri[:, 2] - tri[:, 0])
+    h = np.sqrt(np.linalg.norm(nrm, axis=1, keepdims=True))
+    nrm /= np.linalg.norm(nrm, axis=1, keepdims=True)
+    pts[: npts // 4] = tri.mean(axis=1) + nrm * h * rng.uniform(0.5, 3.0, size=(npts // 4, 1))
+    pts[-40:] = pts[-41]
+    with gpu_lib.Mesh(nodes, elems) as m:
+        for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL)):
+            m.set_far_engine("tree")
+            p = m.evaluate(pts, t, u, prec)
+            assert np.array_equal(p, m.evaluate(pts, t, u, prec))
+            bad = pts.copy()
+            bad[5] = np.nan
+            pb = m.evaluate(bad, t, u, prec)
+            assert np.isnan(pb[5]) and rel_l2(np.delete(pb, 5), np.delete(p, 5)) < tol
+            m.set_far_engine("cuda")
+            assert rel_l2(p, m.evaluate(pts, t, u, prec)) < tol
+        rows = np.linspace(0, npts - 1, 64).astype(int)
+        m.set_far_engine("tree")
+        assert rel_l2(m.evaluate(pts, t, u)[rows], oracle.evaluate(nodes, elems, pts[rows], t, u)) < FP64_TOL
