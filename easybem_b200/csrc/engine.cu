@@ -246,14 +246,6 @@ static int upload(DevBuf& b, const std::vector<T>& v)
   return EB_OK;
 }
 
-template <typename T>
-static int upload(TmpBuf& b, const std::vector<T>& v)
-{
-  EB_CHECK(b.alloc(sizeof(T) * std::max<size_t>(v.size(), 1)));
-  if (!v.empty()) EB_CUDA(cudaMemcpyAsync(b.p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, b.st));
-  return EB_OK;
-}
-
 Mesh::~Mesh()
 {
   if (ev0) cudaEventDestroy(ev0);
@@ -301,196 +293,161 @@ __global__ void dl_gather_kernel(const int* __restrict__ cptr, const int* __rest
 
 // ---------------------------------------------------------------------------
 
-static int build_static(Mesh* m)
-{
-  HostMesh& h = m->h;
-  const int ne = h.ne, Q = h.Q, K = h.K;
-  const int ntt = (h.nitems + kTT - 1) / kTT;
-  std::vector<float4> pos32((size_t)ne * Q), tgt32((size_t)h.nitems * K), tgtw32((size_t)h.nitems * K);
-  std::vector<dq> tgtw64((size_t)h.nitems * K);
-  std::vector<dq> pos64((size_t)ne * Q), trin(ne), tgt64((size_t)h.nitems * K), tcent(h.nitems), tnrm(h.nitems),
-      ccent(h.ncells), snrm(ne), ttile(ntt), twarp((h.nitems + kWarpItems - 1) / kWarpItems), splane64(ne);
-  std::vector<float4> splane32(ne);
-  std::vector<double> wjtab((size_t)ne * Q);
-  std::vector<int4> svid(ne), tvid(h.nitems);
-  std::vector<double> bary(2 * (size_t)Q);
-  for (int b = 0; b < Q; b++) {
-    bary[2 * b] = h.quad.tx[b];
-    bary[2 * b + 1] = h.quad.ty[b];
-  }
-  auto vertex = [&](int s, int k) {
-    const int v = h.elems[3 * h.perm[s] + k];
-    return mk3(h.nodes[3 * v], h.nodes[3 * v + 1], h.nodes[3 * v + 2]);
-  };
-  for (int c = 0; c < h.ncells; c++) {
-    const double* b = &h.cell_ball[4 * (size_t)c];
-    ccent[c] = dq{b[0], b[1], b[2], b[3]};
-  }
-  h.cell_rho.assign(h.ncells, 0.0);
-  for (int s = 0; s < ne; s++) {
-    d3 P[3];
-    for (int k = 0; k < 3; k++) P[k] = vertex(s, k);
-    const int* f = &h.elems[3 * h.perm[s]];
-    const d3 w = P[1] - P[0], z = P[2] - P[0];
-    const d3 n = cross3(w, z);
-    const double J = std::sqrt(dot3(n, n));
-    trin[s] = dq{n.x / J, n.y / J, n.z / J, J};
-    const d3 nu = (1.0 / J) * n;
-    snrm[s] = dq{nu.x, nu.y, nu.z, dot3(P[0], nu)};
-    svid[s] = make_int4(f[0], f[1], f[2], 0);
-    const int cell = s / kCell;
-    const d3 cc = mk3(ccent[cell].x, ccent[cell].y, ccent[cell].z);
-    const double hp = dot3(P[0] - cc, nu);
-    splane64[s] = dq{nu.x, nu.y, nu.z, hp};
-    splane32[s] = make_float4((float)nu.x, (float)nu.y, (float)nu.z, (float)hp);
-    for (int b = 0; b < Q; b++) {
-      const d3 y = P[0] + h.quad.tx[b] * w + h.quad.ty[b] * z;
-      wjtab[(size_t)s * Q + b] = h.quad.tw[b] * J;
-      const d3 yr = y - cc;
-      pos64[(size_t)s * Q + b] = dq{-2.0 * yr.x, -2.0 * yr.y, -2.0 * yr.z, dot3(yr, yr)};
-      h.cell_rho[cell] = std::max(h.cell_rho[cell], dot3(yr, yr));
-      const float fx = (float)yr.x, fy = (float)yr.y, fz = (float)yr.z;
-      const double y2 = (double)fx * fx + (double)fy * fy + (double)fz * fz;
-      pos32[(size_t)s * Q + b] = make_float4(-2.0f * fx, -2.0f * fy, -2.0f * fz, (float)y2);
-    }
-    const d3 cen = (1.0 / 3.0) * (P[0] + P[1] + P[2]);
-    for (int ch = 0; ch < h.nchunk; ch++) {
-      const int item = s * h.nchunk + ch;
-      tcent[item] = dq{cen.x, cen.y, cen.z, 0.0};
-      tnrm[item] = dq{nu.x, nu.y, nu.z, 0.0};
-      tvid[item] = svid[s];
-      for (int a = 0; a < K; a++) {
-        const int pa = ch * K + a;
-        const int pp = std::min(pa, Q - 1);
-        const double wa = pa < Q ? h.quad.tw[pp] : 0.0;
-        const d3 x = P[0] + h.quad.tx[pp] * w + h.quad.ty[pp] * z;
-        const d3 xr = x - cen;
-        tgt64[(size_t)item * K + a] = dq{xr.x, xr.y, xr.z, wa};
-        tgt32[(size_t)item * K + a] = make_float4((float)xr.x, (float)xr.y, (float)xr.z, (float)wa);
-        // P1 test weights w_a (1 - xi - eta, xi, eta) in the triangle's vertex order
-        const double ph0 = 1.0 - h.quad.tx[pp] - h.quad.ty[pp], ph1 = h.quad.tx[pp], ph2 = h.quad.ty[pp];
-        tgtw64[(size_t)item * K + a] = dq{wa * ph0, wa * ph1, wa * ph2, 0.0};
-        tgtw32[(size_t)item * K + a] = make_float4((float)(wa * ph0), (float)(wa * ph1), (float)(wa * ph2), 0.0f);
-      }
-    }
-  }
-  for (double& r : h.cell_rho) r = std::sqrt(r) * (1.0 + 1e-12);
-  // bounding spheres over the triangles of n consecutive target items: per
-  // tile of kTT (the tensor-core kernel's test) and per warp of kWarpItems
-  // (the CUDA-core kernel's: a tighter sphere leaves fewer cells "near")
-  auto item_spheres = [&](int n, std::vector<dq>& out) {
-    for (size_t t = 0; t < out.size(); t++) {
-      const int i0 = (int)t * n, i1 = std::min(h.nitems, i0 + n);
-      double b[4];
-      if (h.nchunk == 1 && n == kCell) std::copy_n(&h.cell_ball[4 * t], 4, b);  // a cell's own triangles
-      else vertex_ball(h, i0 / h.nchunk, (i1 - 1) / h.nchunk + 1, b);
-      out[t] = dq{b[0], b[1], b[2], b[3]};
-    }
-  };
-  item_spheres(kTT, ttile);
-  item_spheres(kWarpItems, twarp);
-  // how the warp x cell blocks split under the CUDA-core kernel's separation test
-  {
-    long long fc = 0, nc = 0;
-    for (size_t t = 0; t < twarp.size(); t++) {
-      const long long nt = std::min<long long>(h.nitems, (long long)(t + 1) * kWarpItems) - (long long)t * kWarpItems;
-      for (int c = 0; c < h.ncells; c++) {
-        const long long ns = std::min(ne, (c + 1) * kCell) - c * kCell;
-        const double dx = ccent[c].x - twarp[t].x, dy = ccent[c].y - twarp[t].y, dz = ccent[c].z - twarp[t].z;
-        const double rr = kFarRatio * (ccent[c].w + twarp[t].w);
-        (dx * dx + dy * dy + dz * dz > rr * rr ? fc : nc) += nt * ns;
-      }
-    }
-    h.far_cell_tri_pairs = fc;
-    h.near_cell_tri_pairs = nc;
-  }
-  // one allocation and one copy for all static tables (a mesh set-up that
-  // runs beside other GPU work pays the per-call latency of the runtime once)
+// Lays buffers out in one allocation (each aligned to 256 bytes).
+struct Arena {
   struct Part {
     DevBuf* dst;
-    const void* src;
     size_t bytes;
   };
-  auto part = [](DevBuf& d, const auto& v) {
-    return Part{&d, (const void*)v.data(), sizeof(v[0]) * v.size()};
-  };
-  const Part parts[] = {part(m->pos32, pos32),   part(m->pos64, pos64),     part(m->wj, wjtab),
-                        part(m->trin, trin),     part(m->svid, svid),       part(m->perm, h.perm),
-                        part(m->iperm, h.iperm), part(m->bary, bary),       part(m->tgt32, tgt32),
-                        part(m->tgt64, tgt64),   part(m->tgtw32, tgtw32),   part(m->tgtw64, tgtw64),
-                        part(m->tcent, tcent),   part(m->tnrm, tnrm),       part(m->snrm, snrm),
-                        part(m->tvid, tvid),     part(m->ccent, ccent),     part(m->ttile, ttile),
-                        part(m->twarp, twarp),
-                        part(m->splane32, splane32), part(m->splane64, splane64)};
-  auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  size_t total = 0;
-  for (const Part& q : parts) total += align(std::max<size_t>(q.bytes, 16));
-  std::vector<unsigned char> staging(total, 0);
-  size_t off = 0;
-  for (const Part& q : parts) {
-    if (q.bytes) std::memcpy(staging.data() + off, q.src, q.bytes);
-    off += align(std::max<size_t>(q.bytes, 16));
-  }
-  const auto ta = std::chrono::steady_clock::now();
-  EB_CHECK(m->arena.alloc(total));
-  const auto tb = std::chrono::steady_clock::now();
-  EB_CHECK(copy_h2d(m->arena.p, staging.data(), total));
-  const auto tc = std::chrono::steady_clock::now();
-  m->setup_s[3] = std::chrono::duration<double>(tb - ta).count();
-  m->setup_s[4] = std::chrono::duration<double>(tc - tb).count();
-  off = 0;
-  for (const Part& q : parts) {
-    const size_t n = align(std::max<size_t>(q.bytes, 16));
-    q.dst->view(static_cast<unsigned char*>(m->arena.p) + off, std::max<size_t>(q.bytes, 16));
-    off += n;
-  }
-  return EB_OK;
-}
-
-static int build_near(Mesh* m)
-{
-  HostMesh& h = m->h;
-  const int npairs = (int)h.sl_col.size();
-  m->npairs = npairs;
-  EB_CHECK(upload(m->sl_rowptr, h.sl_rowptr));
-  EB_CHECK(upload(m->sl_col, h.sl_col));
-  EB_CHECK(upload(m->dl_rowptr, h.dl_rowptr));
-  EB_CHECK(upload(m->dl_col, h.dl_col));
-  EB_CHECK(m->sl_val.alloc(sizeof(double) * std::max(npairs, 1)));
-  const int nslots = (int)h.dl_col.size();
-  EB_CHECK(m->dl_val.alloc(sizeof(double) * std::max(nslots, 1)));
-  // a private stream with stream-ordered temporaries: mesh set-up overlaps
-  // work that other threads run on the GPU and never waits for the device
-  cudaStream_t st = nullptr;
-  EB_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  int rc = EB_OK;
-  cudaError_t e1 = cudaSuccess, e2 = cudaSuccess;
+  std::vector<Part> parts;
+  void add(DevBuf& d, size_t bytes) { parts.push_back({&d, std::max<size_t>(bytes, 16)}); }
+  int make(DevBuf& arena)
   {
-    TmpBuf d_nodes(st), d_elems(st), d_pi(st), d_pj(st), d_dle(st), d_cptr(st), d_contrib(st);
-    rc = upload(d_nodes, h.nodes);
-    if (rc == EB_OK) rc = upload(d_elems, h.elems);
-    if (rc == EB_OK) rc = upload(d_pi, h.pair_i);
-    if (rc == EB_OK) rc = upload(d_pj, h.sl_col);
-    if (rc == EB_OK) rc = upload(d_cptr, h.dl_contrib_ptr);
-    if (rc == EB_OK) rc = upload(d_contrib, h.dl_contrib);
-    if (rc == EB_OK) rc = d_dle.alloc(sizeof(double) * 3 * std::max(npairs, 1));
-    if (rc == EB_OK) {
-      if (npairs > 0)
-        near_values_kernel<<<(npairs + 127) / 128, 128, 0, st>>>(h.quad, d_nodes.as<double>(), d_elems.as<int>(),
-                                                                 d_pi.as<int>(), d_pj.as<int>(), npairs,
-                                                                 m->sl_val.as<double>(), d_dle.as<double>());
-      if (nslots > 0)
-        dl_gather_kernel<<<(nslots + 255) / 256, 256, 0, st>>>(d_cptr.as<int>(), d_contrib.as<int>(),
-                                                              d_dle.as<double>(), nslots, m->dl_val.as<double>());
-      e1 = cudaGetLastError();
+    auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    size_t total = 0;
+    for (const Part& p : parts) total += align(p.bytes);
+    EB_CHECK(arena.alloc(total));
+    unsigned char* at = static_cast<unsigned char*>(arena.p);
+    for (const Part& p : parts) {
+      p.dst->view(at, p.bytes);
+      at += align(p.bytes);
     }
-  }  // temporaries released on st
+    return EB_OK;
+  }
+};
+
+// Copies of a mesh set-up: host arrays collected in the thread's pinned buffer
+// and issued on one stream, waited for only when the buffer is full.
+class SetupCopies {
+ public:
+  explicit SetupCopies(cudaStream_t st) : st_(st), stage_(static_cast<unsigned char*>(staging_buffer())) {}
+  int add(void* dst, const void* src, size_t bytes)
+  {
+    if (!stage_) return set_error(EB_ERR_CUDA, "cannot create the pinned staging buffer");
+    for (size_t off = 0; off < bytes;) {
+      if (used_ == kStageChunk) {
+        EB_CUDA(cudaStreamSynchronize(st_));
+        used_ = 0;
+      }
+      const size_t n = std::min(bytes - off, kStageChunk - used_);
+      std::memcpy(stage_ + used_, static_cast<const unsigned char*>(src) + off, n);
+      EB_CUDA(cudaMemcpyAsync(static_cast<unsigned char*>(dst) + off, stage_ + used_, n, cudaMemcpyHostToDevice, st_));
+      off += n;
+      used_ += n;
+    }
+    return EB_OK;
+  }
+  template <typename T>
+  int add(void* dst, const std::vector<T>& v) { return add(dst, v.data(), sizeof(T) * v.size()); }
+
+ private:
+  cudaStream_t st_;
+  unsigned char* stage_;
+  size_t used_ = 0;
+};
+
+// Static tables and near field of a new mesh: the geometry and the near-pair
+// lists go up in one allocation each, kernels write the rest; the host plans
+// the tree while the near values are computed. One private stream, so that
+// set-up overlaps work that other threads run on the GPU and never waits for
+// the device.
+static int build_tables(Mesh* m, cudaStream_t st)
+{
+  using clk = std::chrono::steady_clock;
+  const auto sec = [](clk::time_point a, clk::time_point b) { return std::chrono::duration<double>(b - a).count(); };
+  const auto t0 = clk::now();
+  HostMesh& h = m->h;
+  const size_t ne = h.ne, nq = ne * h.Q, items = h.nitems, nk = items * h.K;
+  const size_t ntt = (items + kTT - 1) / kTT, nw = (items + kWarpItems - 1) / kWarpItems;
+  const size_t npairs = h.sl_col.size(), nslots = h.dl_col.size();
+  m->npairs = (long long)npairs;
+  Arena a;
+  a.add(m->pos32, sizeof(float4) * nq);
+  a.add(m->pos64, sizeof(dq) * nq);
+  a.add(m->wj, sizeof(double) * nq);
+  a.add(m->trin, sizeof(dq) * ne);
+  a.add(m->svid, sizeof(int4) * ne);
+  a.add(m->perm, sizeof(int) * ne);
+  a.add(m->iperm, sizeof(int) * ne);
+  a.add(m->bary, sizeof(double) * 2 * h.Q);
+  a.add(m->tgt32, sizeof(float4) * nk);
+  a.add(m->tgt64, sizeof(dq) * nk);
+  a.add(m->tgtw32, sizeof(float4) * nk);
+  a.add(m->tgtw64, sizeof(dq) * nk);
+  a.add(m->tcent, sizeof(dq) * items);
+  a.add(m->tnrm, sizeof(dq) * items);
+  a.add(m->snrm, sizeof(dq) * ne);
+  a.add(m->tvid, sizeof(int4) * items);
+  a.add(m->ccent, sizeof(dq) * h.ncells);
+  a.add(m->ttile, sizeof(dq) * ntt);
+  a.add(m->twarp, sizeof(dq) * nw);
+  a.add(m->splane32, sizeof(float4) * ne);
+  a.add(m->splane64, sizeof(dq) * ne);
+  EB_CHECK(a.make(m->arena));
+  Arena b;
+  b.add(m->sl_rowptr, sizeof(int) * h.sl_rowptr.size());
+  b.add(m->sl_col, sizeof(int) * npairs);
+  b.add(m->dl_rowptr, sizeof(int) * h.dl_rowptr.size());
+  b.add(m->dl_col, sizeof(int) * nslots);
+  b.add(m->sl_val, sizeof(double) * npairs);
+  b.add(m->dl_val, sizeof(double) * nslots);
+  EB_CHECK(b.make(m->near_arena));
+  m->setup_s[3] = sec(t0, clk::now());
+  TmpBuf nodes(st), elems(st), tw(st), rho(st), pi(st), dle(st), cptr(st), contrib(st);
+  EB_CHECK(nodes.alloc(sizeof(double) * h.nodes.size()));
+  EB_CHECK(elems.alloc(sizeof(int) * h.elems.size()));
+  EB_CHECK(tw.alloc(sizeof(double) * h.Q));
+  EB_CHECK(rho.alloc(sizeof(double) * h.ncells));
+  EB_CHECK(pi.alloc(sizeof(int) * npairs));
+  EB_CHECK(dle.alloc(sizeof(double) * 3 * npairs));
+  EB_CHECK(cptr.alloc(sizeof(int) * h.dl_contrib_ptr.size()));
+  EB_CHECK(contrib.alloc(sizeof(int) * h.dl_contrib.size()));
+  const auto t1 = clk::now();
+  std::vector<double> bary(2 * (size_t)h.Q);
+  for (int k = 0; k < h.Q; k++) {
+    bary[2 * k] = h.quad.tx[k];
+    bary[2 * k + 1] = h.quad.ty[k];
+  }
+  static_assert(sizeof(dq) == 4 * sizeof(double), "cell balls are copied as they are");
+  SetupCopies up(st);
+  EB_CHECK(up.add(nodes.p, h.nodes));
+  EB_CHECK(up.add(elems.p, h.elems));
+  EB_CHECK(up.add(m->perm.p, h.perm));
+  EB_CHECK(up.add(m->iperm.p, h.iperm));
+  EB_CHECK(up.add(m->bary.p, bary));
+  EB_CHECK(up.add(tw.p, h.quad.tw, sizeof(double) * h.Q));
+  EB_CHECK(up.add(m->ccent.p, h.cell_ball));
+  const StaticTables t{h.ne, h.Q, h.K, h.nchunk, nodes.as<double>(), m->bary.as<double>(), tw.as<double>(),
+                       elems.as<int>(), m->perm.as<int>(), m->ccent.as<dq>(), m->pos32.as<float4>(),
+                       m->tgt32.as<float4>(), m->tgtw32.as<float4>(), m->splane32.as<float4>(), m->pos64.as<dq>(),
+                       m->trin.as<dq>(), m->tgt64.as<dq>(), m->tgtw64.as<dq>(), m->tcent.as<dq>(), m->tnrm.as<dq>(),
+                       m->snrm.as<dq>(), m->splane64.as<dq>(), m->ttile.as<dq>(), m->twarp.as<dq>(),
+                       m->wj.as<double>(), rho.as<double>(), m->svid.as<int4>(), m->tvid.as<int4>()};
+  EB_CUDA(static_tables_launch(t, st));
+  EB_CHECK(up.add(m->sl_rowptr.p, h.sl_rowptr));
+  EB_CHECK(up.add(m->sl_col.p, h.sl_col));
+  EB_CHECK(up.add(m->dl_rowptr.p, h.dl_rowptr));
+  EB_CHECK(up.add(m->dl_col.p, h.dl_col));
+  EB_CHECK(up.add(pi.p, h.pair_i));
+  EB_CHECK(up.add(cptr.p, h.dl_contrib_ptr));
+  EB_CHECK(up.add(contrib.p, h.dl_contrib));
+  h.cell_rho.resize(h.ncells);
+  EB_CUDA(cudaMemcpyAsync(h.cell_rho.data(), rho.p, sizeof(double) * h.ncells, cudaMemcpyDeviceToHost, st));
+  EB_CUDA(cudaStreamSynchronize(st));  // the radii are here
+  const auto t2 = clk::now();
+  m->setup_s[1] = sec(t0, t2);
+  m->setup_s[4] = sec(t1, t2);
+  if (npairs > 0)
+    near_values_kernel<<<((int)npairs + 127) / 128, 128, 0, st>>>(h.quad, nodes.as<double>(), elems.as<int>(),
+                                                                  pi.as<int>(), m->sl_col.as<int>(), (int)npairs,
+                                                                  m->sl_val.as<double>(), dle.as<double>());
+  if (nslots > 0)
+    dl_gather_kernel<<<((int)nslots + 255) / 256, 256, 0, st>>>(cptr.as<int>(), contrib.as<int>(), dle.as<double>(),
+                                                                (int)nslots, m->dl_val.as<double>());
+  EB_CUDA(cudaGetLastError());
   tree_prepare(m);  // host work beside the kernels
-  e2 = cudaStreamSynchronize(st);
-  cudaStreamDestroy(st);
-  EB_CHECK(rc);
-  EB_CUDA(e1);
-  EB_CUDA(e2);
+  EB_CUDA(cudaStreamSynchronize(st));
+  m->setup_s[2] = sec(t2, clk::now());
   return EB_OK;
 }
 
@@ -571,16 +528,18 @@ int mesh_create(int nv, const double* nodes, int ne, const int* elems1, int orde
     m->h.topology_on_device = done;
   }
   if (st == EB_OK) tuned_plan_for(m->h, &m->plan.items_per_sm, &m->plan.tile);
-  const auto t1 = clk::now();
-  if (st == EB_OK) st = build_static(m);
-  const auto t2 = clk::now();
-  if (st == EB_OK) st = build_near(m);
-  const auto t3 = clk::now();
+  m->setup_s[0] = std::chrono::duration<double>(clk::now() - t0).count();
+  if (st == EB_OK) {
+    cudaStream_t priv = nullptr;
+    const cudaError_t es = cudaStreamCreateWithFlags(&priv, cudaStreamNonBlocking);
+    st = es == cudaSuccess ? build_tables(m, priv)
+                           : set_error(EB_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(es));
+    if (priv) {
+      cudaStreamSynchronize(priv);  // nothing queued outlives a failed set-up
+      cudaStreamDestroy(priv);
+    }
+  }
   if (st == EB_OK) st = build_items(m);
-  const auto sec = [](clk::time_point a, clk::time_point b) { return std::chrono::duration<double>(b - a).count(); };
-  m->setup_s[0] = sec(t0, t1);
-  m->setup_s[1] = sec(t1, t2);
-  m->setup_s[2] = sec(t2, t3);
   if (st != EB_OK) {
     delete m;
     return st;
@@ -969,8 +928,23 @@ int eb_mesh_topology_on_device(eb_mesh mesh, int* on_device)
 int eb_mesh_cell_pairs(eb_mesh mesh, long long* far_cell_tri_pairs, long long* near_cell_tri_pairs)
 {
   if (!mesh) return set_error(EB_ERR_INVALID, "null mesh");
-  if (far_cell_tri_pairs) *far_cell_tri_pairs = mesh->m->h.far_cell_tri_pairs;
-  if (near_cell_tri_pairs) *near_cell_tri_pairs = mesh->m->h.near_cell_tri_pairs;
+  // how the warp x cell blocks split under the CUDA-core kernel's separation test
+  const eb::HostMesh& h = mesh->m->h;
+  long long fc = 0, nc = 0;
+  for (int i0 = 0; i0 < h.nitems; i0 += eb::kWarpItems) {
+    const int i1 = std::min(h.nitems, i0 + eb::kWarpItems);
+    double w[4];
+    eb::vertex_ball(h, i0 / h.nchunk, (i1 - 1) / h.nchunk + 1, w);
+    for (int c = 0; c < h.ncells; c++) {
+      const long long ns = std::min(h.ne, (c + 1) * eb::kCell) - c * eb::kCell;
+      const double* b = &h.cell_ball[4 * (size_t)c];
+      const double dx = b[0] - w[0], dy = b[1] - w[1], dz = b[2] - w[2];
+      const double rr = eb::kFarRatio * (b[3] + w[3]);
+      (dx * dx + dy * dy + dz * dz > rr * rr ? fc : nc) += (i1 - i0) * ns;
+    }
+  }
+  if (far_cell_tri_pairs) *far_cell_tri_pairs = fc;
+  if (near_cell_tri_pairs) *near_cell_tri_pairs = nc;
   return EB_OK;
 }
 

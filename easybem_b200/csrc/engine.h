@@ -107,6 +107,8 @@ struct Mesh {
 
   // static geometry (sorted order), views into one allocation (arena)
   DevBuf arena;
+  // the near field's lists and values, views into another
+  DevBuf near_arena;
   DevBuf pos32, pos64, wj, trin, svid, perm, iperm, bary;
   DevBuf tgt32, tgt64, tgtw32, tgtw64, tcent, tnrm, tvid, ccent, snrm, ttile, twarp, splane32, splane64;
   // P1 x P1 single layer near field (built on first use)
@@ -189,6 +191,19 @@ int ensure_tc_static(Mesh* m);
 // EB_ERR_TIMEOUT (and the flag cleared) if the last tensor-core launch on m
 // gave up a bounded wait; EB_OK otherwise. The stream must be synchronised.
 int mesh_check_far_error(Mesh* m);
+// Inputs and outputs of the static-table kernels (device pointers; the tables
+// are described at Mesh and FarMeshDesc).
+struct StaticTables {
+  int ne, Q, K, nchunk;
+  const double *nodes, *bary, *tw;
+  const int *elems, *perm;
+  const dq* ccent;
+  float4 *pos32, *tgt32, *tgtw32, *splane32;
+  dq *pos64, *trin, *tgt64, *tgtw64, *tcent, *tnrm, *snrm, *splane64, *ttile, *twarp;
+  double *wj, *rho;  // rho [ncells]: radius of each cell over its quadrature points
+  int4 *svid, *tvid;
+};
+cudaError_t static_tables_launch(const StaticTables& t, cudaStream_t st);
 // The record and partial-sum scratch of single-mesh calls.
 int ensure_apply_scratch(Mesh* m);
 // The mixed potential evaluation sums cells within this many radii of a point in FP64.

@@ -50,11 +50,6 @@ struct HostMesh {
 
   long long far_quad_pairs = 0;  // regular quadrature-point pairs per apply
   bool topology_on_device = false;  // near-pair lists built by device_topology
-  // (target item, source triangle) pairs in source cells well separated from
-  // the item's warp of target items, and in the others (where a far-field kernel
-  // masks vertex-sharing pairs and forms differences directly); set with the
-  // static tables
-  long long far_cell_tri_pairs = 0, near_cell_tri_pairs = 0;
 };
 
 // Cells of the first half of a range of ncells cells in the bisection.

@@ -49,9 +49,8 @@ static double now_ms()
 static size_t mesh_resident_bytes(const Mesh* m)
 {
   size_t b = 0;
-  // the static tables are views into the arena, which is counted once
-  const DevBuf* bufs[] = {&m->arena, &m->sl_rowptr, &m->sl_col, &m->sl_val, &m->dl_rowptr,
-                          &m->dl_col, &m->dl_val, &m->rec, &m->partial, &m->counter, &m->items, &m->io_t,
+  // static tables and near field are views into the arenas, which are counted once
+  const DevBuf* bufs[] = {&m->arena, &m->near_arena, &m->rec, &m->partial, &m->counter, &m->items, &m->io_t,
                           &m->io_u, &m->io_v, &m->io_q, &m->pc_val};
   for (const DevBuf* d : bufs) b += d->bytes;
   return b + tree_bytes(m);
