@@ -546,15 +546,17 @@ __device__ __forceinline__ void each_harmonic(const TreeTables& tab, const CellP
 }
 
 // Multipoles of one cell: NSL single-layer columns (they share sum_b w_b J
-// R(y_b)), and for ND = 1 the double-layer column blockIdx.y. DIFF: one
-// column, single minus double layer (the representation formula).
-template <int P, int NSL, int ND, bool DIFF = false>
+// R(y_b)), and for ND = 1 the double-layer column blockIdx.y. KIND: both apart,
+// single minus double layer in one column (the representation formula), or
+// the strengths of the double-layer column as charges (P1 single layer).
+enum Sources { kApart, kDiff, kCharges };
+template <int P, int NSL, int ND, int KIND = kApart>
 __global__ void __launch_bounds__(32 * kCellWarps)
     tree_p2m_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh, ApplyArgs one,
                     const ApplyArgs* __restrict__ many, TreeTables tab)
 {
   constexpr int kPairs = tree_pairs(P);
-  constexpr int kRows = 2 * NSL + 6 * ND;
+  constexpr int kRows = KIND == kCharges ? 2 : 2 * NSL + 6 * ND;
   static_assert(kRows <= kSumRows, "one row of lane sums per value");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* s_red = reinterpret_cast<double*>(smem_raw) + (threadIdx.x >> 5) * kSumRows * kSumStride;
@@ -611,10 +613,15 @@ __global__ void __launch_bounds__(32 * kCellWarps)
         gr += s[a] * re[a];
         gi += s[a] * im[a];
       }
+      if constexpr (KIND == kCharges) {
+        s_red[lane] = gr;
+        s_red[kSumStride + lane] = gi;
+      } else {
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        s_red[row++ * kSumStride + lane] = gr * nrm[k];
-        s_red[row++ * kSumStride + lane] = gi * nrm[k];
+        for (int k = 0; k < 3; ++k) {
+          s_red[row++ * kSumStride + lane] = gr * nrm[k];
+          s_red[row++ * kSumStride + lane] = gi * nrm[k];
+        }
       }
     }
     __syncwarp();
@@ -633,11 +640,13 @@ __global__ void __launch_bounds__(32 * kCellWarps)
   const size_t cstride = (size_t)d.nnodes * kPairs;
   double2* out = d.multipole + (size_t)cell * kPairs;
   for (int i = threadIdx.x; i < kPairs; i += 32 * kCellWarps) {
-    if constexpr (!DIFF)
+    if constexpr (KIND == kApart)
 #pragma unroll
       for (int c = 0; c < NSL; ++c)
         out[c * cstride + i] = make_double2(s_sum[2 * c * kPairs + i], s_sum[(2 * c + 1) * kPairs + i]);
-    if constexpr (ND > 0) {
+    if constexpr (KIND == kCharges) {
+      out[i] = make_double2(s_sum[i], s_sum[kPairs + i]);
+    } else if constexpr (ND > 0) {
       // (n.grad) R_n^m from the moments G^k = sum s n_k R of degree n - 1
       const double* g = s_sum + 2 * NSL * kPairs;
       const int info = tab.pair[i];
@@ -672,7 +681,7 @@ __global__ void __launch_bounds__(32 * kCellWarps)
         ar /= rho;
         ai /= rho;
       }
-      if constexpr (DIFF) out[i] = make_double2(s_sum[i] - ar, s_sum[kPairs + i] - ai);
+      if constexpr (KIND == kDiff) out[i] = make_double2(s_sum[i] - ar, s_sum[kPairs + i] - ai);
       else out[((size_t)NSL + blockIdx.y) * cstride + i] = make_double2(ar, ai);
     }
   }
@@ -684,15 +693,18 @@ constexpr size_t p2m_smem()
   return sizeof(double) * (kCellWarps * kSumRows * kSumStride + (2 * NSL + 6 * ND) * tree_pairs(P));
 }
 
-// Far sums of one cell's rows: sum_a w_a phi_c(x_a) for every column c.
-template <int P, int NC>
+// Far sums of one cell's rows: sum_a w_a phi_c(x_a) for every column c; P1T:
+// sum_a w_a phi_k(x_a) phi(x_a) of one column with the triangle's three hat
+// functions.
+template <int P, int NC, bool P1T = false>
 __global__ void __launch_bounds__(32 * kCellWarps)
     tree_l2p_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh, TreeTables tab)
 {
   constexpr int kPairs = tree_pairs(P);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* s_loc = reinterpret_cast<double2*>(smem_raw);  // [NC][kPairs]
-  __shared__ double s_part[kCellWarps][NC][kCell];
+  constexpr int NO = P1T ? 3 : NC;
+  __shared__ double s_part[kCellWarps][NO][kCell];
   int cell = blockIdx.x;
   const TreeDesc& d = descs[tree_entry(off, nmesh, cell)];
   if (d.far.active && *d.far.active == 0) return;
@@ -711,33 +723,47 @@ __global__ void __launch_bounds__(32 * kCellWarps)
   const int sel = on ? tri : cell * kCell;
   CellPoints p;
   load_points(d, sel, 1.0 / d.ball[cell].w, p);
-  double w[kQ], phi[NC];
+  constexpr int NW = P1T ? 3 : 1;
+  double w[NW][kQ], phi[NO];
 #pragma unroll
-  for (int a = 0; a < kQ; ++a) w[a] = d.far.tgt64[(size_t)sel * kQ + a].w;
+  for (int a = 0; a < kQ; ++a) {
+    if constexpr (P1T) {
+      const dq q = d.far.tgtw64[(size_t)sel * kQ + a];
+      w[0][a] = q.x;
+      w[1][a] = q.y;
+      w[2][a] = q.z;
+    } else {
+      w[0][a] = d.far.tgt64[(size_t)sel * kQ + a].w;
+    }
+  }
 #pragma unroll
-  for (int c = 0; c < NC; ++c) phi[c] = 0.0;
+  for (int c = 0; c < NO; ++c) phi[c] = 0.0;
   __syncthreads();
   each_harmonic<P>(tab, p, warp, [&](int n, int m, const double (&re)[kQ], const double (&im)[kQ]) {
-    double hr = 0.0, hi = 0.0;
+    double hr[NW], hi[NW];
 #pragma unroll
-    for (int a = 0; a < kQ; ++a) {
-      hr += w[a] * re[a];
-      hi += w[a] * im[a];
+    for (int k = 0; k < NW; ++k) {
+      hr[k] = hi[k] = 0.0;
+#pragma unroll
+      for (int a = 0; a < kQ; ++a) {
+        hr[k] += w[k][a] * re[a];
+        hi[k] += w[k][a] * im[a];
+      }
     }
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const double2 l = s_loc[c * kPairs + tree_pair(n, m)];
-      phi[c] += l.x * hr + l.y * hi;
+    for (int c = 0; c < NO; ++c) {
+      const double2 l = s_loc[(P1T ? 0 : c) * kPairs + tree_pair(n, m)];
+      phi[c] += l.x * hr[P1T ? c : 0] + l.y * hi[P1T ? c : 0];
     }
   });
 #pragma unroll
-  for (int c = 0; c < NC; ++c) s_part[warp][c][lane] = phi[c];
+  for (int c = 0; c < NO; ++c) s_part[warp][c][lane] = phi[c];
   __syncthreads();
   if (warp == 0) {
     const size_t stride = (size_t)d.slot_off[d.ncells] * kCell;
     double* out = d.partial + d.first_col * stride + (size_t)(d.slot_off[cell + 1] - 1) * kCell + lane;
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
+    for (int c = 0; c < NO; ++c) {
       double v = 0.0;
 #pragma unroll
       for (int k = 0; k < kCellWarps; ++k) v += s_part[k][c][lane];
@@ -983,17 +1009,21 @@ __global__ void __launch_bounds__(32, 8)
     d.partial[c * stride + (size_t)task.w * kCell + lane] = active ? (double)hi[c] + (double)lo[c] : 0.0;
 }
 
-// The same in forward order only, for ND double-layer columns: every cell
-// against all its close cells (the full lists). With four columns a pair costs
-// 15 operations in either order; two symmetric passes of two columns, the most
-// whose sums fit the registers, cost the same.
+// The same in forward order only: every cell against all its close cells (the
+// full lists), for ND double-layer columns or (ND = 0) one single layer tested
+// with the three hat functions. With four columns a pair costs 15 operations
+// in either order; two symmetric passes of two columns, the most whose sums
+// fit the registers, cost the same. P1 charges do not factor over a source's
+// points, which the symmetric sums rely on.
 template <typename T, int ND>
 __global__ void __launch_bounds__(32, 8)
-    tree_near_dl_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh)
+    tree_near_forward_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh)
 {
   using S = typename Slot<T>::type;
   constexpr bool F32 = sizeof(T) == 4;
-  constexpr int NREC = rec_slots(0, ND);
+  constexpr bool P1T = ND == 0;
+  constexpr int NSL = P1T ? 1 : 0, NO = P1T ? 3 : ND, NDX = P1T ? 1 : ND;
+  constexpr int NREC = rec_slots(NSL, ND);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int4 s_vid[kCell];
   __shared__ dq s_nrm[kCell];
@@ -1012,9 +1042,9 @@ __global__ void __launch_bounds__(32, 8)
   const double cen[3] = {cd.x, cd.y, cd.z}, nrm[3] = {nd.x, nd.y, nd.z};
   const int4 tv = active ? md.tvid[tsel] : make_int4(-1, -1, -1, 0);
   const S* grec = reinterpret_cast<const S*>(md.rec);
-  T hi[ND], lo[ND];
+  T hi[NO], lo[NO];
 #pragma unroll
-  for (int c = 0; c < ND; ++c) hi[c] = lo[c] = 0;
+  for (int c = 0; c < NO; ++c) hi[c] = lo[c] = 0;
 #pragma unroll 1
   for (int e = task.y; e < task.z; ++e) {
     const int cell = d.entries[e].x, t0 = cell * kCell;
@@ -1053,7 +1083,7 @@ __global__ void __launch_bounds__(32, 8)
       const double rr = kFarRatio * (cc.w + ball.w);
       const bool far = ddx * ddx + ddy * ddy + ddz * ddz > rr * rr;
       const T o[3] = {(T)(cc.x - cen[0]), (T)(cc.y - cen[1]), (T)(cc.z - cen[2])};
-      T xs[kQ], ys[kQ], zs[kQ], q2[kQ], wq[kQ], sl[1][kQ], dl[ND][kQ];
+      T xs[kQ], ys[kQ], zs[kQ], q2[kQ], wq[kQ], sl[1][kQ], dl[NDX][kQ];
 #pragma unroll
       for (int a = 0; a < kQ; ++a) {
         S p;
@@ -1064,20 +1094,24 @@ __global__ void __launch_bounds__(32, 8)
         wq[a] = p.w;
         sl[0][a] = 0;
 #pragma unroll
-        for (int c = 0; c < ND; ++c) dl[c][a] = 0;
+        for (int c = 0; c < NDX; ++c) dl[c][a] = 0;
       }
       if constexpr (F32) {
-        if (far) eval_cell_sp<kQ, kQ, 0, ND, true>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
-        else eval_cell_sp<kQ, kQ, 0, ND, false>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+        if (far) eval_cell_sp<kQ, kQ, NSL, ND, true>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+        else eval_cell_sp<kQ, kQ, NSL, ND, false>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
       } else {
-        if (far) eval_cell<T, kQ, kQ, 0, ND, true>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
-        else eval_cell<T, kQ, kQ, 0, ND, false>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+        if (far) eval_cell<T, kQ, kQ, NSL, ND, true>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+        else eval_cell<T, kQ, kQ, NSL, ND, false>(s_rec, s_vid, s_nrm, s_plane, 0, ns, kQ, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
       }
 #pragma unroll
-      for (int c = 0; c < ND; ++c) {
+      for (int c = 0; c < NO; ++c) {
         T part = 0;
 #pragma unroll
-        for (int a = 0; a < kQ; ++a) part += wq[a] * dl[c][a];
+        for (int a = 0; a < kQ; ++a) {
+          if constexpr (P1T && F32) part += comp(md.tgtw32[(size_t)tsel * kQ + a], c) * sl[0][a];
+          else if constexpr (P1T) part += comp(md.tgtw64[(size_t)tsel * kQ + a], c) * sl[0][a];
+          else part += wq[a] * dl[c][a];
+        }
         if constexpr (F32) two_sum_add(hi[c], lo[c], part);
         else hi[c] += part;
       }
@@ -1086,7 +1120,7 @@ __global__ void __launch_bounds__(32, 8)
   }
   const size_t stride = (size_t)d.slot_off[d.ncells] * kCell;
 #pragma unroll
-  for (int c = 0; c < ND; ++c)
+  for (int c = 0; c < NO; ++c)
     d.partial[c * stride + (size_t)task.w * kCell + lane] = active ? (double)hi[c] + (double)lo[c] : 0.0;
 }
 
@@ -1241,7 +1275,7 @@ cudaError_t start(void (*fn)(Args...), dim3 grid, int block, size_t smem, cudaSt
   return cudaGetLastError();
 }
 
-template <int P, typename T, int NSL, int ND>
+template <int P, typename T, int NSL, int ND, bool P1 = false>
 int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const ApplyArgs* many, const TreeTables& tab,
                const TreeSide& side, cudaStream_t st)
 {
@@ -1258,16 +1292,23 @@ int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const
   }
   // a single double layer runs the SL+DL sums with zero charges (their records
   // hold zeros there; 1 of 9 or 14 operations), several the forward form
-  if constexpr (ND > 1)
-    EB_CUDA(start(tree_near_dl_kernel<T, ND>, dim3(g.ntasks), 32, (size_t)kCell * kQ * rec_slots(0, ND) * 4 * sizeof(T),
+  if constexpr (P1)
+    EB_CUDA(start(tree_near_forward_kernel<T, 0>, dim3(g.ntasks), 32, (size_t)kCell * kQ * rec_slots(1, 0) * 4 * sizeof(T),
+                  near, d, g.tasks, g.nmesh));
+  else if constexpr (ND > 1)
+    EB_CUDA(start(tree_near_forward_kernel<T, ND>, dim3(g.ntasks), 32, (size_t)kCell * kQ * rec_slots(0, ND) * 4 * sizeof(T),
                   near, d, g.tasks, g.nmesh));
   else
     EB_CUDA(start(tree_near_kernel<T, ND ? 1 : NSL, ND>, dim3(g.ntasks), 32, near_smem<T, ND ? 1 : NSL, ND>(), near, d,
                   g.tasks, g.nmesh));
   if (!g.expansions) return EB_OK;
   EB_CUDA(cudaEventRecord(side.join, side.st));
-  EB_CUDA(start(tree_p2m_kernel<P, NSL, PD>, dim3(g.ncells, ND > 1 ? ND : 1), 32 * kCellWarps, p2m_smem<P, NSL, PD>(), st,
-                d, g.cells, g.nmesh, one, many, tab));
+  if constexpr (P1)
+    EB_CUDA(start(tree_p2m_kernel<P, 0, 1, kCharges>, dim3(g.ncells), 32 * kCellWarps, p2m_smem<P, 0, 1>(), st, d, g.cells,
+                  g.nmesh, one, many, tab));
+  else
+    EB_CUDA(start(tree_p2m_kernel<P, NSL, PD>, dim3(g.ncells, ND > 1 ? ND : 1), 32 * kCellWarps, p2m_smem<P, NSL, PD>(),
+                  st, d, g.cells, g.nmesh, one, many, tab));
   for (int s = 0; s < kTreePasses; s++)
     EB_CUDA(start(tree_move_kernel<P, MC, kUp>, dim3(g.nup[s], NC / MC), b.x, Mv::smem(), st, d, g.up[s],
                   g.nmesh, s, tab));
@@ -1275,7 +1316,7 @@ int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const
                 0, tab));
   EB_CUDA(start(tree_move_kernel<P, MC, kDown>, dim3(g.ncells, NC / MC), b.x, Mv::smem(), st, d, g.cells,
                 g.nmesh, 0, tab));
-  EB_CUDA(start(tree_l2p_kernel<P, NC>, dim3(g.ncells), 32 * kCellWarps, sizeof(double2) * NC * tree_pairs(P), st, d,
+  EB_CUDA(start(tree_l2p_kernel<P, NC, P1>, dim3(g.ncells), 32 * kCellWarps, sizeof(double2) * NC * tree_pairs(P), st, d,
                 g.cells, g.nmesh, tab));
   EB_CUDA(cudaStreamWaitEvent(st, side.join, 0));
   return EB_OK;
@@ -1283,6 +1324,7 @@ int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const
 
 bool tree_variant(int nsl, int nd)
 {
+  if (nsl == kTreeP1) return nd == 0;
   return nd == 0 ? nsl == 1 || nsl == 3 || nsl == 4 : nsl == 0 ? nd == 1 || nd == 4 : nsl == 1 && nd == 1;
 }
 
@@ -1712,7 +1754,7 @@ int evaluate_order(Mesh* m, int n, const double* pts, const double* d_pts, const
   TreeDesc* dd = w.desc.as<TreeDesc>();
   EB_CUDA(cudaMemcpyAsync(dd, &d[0], sizeof(TreeDesc), cudaMemcpyHostToDevice, st));
   using Mv = MoveShape<P, 1>;
-  EB_CUDA(start(tree_p2m_kernel<P, 1, 1, true>, dim3(plan.ncells), 32 * kCellWarps, p2m_smem<P, 1, 1>(), st,
+  EB_CUDA(start(tree_p2m_kernel<P, 1, 1, kDiff>, dim3(plan.ncells), 32 * kCellWarps, p2m_smem<P, 1, 1>(), st,
                 (const TreeDesc*)dd, (const int*)nullptr, 1, A, (const ApplyArgs*)nullptr, tab));
   for (int s = 0; s < kTreePasses; s++)
     EB_CUDA(start(tree_move_kernel<P, 1, kUp>, dim3(d[0].nup[s]), Mv::kThreads, Mv::smem(), st, (const TreeDesc*)dd,
@@ -1789,6 +1831,9 @@ int tree_launch(bool fp32, int nsl, int nd, const TreeDesc* d, const TreeGrid& g
 {
   TreeTables tab = {};
   if (g.expansions) EB_CHECK(tables_for(device, fp32 ? kTreeOrder32 : kTreeOrder64, &tab));
+  if (nsl == kTreeP1 && nd == 0)
+    return fp32 ? launch_all<kTreeOrder32, float, 1, 0, true>(d, g, one, many, tab, side, st)
+                : launch_all<kTreeOrder64, double, 1, 0, true>(d, g, one, many, tab, side, st);
 #define EB_TREE(NSL, ND)                                                                        \
   if (nsl == NSL && nd == ND)                                                                   \
     return fp32 ? launch_all<kTreeOrder32, float, NSL, ND>(d, g, one, many, tab, side, st)            \
@@ -1814,7 +1859,7 @@ void tree_prepare(Mesh* m)
 bool tree_eligible(const Mesh* m, bool fp32, int nsl, int nd)
 {
   return m->plan.engine == 4 && m->tree && m->tree->usable && tree_variant(nsl, nd) &&
-         (fp32 || m->h.ncells >= kTreeMinCells64);
+         (fp32 || m->h.ncells >= (nsl == kTreeP1 ? kTreeMinCells64P1 : kTreeMinCells64));
 }
 
 static int upload_lists(TreeMesh* t)
@@ -1884,12 +1929,16 @@ TreeSide::~TreeSide()
 }
 
 // Close pairs of a variant in both orders at once, or forward only.
-static bool tree_forward(int nd) { return nd > 1; }
+static bool tree_forward(int nsl, int nd) { return nd > 1 || nsl == kTreeP1; }
+// Columns of its expansions and of its slots (a double layer alone leaves the
+// single layer's column unused).
+static int moved_columns(int nsl, int nd) { return nsl == kTreeP1 ? 1 : nsl + nd; }
+static int slot_columns(int nsl, int nd) { return nsl == kTreeP1 ? 3 : nd == 1 ? 2 : nsl + nd; }
 
-long long tree_far_slots(const Mesh* m, int nd)
+long long tree_far_slots(const Mesh* m, int nsl, int nd)
 {
   const TreeMesh& t = *m->tree;
-  return (long long)(tree_forward(nd) ? t.fwd : t.plan.sym).slot_off.back() * kCell;
+  return (long long)(tree_forward(nsl, nd) ? t.fwd : t.plan.sym).slot_off.back() * kCell;
 }
 
 static int upload_forward(TreeMesh* t)
@@ -1917,12 +1966,9 @@ size_t tree_expansion_bytes(const Mesh* m, int order, int cols)
   return m->tree->plan.all_close ? 0 : sizeof(double2) * (size_t)cols * m->tree->plan.nnodes * tree_pairs(order);
 }
 
-// A double layer alone leaves the single layer's column unused.
-static int slot_columns(int nsl, int nd) { return nd == 1 ? 2 : nsl + nd; }
-
 size_t tree_partial_bytes(const Mesh* m, int nsl, int nd)
 {
-  return sizeof(double) * (size_t)slot_columns(nsl, nd) * tree_far_slots(m, nd);
+  return sizeof(double) * (size_t)slot_columns(nsl, nd) * tree_far_slots(m, nsl, nd);
 }
 
 int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, void* local, double* partial,
@@ -1931,19 +1977,19 @@ int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, v
   TreeMesh* t = m->tree.get();
   EB_CHECK(upload_lists(t));
   TreeDesc d = t->base;
-  if (tree_forward(nd)) {
+  if (tree_forward(nsl, nd)) {
     EB_CHECK(upload_forward(t));
     d.tasks = t->fwd_lists.as<int4>();
     d.entries = reinterpret_cast<const int2*>(d.tasks + t->fwd.tasks.size());
     d.slot_off = reinterpret_cast<const int*>(d.entries + t->fwd.entries.size());
     d.ntasks = (int)t->fwd.tasks.size();
   }
-  d.far = mesh_far_desc(m, fp32, nsl, nd, rec, partial);
+  d.far = mesh_far_desc(m, fp32, nsl == kTreeP1 ? 1 : nsl, nd, rec, partial);
   d.pos = m->pos64.as<dq>();
   d.multipole = static_cast<double2*>(multipole);
   d.local = static_cast<double2*>(local);
   d.partial = partial;
-  d.first_col = slot_columns(nsl, nd) - nsl - nd;
+  d.first_col = nsl == 0 && nd == 1 ? 1 : 0;
   *out = d;
   return EB_OK;
 }
@@ -1991,8 +2037,8 @@ int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream
   std::unique_ptr<TreeScratch>& sc = t->scratch[(fp32 ? 64 : 0) + nsl * 5 + nd];
   if (!sc) {
     auto s = std::make_unique<TreeScratch>();
-    if (tree_forward(nd)) EB_CHECK(upload_forward(t));  // its slots are counted below
-    const size_t bytes = tree_expansion_bytes(m, fp32 ? kTreeOrder32 : kTreeOrder64, nsl + nd);
+    if (tree_forward(nsl, nd)) EB_CHECK(upload_forward(t));  // its slots are counted below
+    const size_t bytes = tree_expansion_bytes(m, fp32 ? kTreeOrder32 : kTreeOrder64, moved_columns(nsl, nd));
     if (bytes) {
       EB_CHECK(s->multipole.alloc(bytes));
       EB_CHECK(s->local.alloc(bytes));
@@ -2004,7 +2050,7 @@ int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream
     sc = std::move(s);
   }
   const TreeDesc& d = sc->host;
-  A->partial = d.partial + (size_t)d.first_col * tree_far_slots(m, nd);
+  A->partial = d.partial + (size_t)d.first_col * tree_far_slots(m, nsl, nd);
   A->slot_off = d.slot_off;
   TreeGrid g;
   g.ncells = d.ncells;

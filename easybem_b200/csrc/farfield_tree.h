@@ -32,6 +32,10 @@ struct TreeMovesDev {
   const int* src;
 };
 
+// Operator combinations are (nsl, nd) as elsewhere; this nsl with nd = 0 is the
+// P1 single layer (one column of vertex values in ApplyArgs::u, three outputs).
+constexpr int kTreeP1 = 12;
+
 // Per-mesh view of the kernels (device pointers); a batch passes an array.
 struct TreeDesc {
   FarMeshDesc far;           // records and tables of the close pairs
@@ -109,7 +113,7 @@ bool tree_eligible(const Mesh* m, bool fp32, int nsl, int nd);
 // (A.partial and A.slot_off are set for the finalize).
 int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream_t st);
 // Partial slots (summed over the rows, per output).
-long long tree_far_slots(const Mesh* m, int nd);
+long long tree_far_slots(const Mesh* m, int nsl, int nd);
 // Descriptor of mesh m for one variant over the given scratch (tree_scratch_bytes);
 // uploads the mesh's lists the first time.
 int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, void* local, double* partial,

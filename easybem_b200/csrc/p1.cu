@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "farfield_tree.h"
 #include "pairs.h"
 
 namespace eb {
@@ -55,20 +56,25 @@ __global__ void p1_gather_kernel(const int* __restrict__ cptr, const int* __rest
 __global__ void p1_finalize_kernel(int nv, int nchunk, int nsplit, int nitems, const int* __restrict__ vptr,
                                    const int* __restrict__ vlist, const int* __restrict__ iperm,
                                    const dq* __restrict__ trin, const double* __restrict__ partial,
-                                   const int* __restrict__ rowptr, const int* __restrict__ col,
+                                   const int* __restrict__ slot_off, int ncells, const int* __restrict__ rowptr, const int* __restrict__ col,
                                    const double* __restrict__ val, const double* __restrict__ t,
                                    double* __restrict__ v)
 {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= nv) return;
-  const size_t stride = (size_t)nsplit * nitems;
+  const size_t stride = slot_off ? (size_t)slot_off[ncells] * kCell : (size_t)nsplit * nitems;
   double far = 0.0;
   for (int p = vptr[a]; p < vptr[a + 1]; p++) {
     const int i = vlist[p] >> 2, k = vlist[p] & 3;
     const int s = iperm[i];
     double f = 0.0;
-    for (int sp = 0; sp < nsplit; sp++)
-      for (int ch = 0; ch < nchunk; ch++) f += partial[k * stride + (size_t)sp * nitems + (size_t)s * nchunk + ch];
+    if (slot_off) {  // the tree's slots of the triangle's cell
+      const int c = s / kCell;
+      const double* row = partial + k * stride + (s - c * kCell);
+      for (int q = slot_off[c]; q < slot_off[c + 1]; q++) f += row[(size_t)q * kCell];
+    } else
+      for (int sp = 0; sp < nsplit; sp++)
+        for (int ch = 0; ch < nchunk; ch++) f += partial[k * stride + (size_t)sp * nitems + (size_t)s * nchunk + ch];
     far += trin[s].w * (0.25 / M_PI) * f;
   }
   double nr = 0.0;
@@ -81,39 +87,53 @@ static int ensure_p1_near(Mesh* m)
   if (m->p1_val.p) return EB_OK;
   const HostMesh& h = m->h;
   const int npairs = (int)h.sl_col.size();
-  // entries e = 9p + 3k + l at (test vertex, trial vertex), bucketed by row
-  std::vector<int> erow(9 * (size_t)npairs), ecol(9 * (size_t)npairs);
+  // Entries e = 9p + 3k + l at (test vertex, trial vertex), bucketed by row; in
+  // each row the columns ascend, and the entries of a column. Columns are told
+  // apart by marks and only the distinct ones sorted, about a third of the
+  // time of sorting all entries (first apply of 13,530 triangles: 39 -> 14 ms).
+  std::vector<unsigned short> orders(npairs);  // local vertices of the test and trial triangle, 2 bits each
+  std::vector<int> rcount(h.nv + 1, 0);
   for (int p = 0; p < npairs; p++) {
     const int i = h.pair_i[p], j = h.sl_col[p];
     const PairGeom g = classify_pair(&h.elems[3 * i], &h.elems[3 * j], i == j);
     int oi[3], oj[3];
     p1_local_orders(g, oi, oj);
-    for (int k = 0; k < 3; k++)
-      for (int l = 0; l < 3; l++) {
-        erow[9 * (size_t)p + 3 * k + l] = h.elems[3 * i + oi[k]];
-        ecol[9 * (size_t)p + 3 * k + l] = h.elems[3 * j + oj[l]];
-      }
+    unsigned packed = 0;
+    for (int k = 0; k < 3; k++) {
+      packed |= oi[k] << (2 * k) | oj[k] << (2 * k + 6);
+      rcount[h.elems[3 * i + oi[k]] + 1] += 3;
+    }
+    orders[p] = (unsigned short)packed;
   }
-  std::vector<int> rcount(h.nv + 1, 0);
-  for (int r : erow) rcount[r + 1]++;
   for (int v = 0; v < h.nv; v++) rcount[v + 1] += rcount[v];
-  std::vector<int> byrow(erow.size());
+  const size_t nent = 9 * (size_t)npairs;
+  std::vector<int2> byrow(nent);  // column, entry
   {
     std::vector<int> fill(rcount.begin(), rcount.end() - 1);
-    for (size_t e = 0; e < erow.size(); e++) byrow[fill[erow[e]]++] = (int)e;
-  }
-  std::vector<int> rowptr(h.nv + 1, 0), cols, cptr(1, 0), contrib;
-  contrib.reserve(erow.size());
-  for (int a = 0; a < h.nv; a++) {
-    std::vector<std::pair<int, int>> es;
-    for (int q = rcount[a]; q < rcount[a + 1]; q++) es.push_back({ecol[byrow[q]], byrow[q]});
-    std::sort(es.begin(), es.end());
-    for (size_t q = 0; q < es.size(); q++) {
-      if (q > 0 && es[q].first != es[q - 1].first) cptr.push_back((int)contrib.size());
-      if (q == 0 || es[q].first != es[q - 1].first) cols.push_back(es[q].first);
-      contrib.push_back(es[q].second);
+    for (int p = 0; p < npairs; p++) {
+      const int *vi = &h.elems[3 * (size_t)h.pair_i[p]], *vj = &h.elems[3 * (size_t)h.sl_col[p]];
+      for (int k = 0; k < 3; k++) {
+        int2* row = &byrow[fill[vi[orders[p] >> (2 * k) & 3]]];
+        for (int l = 0; l < 3; l++) row[l] = make_int2(vj[orders[p] >> (2 * l + 6) & 3], 9 * p + 3 * k + l);
+        fill[vi[orders[p] >> (2 * k) & 3]] += 3;
+      }
     }
-    if (!es.empty()) cptr.push_back((int)contrib.size());
+  }
+  std::vector<int> rowptr(h.nv + 1, 0), cols, cptr(1, 0), contrib(nent), count(h.nv, 0);
+  cols.reserve(nent / 9);
+  cptr.reserve(nent / 9 + 1);
+  for (int a = 0; a < h.nv; a++) {
+    const size_t first = cols.size();
+    for (int q = rcount[a]; q < rcount[a + 1]; q++)
+      if (count[byrow[q].x]++ == 0) cols.push_back(byrow[q].x);
+    std::sort(cols.begin() + first, cols.end());
+    for (size_t c = first; c < cols.size(); c++) {
+      const int n = count[cols[c]];
+      count[cols[c]] = cptr.back();  // where the column's next entry goes
+      cptr.push_back(cptr.back() + n);
+    }
+    for (int q = rcount[a]; q < rcount[a + 1]; q++) contrib[count[byrow[q].x]++] = byrow[q].y;
+    for (size_t c = first; c < cols.size(); c++) count[cols[c]] = 0;
     rowptr[a + 1] = (int)cols.size();
   }
   DevBuf d_nodes, d_elems, d_pi, d_pj, d_ent, d_cptr, d_contrib;
@@ -130,7 +150,7 @@ static int ensure_p1_near(Mesh* m)
   EB_CHECK(up(d_contrib, contrib.data(), sizeof(int) * contrib.size()));
   EB_CHECK(up(m->p1_rowptr, rowptr.data(), sizeof(int) * rowptr.size()));
   EB_CHECK(up(m->p1_col, cols.data(), sizeof(int) * cols.size()));
-  EB_CHECK(d_ent.alloc(sizeof(double) * std::max<size_t>(erow.size(), 1)));
+  EB_CHECK(d_ent.alloc(sizeof(double) * std::max<size_t>(nent, 1)));
   EB_CHECK(m->p1_val.alloc(sizeof(double) * std::max<size_t>(cols.size(), 1)));
   cudaStream_t st = nullptr;
   EB_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
@@ -158,12 +178,10 @@ int mesh_apply_sl_p1(Mesh* m, int precision, const double* d_t, double* d_v, cud
   EB_CHECK(ensure_p1_near(m));
   EB_CHECK(ensure_vertex_lists(m));
   const HostMesh& h = m->h;
-  if (!m->rec.p) {
-    EB_CHECK(m->rec.alloc((size_t)h.ne * h.Q * kMaxRecSlots * sizeof(dq)));
-    EB_CHECK(m->partial.alloc(sizeof(double) * (size_t)kMaxOutputs * m->plan.nsplit * h.nitems));
-  }
+  EB_CHECK(ensure_apply_scratch(m));
+  const bool tree = tree_eligible(m, fp32, kTreeP1, 0);
   Mesh::Variant& var = m->variants[100 + (fp32 ? 1 : 0)];
-  if (!var.desc.p) {
+  if (!tree && !var.desc.p) {
     const FarMeshDesc desc = mesh_far_desc(m, fp32, 1, false, m->rec.p, m->partial.as<double>());
     const size_t smem = far_smem_bytes(desc.src_tile, h.Q, rec_slots(1, false), fp32);
     int occ = far_occupancy(fp32, 1, false, h.K, h.Q, smem, true);
@@ -178,15 +196,19 @@ int mesh_apply_sl_p1(Mesh* m, int precision, const double* d_t, double* d_v, cud
   }
   // records: the DL strength slot (w_b J_j u_h(y_b)) is where the single SL
   // charge of the far kernel is read (record slot 1, component 0)
-  const ApplyArgs A = mesh_apply_args(m, fp32, m->rec.p, nullptr, nullptr, h.ne, d_t, nullptr, h.ne, nullptr);
+  ApplyArgs A = mesh_apply_args(m, fp32, m->rec.p, m->partial.as<double>(), nullptr, h.ne, d_t, nullptr, h.ne, nullptr);
   EB_CUDA(prep_launch(fp32, 0, true, A, st));
-  EB_CUDA(cudaMemsetAsync(m->counter.p, 0, sizeof(int), st));
-  EB_CUDA(far_launch(fp32, 1, false, h.K, h.Q, var.desc.as<FarMeshDesc>(), m->items.as<WorkItem>(), m->nitems_work,
-                     m->counter.as<int>(), var.smem, var.grid, st, true));
+  if (tree) {
+    EB_CHECK(tree_far_apply(m, fp32, kTreeP1, 0, &A, st));
+  } else {
+    EB_CUDA(cudaMemsetAsync(m->counter.p, 0, sizeof(int), st));
+    EB_CUDA(far_launch(fp32, 1, false, h.K, h.Q, var.desc.as<FarMeshDesc>(), m->items.as<WorkItem>(), m->nitems_work,
+                       m->counter.as<int>(), var.smem, var.grid, st, true));
+  }
   p1_finalize_kernel<<<(h.nv + 127) / 128, 128, 0, st>>>(
       h.nv, h.nchunk, m->plan.nsplit, h.nitems, m->vtri_ptr.as<int>(), m->vtri_list.as<int>(), m->iperm.as<int>(),
-      m->trin.as<dq>(), m->partial.as<double>(), m->p1_rowptr.as<int>(), m->p1_col.as<int>(), m->p1_val.as<double>(),
-      d_t, d_v);
+      m->trin.as<dq>(), A.partial, A.slot_off, h.ncells, m->p1_rowptr.as<int>(), m->p1_col.as<int>(),
+      m->p1_val.as<double>(), d_t, d_v);
   EB_CUDA(cudaGetLastError());
   return EB_OK;
 }

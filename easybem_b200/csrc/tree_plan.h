@@ -59,7 +59,9 @@ constexpr int kTreeAllCloseCells = 140;
 // Least cells of an FP64 apply on the tree: below, a pair of cells (22 us on an
 // SM quarter) is too coarse a task, and the ordered-pair kernel's finer items
 // finish first (512 triangles, SL+DL: 69 us against 96; 1,200: 134 against 121).
-constexpr int kTreeMinCells64 = 28;
+// The P1 single layer alone costs a third of that (128 triangles, 4 cells: 77
+// against 69 us; 512: 103 against 78; 36 triangles: 67.6 against 69.9).
+constexpr int kTreeMinCells64 = 28, kTreeMinCells64P1 = 4;
 
 // Expansions moved into node tgt[k] from nodes src[ptr[k] .. ptr[k + 1]). The
 // upper 8 bits of a source are the share f / 255 of the degrees that its pair

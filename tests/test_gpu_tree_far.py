@@ -68,6 +68,9 @@ def test_tree_matches_oracle_and_symmetric_kernels(gpu_lib, oracle, name):
             d = m.apply_hypersingular(u, precision=prec)
             qs = m.apply_dl(u, precision=prec)
             assert rel_l2(qs[rows], qo) < tol
+            w = m.apply_sl_p1(u, precision=prec)
+            m.set_far_engine("cuda")
+            assert rel_l2(w, m.apply_sl_p1(u, precision=prec)) < tol
             m.set_far_engine("sym_all")
             vd, qd = m.apply_sl_dl(t, u, precision=prec)
             assert rel_l2(v, vd) < tol and rel_l2(q, qd) < tol
@@ -151,10 +154,12 @@ def test_small_meshes_sum_all_cell_pairs(gpu_lib, oracle, ne):
             m.set_far_engine("tree")
             v, q = m.apply_sl_dl(t, u, precision=prec)
             vs, qs, b, d = m.apply_sl(t, prec), m.apply_dl(u, prec), m.dirichlet_rhs(g, prec), m.apply_hypersingular(u, prec)
+            p = m.apply_sl_p1(u, prec)
             assert rel_l2(v[rows], vo) < tol and rel_l2(vs[rows], vo) < tol
             m.set_far_engine("cuda")
             w, r = m.apply_sl_dl(t, u, precision=prec)
             c, e = m.dirichlet_rhs(g, prec), m.apply_hypersingular(u, prec)
+            assert rel_l2(p, m.apply_sl_p1(u, prec)) < tol
             if ne == 1:  # no pair but the triangle with itself: K u = 0
                 assert not q.any() and not qs.any() and not r.any()
             else:
