@@ -125,6 +125,8 @@ int autotune(Mesh* m, int precision, int operators, int reps, int* best_ips, int
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   const FarPlan start = m->plan;
+  // the plan shapes the direct kernels: a mesh on the tree is timed without it
+  if (m->plan.engine == EB_FAR_TREE) m->plan.engine = EB_FAR_SYMMETRIC;
   const int deft = src_tile_for(h.Q, precision == EB_PREC_MIXED, nsl, dl);
   std::vector<int> tiles{0};
   for (int c : {32, 16})
@@ -156,6 +158,7 @@ int autotune(Mesh* m, int precision, int operators, int reps, int* best_ips, int
   // keep the winner (or put the starting plan back after a failure)
   const int rc2 = rc == EB_OK ? mesh_set_plan(m, best.items_per_sm, best.tile)
                               : mesh_set_plan(m, start.items_per_sm, start.tile);
+  m->plan.engine = start.engine;
   if (rc != EB_OK) return rc;
   EB_CHECK(rc2);
   {

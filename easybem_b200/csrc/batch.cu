@@ -217,6 +217,7 @@ int Batch::build_tree(const std::vector<TreeDesc>& desc, const std::vector<Apply
     return at;
   };
   TreeGrid g;
+  g.rule = Q_;
   g.nmesh = n;
   g.ntasks = blocks([](const TreeDesc& d) { return d.ntasks; });
   g.ncells = blocks([](const TreeDesc& d) { return d.multipole ? d.ncells : 0; });

@@ -635,7 +635,7 @@ bool sym_eligible(const Mesh* m, bool fp32, int nsl, int nd, bool fp64_internal)
 
 long long mesh_far_slots(const Mesh* m, bool fp32, int nsl, int nd)
 {
-  if (tree_eligible(m, fp32, nsl, nd) && (nd <= 1 || !m->tree->fwd.slot_off.empty())) return tree_far_slots(m, nsl, nd);
+  if (tree_eligible(m, fp32, nsl, nd)) return tree_far_slots(m, nsl, nd);
   if (sym_eligible(m, fp32, nsl, nd)) {
     const int r = far_sym_cells_per_item(kSymCellsPerItem);
     long long n = 0;

@@ -481,15 +481,20 @@ __global__ void __launch_bounds__(MoveShape<P, NC>::kThreads, MoveShape<P, NC>::
 constexpr int kCellWarps = 4;
 constexpr int kSumRows = 8, kSumStride = 36;  // conflict-free rows of the lane sums
 
+constexpr int kWideItem = 8;  // target points per item of rules of more than 7
+constexpr int kWideTile = 8;  // source triangles staged at a time for those rules (even)
+
 struct CellPoints {
   double x[kQ], y[kQ], z[kQ], r2[kQ];
 };
 
-__device__ __forceinline__ void load_points(const TreeDesc& d, int tri, double inv_rho, CellPoints& p)
+// Points first .. first + kQ of a rule of Q (the last repeated past its end).
+__device__ __forceinline__ void load_points(const TreeDesc& d, int tri, double inv_rho, CellPoints& p, int Q = kQ,
+                                            int first = 0)
 {
 #pragma unroll
   for (int a = 0; a < kQ; ++a) {
-    const dq q = d.pos[(size_t)tri * kQ + a];
+    const dq q = d.pos[(size_t)tri * Q + min(first + a, Q - 1)];
     p.x[a] = -0.5 * q.x * inv_rho;
     p.y[a] = -0.5 * q.y * inv_rho;
     p.z[a] = -0.5 * q.z * inv_rho;
@@ -549,8 +554,9 @@ __device__ __forceinline__ void each_harmonic(const TreeTables& tab, const CellP
 // R(y_b)), and for ND = 1 the double-layer column blockIdx.y. KIND: both apart,
 // single minus double layer in one column (the representation formula), or
 // the strengths of the double-layer column as charges (P1 single layer).
+// WIDE: a rule of more than kQ points, kQ at a time.
 enum Sources { kApart, kDiff, kCharges };
-template <int P, int NSL, int ND, int KIND = kApart>
+template <int P, int NSL, int ND, int KIND = kApart, bool WIDE = false>
 __global__ void __launch_bounds__(32 * kCellWarps)
     tree_p2m_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh, ApplyArgs one,
                     const ApplyArgs* __restrict__ many, TreeTables tab)
@@ -571,25 +577,29 @@ __global__ void __launch_bounds__(32 * kCellWarps)
   const int tri = cell * kCell + lane;
   const bool on = tri < A.ne;
   const int sel = on ? tri : cell * kCell;
-  CellPoints p;
-  load_points(d, sel, 1.0 / rho, p);
-  double wj[kQ], s[kQ], t[NSL > 0 ? NSL : 1], nrm[3] = {0.0, 0.0, 0.0};
+  double t[NSL > 0 ? NSL : 1], nrm[3] = {0.0, 0.0, 0.0}, u0 = 0.0, u1 = 0.0, u2 = 0.0;
   const int orig = A.perm[sel];
-#pragma unroll
-  for (int a = 0; a < kQ; ++a) wj[a] = on ? A.wj[(size_t)sel * kQ + a] : 0.0;
 #pragma unroll
   for (int c = 0; c < NSL; ++c) t[c] = A.t[(size_t)c * A.tstride + orig];
   if constexpr (ND > 0) {
     const int4 v = A.svid[sel];
     const double* u = A.u + (size_t)blockIdx.y * A.ustride;
-    const double u0 = u[v.x], u1 = u[v.y], u2 = u[v.z];
-#pragma unroll
-    for (int a = 0; a < kQ; ++a) {
-      const double e1 = A.bary[2 * a], e2 = A.bary[2 * a + 1];
-      s[a] = wj[a] * ((1.0 - e1 - e2) * u0 + e1 * u1 + e2 * u2);
-    }
+    u0 = u[v.x]; u1 = u[v.y]; u2 = u[v.z];
     const dq n = A.trin[sel];
     nrm[0] = n.x; nrm[1] = n.y; nrm[2] = n.z;
+  }
+  const int Q = WIDE ? A.Q : kQ;
+#pragma unroll 1
+  for (int first = 0; first < Q; first += kQ) {
+    CellPoints p;
+    load_points(d, sel, 1.0 / rho, p, Q, first);
+    double wj[kQ], s[kQ];
+#pragma unroll
+    for (int a = 0; a < kQ; ++a) {
+      const int b = min(first + a, Q - 1);
+      wj[a] = on && first + a < Q ? A.wj[(size_t)sel * Q + b] : 0.0;
+      const double e1 = A.bary[2 * b], e2 = A.bary[2 * b + 1];
+      s[a] = wj[a] * ((1.0 - e1 - e2) * u0 + e1 * u1 + e2 * u2);
   }
   each_harmonic<P>(tab, p, warp, [&](int n, int m, const double (&re)[kQ], const double (&im)[kQ]) {
     int row = 0;
@@ -633,9 +643,13 @@ __global__ void __launch_bounds__(32 * kCellWarps)
       for (int k = 0; k < 8; ++k) v += s_red[r * kSumStride + part + 4 * k];
     v += __shfl_xor_sync(0xffffffffu, v, 1);
     v += __shfl_xor_sync(0xffffffffu, v, 2);
-    if (part == 0 && r < kRows) s_sum[r * kPairs + tree_pair(n, m)] = v;
+    if (part == 0 && r < kRows) {
+      double* sum = &s_sum[r * kPairs + tree_pair(n, m)];
+      *sum = WIDE && first ? *sum + v : v;  // the same thread every time
+    }
     __syncwarp();
   });
+  }
   __syncthreads();
   const size_t cstride = (size_t)d.nnodes * kPairs;
   double2* out = d.multipole + (size_t)cell * kPairs;
@@ -695,8 +709,8 @@ constexpr size_t p2m_smem()
 
 // Far sums of one cell's rows: sum_a w_a phi_c(x_a) for every column c; P1T:
 // sum_a w_a phi_k(x_a) phi(x_a) of one column with the triangle's three hat
-// functions.
-template <int P, int NC, bool P1T = false>
+// functions. WIDE: a rule of more than kQ points, kQ at a time.
+template <int P, int NC, bool P1T = false, bool WIDE = false>
 __global__ void __launch_bounds__(32 * kCellWarps)
     tree_l2p_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh, TreeTables tab)
 {
@@ -721,24 +735,29 @@ __global__ void __launch_bounds__(32 * kCellWarps)
   const int tri = cell * kCell + lane;
   const bool on = tri < d.far.ne;
   const int sel = on ? tri : cell * kCell;
-  CellPoints p;
-  load_points(d, sel, 1.0 / d.ball[cell].w, p);
   constexpr int NW = P1T ? 3 : 1;
-  double w[NW][kQ], phi[NO];
-#pragma unroll
-  for (int a = 0; a < kQ; ++a) {
-    if constexpr (P1T) {
-      const dq q = d.far.tgtw64[(size_t)sel * kQ + a];
-      w[0][a] = q.x;
-      w[1][a] = q.y;
-      w[2][a] = q.z;
-    } else {
-      w[0][a] = d.far.tgt64[(size_t)sel * kQ + a].w;
-    }
-  }
+  double phi[NO];
 #pragma unroll
   for (int c = 0; c < NO; ++c) phi[c] = 0.0;
   __syncthreads();
+  const int Q = WIDE ? d.far.Q : kQ;
+  const size_t at = (size_t)sel * (WIDE ? d.far.nitems / d.far.ne * kWideItem : kQ);
+#pragma unroll 1
+  for (int first = 0; first < Q; first += kQ) {
+    CellPoints p;
+    load_points(d, sel, 1.0 / d.ball[cell].w, p, Q, first);
+    double w[NW][kQ];
+#pragma unroll
+    for (int a = 0; a < kQ; ++a) {
+      if constexpr (P1T) {
+        const dq q = d.far.tgtw64[at + a];
+        w[0][a] = q.x;
+        w[1][a] = q.y;
+        w[2][a] = q.z;
+      } else {
+        w[0][a] = first + a < Q ? d.far.tgt64[at + first + a].w : 0.0;
+      }
+  }
   each_harmonic<P>(tab, p, warp, [&](int n, int m, const double (&re)[kQ], const double (&im)[kQ]) {
     double hr[NW], hi[NW];
 #pragma unroll
@@ -756,6 +775,7 @@ __global__ void __launch_bounds__(32 * kCellWarps)
       phi[c] += l.x * hr[P1T ? c : 0] + l.y * hi[P1T ? c : 0];
     }
   });
+  }
 #pragma unroll
   for (int c = 0; c < NO; ++c) s_part[warp][c][lane] = phi[c];
   __syncthreads();
@@ -1124,6 +1144,125 @@ __global__ void __launch_bounds__(32, 8)
     d.partial[c * stride + (size_t)task.w * kCell + lane] = active ? (double)hi[c] + (double)lo[c] : 0.0;
 }
 
+// The same for rules of more than 7 points, whose triangles are items of
+// kWideItem target points (the last padded with zero weights): a lane runs its
+// triangle's items one after the other against kWideTile staged sources, so
+// that the FP64 records of a rule of 25 points leave 17 warps on an SM (4 with
+// whole cells). Host apply of one operator, 8,192 triangles: rule of 16
+// points FP64 12.44 -> 2.95 ms, mixed 5.95 -> 1.33; of 25, 38.3 -> 8.1 and
+// 17.9 -> 3.7.
+template <typename T, int NSL, int ND>
+__global__ void __launch_bounds__(32)
+    tree_near_wide_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh)
+{
+  using S = typename Slot<T>::type;
+  constexpr bool F32 = sizeof(T) == 4;
+  constexpr int K = kWideItem, NO = NSL + ND, NSX = NSL > 0 ? NSL : 1, NDX = ND > 0 ? ND : 1;
+  constexpr int NREC = rec_slots(NSL, ND);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int4 s_vid[kWideTile];
+  __shared__ dq s_nrm[kWideTile];
+  __shared__ S s_plane[kWideTile];
+  S* s_rec = reinterpret_cast<S*>(smem_raw);
+  const int lane = threadIdx.x;
+  int k = blockIdx.x;
+  const TreeDesc& d = descs[tree_entry(off, nmesh, k)];
+  const FarMeshDesc& md = d.far;
+  if (md.active && *md.active == 0) return;
+  const int4 task = d.tasks[k];
+  const int ti = task.x * kCell + lane;
+  const bool active = ti < md.ne;
+  const int tsel = active ? ti : task.x * kCell;
+  const int Q = md.Q, nchunk = md.nitems / md.ne, per = Q * NREC;
+  const size_t item0 = (size_t)tsel * nchunk;
+  const dq ball = md.ccent[task.x], cd = md.tcent[item0], nd = md.tnrm[item0];
+  const double cen[3] = {cd.x, cd.y, cd.z}, nrm[3] = {nd.x, nd.y, nd.z};
+  const int4 tv = active ? md.tvid[item0] : make_int4(-1, -1, -1, 0);
+  const S* grec = reinterpret_cast<const S*>(md.rec);
+  T hi[NO], lo[NO];
+#pragma unroll
+  for (int c = 0; c < NO; ++c) hi[c] = lo[c] = 0;
+#pragma unroll 1
+  for (int e = task.y; e < task.z; ++e) {
+    const int cell = d.entries[e].x, end = min(cell * kCell + kCell, md.ne);
+    const dq cc = md.ccent[cell];
+    const double ddx = cc.x - ball.x, ddy = cc.y - ball.y, ddz = cc.z - ball.z;
+    const double rr = kFarRatio * (cc.w + ball.w);
+    const bool far = ddx * ddx + ddy * ddy + ddz * ddz > rr * rr;
+    const T o[3] = {(T)(cc.x - cen[0]), (T)(cc.y - cen[1]), (T)(cc.z - cen[2])};
+#pragma unroll 1
+    for (int t0 = cell * kCell; t0 < end; t0 += kWideTile) {
+      const int ns = min(kWideTile, end - t0);
+      const S* g = grec + (size_t)t0 * per;
+      if constexpr (F32) {  // source-pair layout
+        const int nstage = ((ns + 1) >> 1) * per;
+        for (int i = lane; i < nstage; i += 32) {
+          const int p = i / per, rem = i - p * per;
+          const float4 a = g[(size_t)(2 * p) * per + rem];
+          float4 c;
+          if (2 * p + 1 < ns) c = g[(size_t)(2 * p + 1) * per + rem];
+          else c = rem % NREC == 0 ? make_float4(0.f, 0.f, 0.f, 1.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+          s_rec[2 * i] = make_float4(a.x, c.x, a.y, c.y);
+          s_rec[2 * i + 1] = make_float4(a.z, c.z, a.w, c.w);
+        }
+        if ((ns & 1) && lane == 0) {
+          s_vid[ns] = make_int4(-1, -1, -1, 0);
+          s_nrm[ns] = dq{0.0, 0.0, 0.0, 0.0};
+          s_plane[ns] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      } else {
+        for (int i = lane; i < ns * per; i += 32) s_rec[i] = g[i];
+      }
+      if (lane < ns) {
+        s_vid[lane] = md.svid[t0 + lane];
+        s_nrm[lane] = md.snrm[t0 + lane];
+        if constexpr (F32) s_plane[lane] = md.splane32[t0 + lane];
+        else s_plane[lane] = md.splane64[t0 + lane];
+      }
+      __syncwarp();
+      if (active) {
+#pragma unroll 1
+        for (int ch = 0; ch < nchunk; ++ch) {
+          T xs[K], ys[K], zs[K], q2[K], wq[K], sl[NSX][K], dl[NDX][K];
+#pragma unroll
+          for (int a = 0; a < K; ++a) {
+            S p;
+            if constexpr (F32) p = md.tgt32[(item0 + ch) * K + a];
+            else p = md.tgt64[(item0 + ch) * K + a];
+            xs[a] = p.x - o[0]; ys[a] = p.y - o[1]; zs[a] = p.z - o[2];
+            q2[a] = xs[a] * xs[a] + ys[a] * ys[a] + zs[a] * zs[a];
+            wq[a] = p.w;
+#pragma unroll
+            for (int c = 0; c < NSX; ++c) sl[c][a] = 0;
+#pragma unroll
+            for (int c = 0; c < NDX; ++c) dl[c][a] = 0;
+          }
+          if constexpr (F32) {
+            if (far) eval_cell_sp<K, 0, NSL, ND, true>(s_rec, s_vid, s_nrm, s_plane, 0, ns, Q, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+            else eval_cell_sp<K, 0, NSL, ND, false>(s_rec, s_vid, s_nrm, s_plane, 0, ns, Q, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+          } else {
+            if (far) eval_cell<T, K, 0, NSL, ND, true>(s_rec, s_vid, s_nrm, s_plane, 0, ns, Q, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+            else eval_cell<T, K, 0, NSL, ND, false>(s_rec, s_vid, s_nrm, s_plane, 0, ns, Q, tv, xs, ys, zs, q2, o, cen, nrm, sl, dl);
+          }
+#pragma unroll
+          for (int c = 0; c < NO; ++c) {
+            T part = 0;
+#pragma unroll
+            for (int a = 0; a < K; ++a) part += wq[a] * (c < NSL ? sl[c < NSL ? c : 0][a] : dl[c < NSL ? 0 : c - NSL][a]);
+            if constexpr (F32) two_sum_add(hi[c], lo[c], part);
+            else hi[c] += part;
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+  const size_t stride = (size_t)d.slot_off[d.ncells] * kCell;
+#pragma unroll
+  for (int c = 0; c < NO; ++c)
+    d.partial[c * stride + (size_t)task.w * kCell + lane] = active ? (double)hi[c] + (double)lo[c] : 0.0;
+}
+
 // ---------------------------------------------------------------------------
 // Tables (host, extended precision).
 
@@ -1275,7 +1414,7 @@ cudaError_t start(void (*fn)(Args...), dim3 grid, int block, size_t smem, cudaSt
   return cudaGetLastError();
 }
 
-template <int P, typename T, int NSL, int ND, bool P1 = false>
+template <int P, typename T, int NSL, int ND, bool P1 = false, bool WIDE = false>
 int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const ApplyArgs* many, const TreeTables& tab,
                const TreeSide& side, cudaStream_t st)
 {
@@ -1295,6 +1434,9 @@ int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const
   if constexpr (P1)
     EB_CUDA(start(tree_near_forward_kernel<T, 0>, dim3(g.ntasks), 32, (size_t)kCell * kQ * rec_slots(1, 0) * 4 * sizeof(T),
                   near, d, g.tasks, g.nmesh));
+  else if constexpr (WIDE)
+    EB_CUDA(start(tree_near_wide_kernel<T, NSL, ND>, dim3(g.ntasks), 32,
+                  (size_t)kWideTile * g.rule * rec_slots(NSL, ND) * 4 * sizeof(T), near, d, g.tasks, g.nmesh));
   else if constexpr (ND > 1)
     EB_CUDA(start(tree_near_forward_kernel<T, ND>, dim3(g.ntasks), 32, (size_t)kCell * kQ * rec_slots(0, ND) * 4 * sizeof(T),
                   near, d, g.tasks, g.nmesh));
@@ -1307,7 +1449,7 @@ int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const
     EB_CUDA(start(tree_p2m_kernel<P, 0, 1, kCharges>, dim3(g.ncells), 32 * kCellWarps, p2m_smem<P, 0, 1>(), st, d, g.cells,
                   g.nmesh, one, many, tab));
   else
-    EB_CUDA(start(tree_p2m_kernel<P, NSL, PD>, dim3(g.ncells, ND > 1 ? ND : 1), 32 * kCellWarps, p2m_smem<P, NSL, PD>(),
+    EB_CUDA(start(tree_p2m_kernel<P, NSL, PD, kApart, WIDE>, dim3(g.ncells, ND > 1 ? ND : 1), 32 * kCellWarps, p2m_smem<P, NSL, PD>(),
                   st, d, g.cells, g.nmesh, one, many, tab));
   for (int s = 0; s < kTreePasses; s++)
     EB_CUDA(start(tree_move_kernel<P, MC, kUp>, dim3(g.nup[s], NC / MC), b.x, Mv::smem(), st, d, g.up[s],
@@ -1316,7 +1458,7 @@ int launch_all(const TreeDesc* d, const TreeGrid& g, const ApplyArgs& one, const
                 0, tab));
   EB_CUDA(start(tree_move_kernel<P, MC, kDown>, dim3(g.ncells, NC / MC), b.x, Mv::smem(), st, d, g.cells,
                 g.nmesh, 0, tab));
-  EB_CUDA(start(tree_l2p_kernel<P, NC, P1>, dim3(g.ncells), 32 * kCellWarps, sizeof(double2) * NC * tree_pairs(P), st, d,
+  EB_CUDA(start(tree_l2p_kernel<P, NC, P1, WIDE>, dim3(g.ncells), 32 * kCellWarps, sizeof(double2) * NC * tree_pairs(P), st, d,
                 g.cells, g.nmesh, tab));
   EB_CUDA(cudaStreamWaitEvent(st, side.join, 0));
   return EB_OK;
@@ -1838,6 +1980,14 @@ int tree_launch(bool fp32, int nsl, int nd, const TreeDesc* d, const TreeGrid& g
   if (nsl == NSL && nd == ND)                                                                   \
     return fp32 ? launch_all<kTreeOrder32, float, NSL, ND>(d, g, one, many, tab, side, st)            \
                 : launch_all<kTreeOrder64, double, NSL, ND>(d, g, one, many, tab, side, st);
+#define EB_TREE_WIDE(NSL, ND)                                                                         \
+  if (g.rule > kQ && nsl == NSL && nd == ND)                                                          \
+    return fp32 ? launch_all<kTreeOrder32, float, NSL, ND, false, true>(d, g, one, many, tab, side, st)  \
+                : launch_all<kTreeOrder64, double, NSL, ND, false, true>(d, g, one, many, tab, side, st);
+  EB_TREE_WIDE(1, 1)
+  EB_TREE_WIDE(1, 0)
+  EB_TREE_WIDE(0, 1)
+#undef EB_TREE_WIDE
   EB_TREE(1, 1)
   EB_TREE(1, 0)
   EB_TREE(3, 0)
@@ -1848,17 +1998,25 @@ int tree_launch(bool fp32, int nsl, int nd, const TreeDesc* d, const TreeGrid& g
   return set_error(EB_ERR_INVALID, "no tree far field for this operator combination");
 }
 
+// Rules of 8 points and more take the tree in the single variants, on meshes
+// that have expansions: their close pairs run in forward order only, which
+// gains nothing where every pair is close.
+static bool wide_rule(const HostMesh& h) { return h.K == kWideItem; }
+
 void tree_prepare(Mesh* m)
 {
   const HostMesh& h = m->h;
-  if (h.Q != kSymRule || h.K != kSymRule || h.nchunk != 1) return;
+  m->tree.reset();
+  const bool wide = wide_rule(h);
+  if (!wide && (h.Q != kSymRule || h.K != kSymRule || h.nchunk != 1)) return;
   m->tree = std::make_shared<TreeMesh>();
-  m->tree->usable = make_tree_plan(h, &m->tree->plan);
+  m->tree->usable = make_tree_plan(h, &m->tree->plan) && !(wide && m->tree->plan.all_close);
 }
 
 bool tree_eligible(const Mesh* m, bool fp32, int nsl, int nd)
 {
   return m->plan.engine == 4 && m->tree && m->tree->usable && tree_variant(nsl, nd) &&
+         (!wide_rule(m->h) || (nsl <= 1 && nd <= 1)) &&
          (fp32 || m->h.ncells >= (nsl == kTreeP1 ? kTreeMinCells64P1 : kTreeMinCells64));
 }
 
@@ -1929,23 +2087,33 @@ TreeSide::~TreeSide()
 }
 
 // Close pairs of a variant in both orders at once, or forward only.
-static bool tree_forward(int nsl, int nd) { return nd > 1 || nsl == kTreeP1; }
-// Columns of its expansions and of its slots (a double layer alone leaves the
-// single layer's column unused).
+static bool tree_forward(const Mesh* m, int nsl, int nd) { return nd > 1 || nsl == kTreeP1 || wide_rule(m->h); }
+// Columns of its expansions and of its slots (a double layer alone in both
+// orders leaves the single layer's column unused).
 static int moved_columns(int nsl, int nd) { return nsl == kTreeP1 ? 1 : nsl + nd; }
-static int slot_columns(int nsl, int nd) { return nsl == kTreeP1 ? 3 : nd == 1 ? 2 : nsl + nd; }
+static int unused_columns(const Mesh* m, int nsl, int nd) { return nsl == 0 && nd == 1 && !wide_rule(m->h) ? 1 : 0; }
+static int slot_columns(const Mesh* m, int nsl, int nd)
+{
+  return nsl == kTreeP1 ? 3 : nsl + nd + unused_columns(m, nsl, nd);
+}
+
+static void forward_lists(TreeMesh* t)
+{
+  if (t->fwd.slot_off.empty()) make_near_lists(t->plan, false, &t->fwd);
+}
 
 long long tree_far_slots(const Mesh* m, int nsl, int nd)
 {
-  const TreeMesh& t = *m->tree;
-  return (long long)(tree_forward(nsl, nd) ? t.fwd : t.plan.sym).slot_off.back() * kCell;
+  TreeMesh& t = *m->tree;
+  if (tree_forward(m, nsl, nd)) forward_lists(&t);
+  return (long long)(tree_forward(m, nsl, nd) ? t.fwd : t.plan.sym).slot_off.back() * kCell;
 }
 
 static int upload_forward(TreeMesh* t)
 {
   if (t->fwd_lists.p) return EB_OK;
-  TreeNear& f = t->fwd;
-  make_near_lists(t->plan, false, &f);
+  forward_lists(t);
+  const TreeNear& f = t->fwd;
   const size_t a = f.tasks.size() * sizeof(int4), b = f.entries.size() * sizeof(int2), c = f.slot_off.size() * sizeof(int);
   std::vector<unsigned char> host(a + b + c);
   std::memcpy(host.data(), f.tasks.data(), a);
@@ -1968,7 +2136,7 @@ size_t tree_expansion_bytes(const Mesh* m, int order, int cols)
 
 size_t tree_partial_bytes(const Mesh* m, int nsl, int nd)
 {
-  return sizeof(double) * (size_t)slot_columns(nsl, nd) * tree_far_slots(m, nsl, nd);
+  return sizeof(double) * (size_t)slot_columns(m, nsl, nd) * tree_far_slots(m, nsl, nd);
 }
 
 int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, void* local, double* partial,
@@ -1977,7 +2145,7 @@ int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, v
   TreeMesh* t = m->tree.get();
   EB_CHECK(upload_lists(t));
   TreeDesc d = t->base;
-  if (tree_forward(nsl, nd)) {
+  if (tree_forward(m, nsl, nd)) {
     EB_CHECK(upload_forward(t));
     d.tasks = t->fwd_lists.as<int4>();
     d.entries = reinterpret_cast<const int2*>(d.tasks + t->fwd.tasks.size());
@@ -1989,7 +2157,7 @@ int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, v
   d.multipole = static_cast<double2*>(multipole);
   d.local = static_cast<double2*>(local);
   d.partial = partial;
-  d.first_col = nsl == 0 && nd == 1 ? 1 : 0;
+  d.first_col = unused_columns(m, nsl, nd);
   *out = d;
   return EB_OK;
 }
@@ -1998,7 +2166,7 @@ bool tree_points_eligible(const Mesh* m, bool fp32, int npts)
 {
   const double pairs = (double)npts * m->h.ne;
   return m->plan.engine == 4 && m->tree && m->tree->usable && !m->tree->plan.all_close &&
-         (fp32 ? pairs >= kTreePointPairs32 : pairs >= kTreePointPairs64 && m->h.ne >= kTreePointTriangles64);
+         !wide_rule(m->h) && (fp32 ? pairs >= kTreePointPairs32 : pairs >= kTreePointPairs64 && m->h.ne >= kTreePointTriangles64);
 }
 
 int tree_evaluate(Mesh* m, bool fp32, int npts, const double* pts, const double* d_pts, const double* d_t,
@@ -2037,7 +2205,6 @@ int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream
   std::unique_ptr<TreeScratch>& sc = t->scratch[(fp32 ? 64 : 0) + nsl * 5 + nd];
   if (!sc) {
     auto s = std::make_unique<TreeScratch>();
-    if (tree_forward(nsl, nd)) EB_CHECK(upload_forward(t));  // its slots are counted below
     const size_t bytes = tree_expansion_bytes(m, fp32 ? kTreeOrder32 : kTreeOrder64, moved_columns(nsl, nd));
     if (bytes) {
       EB_CHECK(s->multipole.alloc(bytes));
@@ -2053,6 +2220,7 @@ int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream
   A->partial = d.partial + (size_t)d.first_col * tree_far_slots(m, nsl, nd);
   A->slot_off = d.slot_off;
   TreeGrid g;
+  g.rule = m->h.Q;
   g.ncells = d.ncells;
   g.nm2l = d.nm2l;
   g.ntasks = d.ntasks;

@@ -86,6 +86,7 @@ struct TreeGrid {
   const int *cells = nullptr, *m2l = nullptr, *tasks = nullptr, *up[kTreePasses] = {};
   int ncells = 0, nm2l = 0, ntasks = 0, nup[kTreePasses] = {};
   bool expansions = true;
+  int rule = 0;  // points of the triangle rule
 };
 
 // A mesh's tree: the plan of a new mesh, the rest with the first apply.

@@ -202,3 +202,19 @@ def test_tree_potentials(gpu_lib, oracle, name, npts):
         rows = np.linspace(0, npts - 1, 64).astype(int)
         m.set_far_engine("tree")
         assert rel_l2(m.evaluate(pts, t, u)[rows], oracle.evaluate(nodes, elems, pts[rows], t, u)) < FP64_TOL
+
+
+@pytest.mark.parametrize("order", [6, 7, 9, 10, 18])
+@pytest.mark.parametrize("ne", [4160, 4737, 12831])
+def test_larger_rules(gpu_lib, order, ne):
+    """Rules of 13 to 73 points: against the direct kernels, every row."""
+    nodes, elems = _cut(*meshes.torus(206, 0.25), ne)
+    t, u = _vectors(nodes, elems, order)
+    with gpu_lib.Mesh(nodes, elems, order=order) as m:
+        for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL)):
+            m.set_far_engine("tree")
+            got = [*m.apply_sl_dl(t, u, precision=prec), m.apply_sl(t, prec), m.apply_dl(u, prec)]
+            m.set_far_engine("cuda")
+            ref = [*m.apply_sl_dl(t, u, precision=prec), m.apply_sl(t, prec), m.apply_dl(u, prec)]
+            for g, r in zip(got, ref):
+                assert rel_l2(g, r) < tol
