@@ -55,7 +55,7 @@ int Batch::build(const std::vector<BatchEntry*>& entries, bool fp32, int nsl, in
   K_ = entries[0]->mesh->h.K;
   const int n = (int)entries.size();
   std::vector<char> tree(n);
-  for (int e = 0; e < n; e++) tree[e] = tree_eligible(entries[e]->mesh, fp32, nsl_, nd_);
+  for (int e = 0; e < n; e++) tree[e] = tree_eligible(entries[e]->mesh, nsl_, nd_);
   ntree_ = (int)std::count(tree.begin(), tree.end(), 1);
   tc_ = fp32 && nsl_ == 1 && nd_ == 1 && ntree_ < n;
   for (int e = 0; e < n; e++)

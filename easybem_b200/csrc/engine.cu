@@ -635,7 +635,7 @@ bool sym_eligible(const Mesh* m, bool fp32, int nsl, int nd, bool fp64_internal)
 
 long long mesh_far_slots(const Mesh* m, bool fp32, int nsl, int nd)
 {
-  if (tree_eligible(m, fp32, nsl, nd)) return tree_far_slots(m, nsl, nd);
+  if (tree_eligible(m, nsl, nd)) return tree_far_slots(m, nsl, nd);
   if (sym_eligible(m, fp32, nsl, nd)) {
     const int r = far_sym_cells_per_item(kSymCellsPerItem);
     long long n = 0;
@@ -753,13 +753,12 @@ int mesh_check_far_error(Mesh* m)
 
 // Scratch sized once for the largest variant, so device pointers captured in
 // descriptors (and in CUDA graphs) stay valid.
-int ensure_apply_scratch(Mesh* m)
+int ensure_apply_scratch(Mesh* m, bool tree)
 {
   const HostMesh& h = m->h;
-  if (!m->rec.p) {
-    EB_CHECK(m->rec.alloc((size_t)h.ne * h.Q * kMaxRecSlots * sizeof(dq)));
+  if (!m->rec.p) EB_CHECK(m->rec.alloc((size_t)h.ne * h.Q * kMaxRecSlots * sizeof(dq)));
+  if (!tree && !m->partial.p)
     EB_CHECK(m->partial.alloc(sizeof(double) * (size_t)kMaxOutputs * m->plan.nsplit * h.nitems));
-  }
   return EB_OK;
 }
 
@@ -774,9 +773,10 @@ int mesh_apply(Mesh* m, int precision, int nsl, int nd, const double* d_t, const
   if (!far_variant_supported(nsl, nd)) return set_error(EB_ERR_INVALID, "unsupported operator combination");
   if ((nsl > 0 && (!d_t || !d_v)) || (dl && (!d_u || !d_q))) return set_error(EB_ERR_INVALID, "null vector");
   const int nrec = rec_slots(nsl, nd);
-  EB_CHECK(ensure_apply_scratch(m));
+  const bool tree = tree_eligible(m, nsl, nd);
+  EB_CHECK(ensure_apply_scratch(m, tree));
   Mesh::Variant& var = m->variants[(fp32 ? 64 : 0) + nsl * 5 + nd];
-  if (!var.desc.p) {
+  if (!tree && !var.desc.p) {
     const FarMeshDesc desc = mesh_far_desc(m, fp32, nsl, nd, m->rec.p, m->partial.as<double>());
     const size_t smem = far_smem_bytes(desc.src_tile, h.Q, nrec, fp32);
     int occ = far_occupancy(fp32, nsl, nd, h.K, h.Q, smem);
@@ -789,7 +789,6 @@ int mesh_apply(Mesh* m, int precision, int nsl, int nd, const double* d_t, const
     var.smem = smem;
     var.src_tile = desc.src_tile;
   }
-  const bool tree = tree_eligible(m, fp32, nsl, nd);
   const bool sym = !tree && sym_eligible(m, fp32, nsl, nd);
   ApplyArgs A = mesh_apply_args(m, fp32, m->rec.p, m->partial.as<double>(), d_t, h.ne, d_u, d_v, h.ne, d_q);
   EB_CUDA(prep_launch(fp32, nsl, nd, A, st));
@@ -1132,7 +1131,7 @@ int eb_mesh_get_far_engine(eb_mesh mesh, int precision, int* engine)
 {
   if (!mesh || !engine) return set_error(EB_ERR_INVALID, "null argument");
   const bool fp32 = precision == EB_PREC_MIXED;
-  *engine = eb::tree_eligible(mesh->m, fp32, 1, 1)        ? (mesh->m->tree->plan.all_close ? EB_FAR_SYMMETRIC : EB_FAR_TREE)
+  *engine = eb::tree_eligible(mesh->m, 1, 1)        ? (mesh->m->tree->plan.all_close ? EB_FAR_SYMMETRIC : EB_FAR_TREE)
             : eb::tc_eligible(mesh->m, fp32, 1, 1)  ? EB_FAR_TENSOR_CORES
             : eb::sym_eligible(mesh->m, fp32, 1, 1) ? EB_FAR_SYMMETRIC
                                                     : EB_FAR_CUDA_CORES;

@@ -204,8 +204,9 @@ struct StaticTables {
   int4 *svid, *tvid;
 };
 cudaError_t static_tables_launch(const StaticTables& t, cudaStream_t st);
-// The record and partial-sum scratch of single-mesh calls.
-int ensure_apply_scratch(Mesh* m);
+// The record scratch of single-mesh calls, and unless the call takes the tree
+// (which has its own) the partial sums.
+int ensure_apply_scratch(Mesh* m, bool tree);
 // The mixed potential evaluation sums cells within this many radii of a point in FP64.
 constexpr double kPotNear = 2.5;
 // Device-pointer apply: t has nsl columns (stride ne), v likewise; u has nd

@@ -814,6 +814,18 @@ constexpr size_t near_smem()
   return (size_t)kCell * kQ * kNrec * 4 * sizeof(T) + kCell * near_red_row<T, NSL, ND>();
 }
 
+// Sources of an entry of the close-pair lists.
+struct NearSources {
+  int cell, t0, ns;
+  __device__ __forceinline__ NearSources(int x, int ne)
+  {
+    const int parts = x >> kTreePartsShift, part = x >> kTreePartShift & 7, n = kCell >> parts;
+    cell = x & ((1 << kTreePartShift) - 1);
+    t0 = cell * kCell + part * n;
+    ns = max(0, min(n, ne - t0));
+  }
+};
+
 template <typename T, int NSL, int ND>
 __global__ void __launch_bounds__(32, 8)
     tree_near_kernel(const TreeDesc* __restrict__ descs, const int* __restrict__ off, int nmesh)
@@ -858,8 +870,8 @@ __global__ void __launch_bounds__(32, 8)
 #pragma unroll 1
   for (int e = task.y; e < task.z; ++e) {
     const int2 en = d.entries[e];
-    const int cell = en.x, t0 = cell * kCell;
-    const int ns = min(kCell, md.ne - t0);
+    const NearSources src(en.x, md.ne);
+    const int cell = src.cell, t0 = src.t0, ns = src.ns;
     {
       const S* g = grec + (size_t)t0 * kQ * kNrec;
       if constexpr (F32) {  // source-pair layout, as the symmetric kernel stages it
@@ -1011,7 +1023,7 @@ __global__ void __launch_bounds__(32, 8)
               v2 += rf[(t + 2) * row + at];
               v3 += rf[(t + 3) * row + at];
             }
-            d.partial[c * stride + (size_t)en.y * kCell + h + lane] = (double)((v0 + v1) + (v2 + v3));
+            d.partial[c * stride + (size_t)en.y * kCell + (t0 - cell * kCell) + h + lane] = (double)((v0 + v1) + (v2 + v3));
           }
         }
         __syncwarp();
@@ -1067,8 +1079,8 @@ __global__ void __launch_bounds__(32, 8)
   for (int c = 0; c < NO; ++c) hi[c] = lo[c] = 0;
 #pragma unroll 1
   for (int e = task.y; e < task.z; ++e) {
-    const int cell = d.entries[e].x, t0 = cell * kCell;
-    const int ns = min(kCell, md.ne - t0);
+    const NearSources src(d.entries[e].x, md.ne);
+    const int cell = src.cell, t0 = src.t0, ns = src.ns;
     const S* g = grec + (size_t)t0 * kQ * NREC;
     if constexpr (F32) {  // source-pair layout
       constexpr int per = kQ * NREC;
@@ -1184,14 +1196,15 @@ __global__ void __launch_bounds__(32)
   for (int c = 0; c < NO; ++c) hi[c] = lo[c] = 0;
 #pragma unroll 1
   for (int e = task.y; e < task.z; ++e) {
-    const int cell = d.entries[e].x, end = min(cell * kCell + kCell, md.ne);
+    const NearSources src(d.entries[e].x, md.ne);
+    const int cell = src.cell, end = src.t0 + src.ns;
     const dq cc = md.ccent[cell];
     const double ddx = cc.x - ball.x, ddy = cc.y - ball.y, ddz = cc.z - ball.z;
     const double rr = kFarRatio * (cc.w + ball.w);
     const bool far = ddx * ddx + ddy * ddy + ddz * ddz > rr * rr;
     const T o[3] = {(T)(cc.x - cen[0]), (T)(cc.y - cen[1]), (T)(cc.z - cen[2])};
 #pragma unroll 1
-    for (int t0 = cell * kCell; t0 < end; t0 += kWideTile) {
+    for (int t0 = src.t0; t0 < end; t0 += kWideTile) {
       const int ns = min(kWideTile, end - t0);
       const S* g = grec + (size_t)t0 * per;
       if constexpr (F32) {  // source-pair layout
@@ -2013,11 +2026,10 @@ void tree_prepare(Mesh* m)
   m->tree->usable = make_tree_plan(h, &m->tree->plan) && !(wide && m->tree->plan.all_close);
 }
 
-bool tree_eligible(const Mesh* m, bool fp32, int nsl, int nd)
+bool tree_eligible(const Mesh* m, int nsl, int nd)
 {
   return m->plan.engine == 4 && m->tree && m->tree->usable && tree_variant(nsl, nd) &&
-         (!wide_rule(m->h) || (nsl <= 1 && nd <= 1)) &&
-         (fp32 || m->h.ncells >= (nsl == kTreeP1 ? kTreeMinCells64P1 : kTreeMinCells64));
+         (!wide_rule(m->h) || (nsl <= 1 && nd <= 1));
 }
 
 static int upload_lists(TreeMesh* t)
@@ -2178,7 +2190,7 @@ int tree_evaluate(Mesh* m, bool fp32, int npts, const double* pts, const double*
   const ApplyArgs A = mesh_apply_args(m, false, rec.p, nullptr, d_t, m->h.ne, d_u, nullptr, m->h.ne, nullptr);
   EB_CUDA(prep_launch(false, 1, 1, A, st));
   if (!fp32) return evaluate_order<kTreeOrder64>(m, npts, pts, d_pts, A, nullptr, rec.as<dq>(), d_out, st);
-  EB_CHECK(ensure_apply_scratch(m));
+  EB_CHECK(ensure_apply_scratch(m, true));
   const ApplyArgs A32 = mesh_apply_args(m, true, m->rec.p, nullptr, d_t, m->h.ne, d_u, nullptr, m->h.ne, nullptr);
   EB_CUDA(prep_launch(true, 1, 1, A32, st));
   return evaluate_order<kTreeOrder32>(m, npts, pts, d_pts, A, m->rec.as<float4>(), rec.as<dq>(), d_out, st);

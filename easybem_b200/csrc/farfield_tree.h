@@ -109,7 +109,7 @@ struct TreeMesh {
 // computes the near field of a new mesh).
 void tree_prepare(Mesh* m);
 // True when mesh m applies this far-field variant through the tree.
-bool tree_eligible(const Mesh* m, bool fp32, int nsl, int nd);
+bool tree_eligible(const Mesh* m, int nsl, int nd);
 // The far field of mesh m: expansions and close pairs into the partial slots
 // (A.partial and A.slot_off are set for the finalize).
 int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream_t st);

@@ -178,8 +178,8 @@ int mesh_apply_sl_p1(Mesh* m, int precision, const double* d_t, double* d_v, cud
   EB_CHECK(ensure_p1_near(m));
   EB_CHECK(ensure_vertex_lists(m));
   const HostMesh& h = m->h;
-  EB_CHECK(ensure_apply_scratch(m));
-  const bool tree = tree_eligible(m, fp32, kTreeP1, 0);
+  const bool tree = tree_eligible(m, kTreeP1, 0);
+  EB_CHECK(ensure_apply_scratch(m, tree));
   Mesh::Variant& var = m->variants[100 + (fp32 ? 1 : 0)];
   if (!tree && !var.desc.p) {
     const FarMeshDesc desc = mesh_far_desc(m, fp32, 1, false, m->rec.p, m->partial.as<double>());

@@ -234,7 +234,7 @@ int mesh_evaluate_potential(Mesh* m, int precision, int npts, const double* d_pt
     return set_error(EB_ERR_INVALID, "precision must be EB_PREC_FP64 or EB_PREC_MIXED");
   if (npts < 1) return EB_OK;
   // source records of the fused SL+DL variant (slot1 = (s, c))
-  EB_CHECK(ensure_apply_scratch(m));
+  EB_CHECK(ensure_apply_scratch(m, true));
   const ApplyArgs A = mesh_apply_args(m, fp32, m->rec.p, nullptr, d_t, h.ne, d_u, nullptr, h.ne, nullptr);
   EB_CUDA(prep_launch(fp32, 1, true, A, st));
   if (fp32) {  // FP64 records for the cells close to a point

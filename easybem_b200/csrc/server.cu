@@ -60,7 +60,7 @@ static size_t mesh_resident_bytes(const Mesh* m)
 static size_t batch_far_bytes(const Mesh* m, int nrhs)
 {
   const size_t entries = ((size_t)nrhs + kBatchCols - 1) / kBatchCols;
-  if (tree_eligible(m, true, kBatchCols, 0))
+  if (tree_eligible(m, kBatchCols, 0))
     return entries * (2 * tree_expansion_bytes(m, kTreeOrder64, kBatchCols) + tree_partial_bytes(m, kBatchCols, 0));
   return sym_eligible(m, true, kBatchCols, 0) ? entries * sym_slot_bytes(m->h, kBatchCols) : 0;
 }

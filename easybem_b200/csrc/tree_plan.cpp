@@ -86,6 +86,9 @@ void make_near_lists(const TreePlan& plan, bool both, TreeNear* out)
   const Rows close(nc, plan.near, !both);
   const int pairs = nc + (int)close.col.size();
   const int chunk = std::min(kTreeNearChunk, std::max(1, pairs / kTreeNearTasks));
+  int log_parts = 0;
+  while ((1 << log_parts) < kTreeNearParts && (pairs << log_parts) < kTreeNearTasks) log_parts++;
+  const int parts = 1 << log_parts;  // above 1 with chunk 1 only
   const int far_slots = plan.all_close ? 0 : 1;
   std::vector<int> trans(nc, 0);
   if (both)
@@ -93,14 +96,17 @@ void make_near_lists(const TreePlan& plan, bool both, TreeNear* out)
   out->slot_off.assign(nc + 1, 0);
   for (int c = 0; c < nc; c++)
     out->slot_off[c + 1] =
-        out->slot_off[c] + trans[c] + (close.ptr[c + 1] - close.ptr[c] + chunk) / chunk + far_slots;
+        out->slot_off[c] + trans[c] + (close.ptr[c + 1] - close.ptr[c] + chunk) / chunk * parts + far_slots;
   std::vector<int> next(out->slot_off.begin(), out->slot_off.end() - 1);
-  out->entries.reserve(close.col.size() + nc);
+  out->entries.reserve((close.col.size() + nc) * parts);
   for (int c = 0; c < nc; c++) {
     const int e0 = (int)out->entries.size();
-    out->entries.push_back(make_int2(c, -1));
-    for (int q = close.ptr[c]; q < close.ptr[c + 1]; q++)
-      out->entries.push_back(make_int2(close.col[q], both ? next[close.col[q]]++ : -1));
+    auto add = [&](int cell, int slot) {
+      for (int part = 0; part < parts; part++)
+        out->entries.push_back(make_int2(cell | part << kTreePartShift | log_parts << kTreePartsShift, slot));
+    };
+    add(c, -1);
+    for (int q = close.ptr[c]; q < close.ptr[c + 1]; q++) add(close.col[q], both ? next[close.col[q]]++ : -1);
     const int e1 = (int)out->entries.size();
     int slot = out->slot_off[c] + trans[c];
     for (int e = e0; e < e1; e += chunk)

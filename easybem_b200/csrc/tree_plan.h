@@ -50,19 +50,21 @@ constexpr double kTreePointTheta64 = 0.35;
 // (four warps on each of the 592 SM quarters).
 constexpr int kTreeNearChunk = 4;
 constexpr int kTreeNearTasks = 4 * 592;
+// Where single pairs leave less, a pair is cut into up to kTreeNearParts tasks
+// of consecutive sources: 820 pairs (1,280 triangles) leave 364 of the 592
+// quarters one warp with nothing to hide its latency and give 228 two. FP64,
+// one operator at 1,280 triangles: 94 -> 85 us (the near kernel 65 before);
+// SL+DL at 512: 96 -> 37, where the ordered-pair kernel takes 69.
+constexpr int kTreeNearParts = 4;
+// A pair's source cell in a list entry, with the part of it: x = cell, the
+// part and log2 of the number of parts in the upper bits.
+constexpr int kTreePartShift = 25, kTreePartsShift = 28;
 // Smaller meshes (cells) have no separated clusters worth an expansion: all
 // their cell pairs are close. Up to here the near tasks alone also beat the
 // symmetric kernel, whose items (a 128-triangle tile against 8 cells) leave
 // SMs idle.
 constexpr int kTreeMinCells = 100;
 constexpr int kTreeAllCloseCells = 140;
-// Least cells of an FP64 apply on the tree: below, a pair of cells (22 us on an
-// SM quarter) is too coarse a task, and the ordered-pair kernel's finer items
-// finish first (512 triangles, SL+DL: 69 us against 96; 1,200: 134 against 121).
-// The P1 single layer alone costs a third of that (128 triangles, 4 cells: 77
-// against 69 us; 512: 103 against 78; 36 triangles: 67.6 against 69.9).
-constexpr int kTreeMinCells64 = 28, kTreeMinCells64P1 = 4;
-
 // Expansions moved into node tgt[k] from nodes src[ptr[k] .. ptr[k + 1]). The
 // upper 8 bits of a source are the share f / 255 of the degrees that its pair
 // needs: an expansion of order p is used up to (p + 1) f / 255 - 1 (rounded

@@ -149,7 +149,7 @@ def test_small_meshes_sum_all_cell_pairs(gpu_lib, oracle, ne):
     g = np.stack([u, u[::-1], 2 * u])
     with gpu_lib.Mesh(nodes, elems) as m:
         if ne < 3200:
-            assert m.far_engine("mixed") == "sym" and m.far_engine("fp64") == ("sym" if ne > 27 * 32 else "cuda")
+            assert m.far_engine("mixed") == "sym" and m.far_engine("fp64") == "sym"
         for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL)):
             m.set_far_engine("tree")
             v, q = m.apply_sl_dl(t, u, precision=prec)
