@@ -57,7 +57,8 @@ enum Move { kUp, kAcross, kDown };
 struct TreeTables {
   const double *bmat, *tmat[3];
   const int* pair;     // (n, m): m | n << 8
-  const double2* rec;  // (n, m): R_n^m = rec.x z R_{n-1}^m - rec.y r^2 R_{n-2}^m (n > m)
+  const double2* rec;  // (n, m): R_n^m = rec.x z R_{n-1}^m - rec.y r^2 R_{n-2}^m (n > m);
+                       // (m, m): R_m^m = rec.x (x + i y) R_{m-1}^{m-1}
 };
 
 __device__ __forceinline__ int tree_pair(int n, int m) { return n * (n + 1) / 2 + m; }
@@ -474,9 +475,14 @@ __global__ void __launch_bounds__(MoveShape<P, NC>::kThreads, MoveShape<P, NC>::
 
 // ---------------------------------------------------------------------------
 // Points and expansions. Four warps per cell, one lane per triangle with its
-// seven points in registers; warp w runs the orders m = w, w + 4, ... of the
-// recurrences in n. Both directions use w_a-weighted sums over a triangle's
-// points: sources need sum_b q_b R(y_b), targets sum_a w_a phi(x_a).
+// seven points in registers; a warp runs every fourth order m of the
+// recurrences in n, back and forth (orders 0, 7, 8, ... for warp 0) so that all
+// warps have the same number of degrees. Both directions use w_a-weighted sums
+// over a triangle's points: sources need sum_b q_b R(y_b), targets sum_a w_a
+// phi(x_a). Latency of the recurrence and of the lane sums bounds them. SL+DL
+// apply at 81,920 triangles, mixed / FP64: orders in turn and the factors of
+// R_m^m computed 2.162 / 8.74 ms, even shares and tabulated factors 2.125 /
+// 8.68; eight warps per cell 2.27 / 8.92.
 
 constexpr int kCellWarps = 4;
 constexpr int kSumRows = 8, kSumStride = 36;  // conflict-free rows of the lane sums
@@ -516,7 +522,7 @@ __device__ __forceinline__ void each_harmonic(const TreeTables& tab, const CellP
 #pragma unroll 1
   for (int m = 0; m <= P; ++m) {
     if (m > 0) {
-      const double f = -sqrt((2.0 * m - 1.0) / (2.0 * m));
+      const double f = tab.rec[tree_pair(m, m)].x;
 #pragma unroll
       for (int a = 0; a < kQ; ++a) {
         const double t = f * (p.x[a] * dr[a] - p.y[a] * di[a]);
@@ -524,7 +530,8 @@ __device__ __forceinline__ void each_harmonic(const TreeTables& tab, const CellP
         dr[a] = t;
       }
     }
-    if ((m & (kCellWarps - 1)) != warp) continue;
+    const int w = m & (kCellWarps - 1);
+    if ((m & kCellWarps ? kCellWarps - 1 - w : w) != warp) continue;
     double r1[kQ], i1[kQ], r0[kQ], i0[kQ];
 #pragma unroll
     for (int a = 0; a < kQ; ++a) {
@@ -1368,7 +1375,9 @@ HostTables make_tables(int P)
   for (int n = 0; n <= P; n++)
     for (int m = 0; m <= n; m++) {
       h.pair.push_back(m | n << 8);
-      if (n > m) {
+      if (n == m) {
+        if (m > 0) h.rec[n * (n + 1) / 2 + m].x = -std::sqrt((2.0 * m - 1.0) / (2.0 * m));
+      } else {
         const double q = (double)(n * n - m * m);
         h.rec[n * (n + 1) / 2 + m] =
             make_double2((2 * n - 1) / std::sqrt(q), std::sqrt(((n - 1.0) * (n - 1.0) - m * m) / q));
@@ -1798,7 +1807,7 @@ __global__ void __launch_bounds__(32 * kPointWarps)
 #pragma unroll 1
   for (int m = 0; m <= P; ++m) {
     if (m > 0) {
-      const double f = -sqrt((2.0 * m - 1.0) / (2.0 * m));
+      const double f = tab.rec[tree_pair(m, m)].x;
       const double t = f * (x * dr - y * di);
       di = f * (x * di + y * dr);
       dr = t;
