@@ -26,7 +26,7 @@ __all__ = ["Mesh", "Batch", "Solver", "Server", "solve", "EasyBemError", "init_g
            "apply_gpu_laplace3d_hypersing", "version", "precision_code", "save_plans", "load_plans", "clear_plans"]
 
 
-# far-field engines of the fused mixed SL+DL apply (EB_FAR_* in easybem_gpu.h)
+# far-field engines (EB_FAR_* in easybem_gpu.h)
 FAR_ENGINES = {"cuda": 0, "tensor": 1, "sym": 2, "sym_all": 3, "tree": 4}
 
 
@@ -187,11 +187,13 @@ class Mesh:
         return a.value, b.value
 
     def set_far_engine(self, engine: str = "tensor"):
-        """Far-field engine of the fused mixed SL+DL apply: "tensor" (tcgen05
-        GEMMs for the pair distances), "cuda" (FP32 pipes only, every ordered
-        pair) or "sym" (FP32 pipes, every unordered pair once, added to both
-        rows; the default); "sym_all" takes the symmetric kernel for the FP64
-        apply too."""
+        """Far-field engine: "tree" (separated clusters through multipole and
+        local expansions, close cells point by point, both precisions; the
+        default), or for the fused mixed SL+DL apply over all pairs "tensor"
+        (tcgen05 GEMMs for the pair distances), "cuda" (FP32 pipes only, every
+        ordered pair) or "sym" (FP32 pipes, every unordered pair once, added
+        to both rows); "sym_all" takes the symmetric kernel for the FP64 apply
+        too."""
         check(lib().eb_mesh_set_far_engine(self._h, FAR_ENGINES[engine]))
 
     def far_engine(self, precision="mixed"):

@@ -42,7 +42,8 @@ class Batch {
   // entry's systems carry zeros). nd = 1 adds the double layer (uin -> qout)
   // in the same pass, with nsl 0 or 1 (the fused SL+DL variant). sym_fp64:
   // an FP64 batch inside the library (the solver's residuals) that takes the
-  // symmetric kernels when the meshes' engine is the default.
+  // symmetric kernels on the engines that have them for mixed applies. Meshes
+  // on the tree take its kernels in either precision, the others run together.
   int build(const std::vector<BatchEntry*>& entries, bool fp32, int nsl, int* d_flags, int nd = 0,
             bool sym_fp64 = false);
   // One apply of all entries whose flag is set (inputs tin, outputs vout).

@@ -352,7 +352,7 @@ int eb_mesh_get_plan(eb_mesh mesh, int* items_per_sm, int* src_tile, int* nsplit
  * per 128-triangle tile and row (16 bytes each: ne^2/8 bytes, 0.84 GB at
  * 81,920 triangles, 13.4 GB at 327,680), allocated on its first apply, and
  * takes meshes of up to 524,288 triangles (32 GiB of slots); larger meshes
- * use the CUDA cores. EB_FAR_SYMMETRIC is the default of a new mesh. Other
+ * use the CUDA cores. Other
  * variants always use the CUDA cores; get reports the engine an apply in
  * `precision` with both operators would use. No counterpart in the
  * reference. */
@@ -361,17 +361,26 @@ int eb_mesh_get_plan(eb_mesh mesh, int* items_per_sm, int* src_tile, int* nsplit
 #define EB_FAR_SYMMETRIC 2
 /* EB_FAR_SYMMETRIC for the FP64 applies too (every unordered pair once in
  * FP64: 7 instead of 13 FP64-pipe operations per pair for SL+DL, 5 instead
- * of 10 for the single layer). Opt-in: the FP64 default of the apply entry
- * points stays the plain ordered-pair kernel (the solver's internal FP64
- * residuals take the symmetric kernel on the default engine); get reports
- * EB_FAR_SYMMETRIC for an FP64 apply on this engine. */
+ * of 10 for the single layer). On EB_FAR_SYMMETRIC the FP64 apply entry
+ * points keep the plain ordered-pair kernel (the solver's internal FP64
+ * residuals take the symmetric kernel); get reports EB_FAR_SYMMETRIC for an
+ * FP64 apply on this engine. */
 #define EB_FAR_SYMMETRIC_ALL 3
-/* The default of a new mesh: separated clusters of triangles through multipole
- * and local expansions, close cells of 32 triangles point by point with the
- * EB_FAR_SYMMETRIC inner loops, so an apply costs O(nelems). Taken by meshes
- * large enough to gain (7-point rule; SL+DL and the SL with 1, 3 or 4 columns),
- * EB_FAR_SYMMETRIC's rules otherwise. The expansion orders keep the truncation
- * below the rounding of the point sums in either precision. */
+/* The default of a new mesh, in both precisions: separated clusters of
+ * triangles through multipole and local expansions, close cells of 32
+ * triangles point by point (every unordered pair once), so an apply costs
+ * O(nelems). 7-point rule: every variant (SL with 1, 3 or 4 columns, DL with 1
+ * or 4, SL+DL, the P1 single layer) and the potentials of many points; below
+ * some 4,000 triangles all cells are close and get reports EB_FAR_SYMMETRIC.
+ * Rules of 12 points and more: SL, DL and SL+DL on meshes that have separated
+ * clusters. EB_FAR_SYMMETRIC's rules otherwise, and where more than a third of
+ * the cell pairs of a larger mesh are close. The expansion orders keep the
+ * truncation below the rounding of the point sums in either precision. An
+ * apply runs the close cells on a stream of the mesh's own beside the
+ * expansions; work before and after it on the caller's stream is ordered as
+ * with one stream, also under capture. Scratch, allocated with a variant's
+ * first apply, grows with nelems: the expansions of SL+DL at 81,920 triangles
+ * take 143 MB in FP64 and 39 MB mixed. */
 #define EB_FAR_TREE 4
 int eb_mesh_set_far_engine(eb_mesh mesh, int engine);
 int eb_mesh_get_far_engine(eb_mesh mesh, int precision, int* engine);
@@ -398,7 +407,8 @@ int eb_sym_plan(int nelems, int cells_per_item, int* nitems, int* nslots_max, in
  * and records it in the process-wide plan table under (SM count,
  * floor(log2 nelems), triangle-rule points, precision); meshes created later
  * that match an entry start from it (mixed entries first). start_ms is the
- * time of the plan the mesh had. No counterpart in the reference. */
+ * time of the plan the mesh had. A mesh on EB_FAR_TREE is timed as on
+ * EB_FAR_SYMMETRIC: the plan shapes the direct kernels only. No counterpart in the reference. */
 int eb_autotune(eb_mesh mesh, int precision, int operators, int reps, int* items_per_sm, int* src_tile,
                 double* best_ms, double* start_ms);
 /* Plan table as text: a header line, then "sms bucket points precision
