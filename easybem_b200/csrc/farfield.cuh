@@ -77,7 +77,8 @@ __host__ __device__ constexpr int charge_comp(int r, int nd) { return (r + nd) %
 // ulps to cancellation for the closest pairs (k = kFarRatio; 19 at 1.6).
 // Measured at the L6 icosphere with 128-item groups: 1.6 leaves 9 % of the
 // (target, source triangle) pairs in the other cells (20 % at 2.5) with the
-// same mixed-precision error (9e-8); per warp it leaves 4 %.
+// same mixed-precision error (9e-8); per warp it leaves 4 % (triangles in Morton
+// order; 0.9 % in the bisection order).
 #ifndef EB_FAR_RATIO
 #define EB_FAR_RATIO 1.6
 #endif

@@ -218,3 +218,20 @@ def test_larger_rules(gpu_lib, order, ne):
             ref = [*m.apply_sl_dl(t, u, precision=prec), m.apply_sl(t, prec), m.apply_dl(u, prec)]
             for g, r in zip(got, ref):
                 assert rel_l2(g, r) < tol
+
+
+@pytest.mark.parametrize("order", [7, 9])
+def test_batch_of_larger_rules(gpu_lib, order):
+    """Meshes with and without separated clusters in one batch, against each alone."""
+    meshes_in = [_cut(*meshes.torus(206, 0.25), ne) for ne in (12831, 640, 4737)]
+    vecs = [_vectors(*x, k) for k, x in enumerate(meshes_in)]
+    ms = [gpu_lib.Mesh(*x, order=order) for x in meshes_in]
+    for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL)):
+        bt = gpu_lib.Batch(ms, precision=prec, sl_dl=True)
+        vs, qs = bt.apply_sl_dl([t for t, _ in vecs], [u for _, u in vecs])
+        bt.close()
+        for m, (t, u), v, q in zip(ms, vecs, vs, qs):
+            w, r = m.apply_sl_dl(t, u, precision=prec)
+            assert rel_l2(v, w) < tol and rel_l2(q, r) < tol
+    for m in ms:
+        m.close()
