@@ -54,7 +54,10 @@ constexpr int kTreeNearTasks = 4 * 592;
 // of consecutive sources: 820 pairs (1,280 triangles) leave 364 of the 592
 // quarters one warp with nothing to hide its latency and give 228 two. FP64,
 // one operator at 1,280 triangles: 94 -> 85 us (the near kernel 65 before);
-// SL+DL at 512: 96 -> 37, where the ordered-pair kernel takes 69.
+// SL+DL at 512: 96 -> 37, where the ordered-pair kernel takes 69. Up to 2 parts
+// are slower below 800 triangles (54 at 512); 8 gain at 128 (25 against 34) but
+// give the finalize more slots to add (512: P1 layer 93 against 75; 800 mixed
+// 40 against 37).
 constexpr int kTreeNearParts = 4;
 // A pair's source cell in a list entry, with the part of it: x = cell, the
 // part and log2 of the number of parts in the upper bits.
