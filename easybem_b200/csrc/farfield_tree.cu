@@ -1583,7 +1583,7 @@ static_assert(32 * (kTreePasses * kTreeLevelsPerPass + 2) <= kListStack, "stack 
 // or written at the scanned offsets.
 template <bool FILL>
 __global__ void __launch_bounds__(32 * kListWarps)
-    group_lists_kernel(int ngroups, int root, int ncells, double theta, const dq* __restrict__ nodes,
+    group_lists_kernel(int ngroups, int root, int ncells, double ratio, const dq* __restrict__ nodes,
                        const char* __restrict__ formed, const int2* __restrict__ child, const dq* __restrict__ ball,
                        int* __restrict__ far_ptr, int* __restrict__ near_ptr, int* __restrict__ task_ptr,
                        int* __restrict__ far, int* __restrict__ near)
@@ -1608,17 +1608,14 @@ __global__ void __launch_bounds__(32 * kListWarps)
       const dq x = nodes[k];
       const double dx = x.x - b.x, dy = x.y - b.y, dz = x.z - b.z;
       d2 = dx * dx + dy * dy + dz * dz;
-      r = x.w + b.w;
-      is_far = formed[k] && d2 * (theta * theta) > r * r;
+      r = x.w;
+      is_far = formed[k] && separated(r, b.w, d2, ratio);
       is_near = !is_far && k < ncells;
     }
     const bool split = k >= 0 && !is_far && !is_near;
     const unsigned mf = __ballot_sync(0xffffffffu, is_far), mn = __ballot_sync(0xffffffffu, is_near);
     const unsigned ms = __ballot_sync(0xffffffffu, split);
-    if (FILL && is_far) {
-      const double share = 2.0 * log(theta) / log(r * r / d2);
-      far[nf + __popc(mf & below)] = (int)((unsigned)fmin(255.0, fmax(1.0, ceil(255.0 * share))) << 24 | (unsigned)k);
-    }
+    if (FILL && is_far) far[nf + __popc(mf & below)] = (int)(degree_share(r, b.w, d2, ratio) << 24 | (unsigned)k);
     if (FILL && is_near) near[nn + __popc(mn & below)] = k;
     if (split) {
       const int2 c = child[k - ncells];
@@ -1949,10 +1946,10 @@ int evaluate_order(Mesh* m, int n, const double* pts, const double* d_pts, const
   d[1].m2l.tgt = ids;
   d[1].m2l.ptr = far_ptr;
   EB_CUDA(cudaMemcpyAsync(w.ball.p, d[0].ball, sizeof(dq) * plan.nnodes, cudaMemcpyDeviceToDevice, st));
-  const double root = plan.ball[plan.nnodes - 1].w, theta = P <= kTreeOrder32 ? kTreePointTheta32 : kTreePointTheta64;
+  const double root = plan.ball[plan.nnodes - 1].w, ratio = P <= kTreeOrder32 ? kTreePointRatio32 : kTreePointRatio64;
   group_ball_kernel<<<(ngroups + 3) / 4, 128, 0, st>>>(ngroups, d_gptr, d_pts, d_perm, 1e-4 * root, gball);
   const int gb = (ngroups + kListWarps - 1) / kListWarps;
-  group_lists_kernel<false><<<gb, 32 * kListWarps, 0, st>>>(ngroups, plan.nnodes - 1, plan.ncells, theta, d[0].ball,
+  group_lists_kernel<false><<<gb, 32 * kListWarps, 0, st>>>(ngroups, plan.nnodes - 1, plan.ncells, ratio, d[0].ball,
                                                             t->formed, t->children, gball, far_ptr, near_ptr, task_ptr,
                                                             nullptr, nullptr);
   scan_lists_kernel<<<1, 1024, 0, st>>>(ngroups, far_ptr, near_ptr, task_ptr);
@@ -1968,7 +1965,7 @@ int evaluate_order(Mesh* m, int n, const double* pts, const double* d_pts, const
   EB_CHECK(w.near.alloc(sizeof(int) * std::max(1, total[1])));
   d[1].m2l.src = w.far.as<int>();
   EB_CUDA(cudaMemcpyAsync(dd + 1, &d[1], sizeof(TreeDesc), cudaMemcpyHostToDevice, st));
-  group_lists_kernel<true><<<gb, 32 * kListWarps, 0, st>>>(ngroups, plan.nnodes - 1, plan.ncells, theta, d[0].ball,
+  group_lists_kernel<true><<<gb, 32 * kListWarps, 0, st>>>(ngroups, plan.nnodes - 1, plan.ncells, ratio, d[0].ball,
                                                            t->formed, t->children, gball, far_ptr, near_ptr,
                                                            task_ptr, w.far.as<int>(), w.near.as<int>());
   EB_CUDA(cudaGetLastError());

@@ -187,10 +187,9 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
     }
     const dq &x = p.ball[a], &y = p.ball[b];
     const d3 d = mk3(x.x - y.x, x.y - y.y, x.z - y.z);
-    const double r = x.w + y.w, d2 = dot3(d, d);
-    if (d2 * (kTreeTheta * kTreeTheta) > r * r) {
-      const double share = 2.0 * std::log(kTreeTheta) / std::log(r * r / d2);
-      far.push_back({a, b, 255u - (unsigned)std::min(255.0, std::max(1.0, std::ceil(255.0 * share)))});
+    const double d2 = dot3(d, d);
+    if (separated(x.w, y.w, d2, kTreeRatio)) {
+      far.push_back({a, b, 255u - degree_share(x.w, y.w, d2, kTreeRatio)});
     } else if (A.left < 0 && B.left < 0) {
       near.push_back({std::min(a, b), std::max(a, b)});
       if ((long long)near.size() > limit) return nc <= kTreeAllCloseCells && all_close();

@@ -1,13 +1,14 @@
 // Cluster tree of a mesh's far field (host side): the cells of the sorted
 // order are the leaves, the ranges of the bisection the inner nodes.
 //
-// A pair of nodes is separated when the sum of its radii is below kTreeTheta
-// times the distance of its centres. The traversal of the tree against itself
+// A pair of nodes is separated when its expansions converge fast enough
+// (separation_ratio). The traversal of the tree against itself
 // splits all cell pairs exactly once into separated node pairs (evaluated
 // through multipole and local expansions) and close cell pairs (evaluated
 // point by point).
 #pragma once
 
+#include <cmath>
 #include <utility>
 #include <vector>
 
@@ -16,12 +17,46 @@
 
 namespace eb {
 
-// Separation: measured on the perturbed icosphere L5 and a torus, random
-// densities, far sum against the whole sum. At 0.5, order 14: 1.9e-10 (SL) and
-// 6.8e-9 (DL); order 24: 3.4e-15 and 3.5e-14. A wider ratio trades close cell
-// pairs (16 a cell at 0.5, 11 at 0.6) for higher orders (18 at 0.6 for the
-// accuracy of 14 at 0.5).
-constexpr double kTreeTheta = 0.5;
+// What an expansion of order p leaves out of the sum between two balls falls as
+// the (p + 1)-th power of the larger of r_a / (d - r_b) and r_b / (d - r_a)
+// (the multipole's sources against the nearest target point, the targets
+// against the nearest source), which is the larger ball's ratio. It is below 1
+// for balls that do not touch.
+__host__ __device__ inline double separation_ratio(double ra, double rb, double dist)
+{
+  return ra > rb ? ra / (dist - rb) : rb / (dist - ra);
+}
+// True when that ratio is below q < 1 (d2 = dist^2).
+__host__ __device__ inline bool separated(double ra, double rb, double d2, double q)
+{
+  const double least = ra > rb ? rb + ra / q : ra + rb / q;
+  return d2 > least * least;
+}
+// Degrees that such a pair needs, as f / 255 of those that ratio q needs.
+__host__ __device__ inline unsigned degree_share(double ra, double rb, double d2, double q)
+{
+  const double f = ceil(255.0 * log(q) / log(separation_ratio(ra, rb, sqrt(d2))));
+  return f < 1.0 ? 1u : f < 255.0 ? (unsigned)f : 255u;
+}
+// Closest pairs. Times of the SL+DL apply of a sphere of 81,920 triangles in
+// us, mixed / FP64, and errors against FP64 point sums, random densities.
+// "sphere": 14,208 triangles refined towards a
+// pole by 0.9 per ring, the rows of its smallest quarter (DL; the symmetric
+// kernels 1.6e-7 and 1.4e-12 there); "bodies": two spheres of radius 1 and 0.02
+// at 0.2, the rows of the small one (3.3e-7 and 7.6e-14):
+//   r_a + r_b < 0.5 d   2,128 / 8,720   sphere 2.1e-6, 1.0e-10   bodies 1.2e-6, 3.7e-11
+//   0.33                2,264 / 9,380   sphere 5.9e-8, 1.8e-12   bodies 2.4e-7, 9.0e-14
+//   0.36                2,075 / 8,575   sphere 8.9e-8, 1.8e-12   bodies 2.4e-7, 9.0e-14
+//   0.40                1,810 / 7,485   sphere 4.8e-7, 1.9e-12
+// A sum of the radii says little about unequal balls (a coarse cell beside a
+// small body, which a cell's radius cannot follow), where its bound is 0.5.
+constexpr double kTreeRatio = 0.36;
+// Triangles that share a vertex must stay in close cells. With the outermost
+// points of the 7-point rule at 0.696 of the way from the centroid to a vertex
+// (farther out in the larger rules), a cell's vertices lie within 1.873 of its
+// radius over the points, so separated nodes, at least (1 + 1 / ratio) / 2 of
+// the sum of their radii apart, have no common one.
+static_assert((1.0 + 1.0 / kTreeRatio) / 2.0 > 1.873, "separated nodes share no vertex");
 // Least distance of a node's centre from its descendants' centres, over its radius.
 constexpr double kTreeMinStep = 1e-3;
 // The upward pass covers three levels of the tree per launch (up to eight
@@ -37,14 +72,17 @@ constexpr int kTreeMaxNodes = 1 << 24;
 // 3,280 x 100,000 4.34 -> 4.53.
 constexpr double kTreePointPairs32 = 2e7, kTreePointPairs64 = 1e8;
 constexpr int kTreePointTriangles64 = 5000;
-// Separation of a group of points from a node. Potentials in the volume are
-// small against the contributions that cancel in them (rough double-layer
-// densities above all), so the same orders need smaller ratios than the
-// applies. Error against 64-bit sums, 50,000 points inside an icosphere L5
-// (the direct sums: 8.3e-8 mixed, 7.1e-16 FP64): at 0.5 1.8e-7 and 1.5e-12, at
-// 0.45 2.8e-8 and 5.2e-14, at 0.4 1.5e-15, at 0.35 5.1e-16 in FP64.
-constexpr double kTreePointTheta32 = 0.45;
-constexpr double kTreePointTheta64 = 0.35;
+// Ratio of a group of points and a node. Potentials in the volume are small
+// against the contributions that cancel in them (rough double-layer densities
+// above all), so FP64 needs a smaller one than the applies. 50,000 points
+// around five meshes (sphere, torus, graded sphere and cube, two bodies of
+// size 10 : 1), random densities, against FP64 point sums: mixed 2.6e-8 at 0.36
+// (the direct sums 5.2e-8) inside the sphere of 20,480 triangles, 6.0e-6 (9.1e-6)
+// at a probe of size 0.001 beside it where the potential nearly cancels, 2.0e-5
+// there at 0.38; FP64 2e-15 of the largest potential from 0.21 to 0.32, 5e-14
+// at the probe (rounding), times at 0.25, 0.28, 0.30: 8.0, 6.8, 6.1 ms.
+constexpr double kTreePointRatio32 = 0.36;
+constexpr double kTreePointRatio64 = 0.30;
 // Close cell pairs per near task (one warp's work; the diagonal counts): at
 // most kTreeNearChunk, fewer while that leaves less than kTreeNearTasks tasks
 // (four warps on each of the 592 SM quarters).
@@ -71,9 +109,8 @@ constexpr int kTreeAllCloseCells = 140;
 // Expansions moved into node tgt[k] from nodes src[ptr[k] .. ptr[k + 1]). The
 // upper 8 bits of a source are the share f / 255 of the degrees that its pair
 // needs: an expansion of order p is used up to (p + 1) f / 255 - 1 (rounded
-// up). With radii r and distance d the truncation falls as (r / d)^(order + 1),
-// so f = ln(kTreeTheta) / ln(r / d) gives every pair the bound of the closest
-// ones (0.8 on average: half of the work). Sorted by f, largest first.
+// up). With f = ln(kTreeRatio) / ln(ratio) every pair has the bound of the
+// closest ones (0.8 on average: half of the work). Sorted by f, largest first.
 struct TreeMoves {
   std::vector<int> tgt, ptr = {0}, src;
 };

@@ -374,8 +374,10 @@ int eb_mesh_get_plan(eb_mesh mesh, int* items_per_sm, int* src_tile, int* nsplit
  * some 4,000 triangles all cells are close and get reports EB_FAR_SYMMETRIC.
  * Rules of 12 points and more: SL, DL and SL+DL on meshes that have separated
  * clusters. EB_FAR_SYMMETRIC's rules otherwise, and where more than a third of
- * the cell pairs of a larger mesh are close. The expansion orders keep the
- * truncation below the rounding of the point sums in either precision. An
+ * the cell pairs of a larger mesh are close. What the expansions leave out
+ * was at or below the rounding of the point sums in either precision on every
+ * surface measured: smooth ones, ones graded towards a pole or edges, and two
+ * bodies of size 50 : 1, on the rows of their smallest triangles too. An
  * apply runs the close cells on a stream of the mesh's own beside the
  * expansions; work before and after it on the caller's stream is ordered as
  * with one stream, also under capture. Scratch, allocated with a variant's
