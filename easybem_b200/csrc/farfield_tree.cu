@@ -39,6 +39,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <numeric>
 #include <type_traits>
 
 #include "farfield_sym_eval.cuh"
@@ -1832,22 +1833,66 @@ __global__ void __launch_bounds__(32 * kPointWarps)
   if (on) out[p] = sum * (0.25 / M_PI);
 }
 
-// Sorted order of the points by code (stable two-pass radix sort).
+// The points of an evaluation that groups can hold, and the others: not finite,
+// or so far out that squared distances overflow. One of those in a group would
+// make its ball, and with it the expansion of every other point, infinite; the
+// direct sums treat each point alone.
+struct PointSet {
+  std::vector<int> perm, apart;
+  double lo[3], hi[3];  // box of perm
+  PointSet(int n, const double* pts) : perm(n)
+  {
+    std::iota(perm.begin(), perm.end(), 0);
+    if (box(pts)) return;
+    perm.clear();
+    for (int i = 0; i < n; i++) (inside(pts + 3 * (size_t)i) ? perm : apart).push_back(i);
+    box(pts);
+  }
+
+ private:
+  static bool inside(const double* p)
+  {
+    constexpr double kOutside = 1e150;
+    return (std::fabs(p[0]) < kOutside) & (std::fabs(p[1]) < kOutside) & (std::fabs(p[2]) < kOutside);
+  }
+  // The box of perm; false when one of its points is outside.
+  bool box(const double* pts)
+  {
+    double a[3] = {1e300, 1e300, 1e300}, b[3] = {-1e300, -1e300, -1e300};
+    bool in = true;
+    for (const int i : perm) {
+      const double* p = pts + 3 * (size_t)i;
+      in &= inside(p);
+      for (int d = 0; d < 3; d++) {
+        a[d] = p[d] < a[d] ? p[d] : a[d];
+        b[d] = p[d] > b[d] ? p[d] : b[d];
+      }
+    }
+    std::copy_n(a, 3, lo);
+    std::copy_n(b, 3, hi);
+    return in;
+  }
+};
+
+__global__ void scatter_kernel(int n, const int* __restrict__ at, const double* __restrict__ v, double* __restrict__ out)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[at[i]] = v[i];
+}
+
+// Sorts the points of perm by code (stable two-pass radix sort).
 void order_points(const std::vector<unsigned>& code, std::vector<int>* perm)
 {
-  const size_t n = code.size();
+  const size_t n = perm->size();
   constexpr int kBits = 11, kBins = 1 << kBits;
   static_assert(3 * kCurveBits <= 2 * kBits, "two passes cover the code");
   std::vector<int> a(n), cnt(kBins + 1);
-  perm->resize(n);
   for (int pass = 0; pass < 2; pass++) {
+    std::vector<int>&from = pass ? a : *perm, &to = pass ? *perm : a;
     std::fill(cnt.begin(), cnt.end(), 0);
-    for (size_t i = 0; i < n; i++) cnt[(code[i] >> (pass * kBits) & (kBins - 1)) + 1]++;
+    for (size_t i = 0; i < n; i++) cnt[(code[from[i]] >> (pass * kBits) & (kBins - 1)) + 1]++;
     for (int k = 0; k < kBins; k++) cnt[k + 1] += cnt[k];
-    for (size_t i = 0; i < n; i++) {
-      const int p = pass ? a[i] : (int)i;
-      (pass ? *perm : a)[cnt[code[p] >> (pass * kBits) & (kBins - 1)]++] = p;
-    }
+    for (size_t i = 0; i < n; i++) to[cnt[code[from[i]] >> (pass * kBits) & (kBins - 1)]++] = from[i];
   }
 }
 
@@ -1881,7 +1926,7 @@ void split_groups(const std::vector<unsigned>& code, const std::vector<int>& per
 }
 
 template <int P>
-int evaluate_order(Mesh* m, int n, const double* pts, const double* d_pts, const ApplyArgs& A, const float4* rec32,
+int evaluate_order(Mesh* m, int n, PointSet& set, const double* d_pts, const ApplyArgs& A, const float4* rec32,
                    const dq* rec64, double* d_out, cudaStream_t st)
 {
   TreeMesh* t = m->tree.get();
@@ -1891,14 +1936,7 @@ int evaluate_order(Mesh* m, int n, const double* pts, const double* d_pts, const
   TreeTables tab;
   EB_CHECK(tables_for(m->device, P, &tab));
   // positions on the curve first: the host sorts them while the GPU forms the multipoles
-  double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-  for (int i = 0; i < n; i++)
-    for (int d = 0; d < 3; d++) {
-      const double v = pts[3 * (size_t)i + d];
-      if (!std::isfinite(v)) continue;
-      lo[d] = std::min(lo[d], v);
-      hi[d] = std::max(hi[d], v);
-    }
+  const double *lo = set.lo, *hi = set.hi;
   const double ext = std::max({hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2], 1e-300});
   EB_CHECK(w.code.alloc(sizeof(unsigned) * (size_t)n));
   EB_CHECK(w.perm.alloc(sizeof(int) * (size_t)n));
@@ -1920,12 +1958,13 @@ int evaluate_order(Mesh* m, int n, const double* pts, const double* d_pts, const
   for (int s = 0; s < kTreePasses; s++)
     EB_CUDA(start(tree_move_kernel<P, 1, kUp>, dim3(d[0].nup[s]), Mv::kThreads, Mv::smem(), st, (const TreeDesc*)dd,
                   (const int*)nullptr, 1, s, tab));
-  std::vector<int> perm;
+  std::vector<int>& perm = set.perm;
+  const int npts = (int)perm.size();
   order_points(code, &perm);
   std::vector<int> gptr;
-  split_groups(code, perm, 0, n, 0, &gptr);
+  split_groups(code, perm, 0, npts, 0, &gptr);
   const int ngroups = (int)gptr.size();
-  gptr.push_back(n);
+  gptr.push_back(npts);
   perm.insert(perm.end(), gptr.begin(), gptr.end());  // one copy
   EB_CHECK(w.perm.alloc(sizeof(int) * perm.size()));
   EB_CHECK(w.ptr.alloc(sizeof(int) * 4 * ((size_t)ngroups + 1)));
@@ -1933,7 +1972,7 @@ int evaluate_order(Mesh* m, int n, const double* pts, const double* d_pts, const
   EB_CHECK(w.local.alloc(sizeof(double2) * ((size_t)plan.nnodes + ngroups) * kPairs));
   EB_CUDA(cudaMemcpyAsync(w.perm.p, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice, st));
   const int* d_perm = w.perm.as<int>();
-  const int* d_gptr = d_perm + n;
+  const int* d_gptr = d_perm + npts;
   int* far_ptr = w.ptr.as<int>();
   int* near_ptr = far_ptr + ngroups + 1;
   int* task_ptr = near_ptr + ngroups + 1;
@@ -2187,19 +2226,46 @@ bool tree_points_eligible(const Mesh* m, bool fp32, int npts)
          !wide_rule(m->h) && (fp32 ? pairs >= kTreePointPairs32 : pairs >= kTreePointPairs64 && m->h.ne >= kTreePointTriangles64);
 }
 
+// Direct sums at the points that are set apart.
+static int evaluate_apart(Mesh* m, bool fp32, const std::vector<int>& apart, const double* pts, const double* d_t,
+                          const double* d_u, double* d_out, cudaStream_t st)
+{
+  const size_t n = apart.size();
+  std::vector<double> x(3 * n);
+  for (size_t i = 0; i < n; i++) std::copy_n(pts + 3 * (size_t)apart[i], 3, &x[3 * i]);
+  DevBuf& w = m->tree->points.apart;
+  EB_CHECK(w.alloc(n * (4 * sizeof(double) + sizeof(int))));
+  double *d_x = w.as<double>(), *d_v = d_x + 3 * n;
+  int* d_at = reinterpret_cast<int*>(d_v + n);
+  EB_CUDA(cudaMemcpyAsync(d_x, x.data(), sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
+  EB_CUDA(cudaMemcpyAsync(d_at, apart.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st));
+  EB_CHECK(mesh_evaluate_potential(m, fp32 ? EB_PREC_MIXED : EB_PREC_FP64, (int)n, d_x, d_t, d_u, d_v, st));
+  scatter_kernel<<<((int)n + 255) / 256, 256, 0, st>>>((int)n, d_at, d_v, d_out);
+  EB_CUDA(cudaGetLastError());
+  EB_CUDA(cudaStreamSynchronize(st));  // x is read by the copy
+  return EB_OK;
+}
+
 int tree_evaluate(Mesh* m, bool fp32, int npts, const double* pts, const double* d_pts, const double* d_t,
                   const double* d_u, double* d_out, cudaStream_t st)
 {
-  // FP64 records in either precision (the cells closest to a point), FP32 ones beside them
-  DevBuf& rec = m->pot_rec64;
-  EB_CHECK(rec.alloc((size_t)m->h.ne * m->h.Q * rec_slots(1, 1) * sizeof(dq)));
-  const ApplyArgs A = mesh_apply_args(m, false, rec.p, nullptr, d_t, m->h.ne, d_u, nullptr, m->h.ne, nullptr);
-  EB_CUDA(prep_launch(false, 1, 1, A, st));
-  if (!fp32) return evaluate_order<kTreeOrder64>(m, npts, pts, d_pts, A, nullptr, rec.as<dq>(), d_out, st);
-  EB_CHECK(ensure_apply_scratch(m, true));
-  const ApplyArgs A32 = mesh_apply_args(m, true, m->rec.p, nullptr, d_t, m->h.ne, d_u, nullptr, m->h.ne, nullptr);
-  EB_CUDA(prep_launch(true, 1, 1, A32, st));
-  return evaluate_order<kTreeOrder32>(m, npts, pts, d_pts, A, m->rec.as<float4>(), rec.as<dq>(), d_out, st);
+  PointSet set(npts, pts);
+  if (!set.perm.empty()) {
+    // FP64 records in either precision (the cells closest to a point), FP32 ones beside them
+    DevBuf& rec = m->pot_rec64;
+    EB_CHECK(rec.alloc((size_t)m->h.ne * m->h.Q * rec_slots(1, 1) * sizeof(dq)));
+    const ApplyArgs A = mesh_apply_args(m, false, rec.p, nullptr, d_t, m->h.ne, d_u, nullptr, m->h.ne, nullptr);
+    EB_CUDA(prep_launch(false, 1, 1, A, st));
+    if (fp32) {
+      EB_CHECK(ensure_apply_scratch(m, true));
+      const ApplyArgs A32 = mesh_apply_args(m, true, m->rec.p, nullptr, d_t, m->h.ne, d_u, nullptr, m->h.ne, nullptr);
+      EB_CUDA(prep_launch(true, 1, 1, A32, st));
+      EB_CHECK(evaluate_order<kTreeOrder32>(m, npts, set, d_pts, A, m->rec.as<float4>(), rec.as<dq>(), d_out, st));
+    } else {
+      EB_CHECK(evaluate_order<kTreeOrder64>(m, npts, set, d_pts, A, nullptr, rec.as<dq>(), d_out, st));
+    }
+  }
+  return set.apart.empty() ? EB_OK : evaluate_apart(m, fp32, set.apart, pts, d_t, d_u, d_out, st);
 }
 
 size_t tree_bytes(const Mesh* m)

@@ -76,7 +76,7 @@ struct TreeSide {
 
 // Scratch of the potential evaluation.
 struct TreePoints {
-  DevBuf code, perm, multipole, local, ball, ptr, far, near, part, desc;
+  DevBuf code, perm, multipole, local, ball, ptr, far, near, part, desc, apart;
 };
 
 // Block counts of each kernel over the meshes of a launch and, for more than
