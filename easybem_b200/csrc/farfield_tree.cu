@@ -1575,6 +1575,11 @@ __global__ void group_ball_kernel(int ngroups, const int* __restrict__ gptr, con
 }
 
 constexpr int kPointCells = 4;  // close cells of a task
+// Lists, expansions and partial sums of the groups evaluated at a time, kept by
+// the mesh: only millions of points (150,000 groups in FP64), or groups that
+// are close to hundreds of cells each, are cut. 6 million points, FP64: 2.3 GB
+// at once, 0.4 GB in parts.
+constexpr size_t kPointScratch = (size_t)1 << 30;
 constexpr int kListWarps = 4;
 constexpr int kListStack = 1024;  // 32 nodes leave and at most 64 children enter: at most 32 (height + 1)
 static_assert(32 * (kTreePasses * kTreeLevelsPerPass + 2) <= kListStack, "stack of the deepest tree");
@@ -1636,14 +1641,15 @@ __global__ void __launch_bounds__(32 * kListWarps)
   }
 }
 
-// Exclusive sums of a[0, n), b[0, n) and c[0, n) in place, totals at [n] (one block).
+// Exclusive sums of a[0, n), b[0, n) and c[0, n) in place, totals at [n] and in
+// total (one block). Sums past 2^31 wrap, the totals do not.
 __global__ void __launch_bounds__(1024) scan_lists_kernel(int n, int* __restrict__ a, int* __restrict__ b,
-                                                          int* __restrict__ c)
+                                                          int* __restrict__ c, long long* __restrict__ total)
 {
   __shared__ int warps[3][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int* v[3] = {a, b, c};
-  int base[3] = {0, 0, 0};
+  long long base[3] = {0, 0, 0};
   for (int i0 = 0; i0 < n; i0 += 1024) {
     const int i = i0 + threadIdx.x;
     int x[3], s[3];
@@ -1660,16 +1666,19 @@ __global__ void __launch_bounds__(1024) scan_lists_kernel(int n, int* __restrict
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      int before = base[k];
+      long long before = base[k];
       for (int j = 0; j < 32; ++j) {
         if (j < w) before += warps[k][j];
         base[k] += warps[k][j];
       }
-      if (i < n) v[k][i] = before + s[k] - x[k];
+      if (i < n) v[k][i] = (int)(before + s[k] - x[k]);
     }
     __syncthreads();
   }
-  if (threadIdx.x < 3) v[threadIdx.x][n] = base[threadIdx.x];
+  if (threadIdx.x < 3) {
+    v[threadIdx.x][n] = (int)base[threadIdx.x];
+    total[threadIdx.x] = base[threadIdx.x];
+  }
 }
 
 __global__ void iota_kernel(int n, int first, int* __restrict__ v)
@@ -1967,59 +1976,72 @@ int evaluate_order(Mesh* m, int n, PointSet& set, const double* d_pts, const App
   gptr.push_back(npts);
   perm.insert(perm.end(), gptr.begin(), gptr.end());  // one copy
   EB_CHECK(w.perm.alloc(sizeof(int) * perm.size()));
-  EB_CHECK(w.ptr.alloc(sizeof(int) * 4 * ((size_t)ngroups + 1)));
   EB_CHECK(w.ball.alloc(sizeof(dq) * ((size_t)plan.nnodes + ngroups)));
-  EB_CHECK(w.local.alloc(sizeof(double2) * ((size_t)plan.nnodes + ngroups) * kPairs));
   EB_CUDA(cudaMemcpyAsync(w.perm.p, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice, st));
   const int* d_perm = w.perm.as<int>();
   const int* d_gptr = d_perm + npts;
-  int* far_ptr = w.ptr.as<int>();
-  int* near_ptr = far_ptr + ngroups + 1;
-  int* task_ptr = near_ptr + ngroups + 1;
-  int* ids = task_ptr + ngroups + 1;
   // the groups as targets: nodes nnodes, nnodes + 1, ...
   dq* gball = w.ball.as<dq>() + plan.nnodes;
-  d[1] = d[0];
-  d[1].ball = w.ball.as<dq>();
-  d[1].local = w.local.as<double2>();
-  d[1].m2l.tgt = ids;
-  d[1].m2l.ptr = far_ptr;
   EB_CUDA(cudaMemcpyAsync(w.ball.p, d[0].ball, sizeof(dq) * plan.nnodes, cudaMemcpyDeviceToDevice, st));
   const double root = plan.ball[plan.nnodes - 1].w, ratio = P <= kTreeOrder32 ? kTreePointRatio32 : kTreePointRatio64;
   group_ball_kernel<<<(ngroups + 3) / 4, 128, 0, st>>>(ngroups, d_gptr, d_pts, d_perm, 1e-4 * root, gball);
-  const int gb = (ngroups + kListWarps - 1) / kListWarps;
-  group_lists_kernel<false><<<gb, 32 * kListWarps, 0, st>>>(ngroups, plan.nnodes - 1, plan.ncells, ratio, d[0].ball,
-                                                            t->formed, t->children, gball, far_ptr, near_ptr, task_ptr,
-                                                            nullptr, nullptr);
-  scan_lists_kernel<<<1, 1024, 0, st>>>(ngroups, far_ptr, near_ptr, task_ptr);
-  iota_kernel<<<(ngroups + 255) / 256, 256, 0, st>>>(ngroups, plan.nnodes, ids);
   EB_CUDA(cudaGetLastError());
-  int total[3];
-  EB_CUDA(cudaMemcpyAsync(&total[0], far_ptr + ngroups, sizeof(int), cudaMemcpyDeviceToHost, st));
-  EB_CUDA(cudaMemcpyAsync(&total[1], near_ptr + ngroups, sizeof(int), cudaMemcpyDeviceToHost, st));
-  EB_CUDA(cudaMemcpyAsync(&total[2], task_ptr + ngroups, sizeof(int), cudaMemcpyDeviceToHost, st));
-  EB_CUDA(cudaStreamSynchronize(st));
-  EB_CHECK(w.part.alloc(sizeof(double) * 32 * (size_t)std::max(1, total[2])));
-  EB_CHECK(w.far.alloc(sizeof(int) * std::max(1, total[0])));
-  EB_CHECK(w.near.alloc(sizeof(int) * std::max(1, total[1])));
-  d[1].m2l.src = w.far.as<int>();
-  EB_CUDA(cudaMemcpyAsync(dd + 1, &d[1], sizeof(TreeDesc), cudaMemcpyHostToDevice, st));
-  group_lists_kernel<true><<<gb, 32 * kListWarps, 0, st>>>(ngroups, plan.nnodes - 1, plan.ncells, ratio, d[0].ball,
-                                                           t->formed, t->children, gball, far_ptr, near_ptr,
-                                                           task_ptr, w.far.as<int>(), w.near.as<int>());
-  EB_CUDA(cudaGetLastError());
-  EB_CUDA(start(tree_move_kernel<P, 1, kAcross>, dim3(ngroups), Mv::kThreads, Mv::smem(), st, (const TreeDesc*)(dd + 1),
-                (const int*)nullptr, 1, 0, tab));
-  constexpr bool F32 = P <= kTreeOrder32;
-  EB_CUDA(start(points_near_kernel<F32>, dim3((total[2] + kPointWarps - 1) / kPointWarps), 32 * kPointWarps,
-                (size_t)kPointWarps * kCell * kQ * kNrec * (F32 ? sizeof(float4) : sizeof(dq)), st, ngroups, total[2],
-                d_gptr, d_pts, d_perm, (const int*)task_ptr, (const int*)near_ptr, (const int*)w.near.as<int>(), m->h.ne,
-                rec32, (const float4*)m->splane32.as<float4>(), rec64, (const dq*)m->splane64.as<dq>(),
-                (const dq*)m->ccent.as<dq>(), w.part.as<double>()));
-  EB_CUDA(start(tree_points_kernel<P>, dim3((ngroups + kPointWarps - 1) / kPointWarps), 32 * kPointWarps, 0, st, ngroups,
-                d_gptr, d_pts, d_perm, (const dq*)gball,
-                (const double2*)(w.local.as<double2>() + (size_t)plan.nnodes * kPairs), (const int*)task_ptr,
-                (const double*)w.part.as<double>(), tab, d_out));
+  // All groups at once where their lists, expansions and partial sums fit
+  // kPointScratch, else as many at a time as fit whatever their lists hold.
+  const size_t local_bytes = sizeof(double2) * kPairs, task_bytes = sizeof(double) * 32;
+  const size_t most = local_bytes + 2 * sizeof(int) * (size_t)plan.ncells +
+                      task_bytes * ((plan.ncells + kPointCells - 1) / kPointCells);
+  const int slab = (int)std::max<size_t>(1, std::min<size_t>(ngroups, kPointScratch / most));
+  for (int g0 = 0, step = ngroups; g0 < ngroups;) {
+    const int ng = std::min(step, ngroups - g0);
+    EB_CHECK(w.ptr.alloc(sizeof(long long) * 3 + sizeof(int) * 4 * ((size_t)ng + 1)));
+    long long* d_total = w.ptr.as<long long>();
+    int* far_ptr = reinterpret_cast<int*>(d_total + 3);
+    int* near_ptr = far_ptr + ng + 1;
+    int* task_ptr = near_ptr + ng + 1;
+    int* ids = task_ptr + ng + 1;
+    const int gb = (ng + kListWarps - 1) / kListWarps;
+    group_lists_kernel<false><<<gb, 32 * kListWarps, 0, st>>>(ng, plan.nnodes - 1, plan.ncells, ratio, d[0].ball,
+                                                              t->formed, t->children, gball + g0, far_ptr, near_ptr,
+                                                              task_ptr, nullptr, nullptr);
+    scan_lists_kernel<<<1, 1024, 0, st>>>(ng, far_ptr, near_ptr, task_ptr, d_total);
+    iota_kernel<<<(ng + 255) / 256, 256, 0, st>>>(ng, plan.nnodes + g0, ids);
+    EB_CUDA(cudaGetLastError());
+    long long total[3];
+    EB_CUDA(cudaMemcpyAsync(total, d_total, sizeof(total), cudaMemcpyDeviceToHost, st));
+    EB_CUDA(cudaStreamSynchronize(st));
+    if (step > slab && local_bytes * ng + sizeof(int) * (size_t)(total[0] + total[1]) +
+                               task_bytes * (size_t)total[2] > kPointScratch) {
+      step = slab;
+      continue;
+    }
+    EB_CHECK(w.local.alloc(local_bytes * ng));
+    EB_CHECK(w.part.alloc(task_bytes * (size_t)std::max(1ll, total[2])));
+    EB_CHECK(w.far.alloc(sizeof(int) * (size_t)std::max(1ll, total[0])));
+    EB_CHECK(w.near.alloc(sizeof(int) * (size_t)std::max(1ll, total[1])));
+    d[1] = d[0];
+    d[1].ball = w.ball.as<dq>();
+    d[1].local = w.local.as<double2>() - (size_t)(plan.nnodes + g0) * kPairs;  // the first group's at its node
+    d[1].m2l = TreeMovesDev{ids, far_ptr, w.far.as<int>()};
+    EB_CUDA(cudaMemcpyAsync(dd + 1, &d[1], sizeof(TreeDesc), cudaMemcpyHostToDevice, st));
+    group_lists_kernel<true><<<gb, 32 * kListWarps, 0, st>>>(ng, plan.nnodes - 1, plan.ncells, ratio, d[0].ball,
+                                                             t->formed, t->children, gball + g0, far_ptr, near_ptr,
+                                                             task_ptr, w.far.as<int>(), w.near.as<int>());
+    EB_CUDA(cudaGetLastError());
+    EB_CUDA(start(tree_move_kernel<P, 1, kAcross>, dim3(ng), Mv::kThreads, Mv::smem(), st, (const TreeDesc*)(dd + 1),
+                  (const int*)nullptr, 1, 0, tab));
+    constexpr bool F32 = P <= kTreeOrder32;
+    const int ntasks = (int)total[2];
+    EB_CUDA(start(points_near_kernel<F32>, dim3((ntasks + kPointWarps - 1) / kPointWarps), 32 * kPointWarps,
+                  (size_t)kPointWarps * kCell * kQ * kNrec * (F32 ? sizeof(float4) : sizeof(dq)), st, ng, ntasks,
+                  d_gptr + g0, d_pts, d_perm, (const int*)task_ptr, (const int*)near_ptr, (const int*)w.near.as<int>(),
+                  m->h.ne, rec32, (const float4*)m->splane32.as<float4>(), rec64,
+                  (const dq*)m->splane64.as<dq>(), (const dq*)m->ccent.as<dq>(), w.part.as<double>()));
+    EB_CUDA(start(tree_points_kernel<P>, dim3((ng + kPointWarps - 1) / kPointWarps), 32 * kPointWarps, 0, st, ng,
+                  d_gptr + g0, d_pts, d_perm, (const dq*)(gball + g0), (const double2*)w.local.as<double2>(),
+                  (const int*)task_ptr, (const double*)w.part.as<double>(), tab, d_out));
+    g0 += ng;
+  }
   EB_CUDA(cudaStreamSynchronize(st));  // perm and d are read by the copies
   return EB_OK;
 }
@@ -2274,12 +2296,21 @@ size_t tree_bytes(const Mesh* m)
   size_t b = m->tree->lists.bytes + m->tree->fwd_lists.bytes;
   for (const auto& s : m->tree->scratch)
     b += s.second->multipole.bytes + s.second->local.bytes + s.second->partial.bytes + s.second->desc.bytes;
+  const TreePoints& w = m->tree->points;
+  for (const DevBuf* d : {&w.code, &w.perm, &w.multipole, &w.local, &w.ball, &w.ptr, &w.far, &w.near, &w.part, &w.desc,
+                          &w.apart})
+    b += d->bytes;
   return b;
 }
 
 void tree_release_scratch(Mesh* m)
 {
-  if (m->tree) m->tree->scratch.clear();
+  if (!m->tree) return;
+  m->tree->scratch.clear();
+  TreePoints& w = m->tree->points;
+  for (DevBuf* d : {&w.code, &w.perm, &w.multipole, &w.local, &w.ball, &w.ptr, &w.far, &w.near, &w.part, &w.desc,
+                    &w.apart})
+    d->release();
 }
 
 int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream_t st)

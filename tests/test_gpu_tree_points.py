@@ -47,3 +47,26 @@ def test_points_out_of_range_leave_the_others_alone(surface, bad, count, prec, t
     rest = np.delete(np.arange(len(pts)), at)
     if len(rest):
         assert np.isfinite(p[rest]).all() and rel_l2(p[rest], good[rest]) < tol
+
+
+def test_scratch_of_many_points_is_bounded(gpu_lib):
+    """6 million points: beside arrays of the points' number (positions,
+    potentials, order: below 100 bytes a point) an evaluation keeps 1 GiB at
+    most; 256 MiB for the mesh's own tables and the pool's blocks."""
+    import torch
+
+    n = 6_000_000
+    pts = _inside(n, 2)
+    nodes, elems = meshes.perturbed_icosphere(5, seed=3)
+    rng = np.random.default_rng(4)
+    t, u, rows = rng.normal(size=len(elems)), rng.normal(size=len(nodes)), rng.choice(n, 2000, replace=False)
+    lib = gpu_lib._lib.lib()
+    with gpu_lib.Mesh(nodes, elems) as m:
+        assert lib.eb_release_cached_memory() == 0
+        before = torch.cuda.mem_get_info()[0]
+        p = m.evaluate(pts, t, u, "fp64")
+        assert lib.eb_release_cached_memory() == 0
+        used = before - torch.cuda.mem_get_info()[0]
+        m.set_far_engine("cuda")
+        assert rel_l2(p[rows], m.evaluate(pts[rows], t, u, "fp64")) < 1e-12
+        assert used < (1 << 30) + 100 * n + (256 << 20)
