@@ -2099,9 +2099,10 @@ bool tree_eligible(const Mesh* m, int nsl, int nd)
          (!wide_rule(m->h) || (nsl <= 1 && nd <= 1));
 }
 
+// With t->lists_lock held, as upload_forward.
 static int upload_lists(TreeMesh* t)
 {
-  if (t->lists.p) return EB_OK;
+  if (t->lists_ready) return EB_OK;
   const TreePlan& p = t->plan;
   std::vector<unsigned char> host;
   auto add = [&](const auto& v) {
@@ -2144,6 +2145,7 @@ static int upload_lists(TreeMesh* t)
   d.ncells = p.ncells;
   d.ntasks = (int)p.sym.tasks.size();
   d.nm2l = (int)p.m2l.tgt.size();
+  t->lists_ready = true;
   return EB_OK;
 }
 
@@ -2176,30 +2178,27 @@ static int slot_columns(const Mesh* m, int nsl, int nd)
   return nsl == kTreeP1 ? 3 : nsl + nd + unused_columns(m, nsl, nd);
 }
 
-static void forward_lists(TreeMesh* t)
-{
-  if (t->fwd.slot_off.empty()) make_near_lists(t->plan, false, &t->fwd);
-}
-
 long long tree_far_slots(const Mesh* m, int nsl, int nd)
 {
-  TreeMesh& t = *m->tree;
-  if (tree_forward(m, nsl, nd)) forward_lists(&t);
-  return (long long)(tree_forward(m, nsl, nd) ? t.fwd : t.plan.sym).slot_off.back() * kCell;
+  const TreePlan& p = m->tree->plan;
+  return (long long)(tree_forward(m, nsl, nd) ? p.forward_slots : p.sym.slot_off.back()) * kCell;
 }
 
 static int upload_forward(TreeMesh* t)
 {
-  if (t->fwd_lists.p) return EB_OK;
-  forward_lists(t);
-  const TreeNear& f = t->fwd;
+  if (t->fwd_ready) return EB_OK;
+  TreeNear& f = t->fwd;
+  f = TreeNear();
+  make_near_lists(t->plan, false, &f);
   const size_t a = f.tasks.size() * sizeof(int4), b = f.entries.size() * sizeof(int2), c = f.slot_off.size() * sizeof(int);
   std::vector<unsigned char> host(a + b + c);
   std::memcpy(host.data(), f.tasks.data(), a);
   std::memcpy(host.data() + a, f.entries.data(), b);
   std::memcpy(host.data() + a + b, f.slot_off.data(), c);
   EB_CHECK(t->fwd_lists.alloc(host.size()));
-  return copy_h2d(t->fwd_lists.p, host.data(), host.size());
+  EB_CHECK(copy_h2d(t->fwd_lists.p, host.data(), host.size()));
+  t->fwd_ready = true;
+  return EB_OK;
 }
 
 int tree_tables(bool fp32, int device)
@@ -2222,6 +2221,7 @@ int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, v
               TreeDesc* out)
 {
   TreeMesh* t = m->tree.get();
+  std::lock_guard<std::mutex> g(t->lists_lock);
   EB_CHECK(upload_lists(t));
   TreeDesc d = t->base;
   if (tree_forward(m, nsl, nd)) {
@@ -2293,7 +2293,11 @@ int tree_evaluate(Mesh* m, bool fp32, int npts, const double* pts, const double*
 size_t tree_bytes(const Mesh* m)
 {
   if (!m->tree) return 0;
-  size_t b = m->tree->lists.bytes + m->tree->fwd_lists.bytes;
+  size_t b = 0;
+  {
+    std::lock_guard<std::mutex> g(m->tree->lists_lock);
+    b += m->tree->lists.bytes + m->tree->fwd_lists.bytes;
+  }
   for (const auto& s : m->tree->scratch)
     b += s.second->multipole.bytes + s.second->local.bytes + s.second->partial.bytes + s.second->desc.bytes;
   const TreePoints& w = m->tree->points;

@@ -6,6 +6,7 @@
 
 #include <map>
 #include <memory>
+#include <mutex>
 
 #include "engine.h"
 #include "tree_plan.h"
@@ -93,9 +94,13 @@ struct TreeGrid {
 struct TreeMesh {
   bool usable = false;
   TreePlan plan;
+  // The lists are made once, by the first descriptor that needs them: of a call
+  // on the mesh, or of a batch or solver, which share it between threads.
+  std::mutex lists_lock;
+  bool lists_ready = false, fwd_ready = false;
   DevBuf lists;  // one allocation
   TreeDesc base; // static pointers
-  // close pairs in forward order, made with the first variant that needs them
+  // close pairs in forward order
   TreeNear fwd;
   DevBuf fwd_lists;
   const int2* children = nullptr;  // of the inner nodes (device)

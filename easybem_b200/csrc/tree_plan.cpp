@@ -77,6 +77,30 @@ struct Rows {
   }
 };
 
+// How a list of pairs is cut into tasks, and the slots of a cell's forward sums.
+struct Tasks {
+  int chunk, log_parts = 0;
+  explicit Tasks(int pairs) : chunk(std::min(kTreeNearChunk, std::max(1, pairs / kTreeNearTasks)))
+  {
+    while ((1 << log_parts) < kTreeNearParts && (pairs << log_parts) < kTreeNearTasks) log_parts++;
+  }
+  int parts() const { return 1 << log_parts; }  // above 1 with chunk 1 only
+  int slots(int close) const { return (close + chunk) / chunk * parts(); }  // with the cell itself
+};
+
+int count_forward_slots(const TreePlan& plan)
+{
+  std::vector<int> close(plan.ncells, 0);
+  for (const auto& q : plan.near) {
+    close[q.first]++;
+    close[q.second]++;
+  }
+  const Tasks cut(plan.ncells + 2 * (int)plan.near.size());
+  int n = plan.all_close ? 0 : plan.ncells;  // the far slots
+  for (int c : close) n += cut.slots(c);
+  return n;
+}
+
 }  // namespace
 
 void make_near_lists(const TreePlan& plan, bool both, TreeNear* out)
@@ -84,11 +108,8 @@ void make_near_lists(const TreePlan& plan, bool both, TreeNear* out)
   // transposed slots first, then one forward slot per task, then the far slot
   const int nc = plan.ncells;
   const Rows close(nc, plan.near, !both);
-  const int pairs = nc + (int)close.col.size();
-  const int chunk = std::min(kTreeNearChunk, std::max(1, pairs / kTreeNearTasks));
-  int log_parts = 0;
-  while ((1 << log_parts) < kTreeNearParts && (pairs << log_parts) < kTreeNearTasks) log_parts++;
-  const int parts = 1 << log_parts;  // above 1 with chunk 1 only
+  const Tasks cut(nc + (int)close.col.size());
+  const int parts = cut.parts(), log_parts = cut.log_parts, chunk = cut.chunk;
   const int far_slots = plan.all_close ? 0 : 1;
   std::vector<int> trans(nc, 0);
   if (both)
@@ -96,7 +117,7 @@ void make_near_lists(const TreePlan& plan, bool both, TreeNear* out)
   out->slot_off.assign(nc + 1, 0);
   for (int c = 0; c < nc; c++)
     out->slot_off[c + 1] =
-        out->slot_off[c] + trans[c] + (close.ptr[c + 1] - close.ptr[c] + chunk) / chunk * parts + far_slots;
+        out->slot_off[c] + trans[c] + cut.slots(close.ptr[c + 1] - close.ptr[c]) + far_slots;
   std::vector<int> next(out->slot_off.begin(), out->slot_off.end() - 1);
   out->entries.reserve((close.col.size() + nc) * parts);
   for (int c = 0; c < nc; c++) {
@@ -128,6 +149,7 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
     for (int c = 0; c < nc; c++)
       for (int j = c + 1; j < nc; j++) p.near.push_back({c, j});
     make_near_lists(p, true, &p.sym);
+    p.forward_slots = count_forward_slots(p);
     return true;
   };
   if (nc < kTreeMinCells) return all_close();
@@ -277,6 +299,7 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
 
   p.near.swap(near);
   make_near_lists(p, true, &p.sym);
+  p.forward_slots = count_forward_slots(p);
   return true;
 }
 

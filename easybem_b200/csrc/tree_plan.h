@@ -137,6 +137,7 @@ struct TreePlan {
   std::vector<char> formed;    // per node: the upward passes form its multipole
   std::vector<std::pair<int, int>> near;  // close cells, the earlier one first
   TreeNear sym;  // every unordered pair of cells once
+  int forward_slots = 0;  // of the lists of every ordered pair, which are made when a variant needs them
 };
 
 // False when more than a third of all cell pairs are close in a mesh of more
