@@ -2367,9 +2367,10 @@ int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, v
 
 bool tree_points_eligible(const Mesh* m, bool fp32, int npts)
 {
-  const double pairs = (double)npts * m->h.ne;
-  return m->plan.engine == 4 && m->tree && m->tree->usable && !m->tree->plan.all_close &&
-         !wide_rule(m->h) && (fp32 ? pairs >= kTreePointPairs32 : pairs >= kTreePointPairs64 && m->h.ne >= kTreePointTriangles64);
+  const double n = npts, ne = m->h.ne;
+  const double least = fp32 ? kTreePointPairs32 + kTreePointTriangles32 * ne + kTreePointPoints32 * n
+                            : kTreePointPairs64 + kTreePointTriangles64 * ne + kTreePointPoints64 * n;
+  return m->plan.engine == 4 && m->tree && m->tree->usable && !m->tree->plan.all_close && !wide_rule(m->h) && n * ne >= least;
 }
 
 // Direct sums at the points that are set apart.

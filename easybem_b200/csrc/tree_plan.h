@@ -64,14 +64,21 @@ constexpr double kTreeMinStep = 1e-3;
 constexpr int kTreeLevelsPerPass = 3;
 constexpr int kTreePasses = 6;  // enough for 2^18 cells
 constexpr int kTreeMaxNodes = 1 << 24;
-// Points x triangles from which the potential evaluation takes the tree, and
-// least triangles in FP64 (whose point sums are only 1.5 to 3 times dearer
-// than in the mixed evaluation, while the moves cost eight times the work).
-// Measured, direct -> tree (ms): mixed 5,940 triangles 2,000 points 0.41 -> 0.45,
-// 4,000 0.76 -> 0.47; FP64 17,860 x 4,000 1.09 -> 1.11, 8,000 1.97 -> 1.47;
-// 3,280 x 100,000 4.34 -> 4.53.
-constexpr double kTreePointPairs32 = 2e7, kTreePointPairs64 = 1e8;
-constexpr int kTreePointTriangles64 = 5000;
+// The potential evaluation takes the tree where points x triangles are at least
+// kTreePointPairs + kTreePointTriangles x triangles + kTreePointPoints x points:
+// what the direct sums take for a pair goes into each term of the tree's cost,
+// the launches, the multipoles of all cells and the groups' moves. Direct ->
+// tree in ms, points uniform inside a sphere or torus (points near the surface
+// and around it gain from slightly smaller numbers, in the mixed evaluation
+// points far away from some 3,000):
+//   triangles   mixed                                   FP64
+//     5,120     2,000 0.39 -> 0.48, 4,000 0.63 -> 0.49  100,000 6.66 -> 8.38
+//     8,192     1,000 0.28 -> 0.50, 2,000 0.49 -> 0.50  16,000 1.75 -> 1.87, 50,000 5.27 -> 4.42
+//    20,480     1,000 0.56 -> 0.62, 2,000 0.89 -> 0.64  4,000 1.23 -> 1.52, 8,000 2.26 -> 1.94
+//    81,920     500 0.71 -> 1.19, 1,000 1.18 -> 1.21    2,000 2.19 -> 3.13, 4,000 4.68 -> 3.30
+//   327,680     500 1.04 -> 3.13, 2,000 2.95 -> 3.07    2,000 8.58 -> 9.22, 4,000 18.6 -> 9.5
+constexpr double kTreePointPairs32 = 0.8e7, kTreePointTriangles32 = 900, kTreePointPoints32 = 0;
+constexpr double kTreePointPairs64 = 4.3e7, kTreePointTriangles64 = 2000, kTreePointPoints64 = 5200;
 // Ratio of a group of points and a node. Potentials in the volume are small
 // against the contributions that cancel in them (rough double-layer densities
 // above all), so FP64 needs a smaller one than the applies. 50,000 points

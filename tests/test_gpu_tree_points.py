@@ -116,3 +116,39 @@ def test_points_far_from_all_others(gpu_lib, prec, tol):
             m.set_far_engine("tree")
             assert rel_l2(p[rows], ref) < max(tol, 2 * direct), name
         assert max(seconds.values()) < 3 * seconds["plain"], seconds
+
+
+@pytest.mark.parametrize("level, npts, prec", [(7, 100, "mixed"), (6, 500, "mixed"), (4, 2000, "mixed"),
+                                               (4, 50000, "fp64"), (5, 4000, "fp64"), (6, 2000, "fp64"), (7, 500, "fp64")])
+def test_few_points_keep_the_direct_sums(gpu_lib, level, npts, prec):
+    """Sizes at which the tree was 1.2 to 10 times slower: no slower than the
+    direct engine (15 % for the clock; the least of 20 runs each)."""
+    nodes, elems = meshes.icosphere(level)
+    rng = np.random.default_rng(npts)
+    t, u, pts = rng.normal(size=len(elems)), rng.normal(size=len(nodes)), _inside(npts, 6)
+    with gpu_lib.Mesh(nodes, elems) as m:
+        seconds = {}
+        for engine in ("tree", "cuda"):
+            m.set_far_engine(engine)
+            took = []
+            for _ in range(20):
+                start = time.perf_counter()
+                m.evaluate(pts, t, u, prec)
+                took.append(time.perf_counter() - start)
+            seconds[engine] = min(took)
+        assert seconds["tree"] < 1.15 * seconds["cuda"], seconds
+
+
+@pytest.mark.parametrize("n_u, npts, prec, tol", [(206, 5439, "fp64", 1e-12), (206, 5471, "fp64", 1e-12),
+                                                  (206, 1281, "mixed", 1e-6), (100, 2511, "mixed", 1e-6)])
+def test_least_points_on_the_tree(gpu_lib, n_u, npts, prec, tol):
+    """Just above the sizes at which the tree sets in, ragged last groups."""
+    nodes, elems = meshes.torus(n_u, 0.3)
+    rng = np.random.default_rng(npts)
+    t, u, pts = rng.normal(size=len(elems)), rng.normal(size=len(nodes)), rng.uniform(-1.5, 1.5, size=(npts, 3))
+    with gpu_lib.Mesh(nodes, elems) as m:
+        p = m.evaluate(pts, t, u, prec)
+        m.set_far_engine("cuda")
+        direct = m.evaluate(pts, t, u, prec)
+        assert not np.array_equal(p, direct)  # it was the tree
+        assert rel_l2(p, direct) < tol
