@@ -2220,7 +2220,7 @@ void tree_prepare(Mesh* m)
 bool tree_eligible(const Mesh* m, int nsl, int nd)
 {
   return m->plan.engine == 4 && m->tree && m->tree->usable && tree_variant(nsl, nd) &&
-         (!wide_rule(m->h) || (nsl <= 1 && nd <= 1));
+         (!wide_rule(m->h) || (nsl <= 1 && nd <= 1)) && tree_partial_bytes(m, nsl, nd) <= kTreeMaxSlotBytes;
 }
 
 // With t->lists_lock held, as upload_forward.

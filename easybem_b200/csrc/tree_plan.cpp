@@ -194,7 +194,7 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
   far.reserve(32 * (size_t)nc);
   std::vector<std::pair<int, int>> near;  // close cells, the earlier one first
   near.reserve(20 * (size_t)nc);
-  const long long limit = (long long)nc * nc / 6;
+  const long long limit = std::min((long long)nc * nc / 6, (long long)(kTreeMaxSlotBytes / (kCell * sizeof(double))));
   std::vector<std::pair<int, int>> stack(1, {root, root});
   while (!stack.empty()) {
     const auto [a, b] = stack.back();

@@ -113,6 +113,10 @@ constexpr int kTreePartShift = 25, kTreePartsShift = 28;
 // SMs idle.
 constexpr int kTreeMinCells = 100;
 constexpr int kTreeAllCloseCells = 140;
+// Meshes whose partial slots would pass this in a variant keep the direct
+// kernels there (ordinary surfaces take 80 bytes a triangle and column; the
+// limit is the symmetric kernels').
+constexpr size_t kTreeMaxSlotBytes = (size_t)1 << 35;
 // Expansions moved into node tgt[k] from nodes src[ptr[k] .. ptr[k + 1]). The
 // upper 8 bits of a source are the share f / 255 of the degrees that its pair
 // needs: an expansion of order p is used up to (p + 1) f / 255 - 1 (rounded
@@ -148,7 +152,8 @@ struct TreePlan {
 };
 
 // False when more than a third of all cell pairs are close in a mesh of more
-// than kTreeAllCloseCells (the tree would not pay): the plan is then incomplete.
+// than kTreeAllCloseCells (the tree would not pay), or their slots pass
+// kTreeMaxSlotBytes in every variant: the plan is then incomplete.
 bool make_tree_plan(const HostMesh& h, TreePlan* plan);
 // Tasks and slots of a plan's close pairs: every unordered pair once (both),
 // or every ordered pair.
