@@ -1581,8 +1581,11 @@ constexpr int kPointCells = 4;  // close cells of a task
 // at once, 0.4 GB in parts.
 constexpr size_t kPointScratch = (size_t)1 << 30;
 constexpr int kListWarps = 4;
-constexpr int kListStack = 1024;  // 32 nodes leave and at most 64 children enter: at most 32 (height + 1)
-static_assert(32 * (kTreePasses * kTreeLevelsPerPass + 2) <= kListStack, "stack of the deepest tree");
+// Nodes of a group still to be tested: 32 leave at a time and up to 64 children
+// enter. Where these would reach the last kListReserve entries, one node leaves
+// at a time, which adds at most one per level of the tree.
+constexpr int kListStack = 1024, kListReserve = kTreePasses * kTreeLevelsPerPass + 1;
+static_assert(kListReserve + 64 <= kListStack, "room for a step of 32 nodes");
 
 // The tree against every group, a warp per group testing 32 nodes at a time:
 // separated nodes that have a multipole and close cells, counted (FILL false)
@@ -1604,7 +1607,7 @@ __global__ void __launch_bounds__(32 * kListWarps)
   if (lane == 0) stack[0] = root;
   __syncwarp();
   while (top > 0) {
-    const int take = min(32, top);
+    const int take = min(min(32, top), max(1, kListStack - kListReserve - top));
     const int k = lane < take ? stack[top - 1 - lane] : -1;
     top -= take;
     __syncwarp();

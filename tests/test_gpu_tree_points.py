@@ -152,3 +152,18 @@ def test_least_points_on_the_tree(gpu_lib, n_u, npts, prec, tol):
         direct = m.evaluate(pts, t, u, prec)
         assert not np.array_equal(p, direct)  # it was the tree
         assert rel_l2(p, direct) < tol
+
+
+@pytest.mark.parametrize("prec, tol", PRECISIONS)
+def test_groups_as_large_as_the_mesh(gpu_lib, prec, tol):
+    """Every group close to a large part of 10,240 cells: the longest lists of
+    nodes to be tested."""
+    nodes, elems = meshes.perturbed_icosphere(7, seed=1)
+    rng = np.random.default_rng(8)
+    t, u, pts = rng.normal(size=len(elems)), rng.normal(size=len(nodes)), rng.uniform(-1.2, 1.2, size=(2600, 3))
+    pts[:1300] = pts[:1300] / np.linalg.norm(pts[:1300], axis=1, keepdims=True) * rng.choice([0.4, 1.6], size=(1300, 1))
+    with gpu_lib.Mesh(nodes, elems) as m:
+        p = m.evaluate(pts, t, u, prec)
+        m.set_far_engine("cuda")
+        direct = m.evaluate(pts, t, u, prec)
+        assert not np.array_equal(p, direct) and rel_l2(p, direct) < tol
