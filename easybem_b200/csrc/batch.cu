@@ -128,8 +128,7 @@ int Batch::build(const std::vector<BatchEntry*>& entries, bool fp32, int nsl, in
                               h.ne, nd_ ? be->qout.as<double>() : nullptr);
     args[e].active = d_flags ? d_flags + e : nullptr;
     if (tree[e]) {
-      args[e].partial = tdesc.back().partial;
-      args[e].slot_off = tdesc.back().slot_off;
+      tree_finalize_args(m, nsl_, nd_, tdesc.back(), &args[e]);
       tree_args.push_back(args[e]);
     } else if (sym_) {
       args[e].partial = be->sym_partial.as<double>();

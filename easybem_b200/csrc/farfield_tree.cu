@@ -2368,6 +2368,12 @@ int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, v
   return EB_OK;
 }
 
+void tree_finalize_args(const Mesh* m, int nsl, int nd, const TreeDesc& d, ApplyArgs* A)
+{
+  A->partial = d.partial + (size_t)d.first_col * tree_far_slots(m, nsl, nd);
+  A->slot_off = d.slot_off;
+}
+
 bool tree_points_eligible(const Mesh* m, bool fp32, int npts)
 {
   const double n = npts, ne = m->h.ne;
@@ -2464,8 +2470,7 @@ int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream
     sc = std::move(s);
   }
   const TreeDesc& d = sc->host;
-  A->partial = d.partial + (size_t)d.first_col * tree_far_slots(m, nsl, nd);
-  A->slot_off = d.slot_off;
+  tree_finalize_args(m, nsl, nd, d, A);
   TreeGrid g;
   g.rule = m->h.Q;
   g.ncells = d.ncells;

@@ -124,6 +124,8 @@ long long tree_far_slots(const Mesh* m, int nsl, int nd);
 // uploads the mesh's lists the first time.
 int tree_desc(Mesh* m, bool fp32, int nsl, int nd, void* rec, void* multipole, void* local, double* partial,
               TreeDesc* out);
+// Where the finalize reads the sums of descriptor d (of m and this variant).
+void tree_finalize_args(const Mesh* m, int nsl, int nd, const TreeDesc& d, ApplyArgs* A);
 // Bytes of one of the two expansion buffers, and of the partial slots.
 size_t tree_expansion_bytes(const Mesh* m, int order, int cols);
 size_t tree_partial_bytes(const Mesh* m, int nsl, int nd);
