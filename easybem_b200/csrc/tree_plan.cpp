@@ -194,7 +194,8 @@ bool make_tree_plan(const HostMesh& h, TreePlan* plan)
   far.reserve(32 * (size_t)nc);
   std::vector<std::pair<int, int>> near;  // close cells, the earlier one first
   near.reserve(20 * (size_t)nc);
-  const long long limit = std::min((long long)nc * nc / 6, (long long)(kTreeMaxSlotBytes / (kCell * sizeof(double))));
+  const double share = nc > kTreeSmallCells ? kTreeMaxShare : kTreeSmallShare;
+  const long long limit = std::min((long long)(0.5 * share * nc * nc), (long long)(kTreeMaxSlotBytes / (kCell * sizeof(double))));
   std::vector<std::pair<int, int>> stack(1, {root, root});
   while (!stack.empty()) {
     const auto [a, b] = stack.back();

@@ -108,11 +108,28 @@ constexpr int kTreeNearParts = 4;
 // part and log2 of the number of parts in the upper bits.
 constexpr int kTreePartShift = 25, kTreePartsShift = 28;
 // Smaller meshes (cells) have no separated clusters worth an expansion: all
-// their cell pairs are close. Up to here the near tasks alone also beat the
-// symmetric kernel, whose items (a 128-triangle tile against 8 cells) leave
-// SMs idle.
+// their cell pairs are close. Host applies in us, SL+DL and SL, of tori of r =
+// 0.3 with all pairs close / the tree / the direct default (symmetric mixed,
+// ordered FP64):
+//   cells   mixed SL+DL    SL             FP64 SL+DL      SL
+//      81   163/229/210    107/144/131    329/474/471     189/314/313
+//     100   206/199/318    130/147/190    539/459/639     288/383/436
+//     133   288/246/321    182/177/193    816/574/1,099   425/464/716
+//     169   422/294/434    273/212/278    1,260/759/1,713 677/564/1,117
+//     196   546/312/572    353/225/353    1,653/865/2,268 895/584/1,449
 constexpr int kTreeMinCells = 100;
-constexpr int kTreeAllCloseCells = 140;
+// Largest share of close pairs: half (host applies in us, direct default ->
+// tree, mixed / FP64 SL+DL: 4,992 triangles graded towards a pole, share 0.36,
+// 427 -> 356 and 1,468 -> 813; 20,000 needles, 0.43, 4,680 -> 2,870 and 21.8 ->
+// 9.5 ms). Up to kTreeSmallCells a lower one: with all pairs close the single
+// layer gains what four columns lose (100 cells: above, and 413/284, 1,019/749).
+constexpr double kTreeMaxShare = 0.5, kTreeSmallShare = 0.318;
+constexpr int kTreeSmallCells = 140;
+// Meshes above that share: up to here the near tasks alone beat the direct
+// kernels, whose items (a 128-triangle tile against 8 cells) leave SMs idle, in
+// every variant (above; four columns at 169 cells 885 against 897 and 2,213
+// against 2,445).
+constexpr int kTreeAllCloseCells = 170;
 // Meshes whose partial slots would pass this in a variant keep the direct
 // kernels there (ordinary surfaces take 80 bytes a triangle and column; the
 // limit is the symmetric kernels').
@@ -151,8 +168,8 @@ struct TreePlan {
   int forward_slots = 0;  // of the lists of every ordered pair, which are made when a variant needs them
 };
 
-// False when more than a third of all cell pairs are close in a mesh of more
-// than kTreeAllCloseCells (the tree would not pay), or their slots pass
+// False when more than half of all cell pairs are close in a mesh of more than
+// kTreeAllCloseCells (the tree would not pay), or their slots pass
 // kTreeMaxSlotBytes in every variant: the plan is then incomplete.
 bool make_tree_plan(const HostMesh& h, TreePlan* plan);
 // Tasks and slots of a plan's close pairs: every unordered pair once (both),

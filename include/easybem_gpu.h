@@ -373,7 +373,7 @@ int eb_mesh_get_plan(eb_mesh mesh, int* items_per_sm, int* src_tile, int* nsplit
  * or 4, SL+DL, the P1 single layer) and the potentials of many points; below
  * some 4,000 triangles all cells are close and get reports EB_FAR_SYMMETRIC.
  * Rules of 12 points and more: SL, DL and SL+DL on meshes that have separated
- * clusters. EB_FAR_SYMMETRIC's rules otherwise, and where more than a third of
+ * clusters. EB_FAR_SYMMETRIC's rules otherwise, and where more than half of
  * the cell pairs of a larger mesh are close or their partial sums would take
  * more than 32 GiB. What the expansions leave out
  * was at or below the rounding of the point sums in either precision on every

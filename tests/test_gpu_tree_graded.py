@@ -111,3 +111,19 @@ def test_potentials_at_a_probe(gpu_lib, name):
         m.set_far_engine("tree")
         assert rel_l2(m.evaluate(pts, t, u, "mixed"), ref) < 2 * rel_l2(direct, ref)
         assert rel_l2(m.evaluate(pts, t, u, "fp64"), ref) < FP64_TOL
+
+
+@pytest.mark.parametrize("name, north, south, engine", [("small", 25, 5, "sym"), ("third", 30, 8, "tree")])
+def test_many_close_cells(gpu_lib, name, north, south, engine):
+    """More than a third of the cell pairs close: all of them up to 140 cells
+    (3,968 triangles), the tree for larger meshes; against the ordered pairs."""
+    nodes, elems = pole_graded_sphere(64, 0.9, north, south)
+    rng = np.random.default_rng(north)
+    t, u = rng.normal(size=len(elems)), rng.normal(size=len(nodes))
+    with gpu_lib.Mesh(nodes, elems) as m:
+        assert m.far_engine("fp64") == engine and m.far_engine("mixed") == engine
+        got = {prec: m.apply_sl_dl(t, u, precision=prec) for prec in ("fp64", "mixed")}
+        m.set_far_engine("cuda")
+        v, q = m.apply_sl_dl(t, u)
+    for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL)):
+        assert rel_l2(got[prec][0], v) < tol and rel_l2(got[prec][1], q) < tol
