@@ -635,7 +635,7 @@ bool sym_eligible(const Mesh* m, bool fp32, int nsl, int nd, bool fp64_internal)
 
 long long mesh_far_slots(const Mesh* m, bool fp32, int nsl, int nd)
 {
-  if (tree_eligible(m, nsl, nd)) return tree_far_slots(m, nsl, nd);
+  if (tree_eligible(m, nsl, nd, fp32)) return tree_far_slots(m, nsl, nd);
   if (sym_eligible(m, fp32, nsl, nd)) {
     const int r = far_sym_cells_per_item(kSymCellsPerItem);
     long long n = 0;
@@ -773,7 +773,7 @@ int mesh_apply(Mesh* m, int precision, int nsl, int nd, const double* d_t, const
   if (!far_variant_supported(nsl, nd)) return set_error(EB_ERR_INVALID, "unsupported operator combination");
   if ((nsl > 0 && (!d_t || !d_v)) || (dl && (!d_u || !d_q))) return set_error(EB_ERR_INVALID, "null vector");
   const int nrec = rec_slots(nsl, nd);
-  const bool tree = tree_eligible(m, nsl, nd);
+  const bool tree = tree_eligible(m, nsl, nd, fp32);
   EB_CHECK(ensure_apply_scratch(m, tree));
   Mesh::Variant& var = m->variants[(fp32 ? 64 : 0) + nsl * 5 + nd];
   if (!tree && !var.desc.p) {

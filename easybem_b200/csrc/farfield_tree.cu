@@ -2220,8 +2220,10 @@ void tree_prepare(Mesh* m)
   m->tree->usable = make_tree_plan(h, &m->tree->plan) && !(wide && m->tree->plan.all_close);
 }
 
-bool tree_eligible(const Mesh* m, int nsl, int nd)
+bool tree_eligible(const Mesh* m, int nsl, int nd, bool fp32)
 {
+  if (nd > 1 && m->tree && m->tree->plan.all_close && m->h.ncells > (fp32 ? kTreeForwardCells32 : kTreeForwardCells64))
+    return false;
   return m->plan.engine == 4 && m->tree && m->tree->usable && tree_variant(nsl, nd) &&
          (!wide_rule(m->h) || (nsl <= 1 && nd <= 1)) && tree_partial_bytes(m, nsl, nd) <= kTreeMaxSlotBytes;
 }

@@ -113,8 +113,9 @@ struct TreeMesh {
 // The tree of mesh m when its size allows one (host work, done while the GPU
 // computes the near field of a new mesh).
 void tree_prepare(Mesh* m);
-// True when mesh m applies this far-field variant through the tree.
-bool tree_eligible(const Mesh* m, int nsl, int nd);
+// True when mesh m applies this far-field variant through the tree (the same in
+// both precisions but for several double layers).
+bool tree_eligible(const Mesh* m, int nsl, int nd, bool fp32 = false);
 // The far field of mesh m: expansions and close pairs into the partial slots
 // (A.partial and A.slot_off are set for the finalize).
 int tree_far_apply(Mesh* m, bool fp32, int nsl, int nd, ApplyArgs* A, cudaStream_t st);

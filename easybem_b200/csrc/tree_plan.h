@@ -130,6 +130,12 @@ constexpr int kTreeSmallCells = 140;
 // every variant (above; four columns at 169 cells 885 against 897 and 2,213
 // against 2,445).
 constexpr int kTreeAllCloseCells = 170;
+// Four double layers run their close pairs in both orders one by one: with all
+// pairs close up to here, then the direct kernels. Host right-hand sides in us,
+// all close / direct, mixed and FP64: 10 cells 55/73, 93/136; 40 cells 125/118,
+// 198/254; 66 cells 220/206, 423/485; 91 cells 351/346, 789/795; 100 cells
+// 413/371, 1,019/929.
+constexpr int kTreeForwardCells32 = 32, kTreeForwardCells64 = 90;
 // Meshes whose partial slots would pass this in a variant keep the direct
 // kernels there (ordinary surfaces take 80 bytes a triangle and column; the
 // limit is the symmetric kernels').
