@@ -1,5 +1,5 @@
 // Tree far field: the sum over all pairs of quadrature points in time
-// proportional to their number (7-point rule).
+// proportional to their number (rules of 7 points, and of 8 and more).
 //
 // Clusters of triangles (the nodes of the bisection that orders the mesh) are
 // paired as in tree_plan.h. Between separated clusters the kernel 1/|x - y| is
@@ -608,55 +608,55 @@ __global__ void __launch_bounds__(32 * kCellWarps)
       wj[a] = on && first + a < Q ? A.wj[(size_t)sel * Q + b] : 0.0;
       const double e1 = A.bary[2 * b], e2 = A.bary[2 * b + 1];
       s[a] = wj[a] * ((1.0 - e1 - e2) * u0 + e1 * u1 + e2 * u2);
-  }
-  each_harmonic<P>(tab, p, warp, [&](int n, int m, const double (&re)[kQ], const double (&im)[kQ]) {
-    int row = 0;
-    if constexpr (NSL > 0) {
-      double hr = 0.0, hi = 0.0;
-#pragma unroll
-      for (int a = 0; a < kQ; ++a) {
-        hr += wj[a] * re[a];
-        hi += wj[a] * im[a];
-      }
-#pragma unroll
-      for (int c = 0; c < NSL; ++c) {
-        s_red[row++ * kSumStride + lane] = hr * t[c];
-        s_red[row++ * kSumStride + lane] = hi * t[c];
-      }
     }
-    if constexpr (ND > 0) {
-      double gr = 0.0, gi = 0.0;
+    each_harmonic<P>(tab, p, warp, [&](int n, int m, const double (&re)[kQ], const double (&im)[kQ]) {
+      int row = 0;
+      if constexpr (NSL > 0) {
+        double hr = 0.0, hi = 0.0;
 #pragma unroll
-      for (int a = 0; a < kQ; ++a) {
-        gr += s[a] * re[a];
-        gi += s[a] * im[a];
-      }
-      if constexpr (KIND == kCharges) {
-        s_red[lane] = gr;
-        s_red[kSumStride + lane] = gi;
-      } else {
+        for (int a = 0; a < kQ; ++a) {
+          hr += wj[a] * re[a];
+          hi += wj[a] * im[a];
+        }
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          s_red[row++ * kSumStride + lane] = gr * nrm[k];
-          s_red[row++ * kSumStride + lane] = gi * nrm[k];
+        for (int c = 0; c < NSL; ++c) {
+          s_red[row++ * kSumStride + lane] = hr * t[c];
+          s_red[row++ * kSumStride + lane] = hi * t[c];
         }
       }
-    }
-    __syncwarp();
-    // four lanes add a row of 32
-    const int r = lane >> 2, part = lane & 3;
-    double v = 0.0;
-    if (r < kRows)
+      if constexpr (ND > 0) {
+        double gr = 0.0, gi = 0.0;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v += s_red[r * kSumStride + part + 4 * k];
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    if (part == 0 && r < kRows) {
-      double* sum = &s_sum[r * kPairs + tree_pair(n, m)];
-      *sum = WIDE && first ? *sum + v : v;  // the same thread every time
-    }
-    __syncwarp();
-  });
+        for (int a = 0; a < kQ; ++a) {
+          gr += s[a] * re[a];
+          gi += s[a] * im[a];
+        }
+        if constexpr (KIND == kCharges) {
+          s_red[lane] = gr;
+          s_red[kSumStride + lane] = gi;
+        } else {
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            s_red[row++ * kSumStride + lane] = gr * nrm[k];
+            s_red[row++ * kSumStride + lane] = gi * nrm[k];
+          }
+        }
+      }
+      __syncwarp();
+      // four lanes add a row of 32
+      const int r = lane >> 2, part = lane & 3;
+      double v = 0.0;
+      if (r < kRows)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v += s_red[r * kSumStride + part + 4 * k];
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      if (part == 0 && r < kRows) {
+        double* sum = &s_sum[r * kPairs + tree_pair(n, m)];
+        *sum = WIDE && first ? *sum + v : v;  // the same thread every time
+      }
+      __syncwarp();
+    });
   }
   __syncthreads();
   const size_t cstride = (size_t)d.nnodes * kPairs;
@@ -765,24 +765,24 @@ __global__ void __launch_bounds__(32 * kCellWarps)
       } else {
         w[0][a] = first + a < Q ? d.far.tgt64[at + first + a].w : 0.0;
       }
-  }
-  each_harmonic<P>(tab, p, warp, [&](int n, int m, const double (&re)[kQ], const double (&im)[kQ]) {
-    double hr[NW], hi[NW];
+    }
+    each_harmonic<P>(tab, p, warp, [&](int n, int m, const double (&re)[kQ], const double (&im)[kQ]) {
+      double hr[NW], hi[NW];
 #pragma unroll
-    for (int k = 0; k < NW; ++k) {
-      hr[k] = hi[k] = 0.0;
+      for (int k = 0; k < NW; ++k) {
+        hr[k] = hi[k] = 0.0;
 #pragma unroll
-      for (int a = 0; a < kQ; ++a) {
-        hr[k] += w[k][a] * re[a];
-        hi[k] += w[k][a] * im[a];
+        for (int a = 0; a < kQ; ++a) {
+          hr[k] += w[k][a] * re[a];
+          hi[k] += w[k][a] * im[a];
+        }
       }
-    }
 #pragma unroll
-    for (int c = 0; c < NO; ++c) {
-      const double2 l = s_loc[(P1T ? 0 : c) * kPairs + tree_pair(n, m)];
-      phi[c] += l.x * hr[P1T ? c : 0] + l.y * hi[P1T ? c : 0];
-    }
-  });
+      for (int c = 0; c < NO; ++c) {
+        const double2 l = s_loc[(P1T ? 0 : c) * kPairs + tree_pair(n, m)];
+        phi[c] += l.x * hr[P1T ? c : 0] + l.y * hi[P1T ? c : 0];
+      }
+    });
   }
 #pragma unroll
   for (int c = 0; c < NO; ++c) s_part[warp][c][lane] = phi[c];
@@ -812,8 +812,7 @@ constexpr int near_sources() { return sizeof(T) == 4 ? kCell : kCell / 2; }  // 
 template <typename T, int NSL, int ND>
 constexpr size_t near_red_row()  // bytes of a lane's transposed sums, padded
 {
-  return sizeof(T) == 4 ? (ND > 0 ? 16 * (kCell / 2 + 1) : 8 * (kCell / 2 * NSL + 1))
-                        : (ND > 0 ? 16 * (kCell / 2 + 1) : 8 * (kCell / 2 * NSL + 1));
+  return ND > 0 ? 16 * (kCell / 2 + 1) : 8 * (kCell / 2 * NSL + 1);
 }
 
 template <typename T, int NSL, int ND>
@@ -1291,8 +1290,8 @@ using ld = long double;
 
 std::vector<std::vector<ld>> half_turns(int P)
 {
-  // d^n_{m'm}(90 degrees), [n][(m' + n) (2n + 1) + m + n], by the three-term
-  // recurrence in n (stable upward) from n = max(|m|, |m'|)
+  // Wigner's d^n_{m'm}(90 degrees), [n][(m' + n) (2n + 1) + m + n], by their
+  // three-term recurrence in the degree n (stable upward) from n = max(|m|, |m'|)
   std::vector<std::vector<ld>> d(P + 1);
   for (int n = 0; n <= P; n++) d[n].assign((size_t)(2 * n + 1) * (2 * n + 1), 0.0L);
   auto binom = [](int n, int k) {
