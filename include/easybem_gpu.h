@@ -375,15 +375,16 @@ int eb_mesh_get_plan(eb_mesh mesh, int* items_per_sm, int* src_tile, int* nsplit
  * Rules of 12 points and more: SL, DL and SL+DL on meshes that have separated
  * clusters. EB_FAR_SYMMETRIC's rules otherwise, and where more than half of
  * the cell pairs of a larger mesh are close or their partial sums would take
- * more than 32 GiB. What the expansions leave out
- * was at or below the rounding of the point sums in either precision on every
- * surface measured: smooth ones, ones graded towards a pole or edges, and two
- * bodies of size 50 : 1, on the rows of their smallest triangles too. An
- * apply runs the close cells on a stream of the mesh's own beside the
- * expansions; work before and after it on the caller's stream is ordered as
- * with one stream, also under capture. Scratch, allocated with a variant's
- * first apply, grows with nelems: the expansions of SL+DL at 81,920 triangles
- * take 143 MB in FP64 and 39 MB mixed. */
+ * more than 32 GiB. What the expansions leave out was at or below the rounding
+ * of the point sums in either precision on every surface measured: smooth ones,
+ * ones graded towards a pole or edges, and two bodies of size 50 : 1, on the
+ * rows of their smallest triangles too. An apply runs the close cells on a
+ * stream of the mesh's own beside the expansions; work before and after it on
+ * the caller's stream is ordered as with one stream, also under capture (of an
+ * operator that was applied before). Scratch, allocated with a variant's first
+ * apply, grows with nelems: the expansions of SL+DL at 81,920 triangles take
+ * 143 MB in FP64 and 39 MB mixed. An evaluation of potentials keeps at most
+ * 1 GiB beside arrays of the points' number. */
 #define EB_FAR_TREE 4
 int eb_mesh_set_far_engine(eb_mesh mesh, int engine);
 int eb_mesh_get_far_engine(eb_mesh mesh, int precision, int* engine);
